@@ -175,11 +175,12 @@ bool tc5_eligible(const fa_fwd_params& a, bool is_causal, bool is_local, int wl_
   // any head dim up to 256 that keeps rows 16-byte aligned: the tiles are 64, 128 or 256 columns wide and the TMA
   // unit fills the columns beyond the head dim with zeros
   if (a.d < 8 || a.d > 256 || a.d % 8 != 0 || a.seqlen_q < 128) return false;
-  // varlen: both sides packed, and the number of k / v rows known (TMA bound)
-  if ((a.cu_seqlens_q != nullptr) != (a.cu_seqlens_k != nullptr)) return false;
-  if (a.cu_seqlens_k && a.total_k <= 0) return false;
-  // KV cache without append: per-entry lengths, contiguous or paged with whole 128-key blocks per page
-  if ((a.seqused_k || a.block_table) && (a.cu_seqlens_q || !a.seqused_k)) return false;
+  // packed queries: against packed keys (the number of k / v rows known, a TMA bound) or against a KV cache (a step of
+  // chunked prefill; without new tokens, whose prologue launch takes dense queries)
+  if (a.cu_seqlens_k && (!a.cu_seqlens_q || a.seqused_k || a.total_k <= 0)) return false;
+  if (a.cu_seqlens_q && !a.cu_seqlens_k && (!a.seqused_k || a.k_new || a.total_q <= 0)) return false;
+  // KV cache: per-entry lengths, contiguous or paged with whole 128-key blocks per page
+  if (a.block_table && !a.seqused_k) return false;
   if (a.block_table && (a.page_size <= 0 || a.page_size % tc5::kBlockN != 0)) return false;
   // new tokens (and rotary) are served by a prologue launch in front of the kernel; they need the cache lengths
   if ((a.k_new || a.rotary_cos) && (!a.seqused_k || !a.k_new || !a.v_new)) return false;
@@ -260,29 +261,20 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
   }
   p.status = status_word();
   if (!p.status) { *err = "cannot look up the device status word"; return FA_ERR_CUDA; }
-  const bool varlen = a.cu_seqlens_q != nullptr;
   CUtensorMap tq, tk, tv;
-  bool ok = true;
-  if (varlen) {
-    // Packed sequences: one row axis for the whole tensor.  A tile that runs past the end of its
-    // sequence reads rows of the next one (masked by the key range, never stored), a tile that
-    // runs past the end of the tensor reads the TMA fill value.
-    ok = encode_map(&tq, a.q, a.dtype, a.d, a.h, a.total_q, 1, a.q_head_stride, a.q_row_stride, 0) &&
-         encode_map(&tk, a.k, a.dtype, a.d, a.h_k, a.total_k, 1, a.k_head_stride, a.k_row_stride, 0) &&
-         encode_map(&tv, a.v, a.dtype, a.d, a.h_k, a.total_k, 1, a.v_head_stride, a.v_row_stride, 0);
-  } else if (a.block_table) {
-    // (d, kv head, row in page, page): a block-table entry outside the pool reads zeros, not memory
-    const int64_t n_pages = a.kv_outer;
-    ok = encode_map(&tq, a.q, a.dtype, a.d, a.h, a.seqlen_q, a.b, a.q_head_stride, a.q_row_stride, a.q_batch_stride) &&
-         encode_map(&tk, a.k, a.dtype, a.d, a.h_k, a.page_size, n_pages, a.k_head_stride, a.k_row_stride, a.k_batch_stride) &&
-         encode_map(&tv, a.v, a.dtype, a.d, a.h_k, a.page_size, n_pages, a.v_head_stride, a.v_row_stride, a.v_batch_stride);
-  } else {
-    // with cache_batch_idx the cache may have more rows than the batch; an index outside it reads zeros
-    const int64_t kv_batch = a.cache_batch_idx ? a.kv_outer : a.b;
-    ok = encode_map(&tq, a.q, a.dtype, a.d, a.h, a.seqlen_q, a.b, a.q_head_stride, a.q_row_stride, a.q_batch_stride) &&
-         encode_map(&tk, a.k, a.dtype, a.d, a.h_k, a.seqlen_k, kv_batch, a.k_head_stride, a.k_row_stride, a.k_batch_stride) &&
-         encode_map(&tv, a.v, a.dtype, a.d, a.h_k, a.seqlen_k, kv_batch, a.v_head_stride, a.v_row_stride, a.v_batch_stride);
-  }
+  // Packed sequences: one row axis for the whole tensor.  A tile that runs past the end of its sequence reads rows of
+  // the next one (masked by the key range, never stored), a tile that runs past the end of the tensor reads the TMA
+  // fill value.
+  bool ok = a.cu_seqlens_q
+                ? encode_map(&tq, a.q, a.dtype, a.d, a.h, a.total_q, 1, a.q_head_stride, a.q_row_stride, 0)
+                : encode_map(&tq, a.q, a.dtype, a.d, a.h, a.seqlen_q, a.b, a.q_head_stride, a.q_row_stride, a.q_batch_stride);
+  // (d, kv head, row, batch row) of packed, dense or cached keys, or (d, kv head, row in page, page): a cache_batch_idx
+  // or block-table entry outside the cache reads zeros, not memory
+  const bool packed_k = a.cu_seqlens_k != nullptr;
+  const int64_t k_rows = packed_k ? a.total_k : a.block_table ? a.page_size : a.seqlen_k;
+  const int64_t k_outer = packed_k ? 1 : (a.block_table || a.cache_batch_idx) ? a.kv_outer : a.b;
+  ok = ok && encode_map(&tk, a.k, a.dtype, a.d, a.h_k, k_rows, k_outer, a.k_head_stride, a.k_row_stride, packed_k ? 0 : a.k_batch_stride) &&
+       encode_map(&tv, a.v, a.dtype, a.d, a.h_k, k_rows, k_outer, a.v_head_stride, a.v_row_stride, packed_k ? 0 : a.v_batch_stride);
   if (!ok) { *err = "cuTensorMapEncodeTiled failed"; return FA_ERR_CUDA; }
   cudaError_t e = cudaErrorInvalidValue;
   auto launch = [&](auto kern) {

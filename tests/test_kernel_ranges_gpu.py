@@ -1,0 +1,50 @@
+"""GPU: the edges of the ranges that the planner's kernel choices cover, against the oracle: tile remainders, head dims
+between the tile widths, the smallest and largest row counts, single sequences cut over the whole grid.  Inputs are
+N(0, 1); tolerances are the rules of precision.py (rtol = atol = 1e-2 for 16-bit outputs, and the 99.5 % rule)."""
+import pytest
+import torch
+
+import parity_util as U
+from flash_b200 import lib as L
+from flash_b200 import ops
+from oracle import api as OA
+
+pytestmark = pytest.mark.gpu
+BF, FP = torch.bfloat16, torch.float16
+
+
+def _cuda(t):
+    return None if t is None else t.cuda()
+
+
+def _cache(g, dtype, b, room, hk, d, page):
+    """(k, v, block table or None): contiguous rows, or pages of a shuffled pool."""
+    if not page:
+        return U.normal((b, room, hk, d), dtype, g), U.normal((b, room, hk, d), dtype, g), None
+    per = -(-room // page)
+    bt = torch.randperm(b * per, generator=g).view(b, per).to(torch.int32)
+    return U.normal((b * per, page, hk, d), dtype, g), U.normal((b * per, page, hk, d), dtype, g), bt
+
+
+@pytest.mark.parametrize("page", [0, 128])
+@pytest.mark.parametrize("dtype,d,window", [(BF, 128, -1), (FP, 64, -1), (BF, 192, 100)])
+def test_packed_queries_against_a_cache_on_tcgen05(dtype, d, window, page):
+    import flash_attn_npu_v3 as fa3
+    g = torch.Generator().manual_seed(d + page)
+    h, hk = 4, 2
+    q_lens, k_lens = [1, 127, 128, 129, 257], [1, 500, 128, 640, 300]
+    b, room = len(q_lens), 640
+    cq = torch.tensor([0] + list(torch.tensor(q_lens).cumsum(0)), dtype=torch.int32)
+    q = U.normal((sum(q_lens), h, d), dtype, g)
+    kc, vc, bt = _cache(g, dtype, b, room, hk, d, page)
+    lens = torch.tensor(k_lens, dtype=torch.int32)
+    out, lse, *_ = fa3.flash_attn_with_kvcache(q.cuda(), kc.cuda(), vc.cuda(), cache_seqlens=lens.cuda(), page_table=_cuda(bt),
+                                               cu_seqlens_q=cq.cuda(), max_seqlen_q=max(q_lens), causal=True,
+                                               window_size=(window, -1), return_softmax_lse=True)
+    for i in range(b):
+        rows = slice(int(cq[i]), int(cq[i + 1]))
+        ki, vi, bi = (kc, vc, bt[i:i + 1]) if page else (kc[i:i + 1], vc[i:i + 1], None)
+        # a left window counts from the call's longest sequence; none of these windows covers it
+        go, gl = OA.flash_attn_with_kvcache(q[rows].unsqueeze(0), ki, vi, cache_seqlens=lens[i:i + 1], block_table=bi, causal=True,
+                                            window_size=(window if window < k_lens[i] - 1 else -1, -1))
+        U.check_rules(out[rows].unsqueeze(0), lse[:, rows].unsqueeze(0), go, gl, tag=f"sequence {i}")
