@@ -57,6 +57,8 @@ static void normalize_window(int seqlen_q, int max_k, bool causal, int& wl, int&
 
 static bool s_new_too_long(const fa_fwd_params& a) { return a.seqlen_new > a.seqlen_k; }
 
+constexpr int kMinPersistSlots = 4;  // partials of a unit that persistent decode CTAs share, at least
+
 struct Planned {
   fa_fwd_plan pl;
   KParams kp;
@@ -240,33 +242,46 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
   ns = ceil_div(max_blocks, bps);
 
   // Persistent decode: ragged lengths leave a tail of unequal CTAs; CTAs that stay resident and take
-  // equal shares of the KV blocks of the whole launch do not.  A unit cut by a CTA boundary is
-  // finished by the merge kernel from up to kPersistSlots partials.  (Window-bound ranges are
-  // nearly equal; there the merge launch costs what the balance gains -- measured.)
-  constexpr int kPersistSlots = 4;
+  // equal shares of the KV blocks of the whole launch do not.  A unit (batch entry, packed head group) cut by CTA
+  // boundaries is finished by the merge kernel from its partial slots.  There are enough slots for the units to
+  // cover the whole grid (with four of them, 64 units of 131072 keys kept 192 of 296 CTAs busy: 712 -> 650 us; one
+  // sequence of 2048 keys and 8 kv heads ran on 8 CTAs: 36 -> 14 us with the merge), and for many units four, the most that equal
+  // shares of near-equal units need.
   bool persistent = false;
   long long persist_grid = 0;
+  int persist_slots = kMinPersistSlots;
   if (kernel_id == FA_KERNEL_DECODE && a.num_splits == 0 && !a.cu_seqlens_q && a.kv_total == 0 && !a.partial_out) {
     const bool window_bound = is_local && wl >= 0 && range < max_k_bound;
     const long long resident = std::max(1, (227 * 1024) / std::max(1, ci.smem_bytes));
     persist_grid = (long long)num_sm * resident;
-    const bool can_persist = (a.seqused_k != nullptr || window_bound) && base * max_blocks >= 4 * persist_grid &&
-                             base * (max_blocks + 1) < 0x3fffffffLL;
-    persistent = can_persist && !window_bound && !decode_one_segment_only;
-    if (const char* e = std::getenv("FA_B200_DECODE_PERSISTENT"))  // tuning override: 0 off, 1 default rule, 2 also window-bound
-      persistent = can_persist && !decode_one_segment_only && (std::atoi(e) == 2 || (std::atoi(e) == 1 && !window_bound));
     if (const char* e = std::getenv("FA_B200_DECODE_PERSISTENT_GRID")) persist_grid = std::max(1, std::atoi(e));  // tuning override
-    if (persistent) { ns = kPersistSlots; bps = 0; }
+    // (a unit cut into grid / base shares touches up to two CTAs more than whole shares)
+    persist_slots = persist_grid / base > 3 ? (int)(persist_grid / base + 2) : kMinPersistSlots;
+    // Worth a merge launch when the units do not fill the grid by themselves or are many: at least 8 blocks a unit
+    // (below that a CTA per unit finishes in the time a merge takes), or four blocks for every CTA of the grid.
+    const bool can_persist = (a.seqused_k != nullptr || window_bound) && !decode_one_segment_only &&
+                             (max_blocks >= 8 || base * max_blocks >= 4 * persist_grid) && base * (max_blocks + 1) < 0x3fffffffLL;
+    persistent = can_persist && !window_bound;
+    if (can_persist && window_bound) {
+      // Nearly equal units: the balance only pays where the plain grid's last wave is nearly empty.  In KV blocks, a
+      // CTA's fixed part and the merge being worth 512 keys each (as above).
+      const double fixed = 512.0 / ci.block_n;
+      const double plain = (double)((base * ns + persist_grid - 1) / persist_grid) * (ceil_div(max_blocks, ns) + fixed);
+      const double shared = (double)base * (max_blocks + fixed) / persist_grid + fixed;
+      persistent = shared < 0.85 * plain;
+    }
+    if (const char* e = std::getenv("FA_B200_DECODE_PERSISTENT"))  // tuning override: 0 off, 1 ragged ranges only, 2 wherever possible
+      persistent = can_persist && (std::atoi(e) == 2 || (std::atoi(e) == 1 && !window_bound));
     if (forced && forced->kernel == FA_KERNEL_DECODE && forced->num_splits > 1 && forced->blocks_per_split == 0) {
-      if (!can_persist || decode_one_segment_only || forced->grid <= 0 || forced->num_splits != kPersistSlots)
+      if (!can_persist || forced->grid <= 0 || forced->num_splits < kMinPersistSlots)
         return fail(FA_ERR_UNSUPPORTED, "the plan's persistent decode schedule does not fit this problem");
       persistent = true;
       persist_grid = forced->grid;
-      ns = kPersistSlots;
-      bps = 0;
+      persist_slots = forced->num_splits;
     } else if (forced) {
       persistent = false;
     }
+    if (persistent) { ns = persist_slots; bps = 0; }
   }
   if (forced && forced->kernel != FA_KERNEL_TCGEN05 && !persistent) {
     if (forced->num_splits < 1 || forced->blocks_per_split < 1 ||
@@ -334,11 +349,12 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
 // griddepcontrol.launch_dependents when it starts); the kernel waits for that kernel's completion before it reads
 // (combine.cuh).  This hides most of what a second launch costs behind a kernel of a few hundred microseconds.
 template <typename OutT>
-static cudaError_t launch_combine_t(const fa_combine_params& c, int grid, cudaStream_t st) {
+static cudaError_t launch_combine_t(const fa_combine_params& c, int64_t rows, cudaStream_t st) {
+  const bool wide = c.num_splits > 32;
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kCombineWarps * 32);
+  cfg.gridDim = dim3((unsigned)(wide ? rows : (rows + kCombineWarps - 1) / kCombineWarps));
+  cfg.blockDim = dim3((wide ? kCombineWideWarps : kCombineWarps) * 32);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -346,17 +362,17 @@ static cudaError_t launch_combine_t(const fa_combine_params& c, int grid, cudaSt
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, combine_kernel<OutT>, c);
+  return cudaLaunchKernelEx(&cfg, wide ? combine_wide_kernel<OutT> : combine_kernel<OutT>, c);
 }
 
 static int launch_combine(const fa_combine_params& c, cudaStream_t st) {
   const int64_t rows = (int64_t)c.b * c.s * c.h;
   if (rows == 0) return FA_OK;
-  const int grid = (int)((rows + kCombineWarps - 1) / kCombineWarps);
+  if (rows > 0x7fffffffLL) return fail(FA_ERR_UNSUPPORTED, "too many rows to merge");
   cudaError_t e;
-  if (c.out_dtype == FA_BF16) e = launch_combine_t<__nv_bfloat16>(c, grid, st);
-  else if (c.out_dtype == FA_FP16) e = launch_combine_t<__half>(c, grid, st);
-  else if (c.out_dtype == 2) e = launch_combine_t<float>(c, grid, st);
+  if (c.out_dtype == FA_BF16) e = launch_combine_t<__nv_bfloat16>(c, rows, st);
+  else if (c.out_dtype == FA_FP16) e = launch_combine_t<__half>(c, rows, st);
+  else if (c.out_dtype == 2) e = launch_combine_t<float>(c, rows, st);
   else return fail(FA_ERR_INVALID, "bad out_dtype");
   if (e != cudaSuccess) return fail(FA_ERR_CUDA, std::string("combine launch: ") + cudaGetErrorString(e));
   ++g_launches;

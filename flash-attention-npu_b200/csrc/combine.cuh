@@ -1,4 +1,4 @@
-// Split-KV merge (one warp per output row):
+// Split-KV merge:
 //   m = max_i lse_i;  w_i = exp(lse_i - m);  O = sum_i w_i O_i / sum_i w_i;  LSE = m + ln sum_i w_i
 // the same arithmetic as CombineScale (csrc/arch22/flash_attn_npu_v2/CombineScale.hpp:165-309).
 // An empty partial carries lse = -inf (weight 0, its O is never read).  A row whose every
@@ -70,6 +70,12 @@ __device__ __forceinline__ float4 merge_columns(int n, float l_mine, float w_min
   return acc;
 }
 
+__device__ __forceinline__ void merge_store_lse(const fa_combine_params& p, int bb, int ss, int hh, float m, float tot, bool dead) {
+  const float v = dead ? (p.partial_out ? -INFINITY : INFINITY) : m + logf(tot);
+  p.lse[bb * p.lse_batch_stride + ss * p.lse_row_stride + hh * p.lse_head_stride] = v;
+}
+
+// Up to 32 partials: one warp per output row.
 template <typename OutT>
 __global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const __grid_constant__ fa_combine_params p) {
   // The merge is launched as a programmatic dependent of the kernel in front of it (launch_combine): its CTAs may
@@ -86,51 +92,87 @@ __global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const __gri
   const int bb = (int)(row / ((int64_t)p.h * p.s));
   const float* lp = p.lse_partial + bb * p.lp_batch_stride + ss * p.lp_row_stride + hh * p.lp_head_stride;
   const float* op = p.o_partial + bb * p.op_batch_stride + ss * p.op_row_stride + hh * p.op_head_stride;
-
-  float m, tot;
-  bool dead;
   OutT* out = reinterpret_cast<OutT*>(p.o) + bb * p.o_batch_stride + ss * p.o_row_stride + hh * p.o_head_stride;
-  if (p.num_splits <= 32) {
-    float l_mine, w_mine;
-    merge_weights(p.num_splits, lane, [&](int i) { return lp[(int64_t)i * p.lp_split_stride]; }, l_mine, w_mine, m, tot, dead);
-    for (int c0 = 0; c0 < p.d; c0 += 128) {  // every lane takes part in the shuffles, also one without columns
-      const int c = c0 + lane * 4;
-      const bool on = c < p.d;
-      const float4 acc = merge_columns(p.num_splits, l_mine, w_mine, [&](int i) {
-        return on ? *reinterpret_cast<const float4*>(op + (int64_t)i * p.op_split_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  float m, tot, l_mine, w_mine;
+  bool dead;
+  merge_weights(p.num_splits, lane, [&](int i) { return lp[(int64_t)i * p.lp_split_stride]; }, l_mine, w_mine, m, tot, dead);
+  for (int c0 = 0; c0 < p.d; c0 += 128) {  // every lane takes part in the shuffles, also one without columns
+    const int c = c0 + lane * 4;
+    const bool on = c < p.d;
+    const float4 acc = merge_columns(p.num_splits, l_mine, w_mine, [&](int i) {
+      return on ? *reinterpret_cast<const float4*>(op + (int64_t)i * p.op_split_stride + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    });
+    if (on) store4<OutT>(out + c, acc);
+  }
+  if (p.lse && lane == 0) merge_store_lse(p, bb, ss, hh, m, tot, dead);
+}
+
+// More than 32 partials (one long sequence with few heads, cut over the whole grid): a CTA of 16 warps per output row.
+// Every warp weighs and sums every 16th partial, the warps' sums are added in a fixed order.  Latency-bound: with one
+// warp per row 298 partials are a chain of ~300 dependent loads.
+constexpr int kCombineWideWarps = 16;
+template <typename OutT>
+__global__ void __launch_bounds__(kCombineWideWarps * 32) combine_wide_kernel(const __grid_constant__ fa_combine_params p) {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  __shared__ float s_red[kCombineWideWarps];
+  __shared__ float4 s_acc[kCombineWideWarps][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int hh = (int)(blockIdx.x % p.h);
+  const int ss = (int)((blockIdx.x / p.h) % p.s);
+  const int bb = (int)(blockIdx.x / ((int64_t)p.h * p.s));
+  const float* lp = p.lse_partial + bb * p.lp_batch_stride + ss * p.lp_row_stride + hh * p.lp_head_stride;
+  const float* op = p.o_partial + bb * p.op_batch_stride + ss * p.op_row_stride + hh * p.op_head_stride;
+  OutT* out = reinterpret_cast<OutT*>(p.o) + bb * p.o_batch_stride + ss * p.o_row_stride + hh * p.o_head_stride;
+  auto block_reduce = [&](float v, auto op2) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = op2(v, __shfl_xor_sync(0xffffffffu, v, o));
+    __syncthreads();
+    if (lane == 0) s_red[warp] = v;
+    __syncthreads();
+    v = s_red[0];
+#pragma unroll
+    for (int w = 1; w < kCombineWideWarps; ++w) v = op2(v, s_red[w]);
+    return v;
+  };
+  float m = -INFINITY;
+  for (int i = tid; i < p.num_splits; i += kCombineWideWarps * 32) m = fmaxf(m, lp[(int64_t)i * p.lp_split_stride]);
+  m = block_reduce(m, [](float x, float y) { return fmaxf(x, y); });
+  const bool dead = m == -INFINITY;
+  float tot = 0.f;
+  if (!dead)
+    for (int i = tid; i < p.num_splits; i += kCombineWideWarps * 32) tot += __expf(lp[(int64_t)i * p.lp_split_stride] - m);
+  tot = block_reduce(tot, [](float x, float y) { return x + y; });
+  const float inv = dead ? 0.f : 1.f / tot;
+  for (int c0 = 0; c0 < p.d; c0 += 128) {
+    const int c = c0 + lane * 4;
+    const bool on = c < p.d;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    // this warp's partials are warp + 16 k; lane k - k0 holds the weight of partial k
+    for (int k0 = 0; warp + kCombineWideWarps * k0 < p.num_splits; k0 += 32) {
+      const int mine = warp + kCombineWideWarps * (k0 + lane);
+      const float l = mine < p.num_splits ? lp[(int64_t)mine * p.lp_split_stride] : -INFINITY;
+      const float w = (dead || l == -INFINITY) ? 0.f : __expf(l - m) * inv;
+      const int n = min(32, (p.num_splits - warp + kCombineWideWarps - 1) / kCombineWideWarps - k0);
+      const float4 x = merge_columns(n, l, w, [&](int i) {
+        return on ? *reinterpret_cast<const float4*>(op + (int64_t)(warp + kCombineWideWarps * (k0 + i)) * p.op_split_stride + c)
+                  : make_float4(0.f, 0.f, 0.f, 0.f);
       });
-      if (on) store4<OutT>(out + c, acc);
+      acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
     }
-  } else {
-    m = -INFINITY;
-    for (int i = lane; i < p.num_splits; i += 32) m = fmaxf(m, lp[(int64_t)i * p.lp_split_stride]);
+    s_acc[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0 && on) {
+      float4 r = s_acc[0][lane];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    dead = (m == -INFINITY);
-    tot = 0.f;
-    if (!dead)
-      for (int i = lane; i < p.num_splits; i += 32) tot += __expf(lp[(int64_t)i * p.lp_split_stride] - m);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    const float inv = dead ? 0.f : 1.f / tot;
-    for (int c = lane * 4; c < p.d; c += 128) {
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (!dead) {
-        for (int i = 0; i < p.num_splits; ++i) {
-          const float l = lp[(int64_t)i * p.lp_split_stride];
-          if (l == -INFINITY) continue;
-          const float w = __expf(l - m) * inv;
-          const float4 x = *reinterpret_cast<const float4*>(op + (int64_t)i * p.op_split_stride + c);
-          acc.x += w * x.x; acc.y += w * x.y; acc.z += w * x.z; acc.w += w * x.w;
-        }
+      for (int w = 1; w < kCombineWideWarps; ++w) {
+        const float4 x = s_acc[w][lane];
+        r.x += x.x; r.y += x.y; r.z += x.z; r.w += x.w;
       }
-      store4<OutT>(out + c, acc);
+      store4<OutT>(out + c, r);
     }
+    __syncthreads();
   }
-  if (p.lse && lane == 0) {
-    float v = dead ? (p.partial_out ? -INFINITY : INFINITY) : m + logf(tot);
-    p.lse[bb * p.lse_batch_stride + ss * p.lse_row_stride + hh * p.lse_head_stride] = v;
-  }
+  if (p.lse && tid == 0) merge_store_lse(p, bb, ss, hh, m, tot, dead);
 }
 
 }  // namespace fa

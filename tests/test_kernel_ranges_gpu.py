@@ -48,3 +48,35 @@ def test_packed_queries_against_a_cache_on_tcgen05(dtype, d, window, page):
         go, gl = OA.flash_attn_with_kvcache(q[rows].unsqueeze(0), ki, vi, cache_seqlens=lens[i:i + 1], block_table=bi, causal=True,
                                             window_size=(window if window < k_lens[i] - 1 else -1, -1))
         U.check_rules(out[rows].unsqueeze(0), lse[:, rows].unsqueeze(0), go, gl, tag=f"sequence {i}")
+
+
+@pytest.mark.parametrize("b,hk,d,keys", [(1, 1, 128, 40000), (1, 8, 128, 2048), (3, 4, 128, 512)])
+def test_few_sequences_are_cut_over_the_grid(b, hk, d, keys):
+    """One unit over up to the whole grid: up to ~300 partials, the merge of more than 32 among them."""
+    g = torch.Generator().manual_seed(keys)
+    h = 4 * hk
+    q, kc, vc = U.normal((b, 1, h, d), BF, g), U.normal((b, keys, hk, d), BF, g), U.normal((b, keys, hk, d), BF, g)
+    lens = torch.tensor([keys, 1, keys // 3][:b], dtype=torch.int32)
+    out, lse, pl = ops.attention_forward(q.cuda(), kc.cuda(), vc.cuda(), seqused_k=lens.cuda(), softmax_scale=d ** -0.5, causal=True,
+                                         return_plan=True)
+    assert pl.kernel == L.KERNEL_DECODE and pl.num_splits > 1
+    go, gl = OA.flash_attn_with_kvcache(q, kc, vc, cache_seqlens=lens, causal=True)
+    U.check_rules(out, lse, go, gl, tag=f"b {b} hk {hk} d {d} keys {keys}")
+
+
+@pytest.mark.parametrize("n", [32, 33, 300, 1000])
+@pytest.mark.parametrize("d", [4, 128, 256, 300])
+def test_merge_of_many_partials(n, d):
+    """fp32 partials, fp32 result: the merge's own rounding only, sqrt(n) terms of 2^-24 and two exponentials of 2^-22."""
+    g = torch.Generator().manual_seed(n + d)
+    o, lse = torch.randn((n, 2, 3, 2, d), generator=g), torch.randn((n, 2, 3, 2), generator=g) * 3
+    lse[::3, 0, 1] = float("-inf")
+    lse[:, 1, 2, 1] = float("-inf")
+    o[:, 1, 2, 1] = float("nan")  # an empty partial's values are never read
+    out, l = ops.combine(o.cuda(), lse.cuda())
+    w = torch.softmax(lse.double(), 0).nan_to_num(0.0)
+    want = (w.unsqueeze(-1) * o.double().nan_to_num(0.0)).sum(0)
+    torch.testing.assert_close(out.cpu().double(), want, rtol=1e-5, atol=1e-5)
+    want_l = torch.logsumexp(lse.double(), 0)
+    want_l[want_l == float("-inf")] = float("inf")
+    torch.testing.assert_close(l.cpu().double(), want_l, rtol=1e-5, atol=1e-5)
