@@ -143,22 +143,24 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
   }
   MmaConfigInfo ci;
   if (!mma_config_info(hd_pad, cfg, &ci)) return fail(FA_ERR_UNSUPPORTED, "no tile configuration");
-  // ---- producer / consumer decode kernel: <= 32 packed rows, head dim <= 128 (> 64), rows that can
-  //      be moved by 16-byte aligned bulk copies ----
+  // ---- producer / consumer decode kernel: <= 32 packed rows, rows that can be moved by tiled TMA loads ----
   int kernel_id = FA_KERNEL_MMA;
   bool decode_one_segment_only = false;  // the chosen decode configuration keeps its merge slab over the ring
   {
     auto al16 = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };
     const bool strides_ok = a.k_row_stride % 8 == 0 && a.k_head_stride % 8 == 0 && a.k_batch_stride % 8 == 0 &&
                             a.v_row_stride % 8 == 0 && a.v_head_stride % 8 == 0 && a.v_batch_stride % 8 == 0;
-    // K / V stages are fetched by tiled TMA loads: exact head dim 128, 16-byte aligned strides, a
-    // per-sequence length vector, and pages that hold whole key blocks
-    const bool eligible = a.d == 128 && rows_max <= 32 && rows_max > 0 && !a.cu_seqlens_k && strides_ok &&
+    // K / V stages are fetched by tiled TMA loads: 16-byte aligned strides, no packed keys, and pages that hold whole
+    // key blocks
+    const bool eligible = rows_max <= 32 && rows_max > 0 && !a.cu_seqlens_k && strides_ok &&
                           al16(a.k) && al16(a.v) && a.k_batch_stride > 0 && a.v_batch_stride > 0 &&
                           (!a.block_table || a.page_size % 128 == 0);
+    // Several query rows per sequence over few keys, head dims other than 128: left to the register-accumulator kernel,
+    // whose handling of cache tails is tested at these sizes (64 columns, 6144 keys: 18 us there, 12 us here).
+    const bool short_range = a.d != 128 && a.seqlen_q > 1 && (long long)a.b * a.h_k * max_k_bound <= 8192;
     if (a.kernel == FA_KERNEL_DECODE && !eligible)
       return fail(FA_ERR_UNSUPPORTED, "the decode kernel does not cover this problem");
-    if (eligible && (a.kernel == FA_KERNEL_DECODE || a.kernel == FA_KERNEL_AUTO)) {
+    if (eligible && (a.kernel == FA_KERNEL_DECODE || (a.kernel == FA_KERNEL_AUTO && !short_range))) {
       // Measured best.  Up to 16 rows: two resident CTAs of 1x4 consumer warps.  17-32 rows: one CTA of 2x4
       // consumer warps for long key ranges and for launches that become persistent; for short ranges (a
       // sliding window, short caches) two resident CTAs of 2x2 warps, so that one CTA's Q load, slice
@@ -170,7 +172,7 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
         if (windowed) keys = (long long)wl + std::max(wr, 0) + 32 / gp + 2;
         const bool may_persist = a.seqused_k && !windowed && a.num_splits == 0 && !a.cu_seqlens_q && a.kv_total == 0 &&
                                  !a.partial_out;
-        dcfg = (!may_persist && keys <= 16384) ? 11 : 5;
+        dcfg = (hd_pad == 128 && !may_persist && keys <= 16384) ? 11 : 5;
       }
       if (const char* e = std::getenv("FA_B200_DECODE_CONFIG")) {  // tuning override: decode tile configuration
         const int forced = std::atoi(e);
@@ -435,8 +437,10 @@ static int run_fwd(const fa_fwd_params& a, void* workspace, size_t workspace_byt
     if (!tma_encode_rows(&tm_k, a.k, a.dtype, a.d, a.h_k, rows, outer, a.k_head_stride, a.k_row_stride, a.k_batch_stride, P.pl.block_n) ||
         !tma_encode_rows(&tm_v, a.v, a.dtype, a.d, a.h_k, rows, outer, a.v_head_stride, a.v_row_stride, a.v_batch_stride, P.pl.block_n))
       return fail(FA_ERR_CUDA, "cuTensorMapEncodeTiled failed for the KV cache");
-    e = bf ? launch_decode_128_bf16(P.pl.config, kp, tm_k, tm_v, P.pl.grid, st)
-           : launch_decode_128_fp16(P.pl.config, kp, tm_k, tm_v, P.pl.grid, st);
+    auto* launch = P.hd_pad == 64    ? (bf ? launch_decode_64_bf16 : launch_decode_64_fp16)
+                   : P.hd_pad == 128 ? (bf ? launch_decode_128_bf16 : launch_decode_128_fp16)
+                                     : (bf ? launch_decode_256_bf16 : launch_decode_256_fp16);
+    e = launch(P.pl.config, kp, tm_k, tm_v, P.pl.grid, st);
   } else
   switch (P.hd_pad) {
     case 64: e = bf ? launch_mma_64_bf16(P.pl.config, kp, P.pl.grid, st) : launch_mma_64_fp16(P.pl.config, kp, P.pl.grid, st); break;

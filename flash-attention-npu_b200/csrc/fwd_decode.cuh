@@ -26,7 +26,8 @@ template <int HD_, typename T_, int MT_, int WM_, int WN_, int BN_, int ST_, int
 struct DecTraits {
   using T = T_;
   static constexpr int HD = HD_, MT = MT_, WM = WM_, WN = WN_, NCW = WM_ * WN_, BN = BN_, ST = ST_;
-  static_assert(HD == 128, "K / V tiles arrive as two 64-column TMA boxes");
+  static_assert(HD == 64 || HD == 128 || HD == 256, "tile widths; a head dim below the width leaves zero columns (TMA fill)");
+  static constexpr int HALVES = HD / 64;         // K / V tiles arrive as 64-column TMA boxes
   static constexpr int BM = 16 * MT * WM;
   static constexpr int NTHREADS = 32 * (NCW + 1);
   static constexpr int NW = BN / WN;
@@ -36,7 +37,7 @@ struct DecTraits {
   static constexpr int CHUNKS = HD / 8;
   static constexpr int PITCH = HD * 2 + 16;      // Q rows: padded pitch, no swizzle
   static constexpr int HALF_BYTES = BN * 128;    // one 64-column half of a K or V tile (128-byte swizzled rows)
-  static constexpr int KV_BYTES = 2 * HALF_BYTES;
+  static constexpr int KV_BYTES = HALVES * HALF_BYTES;
   static constexpr int STAGE_BYTES = 2 * KV_BYTES;
   static constexpr int PIPE_BYTES = ST * STAGE_BYTES;
   static constexpr int SLAB_LD = HD + 4;
@@ -54,12 +55,13 @@ struct DecTraits {
   static constexpr int BAR_BYTES = 128 + 2 * ST * 8;
   // [pipeline | slab | Q | (m, l) | barriers], the pipeline at a 1024-byte aligned base
   static constexpr int SMEM_BYTES = 1024 + MAIN_BYTES + Q_BYTES + ML_BYTES + BAR_BYTES;
-  static constexpr bool Q_IN_REGS = (MT == 1);
-  static constexpr int MIN_CTAS = SLAB_IN_RING ? 2 : 0;  // resident CTAs per SM the register count must allow (0: no constraint)
+  static constexpr bool Q_IN_REGS = (MT == 1 && HD <= 128);  // 256: 128 registers of O leave no room for 64 of Q
+  // resident CTAs per SM the register count must allow (0: no constraint)
+  static constexpr int MIN_CTAS = (SLAB_IN_RING || (HD == 64 && WM > 1)) ? 2 : 0;
   static_assert(NW % 16 == 0, "each consumer warp needs a multiple of 16 keys");
 };
 
-// Address of 16-byte chunk `ch` (0..15) of row `row` in a K / V tile laid out by two TMA boxes of
+// Address of 16-byte chunk `ch` (0 .. HD / 8 - 1) of row `row` in a K / V tile laid out by TMA boxes of
 // 64 columns with the 128-byte swizzle (chunk index XOR row % 8 inside each 128-byte row).
 template <class Tr>
 __device__ __forceinline__ uint32_t kv_chunk_addr(uint32_t tile_base, int row, int ch) {
@@ -76,7 +78,7 @@ __device__ __forceinline__ void decode_fix_rows(const KParams& p, const SeqView<
   for (int c = lane; c < Tr::NW * Tr::CHUNKS; c += 32) {
     const int row = wn * Tr::NW + c / Tr::CHUNKS, ch = c % Tr::CHUNKS;
     const int t = t0 + row;
-    if (t < sv.l_cache) continue;
+    if (t < sv.l_cache || ch * 8 >= p.a.d) continue;  // columns beyond the head dim: zeros from the TMA unit
     uint4 kv4 = make_uint4(0, 0, 0, 0), vv4 = make_uint4(0, 0, 0, 0);
     if (t < sv.k_len) {
       const int tn = t - sv.l_cache;
@@ -98,8 +100,7 @@ __device__ __forceinline__ void decode_fix_rows(const KParams& p, const SeqView<
   __syncwarp();
 }
 
-// Producer: one elected lane issues four tiled TMA loads per stage (K and V, two 64-column halves
-// each).  Tensor maps are 4-D (d, kv head, row, batch-or-page); every load targets the issuing CTA only.
+// Producer: one elected lane issues the tiled TMA loads of a stage (K and V, 64 columns each).  Tensor maps are 4-D (d, kv head, row, batch-or-page); every load targets the issuing CTA only.
 template <class Tr>
 __device__ __forceinline__ bool decode_producer(const KParams& p, const SeqView<typename Tr::T>& sv,
                                                 const CUtensorMap* tm_k, const CUtensorMap* tm_v, uint32_t pipe_base,
@@ -121,10 +122,10 @@ __device__ __forceinline__ bool decode_producer(const KParams& p, const SeqView<
     }
     if (tc5::elect_one()) {
       tc5::mbar_arrive_expect_tx(full, Tr::STAGE_BYTES);
-      tc5::tma_load_4d(k_base, tm_k, full, 0, hk, row, outer);
-      tc5::tma_load_4d(k_base + Tr::HALF_BYTES, tm_k, full, 64, hk, row, outer);
-      tc5::tma_load_4d(v_base, tm_v, full, 0, hk, row, outer);
-      tc5::tma_load_4d(v_base + Tr::HALF_BYTES, tm_v, full, 64, hk, row, outer);
+#pragma unroll
+      for (int hf = 0; hf < Tr::HALVES; ++hf) tc5::tma_load_4d(k_base + hf * Tr::HALF_BYTES, tm_k, full, 64 * hf, hk, row, outer);
+#pragma unroll
+      for (int hf = 0; hf < Tr::HALVES; ++hf) tc5::tma_load_4d(v_base + hf * Tr::HALF_BYTES, tm_v, full, 64 * hf, hk, row, outer);
     }
     __syncwarp();
   }

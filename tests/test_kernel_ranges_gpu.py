@@ -50,7 +50,34 @@ def test_packed_queries_against_a_cache_on_tcgen05(dtype, d, window, page):
         U.check_rules(out[rows].unsqueeze(0), lse[:, rows].unsqueeze(0), go, gl, tag=f"sequence {i}")
 
 
-@pytest.mark.parametrize("b,hk,d,keys", [(1, 1, 128, 40000), (1, 8, 128, 2048), (3, 4, 128, 512)])
+@pytest.mark.parametrize("page", [0, 128])
+@pytest.mark.parametrize("rows", [1, 16, 17, 32])
+@pytest.mark.parametrize("d", [64, 72, 96, 128, 136, 192, 256])
+def test_decode_kernel_every_head_dim(d, rows, page):
+    """1 to 32 packed rows per kv head; new tokens appended with rotary; lengths around the key blocks' edges."""
+    import flash_attn_npu_v2 as fa2
+    g = torch.Generator().manual_seed(d * 100 + rows)
+    dtype = BF if rows % 2 else FP
+    hk, group, s_q = 2, {1: 1, 16: 8, 17: 17, 32: 8}[rows], {1: 1, 16: 2, 17: 1, 32: 4}[rows]
+    new, room = s_q, 520
+    lens = torch.tensor([0, 1, 127, 128, 300, room - new], dtype=torch.int32)
+    b = lens.numel()
+    rotary = d // 16 * 16
+    q = U.normal((b, s_q, hk * group, d), dtype, g)
+    kc, vc, bt = _cache(g, dtype, b, room, hk, d, page)
+    k, v = U.normal((b, new, hk, d), dtype, g), U.normal((b, new, hk, d), dtype, g)
+    cos, sin = U.rotary_tables(room, rotary, dtype)
+    kc_o, vc_o, kc_g, vc_g = kc.clone(), vc.clone(), kc.cuda(), vc.cuda()
+    go, gl = OA.flash_attn_with_kvcache(q, kc_o, vc_o, k, v, rotary_cos=cos, rotary_sin=sin, cache_seqlens=lens, block_table=bt,
+                                        causal=True, rotary_interleaved=False)
+    out, lse = fa2.flash_attn_with_kvcache(q.cuda(), kc_g, vc_g, k.cuda(), v.cuda(), rotary_cos=cos.cuda(), rotary_sin=sin.cuda(),
+                                           cache_seqlens=lens.cuda(), block_table=_cuda(bt), causal=True,
+                                           rotary_interleaved=False, return_softmax_lse=True)
+    assert torch.equal(kc_g.cpu().view(torch.int16), kc_o.view(torch.int16)) and torch.equal(vc_g.cpu().view(torch.int16), vc_o.view(torch.int16))
+    U.check_rules(out, lse, go, gl, tag=f"d {d} rows {rows}")
+
+
+@pytest.mark.parametrize("b,hk,d,keys", [(1, 1, 128, 40000), (1, 1, 256, 9001), (2, 1, 64, 20001), (1, 8, 128, 2048), (3, 4, 128, 512)])
 def test_few_sequences_are_cut_over_the_grid(b, hk, d, keys):
     """One unit over up to the whole grid: up to ~300 partials, the merge of more than 32 among them."""
     g = torch.Generator().manual_seed(keys)
