@@ -381,14 +381,33 @@ static int launch_combine(const fa_combine_params& c, cudaStream_t st) {
   return FA_OK;
 }
 
+// Device scratch of one call: given by the caller, or asked for once its size is known.
+struct Workspace {
+  void* ptr;
+  size_t bytes;
+  void* (*alloc)(size_t, void*);
+  void* ctx;
+  bool get(size_t need) {
+    if (need == 0 || (ptr && bytes >= need)) return true;
+    if (!alloc) return false;
+    ptr = alloc(need, ctx);
+    bytes = ptr ? need : 0;
+    return ptr != nullptr;
+  }
+};
+
 // skip_merge: leave the split partials in the workspace (the caller merges them itself); *splits_out = their number.
-static int run_fwd(const fa_fwd_params& a, void* workspace, size_t workspace_bytes, cudaStream_t st,
-                   const fa_fwd_plan* forced = nullptr, bool skip_merge = false, int* splits_out = nullptr) {
+static int run_fwd(const fa_fwd_params& a, Workspace& ws, cudaStream_t st, const fa_fwd_plan* forced = nullptr,
+                   bool skip_merge = false, int* splits_out = nullptr) {
   if (!a.q || !a.k || !a.v || !a.o || !a.lse) return fail(FA_ERR_INVALID, "q, k, v, o and lse must be non-null");
   Planned P;
   int rc = make_plan(a, &P, forced);
   if (rc != FA_OK) return rc;
   if (a.total_q == 0 || a.seqlen_q == 0) return FA_OK;
+  if (P.pl.workspace_bytes) {
+    if (!ws.get(P.pl.workspace_bytes)) return fail(FA_ERR_WORKSPACE, "workspace missing or too small");
+    if ((reinterpret_cast<uintptr_t>(ws.ptr) & 15) != 0) return fail(FA_ERR_WORKSPACE, "workspace must be 16-byte aligned");
+  }
   if (P.pl.kernel == FA_KERNEL_TCGEN05) {
     fa_fwd_params a2 = a;
     if (a.k_new) {
@@ -396,9 +415,7 @@ static int run_fwd(const fa_fwd_params& a, void* workspace, size_t workspace_byt
       // the workspace; the prefill kernel then sees a cache of cache_seqlens + s_new keys.
       void* q_rot = nullptr;
       if (a.rotary_cos) {
-        if (!workspace || workspace_bytes < P.pl.workspace_bytes) return fail(FA_ERR_WORKSPACE, "workspace missing or too small");
-        if ((reinterpret_cast<uintptr_t>(workspace) & 15) != 0) return fail(FA_ERR_WORKSPACE, "workspace must be 16-byte aligned");
-        q_rot = workspace;
+        q_rot = ws.ptr;
         a2.q = q_rot;
         a2.q_head_stride = a.d;
         a2.q_row_stride = (int64_t)a.h * a.d;
@@ -420,12 +437,10 @@ static int run_fwd(const fa_fwd_params& a, void* workspace, size_t workspace_byt
   kp.status = device_status_word();
   if (!kp.status) return fail(FA_ERR_CUDA, "cannot look up the device status word");
   if (P.pl.num_splits > 1) {
-    if (!workspace || workspace_bytes < P.pl.workspace_bytes) return fail(FA_ERR_WORKSPACE, "workspace missing or too small");
-    if ((reinterpret_cast<uintptr_t>(workspace) & 15) != 0) return fail(FA_ERR_WORKSPACE, "workspace must be 16-byte aligned");
-    kp.lse_partial = reinterpret_cast<float*>(workspace);
+    kp.lse_partial = reinterpret_cast<float*>(ws.ptr);
     // O partials start at a 16-byte boundary after the LSE partials
     const size_t lse_bytes = ((size_t)P.pl.num_splits * kp.lse_elems * sizeof(float) + 15) & ~(size_t)15;
-    kp.o_partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + lse_bytes);
+    kp.o_partial = reinterpret_cast<float*>(reinterpret_cast<char*>(ws.ptr) + lse_bytes);
   }
   cudaError_t e = cudaErrorInvalidValue;
   const bool bf = a.dtype == FA_BF16;
@@ -530,7 +545,8 @@ static int run_fwd_noalloc(const fa_fwd_params& a_in, cudaStream_t st) {
   void* scratch = nullptr;
   rc = noalloc_scratch_ptr(&scratch);
   if (rc != FA_OK) return rc;
-  return run_fwd(a, scratch, kNoAllocScratchBytes, st);
+  Workspace ws{scratch, kNoAllocScratchBytes, nullptr, nullptr};
+  return run_fwd(a, ws, st);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -596,7 +612,8 @@ static int run_fwd_exchange(const fa_fwd_params& a_in, void* workspace, size_t w
   a.o_head_stride = (int64_t)a.seqlen_q * a.d;
   a.o_row_stride = a.d;
   int ns = 1;
-  rc = run_fwd(a, workspace, workspace_bytes, st, nullptr, true, &ns);
+  Workspace ws{workspace, workspace_bytes, nullptr, nullptr};
+  rc = run_fwd(a, ws, st, nullptr, true, &ns);
   if (rc != FA_OK) return rc;
   if (ns != ns_plan) return fail(FA_ERR_CUDA, "split plan changed between planning and launch");
 
@@ -687,8 +704,7 @@ static int plan_decode(const void* buf, size_t n, PlanBlob* out) {
   return FA_OK;
 }
 
-static int run_fwd_planned(const fa_fwd_params& a, const void* buf, size_t n, void* workspace, size_t workspace_bytes,
-                           cudaStream_t st) {
+static int run_fwd_planned(const fa_fwd_params& a, const void* buf, size_t n, Workspace& ws, cudaStream_t st) {
   PlanBlob blob;
   int rc = plan_decode(buf, n, &blob);
   if (rc != FA_OK) return rc;
@@ -719,10 +735,10 @@ static int run_fwd_planned(const fa_fwd_params& a, const void* buf, size_t n, vo
       if (a2.block_table) a2.seqlen_k = ceil_div(a2.seqlen_k, a2.page_size) * a2.page_size;
       if (a2.max_seqlen_k_known > blob.seqlen_k) a2.max_seqlen_k_known = blob.seqlen_k;
     }
-    rc = run_fwd(a2, workspace, workspace_bytes, st, &blob.plan);
+    rc = run_fwd(a2, ws, st, &blob.plan);
     if (rc != FA_ERR_UNSUPPORTED) return rc;
   }
-  return run_fwd(a, workspace, workspace_bytes, st);
+  return run_fwd(a, ws, st);
 }
 
 }  // namespace fa
@@ -738,14 +754,25 @@ int fa_b200_fwd_noalloc(const fa_fwd_params* p, void* stream) {
 int fa_b200_fwd(const fa_fwd_params* p, void* workspace, size_t workspace_bytes, void* stream) {
   if (!p) return fa::fail(FA_ERR_INVALID, "null params");
   fa::g_err.clear();
-  return fa::run_fwd(*p, workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream));
+  fa::Workspace ws{workspace, workspace_bytes, nullptr, nullptr};
+  return fa::run_fwd(*p, ws, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int fa_b200_fwd_alloc(const fa_fwd_params* p, const void* plan, size_t plan_bytes, void* (*alloc)(size_t, void*), void* ctx,
+                      void* stream) {
+  if (!p || !alloc) return fa::fail(FA_ERR_INVALID, "null params");
+  fa::g_err.clear();
+  fa::Workspace ws{nullptr, 0, alloc, ctx};
+  const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  return plan ? fa::run_fwd_planned(*p, plan, plan_bytes, ws, st) : fa::run_fwd(*p, ws, st);
 }
 
 int fa_b200_fwd_planned(const fa_fwd_params* p, const void* plan, size_t plan_bytes, void* workspace, size_t workspace_bytes,
                         void* stream) {
   if (!p) return fa::fail(FA_ERR_INVALID, "null params");
   fa::g_err.clear();
-  return fa::run_fwd_planned(*p, plan, plan_bytes, workspace, workspace_bytes, reinterpret_cast<cudaStream_t>(stream));
+  fa::Workspace ws{workspace, workspace_bytes, nullptr, nullptr};
+  return fa::run_fwd_planned(*p, plan, plan_bytes, ws, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int fa_b200_plan_encode(const fa_fwd_params* p, void* buf, size_t buf_bytes) {

@@ -20,7 +20,7 @@ static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 template <int HD, typename T>
 static cudaError_t launch_bwd(const BwdParams& p, int n_kblocks, cudaStream_t st) {
   constexpr int smem = BwdSmem<HD>::BYTES;
-  cudaError_t e = cudaFuncSetAttribute(bwd_kernel<HD, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = allow_smem(reinterpret_cast<const void*>(bwd_kernel<HD, T>), smem);
   if (e != cudaSuccess) return e;
   bwd_kernel<HD, T><<<dim3(n_kblocks, p.h_k, p.b), kBwdThreads, smem, st>>>(p);
   return cudaGetLastError();

@@ -52,7 +52,7 @@ int bwd_tc5_launch(const BwdParams& p, const fa_bwd_params& a, cudaStream_t st, 
   cudaError_t e = cudaMemsetAsync(counters, 0, 2 * sizeof(int32_t), st);
   auto launch = [&](auto kern, dim3 grid, const CUtensorMap& mq, const CUtensorMap& mdo, int32_t* counter) {
     if (e != cudaSuccess) return;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    e = allow_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
     if (e == cudaSuccess) {
       kern<<<grid, kThreads, kSmemBytes, st>>>(p, mq, mdo, tk, tv, status, counter);
       e = cudaGetLastError();

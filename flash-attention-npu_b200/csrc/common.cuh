@@ -32,6 +32,10 @@ struct KParams {
   int32_t* status;    // device status word (bounded waits that gave up), may be null
 };
 
+// cudaFuncSetAttribute(dynamic shared memory) once per kernel and device: it costs about half a microsecond, which a small
+// call would pay on every launch (fwd_tc5.cu).
+cudaError_t allow_smem(const void* kernel, int bytes);
+
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // ---- index tensors are never trusted ----

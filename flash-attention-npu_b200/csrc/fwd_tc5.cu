@@ -9,6 +9,7 @@
 #include <mutex>
 #include <string>
 #include <type_traits>
+#include <unordered_map>
 
 #include "fwd_tc5_roles.cuh"
 #include "fwd_tc5_softmax.cuh"
@@ -278,7 +279,7 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
   if (!ok) { *err = "cuTensorMapEncodeTiled failed"; return FA_ERR_CUDA; }
   cudaError_t e = cudaErrorInvalidValue;
   auto launch = [&](auto kern) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    e = allow_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
     if (e == cudaSuccess) {
       kern<<<pl.grid, kThreads, kSmemBytes, st>>>(p, tq, tk, tv);
       e = cudaGetLastError();
@@ -305,6 +306,23 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
   }
   if (e != cudaSuccess) { *err = std::string("tcgen05 kernel launch: ") + cudaGetErrorString(e); return FA_ERR_CUDA; }
   return FA_OK;
+}
+
+cudaError_t allow_smem(const void* kernel, int bytes) {
+  static std::mutex mu;
+  static std::unordered_map<const void*, uint64_t> done;  // kernel -> devices that have been told (bit per device)
+  int dev = 0;
+  if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
+  if (dev < 64) {
+    std::lock_guard<std::mutex> lock(mu);
+    if ((done[kernel] >> dev) & 1) return cudaSuccess;
+  }
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && dev < 64) {
+    std::lock_guard<std::mutex> lock(mu);
+    done[kernel] |= 1ull << dev;
+  }
+  return e;
 }
 
 int32_t* device_status_word() { return tc5::status_word(); }

@@ -9,6 +9,9 @@ backward go through ``torch.library`` operators of the reference's names (``cust
 ``flash_attn_func`` and ``flash_attn_varlen_func`` (and their packed variants) are differentiable:
 autograd Functions with the structure of the reference's (:774-824, :827-900), whose backward
 calls ``bwd`` / ``varlen_bwd`` of the extension.  The KV-cache entry point is inference only.
+
+Eager calls with ordinary arguments take the native host path (csrc/torch_binding.cpp), which answers NotImplemented for
+anything it leaves to the code here: traced calls, tensor subclasses, head dims to pad, arguments to refuse.
 """
 from __future__ import annotations
 
@@ -18,6 +21,7 @@ import torch
 import torch.nn.functional as F
 
 import flash_attn_npu_arch22_v2 as _ext
+from flash_b200 import _native
 
 from . import custom_ops as _ops  # registers the torch.library operators the calls below go through
 
@@ -106,6 +110,11 @@ def flash_attn_func(q, k, v, dropout_p=0.0, softmax_scale=None, causal=False, wi
     _check_dropout(dropout_p)
     if softmax_scale is None:
         softmax_scale = q.shape[-1] ** (-0.5)
+    if not torch.compiler.is_compiling():
+        r = _native.attention(q, k, v, None, None, 0, 0, alibi_slopes, softmax_scale, causal, window_size[0], window_size[1],
+                              softcap, 0)
+        if r is not NotImplemented:
+            return (*r, torch.empty((0,), dtype=q.dtype, device=q.device)) if return_attn_probs else r[0]
     out, lse, s_dmask = FlashAttnFunc.apply(q, k, v, dropout_p, softmax_scale, causal, tuple(window_size), softcap,
                                             alibi_slopes, deterministic, return_attn_probs)
     return (out, lse, s_dmask) if return_attn_probs else out
@@ -133,6 +142,11 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, ma
     _check_dropout(dropout_p)
     if softmax_scale is None:
         softmax_scale = q.shape[-1] ** (-0.5)
+    if block_table is None and not torch.compiler.is_compiling():
+        r = _native.attention(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, alibi_slopes, softmax_scale,
+                              causal, window_size[0], window_size[1], softcap, 0)
+        if r is not NotImplemented:
+            return (*r, torch.empty((0,), dtype=q.dtype, device=q.device)) if return_attn_probs else r[0]
     out, lse, s_dmask = FlashAttnVarlenFunc.apply(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
                                                   dropout_p, softmax_scale, causal, tuple(window_size), softcap,
                                                   alibi_slopes, deterministic, block_table)
@@ -173,6 +187,12 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, rotary_cos=None
     aligned causal mask, window [i + s_k - s_q - left, i + s_k - s_q + right], rows without a
     visible key give 0.  cache_seqlens is not updated by the call.
     """
+    if cache_leftpad is None and not isinstance(cache_seqlens, int) and not torch.compiler.is_compiling():
+        r = _native.kvcache(q, k_cache, v_cache, k, v, None, 0, cache_seqlens, cache_batch_idx, block_table, rotary_cos, rotary_sin,
+                            rotary_interleaved, alibi_slopes, q.shape[-1] ** (-0.5) if softmax_scale is None else softmax_scale,
+                            causal, window_size[0], window_size[1], softcap, num_splits, None)
+        if r is not NotImplemented:
+            return r if return_softmax_lse else r[0]
     assert k_cache.stride(-1) == 1, "k_cache must have contiguous last dimension"
     assert v_cache.stride(-1) == 1, "v_cache must have contiguous last dimension"
     q, k, v = [maybe_contiguous(x) for x in (q, k, v)]

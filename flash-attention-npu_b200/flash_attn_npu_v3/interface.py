@@ -7,6 +7,9 @@ Arguments the backend does not implement (qv, *_descale, attention_chunk, sequse
 cu_seqlens_k_new, rotary_seqlens, cache_leftpad) must keep their defaults, as in the reference
 (csrc/arch22/flash_attn_npu_v3/flash_api.cpp:150-162).  ``flash_attn_func`` and
 ``flash_attn_varlen_func`` are differentiable (backward through ``flash_attn_npu_arch22_v3.bwd``).
+
+Eager calls with ordinary arguments take the native host path (csrc/torch_binding.cpp), which answers NotImplemented for
+anything it leaves to the code here: traced calls, tensor subclasses, head dims to pad, arguments to refuse.
 """
 from __future__ import annotations
 
@@ -15,6 +18,7 @@ from typing import Optional, Union
 import torch
 
 import flash_attn_npu_arch22_v3 as _ext
+from flash_b200 import _native
 
 from . import custom_ops as _ops  # registers the torch.library operators the calls below go through
 
@@ -97,6 +101,12 @@ def flash_attn_func(q, k, v, softmax_scale=None, causal=False, qv=None, q_descal
     """q (b, s_q, h, d), k / v (b, s_k, h_k, d) -> out, or (out, softmax_lse (b, h, s_q))."""
     if softmax_scale is None:
         softmax_scale = _default_scale(q, qv)
+    if (qv is None and q_descale is None and k_descale is None and v_descale is None and attention_chunk == 0
+            and scheduler_metadata is None and not torch.compiler.is_compiling()):
+        r = _native.attention(q, k, v, None, None, 0, 0, None, softmax_scale, causal, window_size[0], window_size[1], softcap,
+                              num_splits)
+        if r is not NotImplemented:
+            return r if return_attn_probs else r[0]
     out, lse = _AttnFunc.apply(q, k, v, dict(
         qv=qv, q_descale=q_descale, k_descale=k_descale, v_descale=v_descale, softmax_scale=softmax_scale, causal=causal,
         window_size_left=window_size[0], window_size_right=window_size[1], attention_chunk=attention_chunk,
@@ -126,6 +136,12 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, ma
     """q (total_q, h, d), k / v (total_k, h_k, d) -> out, or (out, softmax_lse (h, total_q))."""
     if softmax_scale is None:
         softmax_scale = _default_scale(q, qv)
+    if (qv is None and seqused_q is None and seqused_k is None and q_descale is None and k_descale is None and v_descale is None
+            and attention_chunk == 0 and scheduler_metadata is None and not torch.compiler.is_compiling()):
+        r = _native.attention(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, None, softmax_scale, causal,
+                              window_size[0], window_size[1], softcap, num_splits)
+        if r is not NotImplemented:
+            return r if return_attn_probs else r[0]
     out, lse = _AttnFunc.apply(q, k, v, dict(
         qv=qv, cu_seqlens_q=cu_seqlens_q, cu_seqlens_k=cu_seqlens_k, seqused_q=seqused_q, seqused_k=seqused_k,
         max_seqlen_q=max_seqlen_q, max_seqlen_k=max_seqlen_k, q_descale=q_descale, k_descale=k_descale,
@@ -154,10 +170,21 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, qv=None, rotary
     """KV-cache attention; q is (b, s_q, h, d) or (total_q, h, d) with cu_seqlens_q + max_seqlen_q.
     Returns out, or (out, softmax_lse, out_accum, softmax_lse_accum) when return_softmax_lse
     (the last two are empty tensors, as in the reference :1095)."""
-    assert k_cache.stride(-1) == 1, "k_cache must have contiguous last dimension"
-    assert v_cache.stride(-1) == 1, "v_cache must have contiguous last dimension"
     if softmax_scale is None:
         softmax_scale = _default_scale(q, qv)
+    if (qv is None and cache_leftpad is None and cu_seqlens_k_new is None and rotary_seqlens is None and q_descale is None
+            and k_descale is None and v_descale is None and attention_chunk == 0 and not isinstance(cache_seqlens, int)
+            and not torch.compiler.is_compiling()):
+        plan = None if scheduler_metadata is None else _ext._plan_bytes(scheduler_metadata)
+        r = _native.kvcache(q, k_cache, v_cache, k, v, cu_seqlens_q, max_seqlen_q, cache_seqlens, cache_batch_idx, page_table,
+                            rotary_cos, rotary_sin, rotary_interleaved, None, softmax_scale, causal, window_size[0],
+                            window_size[1], softcap, num_splits, plan)
+        if r is not NotImplemented:
+            if not return_softmax_lse:
+                return r[0]
+            return (*r, torch.empty((0,), device=q.device), torch.empty((0,), device=q.device))
+    assert k_cache.stride(-1) == 1, "k_cache must have contiguous last dimension"
+    assert v_cache.stride(-1) == 1, "v_cache must have contiguous last dimension"
     if cache_seqlens is not None and isinstance(cache_seqlens, int):
         cache_seqlens = torch.full((q.shape[0],), cache_seqlens, dtype=torch.int32, device=k_cache.device)
     out, lse, *rest = _forward(q, k_cache, v_cache, k, v, qv, None, cu_seqlens_q, None, cu_seqlens_k_new, None,

@@ -90,7 +90,7 @@ class Exchange(C.Structure):
 
 # every symbol include/fa_b200.h declares
 EXPORTS = (
-    "fa_b200_fwd", "fa_b200_fwd_noalloc", "fa_b200_fwd_plan", "fa_b200_combine", "fa_b200_normalize_window",
+    "fa_b200_fwd", "fa_b200_fwd_alloc", "fa_b200_fwd_noalloc", "fa_b200_fwd_plan", "fa_b200_combine", "fa_b200_normalize_window",
     "fa_b200_check_status", "fa_b200_last_error", "fa_b200_status_string", "fa_b200_abi_version",
     "fa_b200_launch_count", "fa_b200_bwd", "fa_b200_bwd_workspace_bytes",
     "fa_b200_plan_encode", "fa_b200_plan_decode", "fa_b200_fwd_planned",

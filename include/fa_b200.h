@@ -155,6 +155,11 @@ typedef struct fa_combine_params {
  * aligned) must hold fa_fwd_plan.workspace_bytes; it may be NULL when that is 0. */
 int fa_b200_fwd(const fa_fwd_params* p, void* workspace, size_t workspace_bytes, void* stream);
 
+/* fa_b200_fwd with the workspace taken from a callback, called with the bytes the plan needs once they are known (so
+   that the problem is planned once per call); plan may be NULL, or the bytes of fa_b200_plan_encode as for fa_b200_fwd_planned. */
+int fa_b200_fwd_alloc(const fa_fwd_params* p, const void* plan, size_t plan_bytes, void* (*alloc)(size_t bytes, void* ctx),
+                      void* ctx, void* stream);
+
 /* fa_b200_fwd for callers that must not allocate device memory: same arguments and results,
  * but the split-KV partials go to a 32 MiB array that is part of the library image (every GPU
  * that loads the library holds it until the process exits) instead of a caller workspace, and the
