@@ -13,6 +13,8 @@ namespace fa {
 int fail_bwd(int code, const std::string& msg);  // api.cu: records the thread's last error
 bool bwd_tc5_eligible(const fa_bwd_params& a);   // bwd_tc5.cu
 int bwd_tc5_launch(const BwdParams& p, const fa_bwd_params& a, cudaStream_t st, std::string* err);
+bool bwd_wide_eligible(const fa_bwd_params& a);  // bwd_wide.cu
+int bwd_wide_launch(const BwdParams& p, const fa_bwd_params& a, cudaStream_t st, std::string* err);
 void count_launches(int n);                      // api.cu: fa_b200_launch_count
 
 static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
@@ -114,8 +116,9 @@ int fa_b200_bwd(const fa_bwd_params* a, void* workspace, size_t workspace_bytes,
   const bool tc5 = a->kernel != 1 && bwd_tc5_eligible(*a);
   if (a->kernel == 2 && !tc5)
     return fail_bwd(FA_ERR_UNSUPPORTED, "the tcgen05 backward covers head dims up to 128 (packed input: total_k given)");
+  const bool wide = a->kernel == 0 && bwd_wide_eligible(*a);
   cudaError_t e = cudaSuccess;
-  if (!tc5) e = cudaMemsetAsync(p.dq_accum, 0, acc_bytes, cs);
+  if (!tc5 && !wide) e = cudaMemsetAsync(p.dq_accum, 0, acc_bytes, cs);
   if (e != cudaSuccess) return fail_bwd(FA_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
   const bool bf = a->dtype == FA_BF16;
   const int delta_grid = (int)((rows * a->h + 7) / 8);  // 4 warps x 2 rows per block
@@ -123,11 +126,11 @@ int fa_b200_bwd(const fa_bwd_params* a, void* workspace, size_t workspace_bytes,
   else bwd_delta_kernel<__half><<<delta_grid, 128, 0, cs>>>(p);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail_bwd(FA_ERR_CUDA, std::string("backward (delta) launch: ") + cudaGetErrorString(e));
-  if (tc5) {
+  if (tc5 || wide) {
     std::string err;
-    const int rc = bwd_tc5_launch(p, *a, cs, &err);
+    const int rc = tc5 ? bwd_tc5_launch(p, *a, cs, &err) : bwd_wide_launch(p, *a, cs, &err);
     if (rc != FA_OK) return fail_bwd(rc, err);
-    count_launches(3);
+    count_launches(tc5 ? 3 : 2);
     return FA_OK;
   }
   const int n_kblocks = (a->seqlen_k + kBwdBN - 1) / kBwdBN;

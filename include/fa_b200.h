@@ -236,8 +236,9 @@ typedef struct fa_bwd_params {
 /* Bytes of device scratch fa_b200_bwd needs: rowsum(dO o O), plus the fp32 dQ accumulator where the mma.sync kernel runs
  * (the tcgen05 kernels need 16 bytes instead). */
 size_t fa_b200_bwd_workspace_bytes(const fa_bwd_params* p);
-/* Three launches on `stream`.  Head dims up to 128: rowsum, then two tcgen05 kernels (dK / dV per key block,
- * dQ per query block; no atomics, so the results are bit-reproducible).  Otherwise: a memset of the fp32 dQ accumulator,
+/* Launches on `stream`.  Head dims up to 128: rowsum, then two tcgen05 kernels (dK / dV per key block,
+ * dQ per query block); wider heads: rowsum and one tcgen05 kernel (kernel = 0 only).  No atomics, so the results are
+ * bit-reproducible.  Otherwise (kernel = 1, or packed input without total_k): a memset of the fp32 dQ accumulator,
  * rowsum, the mma.sync kernel (dQ through atomic adds), dQ conversion. */
 int fa_b200_bwd(const fa_bwd_params* p, void* workspace, size_t workspace_bytes, void* stream);
 

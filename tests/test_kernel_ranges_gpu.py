@@ -107,3 +107,50 @@ def test_merge_of_many_partials(n, d):
     want_l = torch.logsumexp(lse.double(), 0)
     want_l[want_l == float("-inf")] = float("inf")
     torch.testing.assert_close(l.cpu().double(), want_l, rtol=1e-5, atol=1e-5)
+
+
+def _backward_inputs(g, dtype, rows_q, rows_k, h, hk, d):
+    """2 (rand - 0.5), the distribution that the reference's backward tolerance (rtol = atol = 1e-2) is meant for."""
+    r = lambda *s: (2.0 * (torch.rand(s, generator=g) - 0.5)).to(dtype)
+    return r(*rows_q, h, d), r(*rows_k, hk, d), r(*rows_k, hk, d), r(*rows_q, h, d)
+
+
+def _check_gradients(got, want):
+    for name, a, b in zip(("dq", "dk", "dv"), got, want):
+        torch.testing.assert_close(a.float().cpu(), b.float(), rtol=1e-2, atol=1e-2, msg=lambda m: f"{name}: {m}")
+    assert L.load().fa_b200_check_status(torch.cuda.current_stream().cuda_stream) == 0
+
+
+@pytest.mark.parametrize("dtype,b,s_q,s_k,h,hk,d,causal,window,softcap", [
+    (BF, 1, 64, 64, 1, 1, 256, False, (-1, -1), 0.0), (FP, 2, 1, 129, 2, 1, 256, True, (-1, -1), 0.0),
+    (BF, 1, 257, 191, 4, 2, 136, True, (-1, -1), 0.0), (BF, 1, 500, 500, 3, 3, 192, True, (-1, -1), 0.0),
+    (FP, 1, 333, 400, 5, 1, 200, False, (-1, -1), 30.0), (BF, 2, 300, 460, 2, 2, 256, False, (70, 40), 0.0),
+    (FP, 1, 640, 640, 2, 1, 192, True, (128, 0), 0.0), (BF, 1, 1100, 1100, 2, 1, 256, True, (-1, -1), 30.0)])
+def test_wide_head_backward(dtype, b, s_q, s_k, h, hk, d, causal, window, softcap):
+    """Head dims 129 .. 256 on the tcgen05 kernel: units and blocks cut off, rows without keys, grouped heads, windows."""
+    from oracle import bwd as OB
+    g = torch.Generator().manual_seed(d + s_q)
+    q, k, v, dout = _backward_inputs(g, dtype, (b, s_q), (b, s_k), h, hk, d)
+    kw = dict(softmax_scale=d ** -0.5, causal=causal, window_left=window[0], window_right=window[1], softcap=softcap)
+    out, lse = ops.attention_forward(q.cuda(), k.cuda(), v.cuda(), **kw)
+    grads = [torch.full_like(t, float("nan")).cuda() for t in (q, k, v)]  # every element must be written, zeros included
+    n0 = L.load().fa_b200_launch_count()
+    ops.attention_backward(dout.cuda(), q.cuda(), k.cuda(), v.cuda(), out, lse, dq=grads[0], dk=grads[1], dv=grads[2], **kw)
+    assert L.load().fa_b200_launch_count() - n0 == 2  # rowsum and the one persistent kernel
+    _check_gradients(grads, OB.attention_backward(q, k, v, dout, lse.cpu(), softmax_scale=d ** -0.5, causal=causal, window=window,
+                                                  softcap=softcap))
+
+
+@pytest.mark.parametrize("d,causal", [(192, True), (256, False)])
+def test_wide_head_backward_packed(d, causal):
+    from oracle import bwd as OB
+    g = torch.Generator().manual_seed(d)
+    lq, lk, h, hk = [130, 0, 1, 64, 300], [200, 77, 5, 64, 280], 4, 2
+    cq, ck = [torch.tensor([0] + list(torch.tensor(x).cumsum(0)), dtype=torch.int32) for x in (lq, lk)]
+    q, k, v, dout = _backward_inputs(g, BF, (sum(lq),), (sum(lk),), h, hk, d)
+    kw = dict(softmax_scale=d ** -0.5, causal=causal, cu_seqlens_q=cq.cuda(), cu_seqlens_k=ck.cuda(), max_seqlen_q=max(lq), max_seqlen_k=max(lk))
+    out, lse = ops.attention_forward(q.cuda(), k.cuda(), v.cuda(), **kw)
+    grads = [torch.full_like(t, float("nan")).cuda() for t in (q, k, v)]
+    ops.attention_backward(dout.cuda(), q.cuda(), k.cuda(), v.cuda(), out, lse, dq=grads[0], dk=grads[1], dv=grads[2], **kw)
+    _check_gradients(grads, OB.attention_varlen_backward(q, k, v, dout, lse.cpu(), cq, ck, softmax_scale=d ** -0.5, causal=causal,
+                                                         window=(-1, -1)))
