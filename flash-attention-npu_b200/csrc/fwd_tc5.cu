@@ -64,6 +64,11 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
     }
     mbar_init(smem_addr(&bar->fix_req), 2);
     mbar_init(smem_addr(&bar->v_fixed), 1);
+    for (int s = 0; s < kQueue; ++s) {
+      mbar_init(smem_addr(&bar->queue.full[s]), 1);
+      mbar_init(smem_addr(&bar->queue.empty[s]), kQueueReaders);
+    }
+    mbar_init(smem_addr(&bar->queue.answered), 1);
     bar->abort_flag = 0;
     bar->fix_seen[0] = bar->fix_seen[1] = 0;
     fence_barrier_init();
@@ -86,10 +91,10 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
   // scores of a row plus working set, the other roles need far fewer.
   if (warp < 8) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kRegsSoftmax));
-    softmax_loop<T, SOFTCAP, Geo<HD>::kRows>(p, bar, tmem, p_smem, warp >> 2, warp & 3, lane);
+    softmax_loop<T, FIX, SOFTCAP, Geo<HD>::kRows>(p, bar, tmem, p_smem, warp >> 2, warp & 3, lane);
   } else if (warp < 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsCorr));
-    correction_loop<T, HD>(p, bar, tmem, warp & 3, lane);
+    correction_loop<T, FIX, HD>(p, bar, tmem, warp & 3, lane);
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsMma));
     // warp-uniform role code; one elected lane issues
@@ -259,6 +264,10 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
     else if (per_m * kv_bytes_per_pair <= l2_budget || chunk * kv_bytes_per_pair > l2_budget) chunk = per_m;
     if (chunk <= 0 || chunk > per_m) chunk = per_m;
     p.chunk_bh = (int)chunk;
+    // Ragged input: as many heads as keep their K / V in L2, whole groups; all heads when one group's do not fit.
+    const long long kv_rows = a.cu_seqlens_k ? a.total_k : (long long)a.b * a.seqlen_k;
+    const long long kv_heads = l2_budget / std::max(1LL, kv_rows * a.d * 4);
+    p.chunk_heads = kv_heads >= 1 && kv_heads < a.h_k ? (int)(kv_heads * p.group) : a.h;
   }
   p.status = status_word();
   if (!p.status) { *err = "cannot look up the device status word"; return FA_ERR_CUDA; }
@@ -277,11 +286,18 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
   ok = ok && encode_map(&tk, a.k, a.dtype, a.d, a.h_k, k_rows, k_outer, a.k_head_stride, a.k_row_stride, packed_k ? 0 : a.k_batch_stride) &&
        encode_map(&tv, a.v, a.dtype, a.d, a.h_k, k_rows, k_outer, a.v_head_stride, a.v_row_stride, packed_k ? 0 : a.v_batch_stride);
   if (!ok) { *err = "cuTensorMapEncodeTiled failed"; return FA_ERR_CUDA; }
+  // Ragged input: a CTA per tile (TileDraw).  Packed sequences have at most total_q / rows + b tiles a head.
+  int grid = pl.grid;
+  if (p.fix_tail) {
+    long long tiles = (long long)pl.m_blocks * a.b;
+    if (a.cu_seqlens_q) tiles = std::min(tiles, (long long)a.total_q / pl.block_m + a.b);
+    grid = (int)(tiles * a.h);
+  }
   cudaError_t e = cudaErrorInvalidValue;
   auto launch = [&](auto kern) {
     e = allow_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
     if (e == cudaSuccess) {
-      kern<<<pl.grid, kThreads, kSmemBytes, st>>>(p, tq, tk, tv);
+      kern<<<grid, kThreads, kSmemBytes, st>>>(p, tq, tk, tv);
       e = cudaGetLastError();
     }
   };

@@ -24,6 +24,8 @@
 // tensor pipe in steady state, and the tensor pipe has two sub-tiles' worth of independent work.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "tc5_ptx.cuh"
 
@@ -78,7 +80,8 @@ struct Tc5Params {
   int32_t total_tiles;
   float scale_log2;
   float softcap_mul, softcap_l2;  // softcap: scores become softcap_l2 * tanh(s * softcap_mul) in the log2 domain (scale / softcap, softcap * log2 e)
-  int32_t chunk_bh;          // (batch, head) pairs per L2 chunk of the tile order (tile_info)
+  int32_t chunk_bh;          // (batch, head) pairs per L2 chunk of the tile order (static_tile)
+  int32_t chunk_heads;       // ragged input: query heads per L2 chunk (TileDraw)
   // 1: the rows behind the last key of a sequence hold foreign data (the unused tail of a KV cache or of a page,
   // the next sequence of a packed tensor) and must be cleared in V before P.V: P is 0 there, but 0 x NaN is NaN.
   // 0: dense input, those rows lie outside the tensor and the TMA unit already returns zeros for them.
@@ -96,37 +99,44 @@ struct TileInfo {
   int ulo, uhi;  // union of the block ranges
 };
 
-// Tile order: the (batch, head) pairs are cut into chunks whose K / V fit in L2 together; inside a
+// Tile order of dense input: the (batch, head) pairs are cut into chunks whose K / V fit in L2 together; inside a
 // chunk all pairs run their last (heaviest, causal) query tile first, then the one before, and so
 // on, so the K / V prefixes a chunk re-reads tile after tile come from L2 and not from HBM.  The
-// chunk length makes a chunk a whole even number of rounds of the grid (TileSched), which keeps the
+// chunk length makes a chunk a whole even number of rounds of the grid (StaticWalk), which keeps the
 // per-CTA sums as even as one chunk over everything would.
-template <int ROWS>  // query rows of a CTA tile: 256 (two sub-tiles) or 128 (sub-tile 0 only)
-__device__ __forceinline__ void tile_info(const Tc5Params& p, int n, TileInfo& ti) {
+struct TileId {
+  int bi, hh, mt;  // batch entry, query head, query tile
+};
+__device__ __forceinline__ TileId static_tile(const Tc5Params& p, int n) {
   const int per_m = p.a.b * p.a.h;
   const int per_chunk = p.chunk_bh * p.m_tiles;
   const int ck = n / per_chunk, r = n - ck * per_chunk;
   const int cnt = min(p.chunk_bh, per_m - ck * p.chunk_bh);  // pairs in this chunk (the last one may be short)
-  const int mt = p.m_tiles - 1 - r / cnt;  // heavy (late, causal) tiles first
   const int rem = ck * p.chunk_bh + r % cnt;
-  ti.bi = rem / p.a.h;
-  ti.hh = rem % p.a.h;
+  return {rem / p.a.h, rem % p.a.h, p.m_tiles - 1 - r / cnt};  // heavy (late, causal) tiles first
+}
+
+__device__ __forceinline__ int q_length(const Tc5Params& p, int bi) {
+  return p.a.cu_seqlens_q ? p.a.cu_seqlens_q[bi + 1] - p.a.cu_seqlens_q[bi] : p.a.seqlen_q;
+}
+__device__ __forceinline__ int k_length(const Tc5Params& p, int bi) {
+  // KV cache (contiguous or paged): keys in use per batch entry, plus the tokens the prologue appended; clamped here,
+  // the producer reports it
+  if (p.a.seqused_k) return cache_len(p.a, bi, nullptr) + p.a.seqlen_new;
+  return p.a.cu_seqlens_k ? p.a.cu_seqlens_k[bi + 1] - p.a.cu_seqlens_k[bi] : p.a.seqlen_k;
+}
+
+template <int ROWS>  // query rows of a CTA tile: 256 (two sub-tiles) or 128 (sub-tile 0 only)
+__device__ __forceinline__ void tile_info(const Tc5Params& p, const TileId id, TileInfo& ti) {
+  const int mt = id.mt;
+  ti.bi = id.bi;
+  ti.hh = id.hh;
   ti.hk = ti.hh / p.group;
-  ti.q_row0 = 0;
-  ti.q_len = p.a.seqlen_q;
-  ti.k_row0 = 0;
-  ti.k_len = p.a.seqlen_k;
-  if (p.a.cu_seqlens_q) {
-    ti.q_row0 = p.a.cu_seqlens_q[ti.bi];
-    ti.q_len = p.a.cu_seqlens_q[ti.bi + 1] - ti.q_row0;
-  }
-  if (p.a.cu_seqlens_k) {
-    ti.k_row0 = p.a.cu_seqlens_k[ti.bi];
-    ti.k_len = p.a.cu_seqlens_k[ti.bi + 1] - ti.k_row0;
-  }
+  ti.q_row0 = p.a.cu_seqlens_q ? p.a.cu_seqlens_q[ti.bi] : 0;
+  ti.q_len = q_length(p, ti.bi);
+  ti.k_row0 = p.a.cu_seqlens_k ? p.a.cu_seqlens_k[ti.bi] : 0;
+  ti.k_len = k_length(p, ti.bi);
   ti.bk = (p.a.cache_batch_idx && !p.a.block_table) ? p.a.cache_batch_idx[ti.bi] : ti.bi;
-  // KV cache (contiguous or paged): keys in use per batch entry, plus the tokens the prologue appended
-  if (p.a.seqused_k) ti.k_len = cache_len(p.a, ti.bi, nullptr) + p.a.seqlen_new;  // clamped; the producer reports it
   ti.koff = ti.k_len - ti.q_len;
   ti.ulo = 0x7fffffff;
   ti.uhi = 0;
@@ -156,23 +166,14 @@ __device__ __forceinline__ void tile_info(const Tc5Params& p, int n, TileInfo& t
   if (ti.uhi == 0) ti.ulo = 0;
 }
 
-// Static tile schedule.  tile_info orders tiles heaviest first; CTA c of G takes tiles
-// c, 2G-1-c, 2G+c, 4G-1-c, ... (serpentine), which evens out the per-CTA sums of a decreasing
-// sequence (causal, 4K: 1 % spread instead of 6 % with a plain stride).
-struct TileSched {
-  int round, total;
-  __device__ explicit TileSched(const Tc5Params& p) : round(0), total(p.total_tiles) {}
-  __device__ __forceinline__ int cur() const {
-    const int g = (int)gridDim.x, c = (int)blockIdx.x;
-    if (round * g >= total) return total;
-    const int n = round * g + ((round & 1) ? g - 1 - c : c);
-    return n < total ? n : total;
-  }
-  __device__ __forceinline__ int first() { return cur(); }
-  __device__ __forceinline__ int next() {
-    ++round;
-    return cur();
-  }
+// Ragged input (TileDraw): the tiles a CTA has drawn, handed by the producer warp to the other roles.
+constexpr int kQueue = 4;
+constexpr int kQueueReaders = 15;  // warps that read every tile
+struct TileQueue {
+  alignas(16) uint32_t response[4];  // of the request for another CTA's tile
+  uint64_t answered;                 // the response has arrived
+  uint64_t full[kQueue], empty[kQueue];
+  int32_t tile[kQueue];              // (batch entry * heads + head) * m_tiles + query tile; total_tiles: no more
 };
 
 struct Barriers {
@@ -195,8 +196,184 @@ struct Barriers {
   uint32_t fix_slot;       // ring slot of the V tile to repair
   float corr[2][kBlockM];
   float row_inv[2][kBlockM];
+  TileQueue queue;
 };
 static_assert(sizeof(Barriers) <= kBarBytes, "barrier block does not fit");
+
+// Static tile schedule of dense input: CTA c of G takes positions c, 2G-1-c, 2G+c, 4G-1-c, ... (serpentine) of an order
+// that starts with the heaviest tiles, which evens out the per-CTA sums of a decreasing sequence (causal, 4K: 1 % spread
+// instead of 6 % with a plain stride).
+struct StaticWalk {
+  int round = 0;
+  __device__ explicit StaticWalk(Barriers*) {}
+  __device__ __forceinline__ int first(const Tc5Params& p) const {
+    const int g = (int)gridDim.x, c = (int)blockIdx.x;
+    if (round * g >= p.total_tiles) return p.total_tiles;
+    const int n = round * g + ((round & 1) ? g - 1 - c : c);
+    return n < p.total_tiles ? n : p.total_tiles;
+  }
+  __device__ __forceinline__ int next(const Tc5Params& p) {
+    ++round;
+    return first(p);
+  }
+};
+
+// Ragged input: tile counts and lengths are on the device, and a fixed deal leaves the CTAs uneven (12 packed sequences
+// of 37 - 2999 rows, 16 heads: the longest CTA has 1.7 x the mean).  The grid has a CTA per tile instead, and a running
+// CTA takes over the tile of one that has not started (clusterlaunchcontrol) until none is left: no counter in memory,
+// nothing to reset.  The producer warp draws and publishes the tile; the other roles read it here.  Kernel time, those
+// sequences (head dim 64) 332 -> 236 us; 4 chunks of 301 - 2048 rows against 1777 - 8192 cached keys 570 -> 508 us a call.
+struct QueueWalk {
+  Barriers* bar;
+  uint32_t k = 0;
+  __device__ explicit QueueWalk(Barriers* b) : bar(b) {}
+  __device__ __forceinline__ int next(const Tc5Params& p) {
+    TileQueue& q = bar->queue;
+    const uint32_t s = k % kQueue;
+    if (!mbar_wait(smem_addr(&q.full[s]), (k / kQueue) & 1, &bar->abort_flag, 61)) return p.total_tiles;
+    const int n = q.tile[s];
+    ++k;
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(smem_addr(&q.empty[s]));
+    return n;
+  }
+  __device__ __forceinline__ int first(const Tc5Params& p) { return next(p); }
+};
+template <bool FIX>
+using TileWalk = typename std::conditional<FIX, QueueWalk, StaticWalk>::type;
+// The tile number that a walk gives -> tile (p.total_tiles: no more).
+template <bool FIX>
+__device__ __forceinline__ TileId tile_id(const Tc5Params& p, int n) {
+  if (!FIX) return static_tile(p, n);
+  const int pair = n / p.m_tiles;
+  return {pair / p.a.h, pair % p.a.h, n % p.m_tiles};
+}
+
+// The producer's side.  Position n (a CTA index) -> tile: the heads are cut into chunks whose K / V stay in L2 together;
+// a chunk runs its tiles by level, highest first, level = query tile + (causal) the tiles' worth of keys in front of the
+// queries, i.e. about the work of the tile; a level holds at most one tile of every batch entry, for all heads of the
+// chunk.  Tiles that do not exist have no position, the grid's surplus positions no tile.
+template <int ROWS>
+struct TileDraw {
+  const Tc5Params& p;
+  Barriers* bar;
+  int lane, pos;
+  uint32_t k = 0, asked = 0;
+  bool pending = false, more = true;
+  int live = 0, top = 0;                         // tiles of one head; highest level
+  int chunk = 0, level = 0, start = 0, cnt = 0;  // of the last position: its level, the level's first position in the chunk and tiles per head
+
+  __device__ __forceinline__ void entry(int bi, int& lo, int& n) const {  // levels [lo, lo + n) of batch entry bi
+    const int q_len = q_length(p, bi);
+    n = min(max(0, ceil_div(q_len, ROWS)), p.m_tiles);
+    lo = (p.is_causal || p.is_local) ? max(0, k_length(p, bi) - q_len) / ROWS : 0;
+  }
+  __device__ TileDraw(const Tc5Params& p_, Barriers* b, int lane_) : p(p_), bar(b), lane(lane_), pos(blockIdx.x) {
+    for (int bi = lane; bi < p.a.b; bi += 32) {
+      int lo, n;
+      entry(bi, lo, n);
+      live += n;
+      if (n > 0) top = max(top, lo + n - 1);
+    }
+    live = __reduce_add_sync(0xffffffffu, live);
+    top = __reduce_max_sync(0xffffffffu, top);
+    level = top + 1;
+  }
+  __device__ __forceinline__ uint32_t members(int b0) const {  // batch entries b0 .. b0 + 31 with a tile in this level
+    int lo = 0, n = 0;
+    if (b0 + lane < p.a.b) entry(b0 + lane, lo, n);
+    return __ballot_sync(0xffffffffu, level >= lo && level < lo + n);
+  }
+  // position -> tile; positions only ever grow.  False: the position has no tile.
+  __device__ __forceinline__ bool locate(int n, int& tile) {
+    if (n >= live * p.a.h) return false;
+    const int ck = n / (live * p.chunk_heads);
+    const int heads = min(p.chunk_heads, p.a.h - ck * p.chunk_heads);
+    n -= ck * live * p.chunk_heads;
+    if (ck != chunk) {
+      chunk = ck;
+      level = top + 1;
+      start = cnt = 0;
+    }
+    while (level > 0 && n >= start + cnt * heads) {  // the levels down to 0 hold `live` tiles per head
+      start += cnt * heads;
+      --level;
+      cnt = 0;
+      for (int b0 = 0; b0 < p.a.b; b0 += 32) cnt += __popc(members(b0));
+    }
+    int r = (n - start) / heads;
+    const int hh = ck * p.chunk_heads + (n - start) % heads;
+    int bi = 0;
+    for (int b0 = 0; b0 < p.a.b; b0 += 32) {
+      uint32_t m = members(b0);
+      const int c = __popc(m);
+      if (r < c) {
+        for (; r > 0; --r) m &= m - 1;  // drop the r lowest members
+        bi = b0 + __ffs(m) - 1;
+        break;
+      }
+      r -= c;
+    }
+    int lo, nt;
+    entry(bi, lo, nt);
+    tile = (bi * p.a.h + hh) * p.m_tiles + level - lo;
+    return true;
+  }
+  __device__ __forceinline__ void ask() {
+    if (lane == 0) {
+      const uint32_t full = smem_addr(&bar->queue.answered);
+      fence_proxy_async();  // the last response has been read
+      mbar_arrive_expect_tx(full, 16);
+      try_cancel(smem_addr(bar->queue.response), full);
+    }
+    __syncwarp();
+    pending = true;
+  }
+  __device__ __forceinline__ bool answer() {  // -> pos, more
+    pending = false;
+    if (!mbar_wait(smem_addr(&bar->queue.answered), asked & 1, &bar->abort_flag, 62)) return false;
+    ++asked;
+    more = canceled_cta(smem_addr(bar->queue.response), pos);
+    __syncwarp();
+    return true;
+  }
+  __device__ __forceinline__ bool publish(int tile) {
+    TileQueue& q = bar->queue;
+    const uint32_t s = k % kQueue;
+    if (!mbar_wait(smem_addr(&q.empty[s]), ((k / kQueue) & 1) ^ 1, &bar->abort_flag, 63)) return false;
+    ++k;
+    if (lane == 0) {
+      q.tile[s] = tile;
+      mbar_arrive(smem_addr(&q.full[s]));
+    }
+    __syncwarp();
+    return true;
+  }
+  // The CTA's next tile, published to the other roles.  A request is always answered and read before the next one, and
+  // none is made after one that found nothing.
+  __device__ __forceinline__ int next(const Tc5Params&) {
+    prefetch();
+    if (!answer()) return p.total_tiles;
+    return first(p);
+  }
+  __device__ __forceinline__ int first(const Tc5Params&) {
+    int tile = p.total_tiles;
+    while (more && !locate(pos, tile)) {
+      ask();
+      if (!answer()) return p.total_tiles;
+    }
+    if (!more) tile = p.total_tiles;
+    return publish(tile) ? tile : p.total_tiles;
+  }
+  // Called when the tile's loads are nearly through: a CTA must not commit itself to a tile a whole tile ahead.
+  __device__ __forceinline__ void prefetch() {
+    if (!pending) ask();
+  }
+};
+struct StaticDraw : StaticWalk {
+  __device__ StaticDraw(const Tc5Params&, Barriers* b, int) : StaticWalk(b) {}
+  __device__ __forceinline__ void prefetch() {}
+};
 
 }  // namespace tc5
 }  // namespace fa

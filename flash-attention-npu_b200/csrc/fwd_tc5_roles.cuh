@@ -41,10 +41,11 @@ __device__ __forceinline__ void producer_loop(const Tc5Params& p, const CUtensor
   const int lane = threadIdx.x & 31;
   const uint64_t q_policy = l2_policy_evict_first();  // Q is read once
   const int pages_per_seq = p.a.block_table ? ceil_div(p.a.seqlen_k, p.a.page_size) : 0;  // entries per block-table row
-  TileSched sched(p);
-  for (int n = sched.first(); n < p.total_tiles; n = sched.next()) {
+  using Draw = typename std::conditional<FIX, TileDraw<G::kRows>, StaticDraw>::type;
+  Draw draw(p, bar, lane);
+  for (int n = draw.first(p); n < p.total_tiles; n = draw.next(p)) {
     TileInfo ti;
-    tile_info<G::kRows>(p, n, ti);
+    tile_info<G::kRows>(p, tile_id<FIX>(p, n), ti);
     if (ti.uhi <= ti.ulo) continue;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
@@ -98,6 +99,7 @@ __device__ __forceinline__ void producer_loop(const Tc5Params& p, const CUtensor
     if (!load(tm_k, ti.ulo)) return;
     for (int j = ti.ulo; j < ti.uhi; ++j) {
       if (j + 1 < ti.uhi && !load(tm_k, j + 1)) return;
+      if (j + 2 >= ti.uhi) draw.prefetch();
       if (!load(tm_v, j)) return;
     }
   }
@@ -113,20 +115,19 @@ __device__ __forceinline__ void producer_loop(const Tc5Params& p, const CUtensor
 // Hand-shake: the issuing warps arrive on fix_req once the tile has landed (at least one of them uses it and has
 // waited for it), this warp clears the rows and arrives on v_fixed, which both issuing warps wait for.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ bool tile_needs_tail_fix(const Tc5Params& p, const TileInfo& ti) {
-  return p.fix_tail && ti.uhi > ti.ulo && ti.uhi * kBlockN > ti.k_len;
+__device__ __forceinline__ bool tile_needs_tail_fix(const TileInfo& ti) {
+  return ti.uhi > ti.ulo && ti.uhi * kBlockN > ti.k_len;
 }
 
 template <int HD>
 __device__ __forceinline__ void tail_fix_loop(const Tc5Params& p, Barriers* bar, uint32_t kv_smem, int lane) {
-  if (!p.fix_tail) return;
   volatile int* abort_flag = &bar->abort_flag;
   uint32_t fix_cnt = 0;  // tails cleared so far
-  TileSched sched(p);
-  for (int n = sched.first(); n < p.total_tiles; n = sched.next()) {
+  TileWalk<true> walk(bar);
+  for (int n = walk.first(p); n < p.total_tiles; n = walk.next(p)) {
     TileInfo ti;
-    tile_info<Geo<HD>::kRows>(p, n, ti);
-    if (!tile_needs_tail_fix(p, ti)) continue;
+    tile_info<Geo<HD>::kRows>(p, tile_id<true>(p, n), ti);
+    if (!tile_needs_tail_fix(ti)) continue;
     if (!mbar_wait_patient(smem_addr(&bar->fix_req), fix_cnt & 1, abort_flag, 51)) return;
     ++fix_cnt;
     const uint32_t slot = bar->fix_slot;  // written by the issuing warps before they arrived
@@ -192,10 +193,10 @@ __device__ __forceinline__ void mma_loop(const Tc5Params& p, Barriers* bar, uint
     return mbar_wait(smem_addr(&bar->v_fixed), n & 1, abort_flag, 22);
   };
 
-  TileSched sched(p);
-  for (int n = sched.first(); n < p.total_tiles; n = sched.next()) {
+  TileWalk<FIX> walk(bar);
+  for (int n = walk.first(p); n < p.total_tiles; n = walk.next(p)) {
     TileInfo ti;
-    tile_info<G::kRows>(p, n, ti);
+    tile_info<G::kRows>(p, tile_id<FIX>(p, n), ti);
     if (ti.uhi <= ti.ulo) continue;
     if (ti.has[t]) {
       if (!mbar_wait(smem_addr(&bar->q_full[t]), q_cnt & 1, abort_flag, 13)) return;
@@ -203,7 +204,7 @@ __device__ __forceinline__ void mma_loop(const Tc5Params& p, Barriers* bar, uint
     }
     const int jlo_t = ti.has[t] ? ti.jlo[t] : 0, jhi_t = ti.has[t] ? ti.jhi[t] : 0;
     const int jlo_o = ti.has[o] ? ti.jlo[o] : 0, jhi_o = ti.has[o] ? ti.jhi[o] : 0;
-    const int fix_j = (FIX && tile_needs_tail_fix(p, ti)) ? ti.uhi - 1 : -1;  // the block whose V tile needs its tail cleared
+    const int fix_j = (FIX && tile_needs_tail_fix(ti)) ? ti.uhi - 1 : -1;  // the block whose V tile needs its tail cleared
 
     // S_t = Q_t K_j^T.  Tiles only the other sub-tile uses need no arrival from this warp (that warp
     // arrives twice); tiles nobody uses cannot occur (the union of two touching intervals has no hole).

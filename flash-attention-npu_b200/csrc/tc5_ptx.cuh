@@ -100,6 +100,27 @@ __device__ __forceinline__ void tma_load_4d_hint(uint32_t dst, const CUtensorMap
       : "memory");
 }
 
+// ---------------- cluster launch control ----------------
+// Asks for the index of a CTA of this grid that has not started yet; if there is one, it will not start.  The 16-byte
+// response arrives like a bulk copy.
+__device__ __forceinline__ void try_cancel(uint32_t response, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];\n" ::"r"(response),
+               "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ bool canceled_cta(uint32_t response, int& x) {
+  uint32_t ok, cx;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\tld.shared.b128 r, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\tselp.b32 %0, 1, 0, p;\n\tmov.b32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, r;\n\t}\n"
+      : "=r"(ok), "=&r"(cx)
+      : "r"(response)
+      : "memory");
+  x = (int)cx;
+  return ok != 0;
+}
+
 // ---------------- TMEM ----------------
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_dst, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_dst), "r"(ncols) : "memory");

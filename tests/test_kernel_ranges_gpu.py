@@ -154,3 +154,41 @@ def test_wide_head_backward_packed(d, causal):
     ops.attention_backward(dout.cuda(), q.cuda(), k.cuda(), v.cuda(), out, lse, dq=grads[0], dk=grads[1], dv=grads[2], **kw)
     _check_gradients(grads, OB.attention_varlen_backward(q, k, v, dout, lse.cpu(), cq, ck, softmax_scale=d ** -0.5, causal=causal,
                                                          window=(-1, -1)))
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("dtype,d", [(BF, 128), (FP, 64), (BF, 256)])
+def test_packed_tiles_of_more_than_32_sequences(dtype, d, causal):
+    """Tiles are drawn by level and batch entry, 32 entries at a time: empty sequences, sequences of one tile and of several,
+    lengths at the tiles' edges, keys longer and shorter than the queries, an entry count that is not a multiple of 32."""
+    import flash_attn_npu_v2 as fa2
+    g = torch.Generator().manual_seed(d + causal)
+    h, hk = 4, 2
+    q_lens = ([0, 1, 127, 128, 129, 255, 256, 257, 513, 3] * 4)[:37]
+    k_lens = [n + x if n else 0 for n, x in zip(q_lens, [0, 5, 300, 0, 640, 1, 0, 128, 77, 0] * 4)]
+    k_lens[7] = 200  # fewer keys than queries
+    cq, ck = (torch.tensor([0] + list(torch.tensor(x).cumsum(0)), dtype=torch.int32) for x in (q_lens, k_lens))
+    q = U.normal((sum(q_lens), h, d), dtype, g)
+    k, v = U.normal((sum(k_lens), hk, d), dtype, g), U.normal((sum(k_lens), hk, d), dtype, g)
+    out, lse, *_ = fa2.flash_attn_varlen_func(q.cuda(), k.cuda(), v.cuda(), cq.cuda(), ck.cuda(), max(q_lens), max(k_lens),
+                                              causal=causal, return_attn_probs=True)
+    for i, n in enumerate(q_lens):
+        if not n:
+            continue
+        rq, rk = slice(int(cq[i]), int(cq[i + 1])), slice(int(ck[i]), int(ck[i + 1]))
+        go, gl = OA.flash_attn_func(q[rq].unsqueeze(0), k[rk].unsqueeze(0), v[rk].unsqueeze(0), causal=causal)
+        U.check_rules(out[rq].unsqueeze(0), lse[:, rq].unsqueeze(0), go, gl, tag=f"sequence {i}")
+
+
+def test_head_chunks_of_a_large_cache():
+    """A cache too large for L2 runs its heads in chunks (here 8 and 4 of 12 query heads)."""
+    import flash_attn_npu_v2 as fa2
+    g = torch.Generator().manual_seed(5)
+    b, s_q, h, hk, d, room = 3, 300, 12, 6, 128, 16384
+    lens = torch.tensor([300, 700, 2049], dtype=torch.int32)
+    kc, vc = torch.zeros((b, room, hk, d), dtype=BF), torch.zeros((b, room, hk, d), dtype=BF)
+    kc[:, :2049], vc[:, :2049] = U.normal((b, 2049, hk, d), BF, g), U.normal((b, 2049, hk, d), BF, g)
+    q = U.normal((b, s_q, h, d), BF, g)
+    out, lse = fa2.flash_attn_with_kvcache(q.cuda(), kc.cuda(), vc.cuda(), cache_seqlens=lens.cuda(), causal=True, return_softmax_lse=True)
+    go, gl = OA.flash_attn_with_kvcache(q, kc[:, :2049].contiguous(), vc[:, :2049].contiguous(), cache_seqlens=lens, causal=True)
+    U.check_rules(out, lse, go, gl, tag="head chunks")
