@@ -18,6 +18,18 @@
 // space is two more Y slots.
 // Warps 0-15 elementwise and epilogue (0-7 the even, 8-15 the odd units), 16 issues S and acc (in this order in one warp:
 // S of unit u + 2 overwrites the operand of acc of unit u, and the tensor pipe keeps the order), 17 issues dP, 19 loads.
+// A parity wait only tells the current phase of a barrier from the one before, so no role may be two phases away from a
+// barrier it waits on, in either direction.  The resident operands and the Y slots are therefore released by both issuers
+// in every item, also in a dV item, where warp 17 has nothing to issue: it waits for a_full and every y_full there and
+// releases them itself.  (Without that it reached the next dQ item's waits while a dV item of one or two units was still
+// loading, passed them on the parity of the item before, and computed dP from stale tiles.)
+// What a wait relies on, phase by phase:
+//   a_full, y_full   the next phase needs both issuers' releases; warp 16 looks at y_full in dV items only, but in the
+//                    other items its acc of a unit follows that unit's dP, and dP follows y_full
+//   x_full, st_full  the next phase needs acc of this unit, which needs pds_full of this unit
+//   pds_full         warp 17 waits for unit g - 2 after y_full of unit g, whose slot (and, behind a dV item, the space of
+//                    A1) was released by acc of unit g - 2 or a later one, hence after pds_full of every unit before that
+//   acc_done, acc_free  each needs the other's phase before it, by all warps
 #pragma once
 
 #include "bwd_tc5_kernel.cuh"
@@ -48,7 +60,7 @@ struct WideGeo {
 
 template <int HD>
 struct BarW {
-  uint64_t a_full, a_empty;  // A0 / A1 of the item have landed; its last S and dP have read them
+  uint64_t a_full, a_empty;  // A0 / A1 of the item have landed; its last S and dP have read them (dV: its last S has, and the dP issuer has seen a_full)
   uint64_t x_full[WideGeo<HD>::XS], x_empty[WideGeo<HD>::XS];
   uint64_t y_full[WideGeo<HD>::YSV], y_empty[WideGeo<HD>::YSV];
   uint64_t stat_full[WideGeo<HD>::kStats];  // LSE / D of a unit are in shared memory (X's own barrier may run on: dV frees X before the elementwise warps look)
@@ -180,14 +192,14 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
   BarW<HD>* bar = reinterpret_cast<BarW<HD>*>(smem + G::kBarOff);
   if (tid == 0) {
     mbar_init(smem_addr(&bar->a_full), 1);
-    mbar_init(smem_addr(&bar->a_empty), 2);  // the S and the dP issuer (dV: the S issuer, twice)
+    mbar_init(smem_addr(&bar->a_empty), 2);  // the S and the dP issuer
     for (int s = 0; s < G::XS; ++s) {
       mbar_init(smem_addr(&bar->x_full[s]), 1);
       mbar_init(smem_addr(&bar->x_empty[s]), 1);
     }
     for (int s = 0; s < G::YSV; ++s) {
       mbar_init(smem_addr(&bar->y_full[s]), 1);
-      mbar_init(smem_addr(&bar->y_empty[s]), 1);
+      mbar_init(smem_addr(&bar->y_empty[s]), 2);  // dK, dQ: the dP issuer, twice; dV: the acc issuer and the dP issuer
     }
     for (int s = 0; s < G::kStats; ++s) mbar_init(smem_addr(&bar->stat_full[s]), 1);
     for (int b = 0; b < 2; ++b) {
@@ -325,10 +337,7 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
             mma_commit(smem_addr(&bar->st_full[b]));
             mma_commit(smem_addr(&bar->x_empty[xs]));
           }
-          if (u == iters - 1) {
-            mma_commit(smem_addr(&bar->a_empty));
-            if (is_v) mma_commit(smem_addr(&bar->a_empty));
-          }
+          if (u == iters - 1) mma_commit(smem_addr(&bar->a_empty));
         }
         __syncwarp();
         return true;
@@ -374,13 +383,16 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
       if (t < 0) break;
       const ItemW w = item_w(p, t);
       int ys = 0;
-      if (w.kind == kWideDV) {
-        for (int it = 0; it < w.iters; ++it) {
+      if (!mbar_wait(smem_addr(&bar->a_full), wi & 1, abort_flag, 69)) break;
+      if (w.kind == kWideDV) {  // nothing to issue: only keeps in step with the barriers
+        if (lane == 0) mbar_arrive(smem_addr(&bar->a_empty));
+        for (int u = 0; u < w.iters; ++u) {
+          if (!mbar_wait(smem_addr(&bar->y_full[ys]), (yph >> ys) & 1, abort_flag, 58)) { ok = false; break; }
           yph ^= 1u << ys;
+          if (lane == 0) mbar_arrive(smem_addr(&bar->y_empty[ys]));
           if (++ys == G::YSV) ys = 0;
         }
       } else {
-        if (!mbar_wait(smem_addr(&bar->a_full), wi & 1, abort_flag, 69)) break;
         for (int u = 0; u < w.iters; ++u) {
           const uint32_t g = gu + u;
           const int b = g & 1;
@@ -396,6 +408,7 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
 #pragma unroll
             for (int ks = 1; ks < HD / 16; ++ks) mma_ss_c<true>(d_tmem, a_desc + kmaj_off(ks), b_desc + unit_off(ks), idesc_s);
             mma_commit(smem_addr(&bar->st_full[b]));
+            mma_commit(smem_addr(&bar->y_empty[ys]));
             mma_commit(smem_addr(&bar->y_empty[ys]));
             if (u == w.iters - 1) mma_commit(smem_addr(&bar->a_empty));
           }

@@ -192,3 +192,26 @@ def test_head_chunks_of_a_large_cache():
     out, lse = fa2.flash_attn_with_kvcache(q.cuda(), kc.cuda(), vc.cuda(), cache_seqlens=lens.cuda(), causal=True, return_softmax_lse=True)
     go, gl = OA.flash_attn_with_kvcache(q, kc[:, :2049].contiguous(), vc[:, :2049].contiguous(), cache_seqlens=lens, causal=True)
     U.check_rules(out, lse, go, gl, tag="head chunks")
+
+
+@pytest.mark.parametrize("d", [192, 256])
+def test_wide_head_backward_short_items(d):
+    """More items than SMs, most of one or two units: a CTA's dV items end while their tiles are still arriving, and the dQ
+    items behind them must wait for their own.  Every repetition gives the same bits."""
+    from oracle import bwd as OB
+    g = torch.Generator().manual_seed(d)
+    lens = ([1, 128, 64, 65, 17, 127, 129, 100] * 10)[:75]
+    h, hk = 4, 2
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32)
+    q, k, v, dout = _backward_inputs(g, BF, (sum(lens),), (sum(lens),), h, hk, d)
+    kw = dict(softmax_scale=d ** -0.5, causal=True, cu_seqlens_q=cu.cuda(), cu_seqlens_k=cu.cuda(), max_seqlen_q=max(lens),
+              max_seqlen_k=max(lens))
+    qg, kg, vg, dg = q.cuda(), k.cuda(), v.cuda(), dout.cuda()
+    out, lse = ops.attention_forward(qg, kg, vg, **kw)
+    grads = ops.attention_backward(dg, qg, kg, vg, out, lse, **kw)
+    for _ in range(20):
+        again = [torch.full_like(t, float("nan")) for t in (qg, kg, vg)]
+        ops.attention_backward(dg, qg, kg, vg, out, lse, dq=again[0], dk=again[1], dv=again[2], **kw)
+        assert all(torch.equal(a, b) for a, b in zip(grads, again))
+    _check_gradients(grads, OB.attention_varlen_backward(q, k, v, dout, lse.cpu(), cu, cu, softmax_scale=d ** -0.5, causal=True,
+                                                         window=(-1, -1)))
