@@ -542,6 +542,13 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
 // =================================================================================================
 // dQ
 // =================================================================================================
+// A parity wait only tells the current phase of a barrier from the one before, so every role that waits on a barrier must
+// keep it from running two phases ahead.  The elementwise warps do so with s_full (the next S needs their s_free), ds_free
+// (the next dS needs their ds_full) and acc_done (the next item's last product needs their ds_full), but not with
+// qdo_full: the products of an item of one key block need s_free of the item before only, so Q / dO of two further items
+// can land while a warp is still in that item's exponentials or epilogue.  They wait for nothing there and read the LSE
+// and D of their own row from global memory instead.  The issuers release qdo_empty and kv_empty themselves; the dQ
+// issuer's commit is one of the two that release a K tile.
 struct BarB {
   uint64_t qdo_full, qdo_empty;  // Q / dO of the item have landed; the item's last S / dP have read them
   uint64_t kv_full[kDqSlots], kv_empty[kDqSlots];
@@ -554,7 +561,6 @@ struct BarB {
   ItemQueue queue;
   uint32_t tmem_base;
   int abort_flag;
-  float nlse2[2][kBlk], ndls[2][kBlk];  // by item parity: -LSE * log2(e) and -D * scale of the block's query rows
 };
 static_assert(sizeof(BarB) <= kBarBytes, "barrier block does not fit");
 
@@ -659,13 +665,6 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
       }
       queue_publish(&bar->queue, wi, t, lane);
       if (!mbar_wait(smem_addr(&bar->qdo_empty), (wi & 1) ^ 1, abort_flag, 70)) break;
-      for (int r = lane; r < kBlk; r += 32) {
-        const int i = w.row0 + r;
-        const int64_t li = (int64_t)sq.bq * p.lse_batch_stride + (int64_t)w.head * p.lse_head_stride + sq.q_row0 + i;
-        bar->nlse2[wi & 1][r] = i < sq.q_len ? -p.lse[li] * kLog2e : -INFINITY;
-        bar->ndls[wi & 1][r] = i < sq.q_len ? -p.delta[li] * p.softmax_scale : 0.f;
-      }
-      __syncwarp();
       if (elect_one()) {
         const uint32_t full = smem_addr(&bar->qdo_full);
         mbar_arrive_expect_tx(full, 2 * (HD / 64) * kHalfBytes);
@@ -788,8 +787,12 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
       int hi = sq.k_len - 1, lo = 0;
       if (sq.wr >= 0) hi = min(hi, i + sq.koff + sq.wr);
       if (sq.wl >= 0) lo = max(0, i + sq.koff - sq.wl);
-      if (!mbar_wait(smem_addr(&bar->qdo_full), wi & 1, abort_flag, 77)) break;
-      const float nl = bar->nlse2[wi & 1][r], nd = bar->ndls[wi & 1][r];
+      float nl = -INFINITY, nd = 0.f;  // -LSE * log2(e) and -D * scale; rows beyond the sequence: P = 0
+      if (i < sq.q_len) {
+        const int64_t li = (int64_t)sq.bq * p.lse_batch_stride + (int64_t)w.head * p.lse_head_stride + sq.q_row0 + i;
+        nl = -p.lse[li] * kLog2e;
+        nd = -p.delta[li] * p.softmax_scale;
+      }
       const uint64_t nlse2 = pack_f32x2(nl, nl), ndls2 = pack_f32x2(nd, nd);
       const int i_max = min(sq.q_len, row0 + kBlk) - 1;
       for (int it = 0; it < w.iters; ++it) {

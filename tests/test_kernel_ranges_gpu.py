@@ -215,3 +215,22 @@ def test_wide_head_backward_short_items(d):
         assert all(torch.equal(a, b) for a, b in zip(grads, again))
     _check_gradients(grads, OB.attention_varlen_backward(q, k, v, dout, lse.cpu(), cu, cu, softmax_scale=d ** -0.5, causal=True,
                                                          window=(-1, -1)))
+
+
+@pytest.mark.parametrize("dtype,d,causal", [(BF, 128, True), (FP, 64, False)])
+def test_backward_of_many_short_sequences(dtype, d, causal):
+    """Several hundred packed sequences of 1 - 128 rows: every dQ item has one key block, so the products of an item may
+    run while the elementwise warps still finish the item before."""
+    from oracle import bwd as OB
+    g = torch.Generator().manual_seed(d)
+    lens = [1 + (37 * i) % 128 for i in range(400)]
+    h, hk = 4, 2
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32)
+    q, k, v, dout = _backward_inputs(g, dtype, (sum(lens),), (sum(lens),), h, hk, d)
+    kw = dict(softmax_scale=d ** -0.5, causal=causal, cu_seqlens_q=cu.cuda(), cu_seqlens_k=cu.cuda(), max_seqlen_q=max(lens),
+              max_seqlen_k=max(lens))
+    out, lse = ops.attention_forward(q.cuda(), k.cuda(), v.cuda(), **kw)
+    grads = [torch.full_like(t, float("nan")).cuda() for t in (q, k, v)]
+    ops.attention_backward(dout.cuda(), q.cuda(), k.cuda(), v.cuda(), out, lse, dq=grads[0], dk=grads[1], dv=grads[2], **kw)
+    _check_gradients(grads, OB.attention_varlen_backward(q, k, v, dout, lse.cpu(), cu, cu, softmax_scale=d ** -0.5, causal=causal,
+                                                         window=(-1, -1)))
