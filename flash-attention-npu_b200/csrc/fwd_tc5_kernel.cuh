@@ -28,6 +28,7 @@
 
 #include "common.cuh"
 #include "tc5_ptx.cuh"
+#include "tile_order.cuh"
 
 namespace fa {
 namespace tc5 {
@@ -250,25 +251,20 @@ __device__ __forceinline__ TileId tile_id(const Tc5Params& p, int n) {
 }
 
 // The producer's side.  Position n (a CTA index) -> tile: the heads are cut into chunks whose K / V stay in L2 together;
-// a chunk runs its tiles by level, highest first, level = query tile + (causal) the tiles' worth of keys in front of the
-// queries, i.e. about the work of the tile; a level holds at most one tile of every batch entry, for all heads of the
-// chunk.  Tiles that do not exist have no position, the grid's surplus positions no tile.
+// a chunk runs its tiles by level (tile_order.cuh), level = query tile + (causal) the tiles' worth of keys in front of the
+// queries, i.e. about the work of the tile.  The grid's surplus positions have no tile.
 template <int ROWS>
-struct TileDraw {
+struct TileLevels {
   const Tc5Params& p;
-  Barriers* bar;
-  int lane, pos;
-  uint32_t k = 0, asked = 0;
-  bool pending = false, more = true;
-  int live = 0, top = 0;                         // tiles of one head; highest level
-  int chunk = 0, level = 0, start = 0, cnt = 0;  // of the last position: its level, the level's first position in the chunk and tiles per head
+  int lane;
+  int live = 0, top = 0;  // tiles of one head; highest level
 
   __device__ __forceinline__ void entry(int bi, int& lo, int& n) const {  // levels [lo, lo + n) of batch entry bi
     const int q_len = q_length(p, bi);
     n = min(max(0, ceil_div(q_len, ROWS)), p.m_tiles);
     lo = (p.is_causal || p.is_local) ? max(0, k_length(p, bi) - q_len) / ROWS : 0;
   }
-  __device__ TileDraw(const Tc5Params& p_, Barriers* b, int lane_) : p(p_), bar(b), lane(lane_), pos(blockIdx.x) {
+  __device__ TileLevels(const Tc5Params& p_, int lane_) : p(p_), lane(lane_) {
     for (int bi = lane; bi < p.a.b; bi += 32) {
       int lo, n;
       entry(bi, lo, n);
@@ -277,35 +273,37 @@ struct TileDraw {
     }
     live = __reduce_add_sync(0xffffffffu, live);
     top = __reduce_max_sync(0xffffffffu, top);
-    level = top + 1;
   }
-  __device__ __forceinline__ uint32_t members(int b0) const {  // batch entries b0 .. b0 + 31 with a tile in this level
+  __device__ __forceinline__ uint32_t members(int level, int b0) const {  // batch entries b0 .. b0 + 31 with a tile in the level
     int lo = 0, n = 0;
     if (b0 + lane < p.a.b) entry(b0 + lane, lo, n);
     return __ballot_sync(0xffffffffu, level >= lo && level < lo + n);
   }
-  // position -> tile; positions only ever grow.  False: the position has no tile.
+  __device__ __forceinline__ int count(int level) const {
+    int c = 0;
+    for (int b0 = 0; b0 < p.a.b; b0 += 32) c += __popc(members(level, b0));
+    return c;
+  }
+};
+
+template <int ROWS>
+struct TileDraw {
+  const Tc5Params& p;
+  Barriers* bar;
+  int lane, pos;
+  uint32_t k = 0, asked = 0;
+  bool pending = false, more = true;
+  TileLevels<ROWS> levels;
+  TileCursor cursor;
+
+  __device__ TileDraw(const Tc5Params& p_, Barriers* b, int lane_) : p(p_), bar(b), lane(lane_), pos(blockIdx.x), levels(p_, lane_) {}
+  // position -> tile.  False: the position has no tile.
   __device__ __forceinline__ bool locate(int n, int& tile) {
-    if (n >= live * p.a.h) return false;
-    const int ck = n / (live * p.chunk_heads);
-    const int heads = min(p.chunk_heads, p.a.h - ck * p.chunk_heads);
-    n -= ck * live * p.chunk_heads;
-    if (ck != chunk) {
-      chunk = ck;
-      level = top + 1;
-      start = cnt = 0;
-    }
-    while (level > 0 && n >= start + cnt * heads) {  // the levels down to 0 hold `live` tiles per head
-      start += cnt * heads;
-      --level;
-      cnt = 0;
-      for (int b0 = 0; b0 < p.a.b; b0 += 32) cnt += __popc(members(b0));
-    }
-    int r = (n - start) / heads;
-    const int hh = ck * p.chunk_heads + (n - start) % heads;
+    int hh, r;
+    if (!tile_locate(cursor, levels, p.a.h, p.chunk_heads, n, hh, r)) return false;
     int bi = 0;
     for (int b0 = 0; b0 < p.a.b; b0 += 32) {
-      uint32_t m = members(b0);
+      uint32_t m = levels.members(cursor.level, b0);
       const int c = __popc(m);
       if (r < c) {
         for (; r > 0; --r) m &= m - 1;  // drop the r lowest members
@@ -315,8 +313,8 @@ struct TileDraw {
       r -= c;
     }
     int lo, nt;
-    entry(bi, lo, nt);
-    tile = (bi * p.a.h + hh) * p.m_tiles + level - lo;
+    levels.entry(bi, lo, nt);
+    tile = (bi * p.a.h + hh) * p.m_tiles + cursor.level - lo;
     return true;
   }
   __device__ __forceinline__ void ask() {

@@ -1,0 +1,48 @@
+// Order of the query tiles of ragged input, as arithmetic that the device (fwd_tc5_kernel.cuh) and a host test share.
+//
+// Position n -> tile: the heads are cut into chunks of chunk_heads; a chunk runs its tiles by level, highest first; a level
+// holds at most one tile of every batch entry, for all heads of the chunk.  Tiles that do not exist have no position.
+// Positions may be asked for in any order: the cursor only saves the walk down from the highest level when they grow,
+// which is what a CTA usually sees (nothing promises it: clusterlaunchcontrol hands out whichever CTA has not started).
+#pragma once
+
+#ifdef __CUDACC__
+#define FA_TILE_HD __host__ __device__ __forceinline__
+#else
+#define FA_TILE_HD inline
+#endif
+
+namespace fa {
+
+// Levels must offer:  int live (tiles of one head over all batch entries), int top (highest level that holds a tile),
+// int count(level) (batch entries with a tile in it).
+struct TileCursor {
+  int chunk = 0;
+  int level = -1;  // of the last position; -1: none yet
+  int start = 0;   // the level's first position in the chunk
+  int cnt = 0;     // tiles per head in the level
+};
+
+// False: position n has no tile.  Otherwise the tile of head `head` is that of the rank-th batch entry of cursor.level.
+template <class Levels>
+FA_TILE_HD bool tile_locate(TileCursor& c, const Levels& lv, int heads_all, int chunk_heads, int n, int& head, int& rank) {
+  if (n >= lv.live * heads_all) return false;
+  const int ck = n / (lv.live * chunk_heads);
+  const int left = heads_all - ck * chunk_heads, heads = chunk_heads < left ? chunk_heads : left;
+  n -= ck * lv.live * chunk_heads;
+  if (c.level < 0 || ck != c.chunk || n < c.start) {  // from the top again
+    c.chunk = ck;
+    c.level = lv.top + 1;
+    c.start = c.cnt = 0;
+  }
+  while (c.level > 0 && n >= c.start + c.cnt * heads) {  // the levels down to 0 hold `live` tiles per head
+    c.start += c.cnt * heads;
+    --c.level;
+    c.cnt = lv.count(c.level);
+  }
+  head = ck * chunk_heads + (n - c.start) % heads;
+  rank = (n - c.start) / heads;
+  return true;
+}
+
+}  // namespace fa
