@@ -183,6 +183,20 @@ __device__ __forceinline__ SeqInfo seq_info(const BwdParams& p, int bi) {
   return s;
 }
 
+// Packed input: the last tile of a sequence that streams past the resident one also holds rows of the next sequence (or the
+// unused rows behind the last one).  Their P and dS are 0, but 0 x NaN is NaN in the products, so the warp that issues the
+// first product on the tile clears rows [first, ROWS) of its PARTS 64-column parts once it has landed (whole 128-byte rows:
+// the swizzle stays inside them).  Later readers of the tile are ordered behind that product.
+template <int PARTS, int ROWS>
+__device__ __forceinline__ void clear_tail_rows(uint32_t tile, int first, int lane) {
+#pragma unroll 1
+  for (int c = 0; c < PARTS; ++c)
+    for (uint32_t o = first * 128 + lane * 16; o < ROWS * 128; o += 512)
+      asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};\n" ::"r"(tile + c * ROWS * 128 + o), "r"(0) : "memory");
+  fence_proxy_async();
+  __syncwarp();
+}
+
 // 32 columns of a row, of which the first n_cols (a multiple of 8, possibly <= 0) exist
 template <typename T>
 __device__ __forceinline__ void store_slice(T* dst, const uint32_t (&a)[32], int n_cols) {

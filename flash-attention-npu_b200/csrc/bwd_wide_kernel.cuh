@@ -130,6 +130,18 @@ __device__ __forceinline__ ItemW item_w(const BwdParams& p, int t) {
   return w;
 }
 
+// Rows of the streamed sequence counted from a unit's first row: below kUnit in the unit that runs past the sequence.
+struct TailRows {
+  int first, last;  // of an item's first unit, and of the last unit that it streams of a head
+  __device__ __forceinline__ TailRows(const BwdParams& p, const ItemW& w) {
+    const int len = w.kind == kWideDQ ? w.sq.k_len : w.sq.q_len;
+    // dense input: the rows behind the sequence lie outside the tensor, the TMA unit has filled them with zeros
+    first = p.cu_seqlens_q ? len - w.u_lo * kUnit : 0x40000000;
+    last = first - (w.nu - 1) * kUnit;
+  }
+  __device__ __forceinline__ int next(int left) const { return left == last ? first : left - kUnit; }  // (the next head starts over)
+};
+
 // Where the item's result goes: first element of resident row 0 (of the item) and the row stride.
 template <typename T>
 __device__ __forceinline__ T* item_out(const BwdParams& p, const ItemW& w, int64_t& row_stride) {
@@ -321,10 +333,14 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
       const ItemW w = item_w(p, t);
       const bool is_v = w.kind == kWideDV;
       const int iters = w.iters, n_y = is_v ? G::YSV : G::YS;
+      const TailRows tail(p, w);
+      int x_left = tail.first, y_left = tail.first;  // rows of the sequence from the next unit of X (dV: of Y) on
       auto issue_s = [&](int u) -> bool {
         const uint32_t g = gu + u;
         const int xs = g % G::XS, b = g & 1;
         if (!mbar_wait(smem_addr(&bar->x_full[xs]), (g / G::XS) & 1, abort_flag, 64)) return false;
+        if (x_left < kUnit) clear_tail_rows<G::kChunks, kUnit>(base + G::kRingOff + xs * G::kSTile, x_left, lane);
+        x_left = tail.next(x_left);
         tc_fence_after();
         if (elect_one()) {
           const uint64_t b_desc = make_smem_desc(base + G::kRingOff + xs * G::kSTile, 16, 1024);
@@ -349,7 +365,11 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
         if (u + 1 < iters && !issue_s(u + 1)) { ok = false; break; }
         const uint32_t g = gu + u;
         const int xs = g % G::XS, b = g & 1;
-        if (is_v && !mbar_wait(smem_addr(&bar->y_full[ys]), (yph >> ys) & 1, abort_flag, 66)) { ok = false; break; }
+        if (is_v) {
+          if (!mbar_wait(smem_addr(&bar->y_full[ys]), (yph >> ys) & 1, abort_flag, 66)) { ok = false; break; }
+          if (y_left < kUnit) clear_tail_rows<G::kChunks, kUnit>(base + G::y_off(ys), y_left, lane);
+          y_left = tail.next(y_left);
+        }
         yph ^= 1u << ys;
         if (!mbar_wait(smem_addr(&bar->pds_full[b]), (g >> 1) & 1, abort_flag, 67)) { ok = false; break; }
         // the epilogue of the previous item must have the accumulator in registers
@@ -393,11 +413,15 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
           if (++ys == G::YSV) ys = 0;
         }
       } else {
+        const TailRows tail(p, w);
+        int y_left = tail.first;
         for (int u = 0; u < w.iters; ++u) {
           const uint32_t g = gu + u;
           const int b = g & 1;
           if (!mbar_wait(smem_addr(&bar->y_full[ys]), (yph >> ys) & 1, abort_flag, 70)) { ok = false; break; }
           yph ^= 1u << ys;
+          if (y_left < kUnit) clear_tail_rows<G::kChunks, kUnit>(base + G::y_off(ys), y_left, lane);
+          y_left = tail.next(y_left);
           // dP of the unit before in this buffer must have been read
           if (g >= 2 && !mbar_wait(smem_addr(&bar->pds_full[b]), ((g - 2) >> 1) & 1, abort_flag, 71)) { ok = false; break; }
           tc_fence_after();

@@ -156,3 +156,39 @@ def test_packed_sequences_do_not_see_their_neighbours(kernel):
         assert torch.isfinite(out[rows].float()).all(), f"sequence {s} picked up its neighbour's NaN"
         U.check_rules(out[rows], lse[:, rows], go[rows], gl[:, rows], tag=f"packed seq {s}")
     del fa2
+
+
+def _poisoned_backward(d, dtype, causal, poison):
+    """Packed sequences that end inside the kernels' tiles, two of them and the rows behind the last one poisoned in one of
+    the inputs: the others' gradients must equal the oracle's."""
+    from oracle import bwd as OB
+    g = torch.Generator().manual_seed(4500 + d + len(poison))
+    h, hk = 4, 2
+    lens_q, lens_k, spare = [200, 130, 300, 65, 1, 70], [333, 190, 257, 65, 30, 129], 100
+    cq, ck = [torch.tensor([0] + list(torch.tensor(x).cumsum(0)), dtype=torch.int32) for x in (lens_q, lens_k)]
+    r = lambda n, heads: (2.0 * (torch.rand((n + spare, heads, d), generator=g) - 0.5)).to(dtype)
+    t = {"q": r(sum(lens_q), h), "k": r(sum(lens_k), hk), "v": r(sum(lens_k), hk), "dout": r(sum(lens_q), h)}
+    kw = dict(softmax_scale=d ** -0.5, causal=causal)
+    args = dict(kw, cu_seqlens_q=cq.cuda(), cu_seqlens_k=ck.cuda(), max_seqlen_q=max(lens_q), max_seqlen_k=max(lens_k))
+    cu = cq if poison in ("q", "dout") else ck
+    clean = {n: x[:(cq if n in ("q", "dout") else ck)[-1]].clone() for n, x in t.items()}
+    for rows in (slice(int(cu[1]), int(cu[2])), slice(int(cu[4]), int(cu[5])), slice(int(cu[-1]), None)):
+        t[poison][rows] = NAN
+    gpu = {n: x.cuda() for n, x in t.items()}
+    out, lse = ops.attention_forward(gpu["q"], gpu["k"], gpu["v"], **args)
+    grads = ops.attention_backward(gpu["dout"], gpu["q"], gpu["k"], gpu["v"], out, lse, **args)
+    _, clean_lse = ops.attention_forward(clean["q"].cuda(), clean["k"].cuda(), clean["v"].cuda(), **args)
+    want = OB.attention_varlen_backward(clean["q"], clean["k"], clean["v"], clean["dout"], clean_lse.cpu(), cq, ck,
+                                        softmax_scale=d ** -0.5, causal=causal, window=(-1, -1))
+    for s in (0, 2, 3, 5):
+        for name, a, b, c in zip(("dq", "dk", "dv"), grads, want, (cq, ck, ck)):
+            rows = slice(int(c[s]), int(c[s + 1]))
+            assert torch.isfinite(a[rows].float()).all(), f"{name} of sequence {s} picked up its neighbour's NaN"
+            torch.testing.assert_close(a[rows].float().cpu(), b[rows].float(), rtol=1e-2, atol=1e-2, msg=lambda m: f"{name} of sequence {s}: {m}")
+    assert L.load().fa_b200_check_status(torch.cuda.current_stream().cuda_stream) == 0
+
+
+@pytest.mark.parametrize("poison", ["q", "k", "v", "dout"])
+@pytest.mark.parametrize("d,dtype,causal", [(192, BF, True), (256, BF, False), (256, FP, True)])
+def test_packed_backward_of_wide_heads_does_not_see_its_neighbours(d, dtype, causal, poison):
+    _poisoned_backward(d, dtype, causal, poison)
