@@ -31,7 +31,7 @@ int bwd_tc5_launch(const BwdParams& p, const fa_bwd_params& a, cudaStream_t st, 
   const int64_t outer = varlen ? 1 : a.b;
   CUtensorMap tq, tdo, tk, tv, tq_u, tdo_u;  // _u: 64-row boxes (the units of the dK / dV kernel)
   // Packed sequences: one row axis for the whole tensor.  A tile that runs past the end of its sequence reads rows of
-  // the next one (their P is 0 by the mask or by LSE = +inf), past the end of the tensor it reads zeros.
+  // the next one (cleared before the products read them: clear_tail_rows), past the end of the tensor it reads zeros.
   const bool ok =
       tma_encode_rows(&tq, a.q, a.dtype, a.d, a.h, q_rows, outer, a.q_head_stride, a.q_row_stride, a.q_batch_stride, kBlk) &&
       tma_encode_rows(&tdo, a.dout, a.dtype, a.d, a.h, q_rows, outer, a.do_head_stride, a.do_row_stride, a.do_batch_stride, kBlk) &&

@@ -413,10 +413,16 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
       if (t < 0) break;
       const ItemA w = item_a(p, t);
       const int iters = w.iters;
+      // rows of the sequence from a unit's first row on: below kUnit in the unit that runs past it (packed input only)
+      const int left_first = p.cu_seqlens_q ? w.sq.q_len - w.u_lo * kUnit : 0x40000000, left_last = left_first - (w.nu - 1) * kUnit;
+      int left = left_first;
       auto issue_st = [&](int u) -> bool {
         const uint32_t g = gu + u;
         const int s = g % kStages, b = g & 1;
         if (!mbar_wait(bar_full0 + 8 * s, (g / kStages) & 1, abort_flag, 63)) return false;
+        // Q or dO: the other chain reads the tile only after both chains' first products of the unit
+        if (left < kUnit) clear_tail_rows<HD / 64, kUnit>(ring + (2 * s + r) * kUnitTile, left, lane);
+        left = left == left_last ? left_first : left - kUnit;  // (the next head of the group starts over)
         tc_fence_after();
         if (elect_one()) {
           const uint64_t b_desc = b_desc0 + (uint64_t)s * kStageStep;
@@ -731,6 +737,9 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
         const uint32_t slot = r ? kDqKSlots + (g & 1) : g % kDqKSlots;  // V(g) or K(g)
         const uint32_t par = r ? (g >> 1) & 1 : (g / kDqKSlots) & 1;
         if (!mbar_wait(bar_full0 + 8 * slot, par, abort_flag, 74)) { ok = false; break; }
+        // K (which dQ += dS K reads after this warp's S) or V
+        const int left = w.sq.k_len - (w.j_lo + it) * kBlk;
+        if (p.cu_seqlens_q && left < kBlk) clear_tail_rows<HD / 64, kBlk>(ring + slot * kTileBytes, left, lane);
         if (g > 0 && !mbar_wait(bar_sfree, (g - 1) & 1, abort_flag, 76)) { ok = false; break; }
         tc_fence_after();
         if (elect_one()) {

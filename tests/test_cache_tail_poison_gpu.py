@@ -192,3 +192,9 @@ def _poisoned_backward(d, dtype, causal, poison):
 @pytest.mark.parametrize("d,dtype,causal", [(192, BF, True), (256, BF, False), (256, FP, True)])
 def test_packed_backward_of_wide_heads_does_not_see_its_neighbours(d, dtype, causal, poison):
     _poisoned_backward(d, dtype, causal, poison)
+
+
+@pytest.mark.parametrize("poison", ["q", "k", "v", "dout"])
+@pytest.mark.parametrize("d,dtype,causal", [(64, FP, True), (128, BF, False), (128, BF, True)])
+def test_packed_backward_does_not_see_its_neighbours(d, dtype, causal, poison):
+    _poisoned_backward(d, dtype, causal, poison)
