@@ -15,6 +15,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/TracerMode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -57,9 +58,10 @@ bool as_bool(PyObject* o, bool& v) {
 }
 PyObject* not_implemented() { Py_RETURN_NOTIMPLEMENTED; }
 
-// No dispatch mode (FakeTensorMode, make_fx, ...) and no functorch transform is active.
+// No dispatch mode (FakeTensorMode, make_fx, ...), no functorch transform and no torch.jit.trace is active: they record
+// or replace operators, and a launch from here is none (a trace would keep the allocation of the outputs alone).
 bool plain_eager() {
-  return c10::impl::TorchDispatchModeTLS::stack_len() == 0 &&
+  return c10::impl::TorchDispatchModeTLS::stack_len() == 0 && !at::tracer::impl::is_dispatch_enabled() &&
          !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
 }
 bool plain(const Tensor& t) {

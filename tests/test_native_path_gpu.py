@@ -1,0 +1,24 @@
+"""GPU: calls that the native host path (csrc/torch_binding.cpp) must leave to the registered operators."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+def _qkv(seed=0, s=64, grad=False):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return [torch.randn((2, s, 4, 64), generator=g, device="cuda", dtype=BF, requires_grad=grad) for _ in range(3)]
+
+
+@pytest.mark.parametrize("api", ["flash_attn_npu_v2", "flash_attn_npu_v3"])
+def test_trace_records_the_attention(api):
+    """A traced function computes attention of the inputs it is called with."""
+    fa = pytest.importorskip(api)
+    fns = [lambda q, k, v: fa.flash_attn_func(q, k, v, causal=True)]
+    if api.endswith("v3"):  # (the cache call of v2 is not a registered operator)
+        fns.append(lambda q, k, v: fa.flash_attn_with_kvcache(q, k, v, causal=True))
+    for fn in fns:
+        traced = torch.jit.trace(fn, tuple(_qkv(1)), check_trace=False)
+        q, k, v = _qkv(2)
+        assert torch.equal(traced(q, k, v), fn(q, k, v))
