@@ -307,6 +307,8 @@ PyObject* attention(PyObject*, PyObject* const* o, Py_ssize_t n) {
       !as_bool(o[9], a.causal) || !as_int(o[10], a.wl) || !as_int(o[11], a.wr) || !as_float(o[12], a.softcap) || !as_int(o[13], a.num_splits))
     return not_implemented();
   if ((a.cu_q != nullptr) != (a.cu_k != nullptr) || !fill_params(a, p)) return not_implemented();
+  for (const Tensor* t : {a.q, a.k, a.v})
+    if (t->_fw_grad(/*level=*/0).defined()) return not_implemented();  // forward-mode differentiation: refused there
   Tensor out, lse;
   if (at::GradMode::is_enabled() && (a.q->requires_grad() || a.k->requires_grad() || a.v->requires_grad())) {
     if (a.alibi) return not_implemented();  // the backward says why not

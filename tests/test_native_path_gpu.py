@@ -22,3 +22,16 @@ def test_trace_records_the_attention(api):
         traced = torch.jit.trace(fn, tuple(_qkv(1)), check_trace=False)
         q, k, v = _qkv(2)
         assert torch.equal(traced(q, k, v), fn(q, k, v))
+
+
+@pytest.mark.parametrize("requires_grad", [False, True])
+@pytest.mark.parametrize("api", ["flash_attn_npu_v2", "flash_attn_npu_v3"])
+def test_forward_mode_differentiation_is_refused(api, requires_grad):
+    """There is no jvp: a dual tensor raises instead of losing its tangent."""
+    import torch.autograd.forward_ad as fwAD
+    fa = pytest.importorskip(api)
+    for which in range(3):
+        with fwAD.dual_level(), pytest.raises(NotImplementedError, match="jvp"):
+            ts = _qkv(3, grad=requires_grad)
+            ts[which] = fwAD.make_dual(ts[which], torch.ones_like(ts[which]))
+            fa.flash_attn_func(*ts, causal=True)
