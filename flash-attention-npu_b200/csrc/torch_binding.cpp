@@ -354,9 +354,13 @@ PyObject* kvcache(PyObject*, PyObject* const* o, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// plain_eager() -> bool: no mode, transform or trace is active that every function here would decline for
+PyObject* py_plain_eager(PyObject*, PyObject*) { return PyBool_FromLong(plain_eager()); }
+
 PyMethodDef methods[] = {
     {"attention", (PyCFunction)(void (*)(void))attention, METH_FASTCALL, "dense or packed attention; NotImplemented: use the Python path"},
     {"kvcache", (PyCFunction)(void (*)(void))kvcache, METH_FASTCALL, "attention over a KV cache; NotImplemented: use the Python path"},
+    {"plain_eager", py_plain_eager, METH_NOARGS, "False: a mode, transform or trace is active and every function here declines"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "Native host path of the public attention calls.", -1, methods};
 

@@ -174,7 +174,9 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, qv=None, rotary
         softmax_scale = _default_scale(q, qv)
     if (qv is None and cache_leftpad is None and cu_seqlens_k_new is None and rotary_seqlens is None and q_descale is None
             and k_descale is None and v_descale is None and attention_chunk == 0 and not isinstance(cache_seqlens, int)
-            and not torch.compiler.is_compiling()):
+            and not torch.compiler.is_compiling()
+            # (the bytes of a plan can only be read from a plain tensor outside every mode)
+            and (scheduler_metadata is None or (type(scheduler_metadata) is torch.Tensor and _native.plain_eager()))):
         plan = None if scheduler_metadata is None else _ext._plan_bytes(scheduler_metadata)
         r = _native.kvcache(q, k_cache, v_cache, k, v, cu_seqlens_q, max_seqlen_q, cache_seqlens, cache_batch_idx, page_table,
                             rotary_cos, rotary_sin, rotary_interleaved, None, softmax_scale, causal, window_size[0],
