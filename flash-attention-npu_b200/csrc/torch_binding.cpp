@@ -326,23 +326,28 @@ PyObject* attention(PyObject*, PyObject* const* o, Py_ssize_t n) {
 
 // kvcache(q, k_cache, v_cache, k, v, cu_seqlens_q, max_seqlen_q, cache_seqlens, cache_batch_idx, block_table, rotary_cos,
 //         rotary_sin, rotary_interleaved, alibi_slopes, softmax_scale, causal, window_left, window_right, softcap, num_splits,
-//         plan bytes or None) -> (out, lse), or NotImplemented
+//         plan bytes or None, refuse_grad) -> (out, lse), or NotImplemented; neither is differentiable.  refuse_grad: also
+//         NotImplemented when an input requires a gradient
 PyObject* kvcache(PyObject*, PyObject* const* o, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   FwdArgs a;
   fa_fwd_params p;
-  if (n != 21 || !plain_eager()) return not_implemented();
+  bool refuse_grad = false;
+  if (n != 22 || !plain_eager()) return not_implemented();
   if (!as_tensor(o[0], a.q) || !as_tensor(o[1], a.k) || !as_tensor(o[2], a.v) || !as_tensor(o[3], a.k_new) || !as_tensor(o[4], a.v_new) ||
       !as_tensor(o[5], a.cu_q) || (a.cu_q && !as_int(o[6], a.max_q)) || !as_tensor(o[7], a.seqused_k) || !as_tensor(o[8], a.batch_idx) ||
       !as_tensor(o[9], a.table) || !as_tensor(o[10], a.cos) || !as_tensor(o[11], a.sin) || !as_bool(o[12], a.interleaved) ||
       !as_tensor(o[13], a.alibi) || !as_float(o[14], a.scale) || !as_bool(o[15], a.causal) || !as_int(o[16], a.wl) ||
-      !as_int(o[17], a.wr) || !as_float(o[18], a.softcap) || !as_int(o[19], a.num_splits))
+      !as_int(o[17], a.wr) || !as_float(o[18], a.softcap) || !as_int(o[19], a.num_splits) || !as_bool(o[21], refuse_grad))
     return not_implemented();
   if (o[20] != Py_None && PyBytes_AsStringAndSize(o[20], const_cast<char**>(&a.plan), &a.plan_bytes) < 0) {
     PyErr_Clear();
     return not_implemented();
   }
   if (!fill_params(a, p)) return not_implemented();
+  if (refuse_grad && at::GradMode::is_enabled())
+    for (const Tensor* t : {a.q, a.k, a.v, a.k_new, a.v_new, a.cos, a.sin})
+      if (t && t->requires_grad()) return not_implemented();
   if (a.k_new && (a.k->is_inference() || a.v->is_inference())) return not_implemented();
   Tensor out, lse;
   if (!launch_forward(a, p, out, lse)) return not_implemented();

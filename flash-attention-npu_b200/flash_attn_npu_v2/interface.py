@@ -190,7 +190,7 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, rotary_cos=None
     if cache_leftpad is None and not isinstance(cache_seqlens, int) and not torch.compiler.is_compiling():
         r = _native.kvcache(q, k_cache, v_cache, k, v, None, 0, cache_seqlens, cache_batch_idx, block_table, rotary_cos, rotary_sin,
                             rotary_interleaved, alibi_slopes, q.shape[-1] ** (-0.5) if softmax_scale is None else softmax_scale,
-                            causal, window_size[0], window_size[1], softcap, num_splits, None)
+                            causal, window_size[0], window_size[1], softcap, num_splits, None, False)
         if r is not NotImplemented:
             return r if return_softmax_lse else r[0]
     assert k_cache.stride(-1) == 1, "k_cache must have contiguous last dimension"

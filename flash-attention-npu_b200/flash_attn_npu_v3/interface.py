@@ -180,7 +180,7 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, qv=None, rotary
         plan = None if scheduler_metadata is None else _ext._plan_bytes(scheduler_metadata)
         r = _native.kvcache(q, k_cache, v_cache, k, v, cu_seqlens_q, max_seqlen_q, cache_seqlens, cache_batch_idx, page_table,
                             rotary_cos, rotary_sin, rotary_interleaved, None, softmax_scale, causal, window_size[0],
-                            window_size[1], softcap, num_splits, plan)
+                            window_size[1], softcap, num_splits, plan, True)
         if r is not NotImplemented:
             if not return_softmax_lse:
                 return r[0]

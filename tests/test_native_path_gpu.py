@@ -35,3 +35,16 @@ def test_forward_mode_differentiation_is_refused(api, requires_grad):
             ts = _qkv(3, grad=requires_grad)
             ts[which] = fwAD.make_dual(ts[which], torch.ones_like(ts[which]))
             fa.flash_attn_func(*ts, causal=True)
+
+
+def test_kvcache_call_on_inputs_that_require_grad():
+    """v3: the call has no autograd formula.  Its output requires a gradient and the backward says so; it is not detached."""
+    import flash_attn_npu_v3 as fa3
+    q, k, v = _qkv(4)
+    q.requires_grad_(True)
+    out = fa3.flash_attn_with_kvcache(q, k, v, causal=True)
+    assert out.requires_grad
+    with pytest.raises(RuntimeError, match="no autograd formula"):
+        out.sum().backward()
+    with torch.no_grad():
+        assert torch.equal(fa3.flash_attn_with_kvcache(q, k, v, causal=True), out)
