@@ -32,10 +32,14 @@ static cudaError_t launch_bwd(const BwdParams& p, int n_kblocks, cudaStream_t st
 
 extern "C" {
 
-// First part of the workspace: the fp32 dQ accumulator of the mma.sync kernel, or the two work-item counters of the
-// tcgen05 kernels (which write dQ directly).
+// Which kernels a call runs on: the two of head dims up to 128, or the one of wider heads; neither: the mma.sync kernel.
+static bool bwd_runs_tc5(const fa_bwd_params* a) { return a->kernel != 1 && fa::bwd_tc5_eligible(*a); }
+static bool bwd_runs_wide(const fa_bwd_params* a) { return a->kernel == 0 && fa::bwd_wide_eligible(*a); }
+
+// First part of the workspace: the fp32 dQ accumulator of the mma.sync kernel, or the work-item counters of the tcgen05
+// kernels (which write dQ directly).
 static size_t bwd_accum_bytes(const fa_bwd_params* a, int64_t rows) {
-  if (a->kernel != 1 && fa::bwd_tc5_eligible(*a)) return 16;
+  if (bwd_runs_tc5(a) || bwd_runs_wide(a)) return 16;
   const int d_pad = a->d <= 64 ? 64 : (a->d <= 128 ? 128 : 256);
   return fa::align16((size_t)rows * a->h * d_pad * sizeof(float));
 }
@@ -113,10 +117,10 @@ int fa_b200_bwd(const fa_bwd_params* a, void* workspace, size_t workspace_bytes,
   p.delta = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + acc_bytes);
 
   if (a->kernel < 0 || a->kernel > 2) return fail_bwd(FA_ERR_INVALID, "kernel must be 0 (automatic), 1 (mma.sync) or 2 (tcgen05)");
-  const bool tc5 = a->kernel != 1 && bwd_tc5_eligible(*a);
+  const bool tc5 = bwd_runs_tc5(a), wide = bwd_runs_wide(a);
   if (a->kernel == 2 && !tc5)
-    return fail_bwd(FA_ERR_UNSUPPORTED, "the tcgen05 backward covers head dims up to 128 (packed input: total_k given)");
-  const bool wide = a->kernel == 0 && bwd_wide_eligible(*a);
+    return fail_bwd(FA_ERR_UNSUPPORTED, "kernel = 2: this tcgen05 backward covers head dims up to 128 (packed input: total_k given); "
+                                        "wider heads have theirs with kernel = 0");
   cudaError_t e = cudaSuccess;
   if (!tc5 && !wide) e = cudaMemsetAsync(p.dq_accum, 0, acc_bytes, cs);
   if (e != cudaSuccess) return fail_bwd(FA_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));

@@ -245,9 +245,13 @@ def test_backward_workspace_and_kernel_choice():
     assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params())) == 16 + delta
     assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params(softcap=30.0, d=64))) == 16 + delta
     assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params(kernel=1))) == rows * h * 128 * 4 + delta
-    assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params(d=256))) == rows * h * 256 * 4 + delta
+    assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params(d=256))) == 16 + delta
+    assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params(d=136, softcap=30.0))) == 16 + delta
+    assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params(d=256, kernel=1))) == rows * h * 256 * 4 + delta
     packed = dict(cu_seqlens_q=256, cu_seqlens_k=256, lse_batch_stride=0, lse_head_stride=1024)
     assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params(total_k=1024, **packed))) == 16 + delta
+    assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params(total_k=1024, d=192, **packed))) == 16 + delta
+    assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params(total_k=0, d=192, **packed))) == rows * h * 256 * 4 + delta
     assert lib.fa_b200_bwd_workspace_bytes(C.byref(_bwd_params(total_k=0, **packed))) == rows * h * 128 * 4 + delta
     for kw, msg in ((dict(kernel=2, d=256), "tcgen05 backward covers"), (dict(kernel=5), "kernel must be"),
                     (dict(h_k=3), "must divide"), (dict(d=100), "multiple of 8")):
