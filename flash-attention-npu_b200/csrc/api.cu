@@ -155,12 +155,9 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
     const bool eligible = rows_max <= 32 && rows_max > 0 && !a.cu_seqlens_k && strides_ok &&
                           al16(a.k) && al16(a.v) && a.k_batch_stride > 0 && a.v_batch_stride > 0 &&
                           (!a.block_table || a.page_size % 128 == 0);
-    // Several query rows per sequence over few keys, head dims other than 128: left to the register-accumulator kernel,
-    // whose handling of cache tails is tested at these sizes (64 columns, 6144 keys: 18 us there, 12 us here).
-    const bool short_range = a.d != 128 && a.seqlen_q > 1 && (long long)a.b * a.h_k * max_k_bound <= 8192;
     if (a.kernel == FA_KERNEL_DECODE && !eligible)
       return fail(FA_ERR_UNSUPPORTED, "the decode kernel does not cover this problem");
-    if (eligible && (a.kernel == FA_KERNEL_DECODE || (a.kernel == FA_KERNEL_AUTO && !short_range))) {
+    if (eligible && (a.kernel == FA_KERNEL_DECODE || a.kernel == FA_KERNEL_AUTO)) {
       // Measured best.  Up to 16 rows: two resident CTAs of 1x4 consumer warps.  17-32 rows: one CTA of 2x4
       // consumer warps for long key ranges and for launches that become persistent; for short ranges (a
       // sliding window, short caches) two resident CTAs of 2x2 warps, so that one CTA's Q load, slice

@@ -52,7 +52,7 @@ def _poisoned_cache(g, dtype, b, s_cache, hk, d, lens, s_new, page, extra_rows=0
     return kc, vc, bt, idx
 
 
-def _check(q, kc, vc, kn, vn, lens, bt, idx, kernel, tag, causal=True, window=(-1, -1), cos=None, sin=None):
+def _check(q, kc, vc, kn, vn, lens, bt, idx, kernel, tag, causal=True, window=(-1, -1), cos=None, sin=None, ask=L.KERNEL_AUTO):
     kc_o, vc_o = kc.clone(), vc.clone()
     go, gl = OA.flash_attn_with_kvcache(q, kc_o, vc_o, kn, vn, rotary_cos=cos, rotary_sin=sin, cache_seqlens=lens,
                                         cache_batch_idx=idx, block_table=bt, causal=causal, window_size=window,
@@ -63,7 +63,7 @@ def _check(q, kc, vc, kn, vn, lens, bt, idx, kernel, tag, causal=True, window=(-
     out, lse, plan = ops.attention_forward(
         c(q), kc_g, vc_g, k_new=c(kn), v_new=c(vn), seqused_k=c(lens), cache_batch_idx=c(idx), block_table=c(bt),
         rotary_cos=c(cos), rotary_sin=c(sin), rotary_interleaved=False, softmax_scale=q.shape[-1] ** -0.5,
-        causal=causal, window_left=window[0], window_right=window[1], return_plan=True)
+        causal=causal, window_left=window[0], window_right=window[1], kernel=ask, return_plan=True)
     torch.cuda.synchronize()
     assert plan.kernel == kernel, f"{tag}: ran on kernel {plan.kernel}, expected {kernel}"
     assert torch.isfinite(out.float()).all(), f"{tag}: NaN / Inf leaked from memory the call does not own"
@@ -99,9 +99,10 @@ def test_tcgen05_prefill_ignores_the_cache_tail(layout, d, append):
 @pytest.mark.parametrize("append", [False, True], ids=["read", "append"])
 @pytest.mark.parametrize("layout", ["contiguous", "page128", "page256", "batch_idx"])
 @pytest.mark.parametrize("s_q", [1, 4])
-def test_decode_kernel_ignores_the_cache_tail(layout, append, s_q):
+@pytest.mark.parametrize("d", [64, 96, 128, 192, 256])
+def test_decode_kernel_ignores_the_cache_tail(layout, append, s_q, d):
     g = torch.Generator().manual_seed(4200 + len(layout) + append + s_q)
-    b, h, hk, d, s_cache = 6, 32, 8, 128, 1536
+    b, h, hk, s_cache = 6, 32, 8, 1536
     s_new = s_q if append else 0
     lens = torch.tensor([333, 1024, 77, 0 if append else 1, s_cache - s_new, 1281], dtype=torch.int32)
     page = {"page128": 128, "page256": 256}.get(layout, 0)
@@ -110,7 +111,7 @@ def test_decode_kernel_ignores_the_cache_tail(layout, append, s_q):
     kn = vn = cos = sin = None
     if append:
         kn, vn = U.normal((b, s_new, hk, d), BF, g), U.normal((b, s_new, hk, d), BF, g)
-        cos, sin = U.rotary_tables(s_cache + 8, 128, BF)
+        cos, sin = U.rotary_tables(s_cache + 8, d, BF)
     _check(q, kc, vc, kn, vn, lens, bt, idx, L.KERNEL_DECODE, f"decode {layout} append={append} s_q={s_q}", cos=cos, sin=sin)
 
 
@@ -118,7 +119,7 @@ def test_decode_kernel_ignores_the_cache_tail(layout, append, s_q):
 @pytest.mark.parametrize("layout,d,dtype", [("contiguous", 64, FP), ("page16", 128, BF), ("page64", 64, BF), ("batch_idx", 256, BF),
                                             ("page256", 96, FP)])
 def test_register_kernel_ignores_the_cache_tail(layout, d, dtype, append):
-    """Head dims other than 128 and pages smaller than a key block run on the register-accumulator kernel."""
+    """Pages smaller than a key block run on the register-accumulator kernel; the other layouts do when it is asked for."""
     g = torch.Generator().manual_seed(4300 + d + append)
     b, s_q, h, hk, s_cache = 4, 3, 8, 2, 768
     s_new = s_q if append else 0
@@ -129,7 +130,8 @@ def test_register_kernel_ignores_the_cache_tail(layout, d, dtype, append):
     kn = vn = None
     if append:
         kn, vn = U.normal((b, s_new, hk, d), dtype, g), U.normal((b, s_new, hk, d), dtype, g)
-    _check(q, kc, vc, kn, vn, lens, bt, idx, L.KERNEL_MMA, f"mma {layout} d={d} append={append}")
+    _check(q, kc, vc, kn, vn, lens, bt, idx, L.KERNEL_MMA, f"mma {layout} d={d} append={append}",
+           ask=L.KERNEL_AUTO if layout in ("page16", "page64") else L.KERNEL_MMA)
 
 
 @pytest.mark.parametrize("kernel", [L.KERNEL_TCGEN05, L.KERNEL_MMA], ids=["tcgen05", "mma"])

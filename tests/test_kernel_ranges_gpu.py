@@ -68,6 +68,9 @@ def test_decode_kernel_every_head_dim(d, rows, page):
     k, v = U.normal((b, new, hk, d), dtype, g), U.normal((b, new, hk, d), dtype, g)
     cos, sin = U.rotary_tables(room, rotary, dtype)
     kc_o, vc_o, kc_g, vc_g = kc.clone(), vc.clone(), kc.cuda(), vc.cuda()
+    plan = ops.attention_forward(q.cuda(), kc.cuda(), vc.cuda(), k_new=k.cuda(), v_new=v.cuda(), seqused_k=lens.cuda(),
+                                 block_table=_cuda(bt), rotary_cos=cos.cuda(), rotary_sin=sin.cuda(), causal=True, return_plan=True)[2]
+    assert plan.kernel == L.KERNEL_DECODE
     go, gl = OA.flash_attn_with_kvcache(q, kc_o, vc_o, k, v, rotary_cos=cos, rotary_sin=sin, cache_seqlens=lens, block_table=bt,
                                         causal=True, rotary_interleaved=False)
     out, lse = fa2.flash_attn_with_kvcache(q.cuda(), kc_g, vc_g, k.cuda(), v.cuda(), rotary_cos=cos.cuda(), rotary_sin=sin.cuda(),
