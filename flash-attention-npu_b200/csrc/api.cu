@@ -59,6 +59,24 @@ static bool s_new_too_long(const fa_fwd_params& a) { return a.seqlen_new > a.seq
 
 constexpr int kMinPersistSlots = 4;  // partials of a unit that persistent decode CTAs share, at least
 
+// Packed queries against a cache, few query rows in all and many keys: the tcgen05 kernel has no key split, so its few
+// tiles keep a few SMs busy for the whole range (2 us per 128 keys), while the mma.sync kernel cuts the keys over the
+// chip.  Its time follows query rows x heads, that of the tcgen05 kernel does not (one wave), so the line is a number of
+// those, by tile width and key range (measured, mma.sync / tcgen05 in us; both sides of the line):
+//   64 columns    4096 keys: 4900 rows 75 / 79, 6384 rows 103 / 80      32768 keys: 5200 rows 390 / 520, 8192 rows 532 / 513
+//   128 columns   4096 keys: 2000 rows 53 / 87, 2640 rows 88 / 83       16384 keys: 3056 rows 242 / 266, 4288 rows (8192 keys) 175 / 148
+//   256 columns   16384 keys: 520 rows 186 / 244, 1000 rows 248 / 242
+// Below 2048 keys (256 columns: 4096) the tcgen05 kernel is as fast or faster everywhere.
+static bool few_tiles_long_range(const fa_fwd_params& a) {
+  if (!a.cu_seqlens_q || a.cu_seqlens_k) return false;
+  long long keys = a.seqlen_k;
+  if (a.window_left >= 0) keys = std::min<long long>(keys, (long long)a.window_left + 256);  // what one tile sees
+  const long long rows = (long long)a.total_q * a.h;
+  if (a.d <= 64) return keys >= 2048 && rows < (keys < 4096 ? 2560 : keys < 16384 ? 5120 : 6656);
+  if (a.d <= 128) return keys >= 2048 && rows < (keys < 8192 ? 2304 : 3072);
+  return keys >= 4096 && rows < 1024;
+}
+
 struct Planned {
   fa_fwd_plan pl;
   KParams kp;
@@ -335,7 +353,8 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
   kp.lse_elems = lse_elems;
 
   // ---- tcgen05 prefill kernel eligibility ----
-  if (a.kernel != FA_KERNEL_MMA && a.kernel != FA_KERNEL_DECODE && tc5_eligible(a, is_causal, is_local, wl_on_device)) {
+  if (a.kernel != FA_KERNEL_MMA && a.kernel != FA_KERNEL_DECODE && !(a.kernel == FA_KERNEL_AUTO && few_tiles_long_range(a)) &&
+      tc5_eligible(a, is_causal, is_local, wl_on_device)) {
     tc5_fill_plan(a, &pl);
   } else if (a.kernel == FA_KERNEL_TCGEN05) {
     return fail(FA_ERR_UNSUPPORTED, "the tcgen05 kernel does not cover this problem");

@@ -50,6 +50,23 @@ def test_packed_queries_against_a_cache_on_tcgen05(dtype, d, window, page):
         U.check_rules(out[rows].unsqueeze(0), lse[:, rows].unsqueeze(0), go, gl, tag=f"sequence {i}")
 
 
+@pytest.mark.parametrize("d,h,hk,rows,keys,kernel", [
+    (64, 4, 2, 1279, 4096, L.KERNEL_MMA), (64, 4, 2, 1280, 4096, L.KERNEL_TCGEN05), (128, 8, 1, 383, 8192, L.KERNEL_MMA),
+    (128, 8, 1, 384, 8192, L.KERNEL_TCGEN05), (96, 8, 8, 287, 2048, L.KERNEL_MMA), (96, 8, 8, 287, 1920, L.KERNEL_TCGEN05),
+    (256, 4, 1, 255, 4096, L.KERNEL_MMA), (256, 4, 1, 256, 4096, L.KERNEL_TCGEN05)])
+def test_few_packed_rows_against_many_keys(d, h, hk, rows, keys, kernel):
+    """Both sides of the line where a chunk is too small to fill the chip with tiles."""
+    g = torch.Generator().manual_seed(rows)
+    q, (kc, vc, bt) = U.normal((rows, h, d), BF, g), _cache(g, BF, 1, keys, hk, d, 128)
+    lens = torch.tensor([keys - 5], dtype=torch.int32)
+    cq = torch.tensor([0, rows], dtype=torch.int32)
+    out, lse, pl = ops.attention_forward(q.cuda(), kc.cuda(), vc.cuda(), seqused_k=lens.cuda(), block_table=bt.cuda(), cu_seqlens_q=cq.cuda(),
+                                         max_seqlen_q=rows, softmax_scale=d ** -0.5, causal=True, return_plan=True)
+    assert pl.kernel == kernel and (kernel == L.KERNEL_TCGEN05 or pl.num_splits > 1)
+    go, gl = OA.flash_attn_with_kvcache(q.unsqueeze(0), kc, vc, cache_seqlens=lens, block_table=bt, causal=True)
+    U.check_rules(out.unsqueeze(0), lse.unsqueeze(0), go, gl, tag=f"d {d} rows {rows} keys {keys}")
+
+
 @pytest.mark.parametrize("page", [0, 128])
 @pytest.mark.parametrize("rows", [1, 16, 17, 32])
 @pytest.mark.parametrize("d", [64, 72, 96, 128, 136, 192, 256])
