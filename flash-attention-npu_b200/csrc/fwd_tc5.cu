@@ -22,7 +22,7 @@ namespace tc5 {
 // data: warp 15 clears them in the last V tile (tail_fix_loop) and the producer checks the index tensors.  Dense
 // input needs neither, and its instance carries none of that code (the issuing warps' instruction stream is on
 // the kernel's critical path: measured 3-8 % on causal 4K).
-template <typename T, uint32_t AB_FMT, bool FIX, bool SOFTCAP, int HD>
+template <typename T, uint32_t AB_FMT, bool FIX, int CAP, int HD>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUtensorMap tm_q,
                const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v) {
@@ -91,7 +91,7 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
   // scores of a row plus working set, the other roles need far fewer.
   if (warp < 8) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kRegsSoftmax));
-    softmax_loop<T, FIX, SOFTCAP, Geo<HD>::kRows>(p, bar, tmem, p_smem, warp >> 2, warp & 3, lane);
+    softmax_loop<T, FIX, CAP, Geo<HD>::kRows>(p, bar, tmem, p_smem, warp >> 2, warp & 3, lane);
   } else if (warp < 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsCorr));
     correction_loop<T, FIX, HD>(p, bar, tmem, warp & 3, lane);
@@ -301,10 +301,11 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
       e = cudaGetLastError();
     }
   };
-  const bool bf = a.dtype == FA_BF16, cap = a.softcap > 0.f;
+  const bool bf = a.dtype == FA_BF16;
+  const int cap = !(a.softcap > 0.f) ? kCapNone : (a.cu_seqlens_q && !a.cu_seqlens_k) ? kCapFine : kCapApprox;
   auto pick = [&](auto fix_tag, auto cap_tag, auto hd_tag) {
-    constexpr bool F = decltype(fix_tag)::value, C = decltype(cap_tag)::value;
-    constexpr int HD = decltype(hd_tag)::value;
+    constexpr bool F = decltype(fix_tag)::value;
+    constexpr int C = decltype(cap_tag)::value, HD = decltype(hd_tag)::value;
     if (bf) launch(fwd_tc5_kernel<__nv_bfloat16, 1, F, C, HD>);
     else launch(fwd_tc5_kernel<__half, 0, F, C, HD>);
   };
@@ -313,12 +314,15 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
     else if (a.d <= 128) pick(fix_tag, cap_tag, std::integral_constant<int, 128>{});
     else pick(fix_tag, cap_tag, std::integral_constant<int, 256>{});
   };
+  using None = std::integral_constant<int, kCapNone>;
+  using Approx = std::integral_constant<int, kCapApprox>;
   if (p.fix_tail) {
-    if (cap) pick_hd(std::true_type{}, std::true_type{});
-    else pick_hd(std::true_type{}, std::false_type{});
+    if (cap == kCapFine) pick_hd(std::true_type{}, std::integral_constant<int, kCapFine>{});
+    else if (cap == kCapApprox) pick_hd(std::true_type{}, Approx{});
+    else pick_hd(std::true_type{}, None{});
   } else {
-    if (cap) pick_hd(std::false_type{}, std::true_type{});
-    else pick_hd(std::false_type{}, std::false_type{});
+    if (cap) pick_hd(std::false_type{}, Approx{});
+    else pick_hd(std::false_type{}, None{});
   }
   if (e != cudaSuccess) { *err = std::string("tcgen05 kernel launch: ") + cudaGetErrorString(e); return FA_ERR_CUDA; }
   return FA_OK;

@@ -73,6 +73,9 @@ struct Geo {
   static_assert(kRingOff + kRing * kSlotBytes + kBarBytes <= kSmemBytes, "shared memory layout");
 };
 
+// Softcap of a kernel instance: none, by tanh.approx, or by the finer form (packed queries against a cache; softmax role).
+enum CapKind { kCapNone = 0, kCapApprox = 1, kCapFine = 2 };
+
 struct Tc5Params {
   fa_fwd_params a;
   int32_t is_causal, is_local, wl, wr;

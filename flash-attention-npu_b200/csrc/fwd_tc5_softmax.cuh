@@ -48,7 +48,8 @@ __device__ __forceinline__ void chunk_mask(uint32_t (&a)[32], int col_first, int
 }
 
 // softcap: s -> softcap * tanh(s * scale / softcap), here straight into the log2 domain (tests/test_flash_attn_npu_v2.py:
-// the golden applies it to the scaled scores before the mask).  tanh.approx has a relative error of 2^-11.
+// the golden applies it to the scaled scores before the mask).  tanh.approx has a relative error of 2^-11: one unit of the
+// last place of a capped score of 30 .. 50 is 0.02.
 __device__ __forceinline__ void chunk_softcap(uint32_t (&a)[32], float mul, float cap_l2) {
 #pragma unroll
   for (int e = 0; e < 32; ++e) {
@@ -102,7 +103,18 @@ __device__ __forceinline__ void store_p_chunk(uint32_t p_row, uint32_t p_xor, in
   }
 }
 
-template <typename T, bool FIX, bool SOFTCAP, int ROWS>
+// The same through an exponential and a division, 1 - 2 / (e^2y + 1), as the mma.sync and decode kernels compute it: the
+// form of the calls that those kernels served before (packed queries against a cache).  Two special-function results per
+// score instead of one.
+__device__ __forceinline__ void chunk_softcap_fine(uint32_t (&a)[32], float mul, float cap_l2) {
+#pragma unroll
+  for (int e = 0; e < 32; ++e) {
+    const float ex = __expf(2.f * (__uint_as_float(a[e]) * mul));
+    a[e] = __float_as_uint(cap_l2 * (1.f - __fdividef(2.f, ex + 1.f)));
+  }
+}
+
+template <typename T, bool FIX, int CAP, int ROWS>
 __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, uint32_t tmem, uint32_t p_smem, int t,
                                              int warp_in_wg, int lane) {
   volatile int* abort_flag = &bar->abort_flag;
@@ -116,8 +128,8 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
   const uint32_t bar_sfree = smem_addr(&bar->s_free[t]), bar_odone = smem_addr(&bar->o_done[t]);
   const uint32_t bar_oready = smem_addr(&bar->o_ready[t]), bar_ofree = smem_addr(&bar->o_free[t]);
   // with softcap the scores are in the log2 domain once they have been capped: the scale is part of the cap
-  const float scale_log2 = SOFTCAP ? 1.f : p.scale_log2;
-  const float lse_scale = SOFTCAP ? 0.6931471805599453f : p.a.softmax_scale;  // running maximum -> natural log
+  const float scale_log2 = CAP ? 1.f : p.scale_log2;
+  const float lse_scale = CAP ? 0.6931471805599453f : p.a.softmax_scale;  // running maximum -> natural log
   const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
 
   TileWalk<FIX> walk(bar);
@@ -163,9 +175,12 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_sfree);
-      if (SOFTCAP) {
+      if (CAP) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) chunk_softcap(sc[c], p.softcap_mul, p.softcap_l2);
+        for (int c = 0; c < 4; ++c) {
+          if (CAP == kCapFine) chunk_softcap_fine(sc[c], p.softcap_mul, p.softcap_l2);
+          else chunk_softcap(sc[c], p.softcap_mul, p.softcap_l2);
+        }
       }
       if (need_mask) {
 #pragma unroll

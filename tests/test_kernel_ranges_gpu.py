@@ -50,6 +50,26 @@ def test_packed_queries_against_a_cache_on_tcgen05(dtype, d, window, page):
         U.check_rules(out[rows].unsqueeze(0), lse[:, rows].unsqueeze(0), go, gl, tag=f"sequence {i}")
 
 
+@pytest.mark.parametrize("dtype,d", [(FP, 64), (FP, 128), (BF, 256)])
+def test_softcap_of_packed_queries_against_a_cache(dtype, d):
+    """Capped scores as exact as on the kernels that served these calls before (1 - 2 / (e^2y + 1): a few units of 2^-24
+    of the cap, times log2 e).  Scores reach the cap here; the LSE shows their error without the rounding of P.  Sums of
+    fp32 products: sqrt(d) * 2^-24 of the largest partial sums (about 100), 1e-4 in all; tanh.approx gives 3e-4 and more."""
+    g = torch.Generator().manual_seed(d)
+    n, h, hk, cap = 700, 4, 2, 50.0
+    q, k, v = U.normal((n, h, d), dtype, g) * 6, U.normal((1, n, hk, d), dtype, g), U.normal((1, n, hk, d), dtype, g)
+    cq, lens = torch.tensor([0, n], dtype=torch.int32), torch.tensor([n], dtype=torch.int32)
+    out, lse, pl = ops.attention_forward(q.cuda(), k.cuda(), v.cuda(), cu_seqlens_q=cq.cuda(), max_seqlen_q=n, seqused_k=lens.cuda(),
+                                         softmax_scale=d ** -0.5, causal=True, softcap=cap, return_plan=True)
+    assert pl.kernel == L.KERNEL_TCGEN05
+    kk, vv = (t[0].double().repeat_interleave(h // hk, 1).transpose(0, 1) for t in (k, v))
+    x = cap * torch.tanh(q.double().transpose(0, 1) @ kk.transpose(1, 2) * d ** -0.5 / cap)
+    x = x.masked_fill(torch.ones(n, n, dtype=torch.bool).triu(1), float("-inf"))
+    want = torch.logsumexp(x, 2)
+    assert float((lse.cpu().double() - want).abs().max()) < 1e-4
+    torch.testing.assert_close(out.cpu().double(), (torch.softmax(x, 2) @ vv).transpose(0, 1), rtol=1e-2, atol=1e-2)
+
+
 @pytest.mark.parametrize("d,h,hk,rows,keys,kernel", [
     (64, 4, 2, 1279, 4096, L.KERNEL_MMA), (64, 4, 2, 1280, 4096, L.KERNEL_TCGEN05), (128, 8, 1, 383, 8192, L.KERNEL_MMA),
     (128, 8, 1, 384, 8192, L.KERNEL_TCGEN05), (96, 8, 8, 287, 2048, L.KERNEL_MMA), (96, 8, 8, 287, 1920, L.KERNEL_TCGEN05),
