@@ -197,6 +197,8 @@ bool tc5_eligible(const fa_fwd_params& a, bool is_causal, bool is_local, int wl_
   // other kernels decide that on the device: such calls are left to them so that every kernel gives one answer.
   if (wl_on_device && a.rotary_cos) return false;
   if (a.partial_out || a.kv_total > 0) return false;
+  // The row maximum is taken of the raw scores, which a negative scale would turn into the minimum (softcap scales first).
+  if (!(a.softmax_scale >= 0.f) && !(a.softcap > 0.f)) return false;
   // TMA: 16-byte aligned bases and strides
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (!al(a.q) || !al(a.k) || !al(a.v) || !al(a.o)) return false;

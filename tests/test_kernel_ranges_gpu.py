@@ -50,6 +50,32 @@ def test_packed_queries_against_a_cache_on_tcgen05(dtype, d, window, page):
         U.check_rules(out[rows].unsqueeze(0), lse[:, rows].unsqueeze(0), go, gl, tag=f"sequence {i}")
 
 
+@pytest.mark.parametrize("softcap", [0.0, 30.0])
+@pytest.mark.parametrize("kind", ["dense", "packed", "chunk", "decode"])
+def test_negative_softmax_scale(kind, softcap):
+    g = torch.Generator().manual_seed(3)
+    n, h, hk, d, scale = 1 if kind == "decode" else 300, 4, 2, 128, -0.5
+    m = 600 if kind in ("chunk", "decode") else n
+    q, k, v = U.normal((n, h, d), BF, g), U.normal((m, hk, d), BF, g), U.normal((m, hk, d), BF, g)
+    cq, ck, lens = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0, n], [0, m], [m]))
+    kw = dict(softmax_scale=scale, causal=True, softcap=softcap)
+    if kind == "dense":
+        out, lse = ops.attention_forward(q[None].cuda(), k[None].cuda(), v[None].cuda(), **kw)
+    elif kind == "packed":
+        out, lse = ops.attention_forward(q.cuda(), k.cuda(), v.cuda(), cu_seqlens_q=cq, cu_seqlens_k=ck, max_seqlen_q=n, max_seqlen_k=m, **kw)
+    elif kind == "chunk":
+        out, lse = ops.attention_forward(q.cuda(), k[None].cuda(), v[None].cuda(), cu_seqlens_q=cq, max_seqlen_q=n, seqused_k=lens, **kw)
+    else:
+        out, lse = ops.attention_forward(q[None].cuda(), k[None].cuda(), v[None].cuda(), seqused_k=lens, **kw)
+    kk, vv = (t.double().repeat_interleave(h // hk, 1).transpose(0, 1) for t in (k, v))
+    x = q.double().transpose(0, 1) @ kk.transpose(1, 2) * scale
+    if softcap:
+        x = softcap * torch.tanh(x / softcap)
+    x = x.masked_fill(torch.ones(n, m, dtype=torch.bool).triu(1 + m - n), float("-inf"))
+    torch.testing.assert_close(out.cpu().double().view(n, h, d), (torch.softmax(x, 2) @ vv).transpose(0, 1), rtol=1e-2, atol=1e-2)
+    torch.testing.assert_close(lse.cpu().double().view(h, n), torch.logsumexp(x, 2), rtol=1e-2, atol=1e-2)
+
+
 @pytest.mark.parametrize("dtype,d", [(FP, 64), (FP, 128), (BF, 256)])
 def test_softcap_of_packed_queries_against_a_cache(dtype, d):
     """Capped scores as exact as on the kernels that served these calls before (1 - 2 / (e^2y + 1): a few units of 2^-24
