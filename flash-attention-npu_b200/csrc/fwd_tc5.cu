@@ -18,11 +18,11 @@
 namespace fa {
 namespace tc5 {
 
-// FIX: the input is a KV cache or packed sequences, where the rows behind the last key of a sequence hold foreign
+// IN: with a KV cache or packed sequences (ragged input) the rows behind the last key of a sequence hold foreign
 // data: warp 15 clears them in the last V tile (tail_fix_loop) and the producer checks the index tensors.  Dense
 // input needs neither, and its instance carries none of that code (the issuing warps' instruction stream is on
 // the kernel's critical path: measured 3-8 % on causal 4K).
-template <typename T, uint32_t AB_FMT, bool FIX, int CAP, int HD>
+template <typename T, uint32_t AB_FMT, int IN, int CAP, int HD>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUtensorMap tm_q,
                const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v) {
@@ -91,16 +91,16 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
   // scores of a row plus working set, the other roles need far fewer.
   if (warp < 8) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kRegsSoftmax));
-    softmax_loop<T, FIX, CAP, Geo<HD>::kRows>(p, bar, tmem, p_smem, warp >> 2, warp & 3, lane);
+    softmax_loop<T, IN, CAP, Geo<HD>::kRows>(p, bar, tmem, p_smem, warp >> 2, warp & 3, lane);
   } else if (warp < 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsCorr));
-    correction_loop<T, FIX, HD>(p, bar, tmem, warp & 3, lane);
+    correction_loop<T, IN, HD>(p, bar, tmem, warp & 3, lane);
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsMma));
     // warp-uniform role code; one elected lane issues
-    if (warp == kMmaWarp || warp == kMmaWarp + 1) mma_loop<AB_FMT, FIX, HD>(p, bar, q_smem, p_smem, kv_smem, tmem, warp - kMmaWarp);
-    else if (warp == kTmaWarp) producer_loop<FIX, HD>(p, &tm_q, &tm_k, &tm_v, bar, q_smem, kv_smem);
-    else if (FIX) tail_fix_loop<HD>(p, bar, kv_smem, lane);
+    if (warp == kMmaWarp || warp == kMmaWarp + 1) mma_loop<AB_FMT, IN, HD>(p, bar, q_smem, p_smem, kv_smem, tmem, warp - kMmaWarp);
+    else if (warp == kTmaWarp) producer_loop<IN, HD>(p, &tm_q, &tm_k, &tm_v, bar, q_smem, kv_smem);
+    else if (IN != kDense) tail_fix_loop<IN, HD>(p, bar, kv_smem, lane);
   }
 
   tc_fence_before();
@@ -288,12 +288,16 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
   ok = ok && encode_map(&tk, a.k, a.dtype, a.d, a.h_k, k_rows, k_outer, a.k_head_stride, a.k_row_stride, packed_k ? 0 : a.k_batch_stride) &&
        encode_map(&tv, a.v, a.dtype, a.d, a.h_k, k_rows, k_outer, a.v_head_stride, a.v_row_stride, packed_k ? 0 : a.v_batch_stride);
   if (!ok) { *err = "cuTensorMapEncodeTiled failed"; return FA_ERR_CUDA; }
-  // Ragged input: a CTA per tile (TileDraw).  Packed sequences have at most total_q / rows + b tiles a head.
-  int grid = pl.grid;
+  // Ragged input: a CTA per tile, drawn at run time (TileDraw).  Packed sequences have at most total_q / rows + b tiles a
+  // head.  Where these are no more than the SMs (and the tiles that every entry would have at the longest length, which the
+  // fixed deal walks over, not twice as many) the tiles are dealt out instead.
+  int grid = pl.grid, in = kDense;
   if (p.fix_tail) {
     long long tiles = (long long)pl.m_blocks * a.b;
     if (a.cu_seqlens_q) tiles = std::min(tiles, (long long)a.total_q / pl.block_m + a.b);
-    grid = (int)(tiles * a.h);
+    const long long num_sm = a.num_sm > 0 ? a.num_sm : 148;
+    in = tiles * a.h > num_sm || p.total_tiles > 2 * num_sm ? kRaggedDraw : kRaggedFixed;
+    if (in == kRaggedDraw) grid = (int)(tiles * a.h);
   }
   cudaError_t e = cudaErrorInvalidValue;
   auto launch = [&](auto kern) {
@@ -305,27 +309,25 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
   };
   const bool bf = a.dtype == FA_BF16;
   const int cap = !(a.softcap > 0.f) ? kCapNone : (a.cu_seqlens_q && !a.cu_seqlens_k) ? kCapFine : kCapApprox;
-  auto pick = [&](auto fix_tag, auto cap_tag, auto hd_tag) {
-    constexpr bool F = decltype(fix_tag)::value;
-    constexpr int C = decltype(cap_tag)::value, HD = decltype(hd_tag)::value;
-    if (bf) launch(fwd_tc5_kernel<__nv_bfloat16, 1, F, C, HD>);
-    else launch(fwd_tc5_kernel<__half, 0, F, C, HD>);
+  auto pick = [&](auto in_tag, auto cap_tag, auto hd_tag) {
+    constexpr int I = decltype(in_tag)::value, C = decltype(cap_tag)::value, HD = decltype(hd_tag)::value;
+    if (bf) launch(fwd_tc5_kernel<__nv_bfloat16, 1, I, C, HD>);
+    else launch(fwd_tc5_kernel<__half, 0, I, C, HD>);
   };
-  auto pick_hd = [&](auto fix_tag, auto cap_tag) {
-    if (a.d <= 64) pick(fix_tag, cap_tag, std::integral_constant<int, 64>{});
-    else if (a.d <= 128) pick(fix_tag, cap_tag, std::integral_constant<int, 128>{});
-    else pick(fix_tag, cap_tag, std::integral_constant<int, 256>{});
+  auto pick_hd = [&](auto in_tag, auto cap_tag) {
+    if (a.d <= 64) pick(in_tag, cap_tag, std::integral_constant<int, 64>{});
+    else if (a.d <= 128) pick(in_tag, cap_tag, std::integral_constant<int, 128>{});
+    else pick(in_tag, cap_tag, std::integral_constant<int, 256>{});
   };
-  using None = std::integral_constant<int, kCapNone>;
-  using Approx = std::integral_constant<int, kCapApprox>;
-  if (p.fix_tail) {
-    if (cap == kCapFine) pick_hd(std::true_type{}, std::integral_constant<int, kCapFine>{});
-    else if (cap == kCapApprox) pick_hd(std::true_type{}, Approx{});
-    else pick_hd(std::true_type{}, None{});
-  } else {
-    if (cap) pick_hd(std::false_type{}, Approx{});
-    else pick_hd(std::false_type{}, None{});
-  }
+  auto pick_cap = [&](auto in_tag) {
+    constexpr int kCapped = decltype(in_tag)::value == kDense ? kCapApprox : kCapFine;  // dense queries never take the finer form
+    if (cap == kCapNone) pick_hd(in_tag, std::integral_constant<int, kCapNone>{});
+    else if (cap == kCapApprox) pick_hd(in_tag, std::integral_constant<int, kCapApprox>{});
+    else pick_hd(in_tag, std::integral_constant<int, kCapped>{});
+  };
+  if (in == kDense) pick_cap(std::integral_constant<int, kDense>{});
+  else if (in == kRaggedFixed) pick_cap(std::integral_constant<int, kRaggedFixed>{});
+  else pick_cap(std::integral_constant<int, kRaggedDraw>{});
   if (e != cudaSuccess) { *err = std::string("tcgen05 kernel launch: ") + cudaGetErrorString(e); return FA_ERR_CUDA; }
   return FA_OK;
 }

@@ -73,6 +73,9 @@ struct Geo {
   static_assert(kRingOff + kRing * kSlotBytes + kBarBytes <= kSmemBytes, "shared memory layout");
 };
 
+// Input of a kernel instance: dense, or ragged (a KV cache or packed sequences: tiles and tails differ by batch entry),
+// whose tiles are dealt out in a fixed order or drawn at run time.
+enum InputKind { kDense = 0, kRaggedFixed = 1, kRaggedDraw = 2 };
 // Softcap of a kernel instance: none, by tanh.approx, or by the finer form (packed queries against a cache; softmax role).
 enum CapKind { kCapNone = 0, kCapApprox = 1, kCapFine = 2 };
 
@@ -103,7 +106,7 @@ struct TileInfo {
   int ulo, uhi;  // union of the block ranges
 };
 
-// Tile order of dense input: the (batch, head) pairs are cut into chunks whose K / V fit in L2 together; inside a
+// Tile order of dense input (and of ragged input whose tiles are dealt out): the (batch, head) pairs are cut into chunks whose K / V fit in L2 together; inside a
 // chunk all pairs run their last (heaviest, causal) query tile first, then the one before, and so
 // on, so the K / V prefixes a chunk re-reads tile after tile come from L2 and not from HBM.  The
 // chunk length makes a chunk a whole even number of rounds of the grid (StaticWalk), which keeps the
@@ -170,7 +173,7 @@ __device__ __forceinline__ void tile_info(const Tc5Params& p, const TileId id, T
   if (ti.uhi == 0) ti.ulo = 0;
 }
 
-// Ragged input (TileDraw): the tiles a CTA has drawn, handed by the producer warp to the other roles.
+// Ragged input whose tiles are drawn (TileDraw): the tiles a CTA has drawn, handed by the producer warp to the other roles.
 constexpr int kQueue = 4;
 constexpr int kQueueReaders = 15;  // warps that read every tile
 struct TileQueue {
@@ -204,7 +207,7 @@ struct Barriers {
 };
 static_assert(sizeof(Barriers) <= kBarBytes, "barrier block does not fit");
 
-// Static tile schedule of dense input: CTA c of G takes positions c, 2G-1-c, 2G+c, 4G-1-c, ... (serpentine) of an order
+// Static tile schedule of dense input and of ragged input with few tiles: CTA c of G takes positions c, 2G-1-c, 2G+c, 4G-1-c, ... (serpentine) of an order
 // that starts with the heaviest tiles, which evens out the per-CTA sums of a decreasing sequence (causal, 4K: 1 % spread
 // instead of 6 % with a plain stride).
 struct StaticWalk {
@@ -227,6 +230,9 @@ struct StaticWalk {
 // CTA takes over the tile of one that has not started (clusterlaunchcontrol) until none is left: no counter in memory,
 // nothing to reset.  The producer warp draws and publishes the tile; the other roles read it here.  Kernel time, those
 // sequences (head dim 64) 332 -> 236 us; 4 chunks of 301 - 2048 rows against 1777 - 8192 cached keys 570 -> 508 us a call.
+// With no more tiles than SMs there is nothing to even out and the draw costs 2 - 5 us a call (its loads of the lengths,
+// the hand-over, the last request): such launches keep the fixed deal.  300 + 200 packed rows, 32 heads: 18.5 us dealt,
+// 22.5 us drawn; two chunks of 256 rows against 4096 keys 79 and 84 us.
 struct QueueWalk {
   Barriers* bar;
   uint32_t k = 0;
@@ -243,12 +249,12 @@ struct QueueWalk {
   }
   __device__ __forceinline__ int first(const Tc5Params& p) { return next(p); }
 };
-template <bool FIX>
-using TileWalk = typename std::conditional<FIX, QueueWalk, StaticWalk>::type;
+template <int IN>
+using TileWalk = typename std::conditional<IN == kRaggedDraw, QueueWalk, StaticWalk>::type;
 // The tile number that a walk gives -> tile (p.total_tiles: no more).
-template <bool FIX>
+template <int IN>
 __device__ __forceinline__ TileId tile_id(const Tc5Params& p, int n) {
-  if (!FIX) return static_tile(p, n);
+  if (IN != kRaggedDraw) return static_tile(p, n);
   const int pair = n / p.m_tiles;
   return {pair / p.a.h, pair % p.a.h, n % p.m_tiles};
 }

@@ -30,7 +30,7 @@ struct RingPos {
 // 32 consecutive entries in registers, one per lane).
 // ---------------------------------------------------------------------------------------------
 // HD (64 or 128) is the head dim: with 64 a Q / K / V tile is the first 64-column half of its 32 KiB slot only.
-template <bool FIX, int HD>
+template <int IN, int HD>
 __device__ __forceinline__ void producer_loop(const Tc5Params& p, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
                                               const CUtensorMap* tm_v, Barriers* bar, uint32_t q_smem, uint32_t kv_smem) {
   volatile int* abort_flag = &bar->abort_flag;
@@ -41,11 +41,11 @@ __device__ __forceinline__ void producer_loop(const Tc5Params& p, const CUtensor
   const int lane = threadIdx.x & 31;
   const uint64_t q_policy = l2_policy_evict_first();  // Q is read once
   const int pages_per_seq = p.a.block_table ? ceil_div(p.a.seqlen_k, p.a.page_size) : 0;  // entries per block-table row
-  using Draw = typename std::conditional<FIX, TileDraw<G::kRows>, StaticDraw>::type;
+  using Draw = typename std::conditional<IN == kRaggedDraw, TileDraw<G::kRows>, StaticDraw>::type;
   Draw draw(p, bar, lane);
   for (int n = draw.first(p); n < p.total_tiles; n = draw.next(p)) {
     TileInfo ti;
-    tile_info<G::kRows>(p, tile_id<FIX>(p, n), ti);
+    tile_info<G::kRows>(p, tile_id<IN>(p, n), ti);
     if (ti.uhi <= ti.ulo) continue;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
@@ -64,7 +64,7 @@ __device__ __forceinline__ void producer_loop(const Tc5Params& p, const CUtensor
       __syncwarp();
     }
     const int bk = varlen_k ? 0 : ti.bk;
-    if (FIX && lane == 0 && p.a.seqused_k) {  // every role clamps these silently (tile_info); this one reports them
+    if (IN != kDense && lane == 0 && p.a.seqused_k) {  // every role clamps these silently (tile_info); this one reports them
       cache_len(p.a, ti.bi, p.status);
       if (p.a.cache_batch_idx && !p.a.block_table) check_outer_index(p.a, bk, p.status);
     }
@@ -82,7 +82,7 @@ __device__ __forceinline__ void producer_loop(const Tc5Params& p, const CUtensor
           pg_reg = idx < pages_per_seq ? pages[idx] : 0;
         }
         outer = __shfl_sync(0xffffffffu, pg_reg, pg - pg_base);
-        if (FIX && lane == 0) check_outer_index(p.a, outer, p.status);  // out of range: the TMA returns zeros
+        if (IN != kDense && lane == 0) check_outer_index(p.a, outer, p.status);  // out of range: the TMA returns zeros
         row = j * kBlockN - pg * p.a.page_size;
       }
       if (!mbar_wait(smem_addr(&bar->kv_empty[slot]), par ^ 1, abort_flag, 12)) return false;
@@ -119,14 +119,14 @@ __device__ __forceinline__ bool tile_needs_tail_fix(const TileInfo& ti) {
   return ti.uhi > ti.ulo && ti.uhi * kBlockN > ti.k_len;
 }
 
-template <int HD>
+template <int IN, int HD>
 __device__ __forceinline__ void tail_fix_loop(const Tc5Params& p, Barriers* bar, uint32_t kv_smem, int lane) {
   volatile int* abort_flag = &bar->abort_flag;
   uint32_t fix_cnt = 0;  // tails cleared so far
-  TileWalk<true> walk(bar);
+  TileWalk<IN> walk(bar);
   for (int n = walk.first(p); n < p.total_tiles; n = walk.next(p)) {
     TileInfo ti;
-    tile_info<Geo<HD>::kRows>(p, tile_id<true>(p, n), ti);
+    tile_info<Geo<HD>::kRows>(p, tile_id<IN>(p, n), ti);
     if (!tile_needs_tail_fix(ti)) continue;
     if (!mbar_wait_patient(smem_addr(&bar->fix_req), fix_cnt & 1, abort_flag, 51)) return;
     ++fix_cnt;
@@ -153,9 +153,10 @@ __device__ __forceinline__ void tail_fix_loop(const Tc5Params& p, Barriers* bar,
 // threads to have copied S_t into registers, so it runs under this block's exponentials.
 // A K / V slot is released by two arrivals: one per sub-tile, or both from the only user.
 // ---------------------------------------------------------------------------------------------
-template <uint32_t AB_FMT, bool FIX, int HD>
+template <uint32_t AB_FMT, int IN, int HD>
 __device__ __forceinline__ void mma_loop(const Tc5Params& p, Barriers* bar, uint32_t q_smem, uint32_t p_smem,
                                          uint32_t kv_smem, uint32_t tmem, const int t) {
+  constexpr bool FIX = IN != kDense;
   volatile int* abort_flag = &bar->abort_flag;
   constexpr uint32_t idesc_qk = make_idesc(AB_FMT, kBlockM, kBlockN, 0);
   constexpr uint32_t idesc_pv = make_idesc(AB_FMT, kBlockM, HD, 1);
@@ -193,10 +194,10 @@ __device__ __forceinline__ void mma_loop(const Tc5Params& p, Barriers* bar, uint
     return mbar_wait(smem_addr(&bar->v_fixed), n & 1, abort_flag, 22);
   };
 
-  TileWalk<FIX> walk(bar);
+  TileWalk<IN> walk(bar);
   for (int n = walk.first(p); n < p.total_tiles; n = walk.next(p)) {
     TileInfo ti;
-    tile_info<G::kRows>(p, tile_id<FIX>(p, n), ti);
+    tile_info<G::kRows>(p, tile_id<IN>(p, n), ti);
     if (ti.uhi <= ti.ulo) continue;
     if (ti.has[t]) {
       if (!mbar_wait(smem_addr(&bar->q_full[t]), q_cnt & 1, abort_flag, 13)) return;

@@ -114,7 +114,7 @@ __device__ __forceinline__ void chunk_softcap_fine(uint32_t (&a)[32], float mul,
   }
 }
 
-template <typename T, bool FIX, int CAP, int ROWS>
+template <typename T, int IN, int CAP, int ROWS>
 __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, uint32_t tmem, uint32_t p_smem, int t,
                                              int warp_in_wg, int lane) {
   volatile int* abort_flag = &bar->abort_flag;
@@ -132,10 +132,10 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
   const float lse_scale = CAP ? 0.6931471805599453f : p.a.softmax_scale;  // running maximum -> natural log
   const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
 
-  TileWalk<FIX> walk(bar);
+  TileWalk<IN> walk(bar);
   for (int n = walk.first(p); n < p.total_tiles; n = walk.next(p)) {
     TileInfo ti;
-    tile_info<ROWS>(p, tile_id<FIX>(p, n), ti);
+    tile_info<ROWS>(p, tile_id<IN>(p, n), ti);
     if (ti.row0[t] >= ti.q_len) continue;
     const int i = ti.row0[t] + row;
     if (!ti.has[t]) {  // no visible key for the whole sub-tile: O = 0, LSE = +inf
@@ -279,7 +279,7 @@ __device__ __forceinline__ void rescale_o(uint32_t o_tmem, float f) {
   tmem_wait_st();
 }
 
-template <typename T, bool FIX, int HD>
+template <typename T, int IN, int HD>
 __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* bar, uint32_t tmem, int warp_in_wg,
                                                 int lane) {
   volatile int* abort_flag = &bar->abort_flag;
@@ -288,10 +288,10 @@ __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* ba
   uint32_t cr_cnt[2] = {0, 0}, od_cnt[2] = {0, 0}, st_cnt[2] = {0, 0};
   const int d_cols = p.a.d;
 
-  TileWalk<FIX> walk(bar);
+  TileWalk<IN> walk(bar);
   for (int n = walk.first(p); n < p.total_tiles; n = walk.next(p)) {
     TileInfo ti;
-    tile_info<Geo<HD>::kRows>(p, tile_id<FIX>(p, n), ti);
+    tile_info<Geo<HD>::kRows>(p, tile_id<IN>(p, n), ti);
     if (ti.uhi <= ti.ulo) continue;
     for (int j = ti.ulo; j < ti.uhi; ++j) {
 #pragma unroll

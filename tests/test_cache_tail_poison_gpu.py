@@ -200,3 +200,34 @@ def test_packed_backward_of_wide_heads_does_not_see_its_neighbours(d, dtype, cau
 @pytest.mark.parametrize("d,dtype,causal", [(64, FP, True), (128, BF, False), (128, BF, True)])
 def test_packed_backward_does_not_see_its_neighbours(d, dtype, causal, poison):
     _poisoned_backward(d, dtype, causal, poison)
+
+
+@pytest.mark.parametrize("h", [24, 25, 32])
+@pytest.mark.parametrize("layout,d", [("contiguous", 64), ("page128", 128), ("batch_idx", 256)])
+def test_tcgen05_prefill_ignores_the_cache_tail_on_both_sides_of_the_tile_draw(layout, d, h):
+    """144, 150 and 192 tiles (256 columns: twice as many) on 148 SMs: dealt out in a fixed order or drawn at run time."""
+    g = torch.Generator().manual_seed(4600 + h + d)
+    b, s_q, s_cache = 6, 200, 1024
+    lens = torch.tensor([333, 1024, 77, 0, 640, 1000], dtype=torch.int32)
+    kc, vc, bt, idx = _poisoned_cache(g, BF, b, s_cache, 1, d, lens, 0, 128 if layout == "page128" else 0, extra_rows=3 if layout == "batch_idx" else 0)
+    q = U.normal((b, s_q, h, d), BF, g)
+    _check(q, kc, vc, None, None, lens, bt, idx, L.KERNEL_TCGEN05, f"tcgen05 {layout} h={h}")
+
+
+@pytest.mark.parametrize("h", [4, 64])
+def test_packed_forward_does_not_see_its_neighbours_on_both_sides_of_the_tile_draw(h):
+    g = torch.Generator().manual_seed(4700 + h)
+    hk, d, n = h // 2, 128, [200, 130, 300, 1, 257]
+    cu = torch.tensor([0] + list(torch.tensor(n).cumsum(0)), dtype=torch.int32)
+    q, k, v = U.normal((sum(n), h, d), BF, g), U.normal((sum(n), hk, d), BF, g), U.normal((sum(n), hk, d), BF, g)
+    for s in (1, 3):
+        k[cu[s]:cu[s + 1]] = NAN
+        v[cu[s]:cu[s + 1]] = NAN
+    go, gl = OA.flash_attn_varlen_func(q, k, v, cu, cu, max(n), max(n), causal=True)
+    out, lse, plan = ops.attention_forward(q.cuda(), k.cuda(), v.cuda(), cu_seqlens_q=cu.cuda(), cu_seqlens_k=cu.cuda(), max_seqlen_q=max(n),
+                                           max_seqlen_k=max(n), softmax_scale=d ** -0.5, causal=True, return_plan=True)
+    assert plan.kernel == L.KERNEL_TCGEN05
+    for s in (0, 2, 4):
+        rows = slice(int(cu[s]), int(cu[s + 1]))
+        assert torch.isfinite(out[rows].float()).all(), f"sequence {s} picked up its neighbour's NaN"
+        U.check_rules(out[rows], lse[:, rows], go[rows], gl[:, rows], tag=f"packed seq {s}")
