@@ -281,11 +281,16 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
     persistent = can_persist && !window_bound;
     if (can_persist && window_bound) {
       // Nearly equal units: the balance only pays where the plain grid's last wave is nearly empty.  In KV blocks, a
-      // CTA's fixed part and the merge being worth 512 keys each (as above).
+      // CTA's fixed part and the merge being worth 512 keys each (as above).  One wave has no last wave to fill (one
+      // sequence, 8 query heads, window 1024: plain 15.4 us, shared 27.6 - 34.8), and with tiles below 128 columns the
+      // plain grid is the better one at any size (64 columns, 56 sequences of 8 kv heads, window 4096: 98 / 140 us; 96
+      // columns, 80 sequences: 216 / 296).  Inside these limits shared / plain is 0.86 .. 1.02 (2 .. 7 waves, 128 - 256
+      // columns; 40 sequences of 8 kv heads, head dim 128, window 1024: 64.5 -> 56.3 us).
       const double fixed = 512.0 / ci.block_n;
-      const double plain = (double)((base * ns + persist_grid - 1) / persist_grid) * (ceil_div(max_blocks, ns) + fixed);
+      const long long waves = (base * ns + persist_grid - 1) / persist_grid;
+      const double plain = (double)waves * (ceil_div(max_blocks, ns) + fixed);
       const double shared = (double)base * (max_blocks + fixed) / persist_grid + fixed;
-      persistent = shared < 0.85 * plain;
+      persistent = waves >= 2 && a.d >= 128 && shared < 0.85 * plain;
     }
     if (const char* e = std::getenv("FA_B200_DECODE_PERSISTENT"))  // tuning override: 0 off, 1 ragged ranges only, 2 wherever possible
       persistent = can_persist && (std::atoi(e) == 2 || (std::atoi(e) == 1 && !window_bound));

@@ -164,6 +164,18 @@ def test_plan_persistent_decode_for_ragged_lengths_only():
     assert rc == 0 and pl.kernel == L.KERNEL_DECODE and pl.grid % (64 * 8) == 0  # plain grid: units x splits
 
 
+@pytest.mark.parametrize("b,h,hk,d,shared", [(40, 32, 8, 128, True), (40, 32, 8, 256, True), (1, 8, 1, 128, False), (4, 8, 1, 256, False),
+                                             (20, 32, 8, 128, False), (40, 32, 8, 64, False), (40, 32, 8, 96, False)])
+def test_plan_window_bound_decode_shares_blocks_only_to_fill_a_last_wave(b, h, hk, d, shared):
+    """Nearly equal units (a sliding window) keep the plain grid while that is one wave, and for tiles below 128 columns."""
+    rc, pl = _plan(_params(b=b, h=h, h_k=hk, d=d, seqlen_k=32768, total_q=b, seqused_k=256, causal=1, window_left=1024, window_right=0,
+                           q_batch_stride=h * d, q_row_stride=h * d, q_head_stride=d, lse_batch_stride=h, lse_head_stride=1,
+                           k_batch_stride=32768 * hk * d, k_row_stride=hk * d, k_head_stride=d,
+                           v_batch_stride=32768 * hk * d, v_row_stride=hk * d, v_head_stride=d))
+    assert rc == 0 and pl.kernel == L.KERNEL_DECODE and pl.is_local
+    assert (pl.blocks_per_split == 0) == shared
+
+
 def test_plan_32_row_decode_configuration_follows_the_key_range():
     """17-32 packed rows: short key ranges (a sliding window) run two resident CTAs of 2x2 consumer warps with
     64-key blocks (one launch, no partials); long ranges and ragged launches that become persistent keep the
