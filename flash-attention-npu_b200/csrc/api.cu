@@ -272,12 +272,18 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
     const long long resident = std::max(1, (227 * 1024) / std::max(1, ci.smem_bytes));
     persist_grid = (long long)num_sm * resident;
     if (const char* e = std::getenv("FA_B200_DECODE_PERSISTENT_GRID")) persist_grid = std::max(1, std::atoi(e));  // tuning override
-    // (a unit cut into grid / base shares touches up to two CTAs more than whole shares)
-    persist_slots = persist_grid / base > 3 ? (int)(persist_grid / base + 2) : kMinPersistSlots;
-    // Worth a merge launch when the units do not fill the grid by themselves or are many: at least 8 blocks a unit
-    // (below that a CTA per unit finishes in the time a merge takes), or four blocks for every CTA of the grid.
+    // (a unit cut into grid / base shares touches up to two CTAs more than whole shares.)  A share is two blocks at
+    // least: the merge reads every slot (one sequence, one kv head, 1560 keys: 298 slots 28.7 us, 14 slots 18).
+    if (persist_grid / base > 3)
+      persist_slots = (int)std::max<long long>(kMinPersistSlots, std::min(persist_grid / base + 2, (long long)max_blocks / 2 + 1));
+    // Worth a merge launch when the units do not fill the grid by themselves or are many: at least 896 keys a unit (below
+    // that a CTA per unit finishes in the time a merge takes: 104 units of 654 keys 22.5 us plain, 25.6 shared; 16 units of
+    // 909 keys 28.6 and 20.7), 512 for the fewest units (16 units of 642 keys 22.5 and 18.5), 1536 for more than 16 rows,
+    // whose merge takes longer; or four blocks for every CTA of the grid.
+    const long long least_keys = ci.block_m > 16 ? 1536 : base * 16 <= persist_grid ? 512 : 896;
+    const bool long_units = max_blocks >= 8 && max_blocks * (long long)ci.block_n >= least_keys;
     const bool can_persist = (a.seqused_k != nullptr || window_bound) && !decode_one_segment_only &&
-                             (max_blocks >= 8 || base * max_blocks >= 4 * persist_grid) && base * (max_blocks + 1) < 0x3fffffffLL;
+                             (long_units || base * max_blocks >= 4 * persist_grid) && base * (max_blocks + 1) < 0x3fffffffLL;
     persistent = can_persist && !window_bound;
     if (can_persist && window_bound) {
       // Nearly equal units: the balance only pays where the plain grid's last wave is nearly empty.  In KV blocks, a

@@ -176,6 +176,19 @@ def test_plan_window_bound_decode_shares_blocks_only_to_fill_a_last_wave(b, h, h
     assert (pl.blocks_per_split == 0) == shared
 
 
+@pytest.mark.parametrize("b,h,hk,d,keys,slots", [(1, 32, 8, 128, 2048, 17), (1, 8, 1, 128, 1600, 13), (13, 64, 8, 128, 654, 0), (2, 16, 8, 128, 900, 8),
+                                                 (1, 8, 1, 128, 131072, 298), (64, 32, 8, 128, 654, 4), (1, 4, 4, 256, 800, 7), (11, 4, 4, 256, 800, 0),
+                                                 (3, 4, 4, 128, 512, 5)])
+def test_plan_decode_partials_follow_the_key_range(b, h, hk, d, keys, slots):
+    """Units are shared by CTAs from 896 keys on (512 when they are fewest, or when they are many), with at most one partial per two key blocks."""
+    rc, pl = _plan(_params(b=b, h=h, h_k=hk, d=d, seqlen_k=keys, total_q=b, seqused_k=256, causal=1,
+                           q_batch_stride=h * d, q_row_stride=h * d, q_head_stride=d, lse_batch_stride=h, lse_head_stride=1,
+                           k_batch_stride=keys * hk * d, k_row_stride=hk * d, k_head_stride=d,
+                           v_batch_stride=keys * hk * d, v_row_stride=hk * d, v_head_stride=d))
+    assert rc == 0 and pl.kernel == L.KERNEL_DECODE
+    assert (pl.num_splits if pl.blocks_per_split == 0 else 0) == slots
+
+
 def test_plan_32_row_decode_configuration_follows_the_key_range():
     """17-32 packed rows: short key ranges (a sliding window) run two resident CTAs of 2x2 consumer warps with
     64-key blocks (one launch, no partials); long ranges and ragged launches that become persistent keep the
