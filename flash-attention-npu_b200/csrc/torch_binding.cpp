@@ -26,6 +26,7 @@
 #include <torch/csrc/autograd/variable.h>
 
 #include <cstring>
+#include <exception>
 
 #include "fa_b200.h"
 
@@ -184,10 +185,20 @@ struct NoGil {  // a launch blocks when the queue is full: other Python threads 
   }
 };
 
+struct Scratch {
+  c10::Device device;
+  Tensor tensor;
+  std::exception_ptr error;  // out of memory: kept out of the C entry point the callback runs under
+};
 void* alloc_workspace(size_t bytes, void* ctx) {  // from torch's caching allocator, in the order of the current stream
-  auto* slot = static_cast<std::pair<Tensor, c10::Device>*>(ctx);
-  slot->first = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(slot->second));
-  return slot->first.data_ptr();
+  auto* s = static_cast<Scratch*>(ctx);
+  try {
+    s->tensor = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(s->device));
+    return s->tensor.data_ptr();
+  } catch (...) {
+    s->error = std::current_exception();
+    return nullptr;
+  }
 }
 
 // Allocates the outputs and launches; false: the library refused the call (the Python path repeats it for the message).
@@ -207,10 +218,12 @@ bool launch_forward(const FwdArgs& a, fa_fwd_params& p, Tensor& out, Tensor& lse
   }
   p.o = out.data_ptr();
   p.lse = (float*)lse.data_ptr();
-  std::pair<Tensor, c10::Device> ws(Tensor(), q.device());
+  Scratch ws{q.device(), Tensor(), nullptr};
   void* stream = at::cuda::getCurrentCUDAStream(q.device().index()).stream();
   NoGil nogil;
-  return fa_b200_fwd_alloc(&p, a.plan, (size_t)a.plan_bytes, alloc_workspace, &ws, stream) == FA_OK;
+  const int rc = fa_b200_fwd_alloc(&p, a.plan, (size_t)a.plan_bytes, alloc_workspace, &ws, stream);
+  if (ws.error) std::rethrow_exception(ws.error);
+  return rc == FA_OK;
 }
 
 // ------------------------------------------------------------------------------------------------ backward

@@ -48,3 +48,23 @@ def test_kvcache_call_on_inputs_that_require_grad():
         out.sum().backward()
     with torch.no_grad():
         assert torch.equal(fa3.flash_attn_with_kvcache(q, k, v, causal=True), out)
+
+
+def test_workspace_that_does_not_fit_is_an_out_of_memory_error():
+    """The partials of a split call are allocated through a callback of the C library; its failure is torch's own error."""
+    import flash_attn_npu_v2 as fa2
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q = torch.randn((16, 4, 64, 128), generator=g, device="cuda", dtype=BF)  # 64 splits: 135 MB of partials
+    k, v = (torch.randn((16, 8192, 8, 128), generator=g, device="cuda", dtype=BF) for _ in range(2))
+    lens = torch.full((16,), 8192, dtype=torch.int32, device="cuda")
+    call = lambda: fa2.flash_attn_with_kvcache(q, k, v, cache_seqlens=lens, causal=True, num_splits=64)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (60 << 20)) / total)
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            call()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.isfinite(call().float()).all()
