@@ -129,9 +129,10 @@ __device__ __forceinline__ void ew_pair(const bool poly, uint32_t s0, uint32_t s
 // Work items are handed out dynamically: the producer warp draws the next item number from a global counter and
 // publishes it to the other roles of its CTA through a small ring in shared memory (slot k % 8 for the CTA's k-th
 // published item, -1 = no more items).  Items without work (keys nobody sees, rows that see no key) are not
-// published: the producer warp writes their zeros itself.  The ring needs no "empty" barrier: for items with work the
-// producer cannot be more than two items ahead of any other role (it waits for the previous item's last read of the
-// resident tiles, the issuing warps wait for the epilogue of the item before that), and the ring has eight slots.
+// published: the producer warp writes their zeros itself.  The ring needs no "empty" barrier: the producer publishes item
+// n + 1 after the last S of item n - 1, and with items of one block or unit that S has waited for the elementwise warps in
+// item n - 2 or n - 3 and those for the accumulating issuer one item behind; so it is at most five items ahead of any
+// other role, and the ring has eight slots.
 constexpr int kQueue = 8;
 struct ItemQueue {
   uint64_t full[kQueue];

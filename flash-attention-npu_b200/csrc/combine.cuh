@@ -33,8 +33,7 @@ __device__ __forceinline__ void store4<__half>(__half* dst, float4 v) {
 
 // One row's merge weights for n <= 32 partials, one partial per lane: lane i loads LSE_i (one round trip for all of
 // them instead of a chain of dependent loads), the maximum and the sum go through the warp.  Returns this lane's LSE
-// and weight exp(LSE_i - m) / sum; m, tot and dead are the row's.  The arithmetic and its order are those of the
-// sequential form below (lane i contributes term i, the same xor tree adds them up).
+// and weight exp(LSE_i - m) / sum; m, tot and dead are the row's.
 template <typename LoadLse>
 __device__ __forceinline__ void merge_weights(int n, int lane, LoadLse lse_of, float& l_mine, float& w_mine, float& m, float& tot,
                                               bool& dead) {

@@ -130,7 +130,7 @@ typedef struct fa_fwd_plan {
   int32_t m_blocks;
   int32_t num_splits;   /* KV splits launched (1 = none) */
   int32_t blocks_per_split;
-  int32_t grid, threads, smem_bytes;
+  int32_t grid, threads, smem_bytes; /* grid: of the tcgen05 kernel's fixed deal; ragged input with more tiles than SMs launches a CTA per tile */
   int32_t is_causal, is_local, window_left, window_right; /* after host normalisation */
   int32_t launches;     /* kernel launches fa_b200_fwd will make */
   size_t workspace_bytes;
@@ -230,7 +230,7 @@ typedef struct fa_bwd_params {
   float softmax_scale;
   float softcap; /* 0 = off */
   int32_t total_k; /* rows of k / v for packed input (the tcgen05 kernels' TMA bounds); 0 = not given */
-  int32_t kernel;  /* 0 automatic; 1 force the mma.sync kernel; 2 force the tcgen05 kernels (FA_ERR_UNSUPPORTED if they do not cover the problem) */
+  int32_t kernel;  /* 0 automatic; 1 force the mma.sync kernel; 2 force the tcgen05 kernels of head dims up to 128 (FA_ERR_UNSUPPORTED if they do not cover the problem) */
 } fa_bwd_params;
 
 /* Bytes of device scratch fa_b200_bwd needs: rowsum(dO o O), plus the fp32 dQ accumulator where the mma.sync kernel runs
