@@ -125,9 +125,13 @@ int fa_b200_bwd(const fa_bwd_params* a, void* workspace, size_t workspace_bytes,
   if (!tc5 && !wide) e = cudaMemsetAsync(p.dq_accum, 0, acc_bytes, cs);
   if (e != cudaSuccess) return fail_bwd(FA_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
   const bool bf = a->dtype == FA_BF16;
-  const int delta_grid = (int)((rows * a->h + 7) / 8);  // 4 warps x 2 rows per block
-  if (bf) bwd_delta_kernel<__nv_bfloat16><<<delta_grid, 128, 0, cs>>>(p);
-  else bwd_delta_kernel<__half><<<delta_grid, 128, 0, cs>>>(p);
+  auto launch_delta = [&](auto kern, int lanes) {
+    const int64_t per_block = kDeltaThreads / lanes * kDeltaRows, n_rows = varlen ? rows : a->seqlen_q;
+    const int64_t grid = (n_rows + per_block - 1) / per_block * a->h * (varlen ? 1 : a->b);
+    kern<<<(unsigned)grid, kDeltaThreads, 0, cs>>>(p);
+  };
+  if (a->d <= 64) bf ? launch_delta(bwd_delta_kernel<__nv_bfloat16, 8>, 8) : launch_delta(bwd_delta_kernel<__half, 8>, 8);
+  else bf ? launch_delta(bwd_delta_kernel<__nv_bfloat16, 16>, 16) : launch_delta(bwd_delta_kernel<__half, 16>, 16);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail_bwd(FA_ERR_CUDA, std::string("backward (delta) launch: ") + cudaGetErrorString(e));
   if (tc5 || wide) {

@@ -55,36 +55,49 @@ struct BwdSmem {
   static constexpr int BYTES = DELTA_OFF + 64 * 4;
 };
 
-// D_i = sum_d dO_id * O_id.  Half a warp per (row, head): 16 lanes x 16 bytes cover 128 columns per step, so a row of
-// O and of dO is one 256-byte transaction each (the head dim is a multiple of 8, rows are 16-byte aligned).
-template <typename T>
-__global__ void __launch_bounds__(128) bwd_delta_kernel(const __grid_constant__ BwdParams p) {
-  const int lane = threadIdx.x & 31, l16 = lane & 15;
-  const int64_t idx = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 2 + (lane >> 4);
-  const bool varlen = p.cu_seqlens_q != nullptr;
-  const int64_t rows = varlen ? p.total_q : (int64_t)p.b * p.seqlen_q;
-  const bool live = idx < rows * p.h;
-  const int head = live ? (int)(idx % p.h) : 0;
-  const int64_t row = live ? idx / p.h : 0;
-  const int bi = varlen ? 0 : (int)(row / p.seqlen_q);
-  const int64_t i = varlen ? row : row % p.seqlen_q;
-  const T* o = reinterpret_cast<const T*>(p.o) + bi * p.o_batch_stride + i * p.o_row_stride + head * p.o_head_stride;
-  const T* g = reinterpret_cast<const T*>(p.dout) + bi * p.do_batch_stride + i * p.do_row_stride + head * p.do_head_stride;
-  float acc = 0.f;
-  if (live) {
-    for (int c = l16 * 8; c < p.d; c += 128) {
-      Vec16 a, b;
-      a.u = *reinterpret_cast<const uint4*>(o + c);
-      b.u = *reinterpret_cast<const uint4*>(g + c);
-      const T* av = reinterpret_cast<const T*>(&a);
-      const T* bv = reinterpret_cast<const T*>(&b);
+// D_i = sum_d dO_id * O_id.  Bound by memory: O and dO are read once.  LANES lanes per (row, head), 16 bytes of O and of dO
+// each per 8 * LANES columns (the head dim is a multiple of 8, rows are 16-byte aligned); a group of lanes takes kDeltaRows
+// rows of one head and asks for all of them before it adds anything up.  The rows of a block are consecutive, so the results
+// are written in whole sectors; the heads of the same rows are neighbours in the grid, so the 2 * d bytes of a row and head
+// come from open DRAM pages.  One division per block (a 64-bit one per row and two loads in flight per lane before).
+// b 4, s 4096, 32 heads, d 128 (268 MB read): 87 -> 48 us; 18 K packed rows, 16 heads, d 64 (75 MB): 38 -> 15 us.
+constexpr int kDeltaThreads = 256, kDeltaRows = 4;
+template <typename T, int LANES>
+__global__ void __launch_bounds__(kDeltaThreads) bwd_delta_kernel(const __grid_constant__ BwdParams p) {
+  constexpr int kGroups = kDeltaThreads / LANES;
+  const int lane = threadIdx.x % LANES, grp = threadIdx.x / LANES;
+  const int rows = p.cu_seqlens_q ? p.total_q : p.seqlen_q;  // of one batch entry; packed input is one long entry
+  const int blocks = ceil_div(rows, kGroups * kDeltaRows);
+  const int head = blockIdx.x % p.h, n = blockIdx.x / p.h;
+  const int bi = n / blocks, row0 = (n - bi * blocks) * kGroups * kDeltaRows + grp;
+  const T* o = reinterpret_cast<const T*>(p.o) + bi * p.o_batch_stride + head * p.o_head_stride;
+  const T* g = reinterpret_cast<const T*>(p.dout) + bi * p.do_batch_stride + head * p.do_head_stride;
+  float acc[kDeltaRows];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc += to_f32<T>(av[e]) * to_f32<T>(bv[e]);
+  for (int r = 0; r < kDeltaRows; ++r) acc[r] = 0.f;
+  for (int c = lane * 8; c < p.d; c += 8 * LANES) {
+    Vec16 a[kDeltaRows], b[kDeltaRows];
+#pragma unroll
+    for (int r = 0; r < kDeltaRows; ++r) {
+      const int64_t i = min(row0 + r * kGroups, rows - 1);  // (past the end: the last row again, not stored)
+      a[r].u = __ldcs(reinterpret_cast<const uint4*>(o + i * p.o_row_stride + c));
+      b[r].u = *reinterpret_cast<const uint4*>(g + i * p.do_row_stride + c);
+    }
+#pragma unroll
+    for (int r = 0; r < kDeltaRows; ++r) {
+      const T* av = reinterpret_cast<const T*>(&a[r]);
+      const T* bv = reinterpret_cast<const T*>(&b[r]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[r] += to_f32<T>(av[e]) * to_f32<T>(bv[e]);
     }
   }
 #pragma unroll
-  for (int s = 8; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-  if (live && l16 == 0) p.delta[bi * p.lse_batch_stride + head * p.lse_head_stride + i] = acc;
+  for (int r = 0; r < kDeltaRows; ++r) {
+#pragma unroll
+    for (int s = LANES / 2; s > 0; s >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], s);
+    const int i = row0 + r * kGroups;
+    if (lane == 0 && i < rows) p.delta[bi * p.lse_batch_stride + head * p.lse_head_stride + i] = acc[r];
+  }
 }
 
 // fp32 dQ accumulator -> dq in the output dtype.
