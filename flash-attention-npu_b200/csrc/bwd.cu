@@ -19,6 +19,14 @@ void count_launches(int n);                      // api.cu: fa_b200_launch_count
 
 static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
+// Pairs per chunk of the work-item order (item_place in tile_order.cuh): all of them when what they stream (two 16-bit
+// tensors of `rows` rows and `heads` heads) stays in L2 together, otherwise one (the 4 K causal case, 268 MB, in chunks of ten
+// pairs: dK / dV kernel 917 -> 1017 us).  Only a causal mask makes the blocks of a pair unequal; without one a pair at a time.
+static int bwd_chunk(bool causal, int pairs, int64_t rows, int heads, int d) {
+  constexpr int64_t kL2Budget = 96ll << 20;
+  return causal && 4 * rows * heads * d <= kL2Budget ? pairs : 1;
+}
+
 template <int HD, typename T>
 static cudaError_t launch_bwd(const BwdParams& p, int n_kblocks, cudaStream_t st) {
   constexpr int smem = BwdSmem<HD>::BYTES;
@@ -112,6 +120,11 @@ int fa_b200_bwd(const fa_bwd_params* a, void* workspace, size_t workspace_bytes,
   p.softmax_scale = a->softmax_scale;
   p.scale_log2 = a->softmax_scale * kLog2e;
   p.softcap = a->softcap;
+  {
+    const int64_t k_rows = varlen ? a->total_k : (int64_t)a->b * a->seqlen_k;
+    p.chunk_kv = bwd_chunk(p.is_causal, a->h_k * a->b, rows, a->h, a->d);
+    p.chunk_q = bwd_chunk(p.is_causal, a->h * a->b, k_rows, a->h_k, a->d);
+  }
   const size_t acc_bytes = bwd_accum_bytes(a, rows);
   p.dq_accum = reinterpret_cast<float*>(workspace);
   p.delta = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + acc_bytes);

@@ -36,6 +36,7 @@
 
 #include "bwd_kernel.cuh"
 #include "tc5_ptx.cuh"
+#include "tile_order.cuh"
 
 namespace fa {
 namespace btc5 {
@@ -246,10 +247,9 @@ struct BarA {
 };
 static_assert(sizeof(BarA) <= kBarBytes, "barrier block does not fit");
 
-// Work item t of the dK / dV kernel: 128 keys of one (kv head, batch entry).  The key blocks of a pair are
-// neighbours in the order, so the CTAs running at one time stream the same few heads' Q / dO and find them in L2
-// (with one key block index across all pairs at a time every item read its Q / dO from HBM: 2.3 ms against 1.8 on the
-// 4 K causal case); block 0 first: under a causal mask it has the most work, and the launch ends on light items.
+// Work item t of the dK / dV kernel: 128 keys of one (kv head, batch entry).  The order (item_place) keeps few heads in flight, so that
+// their Q / dO come from L2 (with one key block index across all 128 pairs at a time every item read its Q / dO from HBM:
+// 2.3 ms against 1.8 on the 4 K causal case); block 0 first: under a causal mask it has the most work.
 struct ItemA {
   SeqInfo sq;
   int hk, bi, key0, u_lo, nu, iters;  // iters = units x query heads of the group; 0 = nobody sees the keys
@@ -258,11 +258,11 @@ struct ItemA {
 __device__ __forceinline__ ItemA item_a(const BwdParams& p, int t) {
   ItemA w;
   const int n_kblocks = ceil_div(p.seqlen_k, kBlk);
-  const int pair = t / n_kblocks, nb = t - pair * n_kblocks;
-  w.hk = pair % p.h_k;
-  w.bi = pair / p.h_k;
+  const ItemPlace at = item_place(t, n_kblocks, p.h_k * p.b, p.chunk_kv);
+  w.hk = at.pair % p.h_k;
+  w.bi = at.pair / p.h_k;
   w.sq = seq_info(p, w.bi);
-  w.key0 = nb * kBlk;
+  w.key0 = at.block * kBlk;
   w.live = w.key0 < w.sq.k_len;
   w.u_lo = w.nu = w.iters = 0;
   if (w.live) {
@@ -585,8 +585,8 @@ struct BarB {
 };
 static_assert(sizeof(BarB) <= kBarBytes, "barrier block does not fit");
 
-// Work item t of the dQ kernel: 128 query rows of one (head, batch entry); the query blocks of a pair are neighbours
-// in the order (they stream the same K / V), the last one (under a causal mask: the heaviest) first.
+// Work item t of the dQ kernel: 128 query rows of one (head, batch entry); the last block (under a causal mask: the
+// heaviest) first.
 struct ItemB {
   SeqInfo sq;
   int head, hk, bi, row0, j_lo, iters;  // iters = key blocks; 0 = the rows see no key
@@ -595,12 +595,12 @@ struct ItemB {
 __device__ __forceinline__ ItemB item_b(const BwdParams& p, int t) {
   ItemB w;
   const int m_blocks = ceil_div(p.seqlen_q, kBlk);
-  const int pair = t / m_blocks, mi = t - pair * m_blocks;
-  w.head = pair % p.h;
-  w.bi = pair / p.h;
+  const ItemPlace at = item_place(t, m_blocks, p.h * p.b, p.chunk_q);
+  w.head = at.pair % p.h;
+  w.bi = at.pair / p.h;
   w.hk = w.head / (p.h / p.h_k);
   w.sq = seq_info(p, w.bi);
-  w.row0 = (m_blocks - 1 - mi) * kBlk;
+  w.row0 = (m_blocks - 1 - at.block) * kBlk;
   w.live = w.row0 < w.sq.q_len;
   w.j_lo = w.iters = 0;
   if (w.live) {

@@ -84,8 +84,8 @@ struct ItemW {
   int kind, head, hk, bi, row0, u_lo, nu, iters;  // head: dQ only; row0: first resident row (key or query row); iters = 0: nothing visible
   bool live;                                      // false: the sequence has no such rows
 };
-// Items: all dK, then all dV, then all dQ (with grouped heads the smallest ones come last).  Inside a kind a pair's blocks
-// are neighbours (they stream the same tiles from L2), its heaviest under a causal mask first.
+// Items: all dK, then all dV, then all dQ (with grouped heads the smallest ones come last).  Inside a kind in the order of
+// item_place, the heaviest block under a causal mask first.
 __device__ __forceinline__ ItemW item_w(const BwdParams& p, int t) {
   ItemW w;
   const int n_kblocks = ceil_div(p.seqlen_k, kBlk), n_kv = n_kblocks * p.h_k * p.b;
@@ -93,12 +93,12 @@ __device__ __forceinline__ ItemW item_w(const BwdParams& p, int t) {
   if (t < 2 * n_kv) {
     w.kind = t < n_kv ? kWideDK : kWideDV;
     if (t >= n_kv) t -= n_kv;
-    const int pair = t / n_kblocks;
-    w.hk = pair % p.h_k;
-    w.bi = pair / p.h_k;
+    const ItemPlace at = item_place(t, n_kblocks, p.h_k * p.b, p.chunk_kv);
+    w.hk = at.pair % p.h_k;
+    w.bi = at.pair / p.h_k;
     w.head = 0;
     w.sq = seq_info(p, w.bi);
-    w.row0 = (t - pair * n_kblocks) * kBlk;
+    w.row0 = at.block * kBlk;
     w.live = w.row0 < w.sq.k_len;
     if (w.live) {  // query rows that see at least one key of the block
       const int k1 = min(w.sq.k_len, w.row0 + kBlk) - 1;
@@ -112,12 +112,12 @@ __device__ __forceinline__ ItemW item_w(const BwdParams& p, int t) {
     w.kind = kWideDQ;
     t -= 2 * n_kv;
     const int m_blocks = ceil_div(p.seqlen_q, kBlk);
-    const int pair = t / m_blocks;
-    w.head = pair % p.h;
-    w.bi = pair / p.h;
+    const ItemPlace at = item_place(t, m_blocks, p.h * p.b, p.chunk_q);
+    w.head = at.pair % p.h;
+    w.bi = at.pair / p.h;
     w.hk = w.head / (p.h / p.h_k);
     w.sq = seq_info(p, w.bi);
-    w.row0 = (m_blocks - 1 - (t - pair * m_blocks)) * kBlk;
+    w.row0 = (m_blocks - 1 - at.block) * kBlk;
     w.live = w.row0 < w.sq.q_len;
     if (w.live) {  // keys that at least one row of the block sees
       const int r1 = min(w.sq.q_len, w.row0 + kBlk) - 1;
