@@ -214,6 +214,30 @@ __device__ __forceinline__ void store_slice(T* dst, const uint32_t (&a)[32], int
   }
 }
 
+// LSE and D of the 64 query rows of a unit, two rows per lane.  The producer warp asks for those of the next unit before it
+// waits for the ring, so that a unit does not cost it a round trip to memory: with the loads behind the wait the dK / dV kernel
+// was bound by its producer for head dim 64 (12 packed sequences of 37 - 2999 rows, 16 heads of 4 groups: 272 -> 217 us).
+struct UnitStats {
+  float lse[2], delta[2];
+  __device__ __forceinline__ void ask(const BwdParams& p, const SeqInfo& sq, int head, int row0, bool with_delta, int lane) {
+    const int64_t base = (int64_t)sq.bq * p.lse_batch_stride + (int64_t)head * p.lse_head_stride + sq.q_row0;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int i = row0 + lane + 32 * e;
+      const bool valid = i < sq.q_len;
+      lse[e] = valid ? p.lse[base + i] : INFINITY;  // rows beyond the sequence: P = 0
+      delta[e] = valid && with_delta ? p.delta[base + i] : 0.f;
+    }
+  }
+  __device__ __forceinline__ void put(float* nlse2, float* ndls, float scale, int lane) const {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      nlse2[lane + 32 * e] = -lse[e] * kLog2e;
+      ndls[lane + 32 * e] = -delta[e] * scale;
+    }
+  }
+};
+
 __device__ __forceinline__ void finish(int32_t* status, int aborted, int tid) {
   if (aborted) {
     for (int i = 0; i < 64; ++i) __nanosleep(2000);  // copies in flight may still land in this CTA's shared memory
@@ -365,16 +389,14 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
         if (HD > 64) tma_load_4d(v_smem + kHalfBytes, &tm_v, full, 64, w.hk, sq.k_row0 + w.key0, sq.bq);
       }
       __syncwarp();
+      int head = w.hk * group, u = 0;
+      UnitStats stats;
+      stats.ask(p, sq, head, w.u_lo * kUnit, true, lane);
       for (int it = 0; it < w.iters; ++it) {
         const uint32_t g = gu + it;
-        const int s = g % kStages, head = w.hk * group + it / w.nu, row0 = (w.u_lo + it % w.nu) * kUnit;
+        const int s = g % kStages, row0 = (w.u_lo + u) * kUnit;
         if (!mbar_wait(smem_addr(&bar->qdo_empty[s]), ((g / kStages) & 1) ^ 1, abort_flag, 61)) { ok = false; break; }
-        for (int r = lane; r < kUnit; r += 32) {
-          const int i = row0 + r;
-          const int64_t li = (int64_t)sq.bq * p.lse_batch_stride + (int64_t)head * p.lse_head_stride + sq.q_row0 + i;
-          bar->nlse2[s][r] = i < sq.q_len ? -p.lse[li] * kLog2e : -INFINITY;  // rows beyond the sequence: P = 0
-          bar->ndls[s][r] = i < sq.q_len ? -p.delta[li] * p.softmax_scale : 0.f;
-        }
+        stats.put(bar->nlse2[s], bar->ndls[s], p.softmax_scale, lane);
         __syncwarp();
         if (elect_one()) {
           const uint32_t full = smem_addr(&bar->qdo_full[s]);
@@ -386,6 +408,8 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
           if (HD > 64) tma_load_4d(do_dst + kUnitHalf, &tm_do, full, 64, head, sq.q_row0 + row0, sq.bq);
         }
         __syncwarp();
+        if (++u == w.nu) { u = 0; ++head; }
+        if (it + 1 < w.iters) stats.ask(p, sq, head, (w.u_lo + u) * kUnit, true, lane);
       }
       ++wi;
       gu += w.iters;

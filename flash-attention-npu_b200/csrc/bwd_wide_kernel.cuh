@@ -283,18 +283,14 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
       __syncwarp();
       const int s_row0 = is_q ? sq.k_row0 : sq.q_row0;
       int s_head = is_q ? w.hk : w.hk * group, u = 0, ys = 0;
+      UnitStats stats;
+      if (!is_q) stats.ask(p, sq, s_head, w.u_lo * kUnit, !is_v, lane);
       for (int it = 0; it < w.iters; ++it) {
         const uint32_t g = gu + it;
         const int xs = g % G::XS, row = (w.u_lo + u) * kUnit;
         if (!mbar_wait(smem_addr(&bar->x_empty[xs]), ((g / G::XS) & 1) ^ 1, abort_flag, 62)) { ok = false; break; }
         if (!is_q) {
-          const int st = g % G::kStats;
-          for (int r = lane; r < kUnit; r += 32) {
-            const int i = row + r;
-            const int64_t li = (int64_t)sq.bq * p.lse_batch_stride + (int64_t)s_head * p.lse_head_stride + sq.q_row0 + i;
-            bar->nlse2[st][r] = i < sq.q_len ? -p.lse[li] * kLog2e : -INFINITY;  // rows beyond the sequence: P = 0
-            bar->ndls[st][r] = (i < sq.q_len && !is_v) ? -p.delta[li] * p.softmax_scale : 0.f;
-          }
+          stats.put(bar->nlse2[g % G::kStats], bar->ndls[g % G::kStats], p.softmax_scale, lane);
           __syncwarp();
         }
         if (lane == 0) mbar_arrive(smem_addr(&bar->stat_full[g % G::kStats]));
@@ -316,6 +312,7 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
         __syncwarp();
         if (++ys == n_y) ys = 0;
         if (++u == w.nu) { u = 0; ++s_head; }
+        if (!is_q && it + 1 < w.iters) stats.ask(p, sq, s_head, (w.u_lo + u) * kUnit, !is_v, lane);
       }
       ++wi;
       gu += w.iters;
