@@ -66,6 +66,8 @@ constexpr int kDeltaThreads = 256, kDeltaRows = 4;
 template <typename T, int LANES>
 __global__ void __launch_bounds__(kDeltaThreads) bwd_delta_kernel(const __grid_constant__ BwdParams p) {
   constexpr int kGroups = kDeltaThreads / LANES;
+  // the work-item counters of the tcgen05 kernels behind this one (the mma.sync kernel's accumulator has been cleared as a whole)
+  if (blockIdx.x == 0 && threadIdx.x < 4) reinterpret_cast<int32_t*>(p.dq_accum)[threadIdx.x] = 0;
   const int lane = threadIdx.x % LANES, grp = threadIdx.x / LANES;
   const int rows = p.cu_seqlens_q ? p.total_q : p.seqlen_q;  // of one batch entry; packed input is one long entry
   const int blocks = ceil_div(rows, kGroups * kDeltaRows);

@@ -39,8 +39,9 @@ int bwd_wide_launch(const BwdParams& p, const fa_bwd_params& a, cudaStream_t st,
   const long long items = 2LL * ((a.seqlen_k + kBlk - 1) / kBlk) * a.h_k * a.b + (long long)((a.seqlen_q + kBlk - 1) / kBlk) * a.h * a.b;
   if (items > 0x7fffffffLL) { *err = "too many work items"; return FA_ERR_UNSUPPORTED; }
   const unsigned grid = (unsigned)std::min<long long>(items, num_sm);
-  int32_t* counter = reinterpret_cast<int32_t*>(p.dq_accum);  // the work-item counter: the first bytes of the workspace
-  cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int32_t), st);
+  // the work-item counter: the first bytes of the workspace, cleared by the kernel in front (bwd_delta_kernel)
+  int32_t* counter = reinterpret_cast<int32_t*>(p.dq_accum);
+  cudaError_t e = cudaSuccess;
   auto launch = [&](auto kern, int smem) {
     if (e == cudaSuccess) e = allow_smem(reinterpret_cast<const void*>(kern), smem);
     if (e == cudaSuccess) {
