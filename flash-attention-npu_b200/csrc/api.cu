@@ -373,25 +373,13 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
   return FA_OK;
 }
 
-// The merge kernel is launched with programmatic stream serialisation: the launch itself and the start of its CTAs
-// overlap the tail of the kernel in front of it on the stream (the split-KV attention kernel, which signals
-// griddepcontrol.launch_dependents when it starts); the kernel waits for that kernel's completion before it reads
-// (combine.cuh).  This hides most of what a second launch costs behind a kernel of a few hundred microseconds.
+// The merge kernel is launched as a programmatic dependent (launch_dependent, common.cuh): the launch itself and the start of
+// its CTAs overlap the tail of the split-KV attention kernel in front of it, which hides most of what a second launch costs.
 template <typename OutT>
 static cudaError_t launch_combine_t(const fa_combine_params& c, int64_t rows, cudaStream_t st) {
   const bool wide = c.num_splits > 32;
-  cudaLaunchConfig_t cfg;
-  std::memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)(wide ? rows : (rows + kCombineWarps - 1) / kCombineWarps));
-  cfg.blockDim = dim3((wide ? kCombineWideWarps : kCombineWarps) * 32);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, wide ? combine_wide_kernel<OutT> : combine_kernel<OutT>, c);
+  if (wide) return launch_dependent(combine_wide_kernel<OutT>, dim3((unsigned)rows), kCombineWideWarps * 32, 0, st, c);
+  return launch_dependent(combine_kernel<OutT>, dim3((unsigned)((rows + kCombineWarps - 1) / kCombineWarps)), kCombineWarps * 32, 0, st, c);
 }
 
 static int launch_combine(const fa_combine_params& c, cudaStream_t st) {
@@ -588,21 +576,6 @@ static size_t exchange_workspace(const fa_fwd_params& a, int ns) {
   return (((size_t)ns * lse_elems * sizeof(float) + 15) & ~(size_t)15) + (size_t)ns * lse_elems * a.d * sizeof(float);
 }
 
-template <typename Kern>
-static cudaError_t launch_dependent(Kern kern, const XchgParams& xp, int grid, cudaStream_t st) {
-  cudaLaunchConfig_t cfg;
-  std::memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kCombineWarps * 32);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, xp);
-}
-
 static int run_fwd_exchange(const fa_fwd_params& a_in, void* workspace, size_t workspace_bytes, const fa_exchange& x,
                             cudaStream_t st) {
   if (!a_in.q || !a_in.k || !a_in.v || !a_in.o || !a_in.lse) return fail(FA_ERR_INVALID, "q, k, v, o and lse must be non-null");
@@ -670,11 +643,11 @@ static int run_fwd_exchange(const fa_fwd_params& a_in, void* workspace, size_t w
   xp.timeout_cycles = x.timeout_cycles > 0 ? x.timeout_cycles : 4000000000LL;  // about two seconds of SM clock
   xp.status = device_status_word();
   const int grid = (int)((rows + kCombineWarps - 1) / kCombineWarps);
-  cudaError_t e = launch_dependent(xchg_push_kernel, xp, grid, st);
+  cudaError_t e = launch_dependent(xchg_push_kernel, dim3(grid), kCombineWarps * 32, 0, st, xp);
   if (e != cudaSuccess) return fail(FA_ERR_CUDA, std::string("exchange push launch: ") + cudaGetErrorString(e));
   ++g_launches;
-  e = a_in.dtype == FA_BF16 ? launch_dependent(xchg_merge_kernel<__nv_bfloat16>, xp, grid, st)
-                            : launch_dependent(xchg_merge_kernel<__half>, xp, grid, st);
+  e = a_in.dtype == FA_BF16 ? launch_dependent(xchg_merge_kernel<__nv_bfloat16>, dim3(grid), kCombineWarps * 32, 0, st, xp)
+                            : launch_dependent(xchg_merge_kernel<__half>, dim3(grid), kCombineWarps * 32, 0, st, xp);
   if (e != cudaSuccess) return fail(FA_ERR_CUDA, std::string("exchange merge launch: ") + cudaGetErrorString(e));
   ++g_launches;
   return FA_OK;

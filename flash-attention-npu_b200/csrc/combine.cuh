@@ -77,10 +77,8 @@ __device__ __forceinline__ void merge_store_lse(const fa_combine_params& p, int 
 // Up to 32 partials: one warp per output row.
 template <typename OutT>
 __global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const __grid_constant__ fa_combine_params p) {
-  // The merge is launched as a programmatic dependent of the kernel in front of it (launch_combine): its CTAs may
-  // become resident while that kernel still runs and wait here until it has completed and its writes are visible.
-  // Without such a kernel in front this returns at once.
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  grid_trigger();
+  grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * kCombineWarps + (threadIdx.x >> 5);
   const int64_t n_rows = (int64_t)p.b * p.s * p.h;
@@ -112,7 +110,8 @@ __global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const __gri
 constexpr int kCombineWideWarps = 16;
 template <typename OutT>
 __global__ void __launch_bounds__(kCombineWideWarps * 32) combine_wide_kernel(const __grid_constant__ fa_combine_params p) {
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  grid_trigger();
+  grid_wait();
   __shared__ float s_red[kCombineWideWarps];
   __shared__ float4 s_acc[kCombineWideWarps][32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

@@ -43,7 +43,7 @@ __device__ __forceinline__ float* xchg_row(char* buf, int parity, int world, int
 }
 
 __global__ void __launch_bounds__(kCombineWarps * 32) xchg_push_kernel(const __grid_constant__ XchgParams p) {
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the attention kernel in front has completed
+  grid_wait();  // the attention kernel in front has completed
   const fa_combine_params& c = p.c;
   XchgHeader* hdr = reinterpret_cast<XchgHeader*>(p.bufs[p.rank]);
   const unsigned int epoch = *reinterpret_cast<volatile unsigned int*>(&hdr->epoch) + 1u;  // this step
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(kCombineWarps * 32) xchg_push_kernel(const __g
 
 template <typename OutT>
 __global__ void __launch_bounds__(kCombineWarps * 32) xchg_merge_kernel(const __grid_constant__ XchgParams p) {
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");  // this rank's push kernel has completed (and set the epoch)
+  grid_wait();  // this rank's push kernel has completed (and set the epoch)
   const fa_combine_params& c = p.c;
   char* buf = p.bufs[p.rank];
   XchgHeader* hdr = reinterpret_cast<XchgHeader*>(buf);

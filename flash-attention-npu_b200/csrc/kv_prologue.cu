@@ -19,6 +19,8 @@ struct PrologueTraits {
 template <typename T>
 __global__ void __launch_bounds__(256) kv_prologue_kernel(const __grid_constant__ KParams p, T* q_rot, int rot_per_token) {
   using Tr = PrologueTraits<T>;
+  grid_trigger();
+  grid_wait();
   const int bi = blockIdx.y, unit = blockIdx.x, tid = threadIdx.x;
   const int l_cache = cache_len(p.a, bi, p.status);
   if (unit < p.a.h_k) {
@@ -66,10 +68,8 @@ __global__ void __launch_bounds__(256) kv_prologue_kernel(const __grid_constant_
 cudaError_t launch_kv_prologue(const KParams& p, void* q_rot, bool rot_per_token, cudaStream_t st) {
   const dim3 grid(p.a.h_k + (q_rot ? p.a.h : 0), p.a.b);
   if (p.a.dtype == FA_BF16)
-    kv_prologue_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p, reinterpret_cast<__nv_bfloat16*>(q_rot), rot_per_token ? 1 : 0);
-  else
-    kv_prologue_kernel<__half><<<grid, 256, 0, st>>>(p, reinterpret_cast<__half*>(q_rot), rot_per_token ? 1 : 0);
-  return cudaGetLastError();
+    return launch_dependent(kv_prologue_kernel<__nv_bfloat16>, grid, 256, 0, st, p, reinterpret_cast<__nv_bfloat16*>(q_rot), rot_per_token ? 1 : 0);
+  return launch_dependent(kv_prologue_kernel<__half>, grid, 256, 0, st, p, reinterpret_cast<__half*>(q_rot), rot_per_token ? 1 : 0);
 }
 
 }  // namespace fa
