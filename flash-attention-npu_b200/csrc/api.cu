@@ -81,6 +81,7 @@ struct Planned {
   fa_fwd_plan pl;
   KParams kp;
   int hd_pad;
+  int cluster = 0;  // decode: CTAs of a cluster that share a unit's keys instead of the plan's partials; 0: as planned
 };
 
 // `forced`: a plan made earlier for the same problem (fa_b200_plan_encode): its kernel family, tile configuration
@@ -327,6 +328,28 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
     if (!canonical) { ns = 1; bps = max_blocks; persistent = false; }
   }
 
+  // Few units with short ranges run their key splits as one thread-block cluster each and merge them through shared memory
+  // (fwd_decode_kernel<., true>): no partials in memory, no merge launch.  The plan still says how the call would be shared out
+  // otherwise; splits that the caller or a plan asks for are kept.
+  out->cluster = 0;
+  if (kernel_id == FA_KERNEL_DECODE && cfg == 3 && m_blocks == 1 && a.num_splits == 0 && !a.cu_seqlens_q && a.kv_total == 0 &&
+      !a.partial_out && (!forced || persistent)) {
+    // Clusters of up to 8 CTAs, all resident at once; with one CTA per SM a GPC may not have room for its second cluster
+    // of 8 (16 units of head dim 256, 128 CTAs: 17.4 us against 16.5 with a merge launch).
+    const long long per_sm = std::max(1, (227 * 1024) / std::max(1, ci.smem_bytes));
+    int cs = kDecodeMaxCluster;
+    while (cs > 1 && (cs > max_blocks || base * cs > (per_sm > 1 ? num_sm : cs > 2 ? num_sm / 2 : num_sm * 7 / 8))) cs >>= 1;
+    // Worth it while a call is bound by latencies and not by the chip's memory rate.  us a call, merge launch / cluster, 8 kv
+    // heads: one sequence of 512 .. 2048 .. 3072 keys 16.5 / 10.6, 14.1 / 10.9, 15.3 / 12.8, of 4096 14.1 / 14.7 (the other half
+    // of the chip is idle); two of 4096 19.2 / 16.8, four of 2048 19.8 / 16.9, eight of 1024 19.8 / 17.1, of 2048 23.7 / 25.3.
+    // Head dim 64: one sequence of 6144 15.1 / 13.6, of 8192 13.9 / 16.0; 256: one of 8192 30.0 / 27.3, of 12288 35.9 / 36.1.
+    // Several sequences may differ in length, and a cluster's share follows the longest: 512 keys a CTA.
+    const int most = a.b > 1 ? 512 : hd_pad == 64 ? 768 : hd_pad == 128 ? 384 : 1024;
+    bool use = cs > 1 && ceil_div(max_blocks, cs) * ci.block_n <= most;
+    if (const char* e = std::getenv("FA_B200_DECODE_CLUSTER")) use = cs > 1 && std::atoi(e) != 0;  // tuning override
+    if (use) out->cluster = cs;
+  }
+
   fa_fwd_plan& pl = out->pl;
   pl.kernel = kernel_id;
   pl.config = cfg;
@@ -343,7 +366,7 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
   pl.is_local = is_local;
   pl.window_left = wl;
   pl.window_right = wr;
-  pl.launches = ns > 1 ? 2 : 1;
+  pl.launches = ns > 1 && !out->cluster ? 2 : 1;
   pl.workspace_bytes = ns > 1 ? (((size_t)ns * lse_elems * sizeof(float) + 15) & ~(size_t)15) + (size_t)ns * lse_elems * a.d * sizeof(float) : 0;
   if (base * ns > 0x7fffffffLL) return fail(FA_ERR_UNSUPPORTED, "grid too large");
 
@@ -419,7 +442,8 @@ static int run_fwd(const fa_fwd_params& a, Workspace& ws, cudaStream_t st, const
   int rc = make_plan(a, &P, forced);
   if (rc != FA_OK) return rc;
   if (a.total_q == 0 || a.seqlen_q == 0) return FA_OK;
-  if (P.pl.workspace_bytes) {
+  if (P.pl.kernel != FA_KERNEL_DECODE) P.cluster = 0;
+  if (P.pl.workspace_bytes && !P.cluster) {
     if (!ws.get(P.pl.workspace_bytes)) return fail(FA_ERR_WORKSPACE, "workspace missing or too small");
     if ((reinterpret_cast<uintptr_t>(ws.ptr) & 15) != 0) return fail(FA_ERR_WORKSPACE, "workspace must be 16-byte aligned");
   }
@@ -451,7 +475,7 @@ static int run_fwd(const fa_fwd_params& a, Workspace& ws, cudaStream_t st, const
   KParams& kp = P.kp;
   kp.status = device_status_word();
   if (!kp.status) return fail(FA_ERR_CUDA, "cannot look up the device status word");
-  if (P.pl.num_splits > 1) {
+  if (P.pl.num_splits > 1 && !P.cluster) {
     kp.lse_partial = reinterpret_cast<float*>(ws.ptr);
     // O partials start at a 16-byte boundary after the LSE partials
     const size_t lse_bytes = ((size_t)P.pl.num_splits * kp.lse_elems * sizeof(float) + 15) & ~(size_t)15;
@@ -470,7 +494,13 @@ static int run_fwd(const fa_fwd_params& a, Workspace& ws, cudaStream_t st, const
     auto* launch = P.hd_pad == 64    ? (bf ? launch_decode_64_bf16 : launch_decode_64_fp16)
                    : P.hd_pad == 128 ? (bf ? launch_decode_128_bf16 : launch_decode_128_fp16)
                                      : (bf ? launch_decode_256_bf16 : launch_decode_256_fp16);
-    e = launch(P.pl.config, kp, tm_k, tm_v, P.pl.grid, st);
+    if (P.cluster) {
+      kp.num_splits = P.cluster;
+      kp.persistent = 0;
+      e = launch(kDecodeClusterConfig, kp, tm_k, tm_v, kp.heads_eff * a.b * P.cluster, st);
+    } else {
+      e = launch(P.pl.config, kp, tm_k, tm_v, P.pl.grid, st);
+    }
   } else
   switch (P.hd_pad) {
     case 64: e = bf ? launch_mma_64_bf16(P.pl.config, kp, P.pl.grid, st) : launch_mma_64_fp16(P.pl.config, kp, P.pl.grid, st); break;
@@ -481,7 +511,7 @@ static int run_fwd(const fa_fwd_params& a, Workspace& ws, cudaStream_t st, const
   ++g_launches;
   if (splits_out) *splits_out = P.pl.num_splits;
 
-  if (P.pl.num_splits > 1 && !skip_merge) {
+  if (P.pl.num_splits > 1 && !P.cluster && !skip_merge) {
     fa_combine_params c;
     std::memset(&c, 0, sizeof(c));
     const bool varlen_q = a.cu_seqlens_q != nullptr;

@@ -48,18 +48,26 @@ cudaError_t allow_smem(const void* kernel, int bytes);
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 template <typename... Params, typename... Args>
-inline cudaError_t launch_dependent(void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+inline cudaError_t launch_dependent_clusters(void (*kern)(Params...), dim3 grid, int cluster, int threads, size_t smem, cudaStream_t st,
+                                             const Args&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, Params(args)...);
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent(void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+  return launch_dependent_clusters(kern, grid, 1, threads, smem, st, args...);
 }
 
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }

@@ -22,6 +22,9 @@ namespace fa {
 
 // Consumer warps form a WM x WN grid: WM splits the packed query rows (16 * MT rows per warp), WN
 // splits the keys of a stage.
+constexpr int kDecodeClusterConfig = -3;  // to the launchers: configuration 3, key splits as one thread-block cluster
+constexpr int kDecodeMaxCluster = 8;      // the portable limit
+
 template <int HD_, typename T_, int MT_, int WM_, int WN_, int BN_, int ST_, int SR_ = 0>
 struct DecTraits {
   using T = T_;
@@ -60,6 +63,10 @@ struct DecTraits {
   static constexpr int MIN_CTAS = (SLAB_IN_RING || (HD == 64 && WM > 1)) ? 2 : 0;
   static_assert(NW % 16 == 0, "each consumer warp needs a multiple of 16 keys");
 };
+
+// Configuration 3 (decode_configs.cuh), the one that also runs as clusters.
+template <int HD, typename T>
+using DecClusterTraits = DecTraits<HD, T, 1, 1, 4, HD == 64 ? 128 : 64, 3, 0>;
 
 // Address of 16-byte chunk `ch` (0 .. HD / 8 - 1) of row `row` in a K / V tile laid out by TMA boxes of
 // 64 columns with the 128-byte swizzle (chunk index XOR row % 8 inside each 128-byte row).

@@ -15,7 +15,74 @@ struct DecWalk {
   int bi, hh, nb_lo, nb_hi, n_b, quota, cur, g1, ustart;
 };
 
+// Shared memory of another CTA of the cluster, at the address that `addr` has in this one.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float ld_cluster(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+
+// Merge of a unit whose key splits are the CTAs of one cluster: every CTA has its rows (fp32, normalised) in its slab and
+// their LSE in lse_s; the CTAs take the columns of all rows in turn and read the parts from one another's shared memory.
+// Arithmetic and conventions of the merge kernel (combine.cuh).
 template <class Tr>
+__device__ __forceinline__ void cluster_merge(const KParams& p, uint32_t slab, uint32_t lse_s, int bi, int hh, int rank, int tid) {
+  using T = typename Tr::T;
+  const int rows_total = p.a.seqlen_q * p.gp, ns = p.num_splits;
+  for (int c = rank * Tr::NTHREADS + tid; c < rows_total * (Tr::HD / 4); c += ns * Tr::NTHREADS) {
+    const int trow = c / (Tr::HD / 4), c4 = (c % (Tr::HD / 4)) * 4;
+    const int i = trow / p.gp, head = hh * p.gp + (trow - i * p.gp);
+    float l[kDecodeMaxCluster], m = -INFINITY, tot = 0.f;
+    float4 x[kDecodeMaxCluster];
+#pragma unroll
+    for (int k = 0; k < kDecodeMaxCluster; ++k) {
+      l[k] = k < ns ? ld_cluster(cluster_addr(lse_s + trow * 4, k)) : -INFINITY;
+      x[k] = k < ns ? ld_cluster4(cluster_addr(slab + (trow * Tr::SLAB_LD + c4) * 4, k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < kDecodeMaxCluster; ++k) m = fmaxf(m, l[k]);
+    const bool dead = m == -INFINITY;
+#pragma unroll
+    for (int k = 0; k < kDecodeMaxCluster; ++k) tot += dead ? 0.f : __expf(l[k] - m);
+    const float inv = dead ? 0.f : 1.f / tot;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < kDecodeMaxCluster; ++k) {
+      if (l[k] == -INFINITY) continue;
+      const float w = __expf(l[k] - m) * inv;
+      acc.x += w * x[k].x;
+      acc.y += w * x[k].y;
+      acc.z += w * x[k].z;
+      acc.w += w * x[k].w;
+    }
+    if (c4 == 0)
+      p.a.lse[(int64_t)bi * p.a.lse_batch_stride + (int64_t)head * p.a.lse_head_stride + i] = dead ? INFINITY : m + logf(tot);
+    if (c4 < p.a.d) {
+      uint2 w2;
+      w2.x = pack2<T>(acc.x, acc.y);
+      w2.y = pack2<T>(acc.z, acc.w);
+      *reinterpret_cast<uint2*>(reinterpret_cast<T*>(p.a.o) + (int64_t)bi * p.a.o_batch_stride + (int64_t)i * p.a.o_row_stride +
+                                (int64_t)head * p.a.o_head_stride + c4) = w2;
+    }
+  }
+}
+
+// CL: the key splits of a unit are the CTAs of one cluster (cluster_merge), an instance of its own: the merge code would
+// cost the streaming loop of the others registers.
+template <class Tr, bool CL>
 __global__ void __launch_bounds__(Tr::NTHREADS, Tr::MIN_CTAS)
 fwd_decode_kernel(const __grid_constant__ KParams p, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v) {
@@ -107,6 +174,14 @@ fwd_decode_kernel(const __grid_constant__ KParams p, const __grid_constant__ CUt
   // warp-collective: first segment of this CTA (and the cursor, persistent mode)
   auto walk_first = [&](DecWalk& w, DecSeg& sg) {
     w = DecWalk{0, 0, 0, 0, 1, 1, 0, 0, 0};
+    if (CL) {  // split fastest; every unit's own blocks in equal shares
+      const int split = blockIdx.x % p.num_splits, unit = blockIdx.x / p.num_splits, bi = unit / he;
+      int nb_lo, nb_hi;
+      batch_range(bi, p.a.seqlen_q, nb_lo, nb_hi);
+      const int share = ceil_div(nb_hi - nb_lo, p.num_splits), lo = nb_lo + split * share;
+      sg = DecSeg{bi, unit % he, lo, max(0, min(nb_hi, lo + share) - lo), split, p.num_splits, split == 0, 0, 1};
+      return;
+    }
     if (!p.persistent) {
       int idx = blockIdx.x;
       const int hh = idx % he;
@@ -543,7 +618,7 @@ fwd_decode_kernel(const __grid_constant__ KParams p, const __grid_constant__ CUt
           }
 
           const bool f32_out = to_partial || p.a.partial_out;
-          for (int c = tid; c < BM * (Tr::HD / 4); c += NCT) {
+          for (int c = tid; !CL && c < BM * (Tr::HD / 4); c += NCT) {
             const int trow = c / (Tr::HD / 4), c4 = (c % (Tr::HD / 4)) * 4;
             if (trow >= rows_total) continue;
             const int i = trow / p.gp, head = hh * p.gp + (trow - i * p.gp);
@@ -577,7 +652,7 @@ fwd_decode_kernel(const __grid_constant__ KParams p, const __grid_constant__ CUt
           }
         }
       }
-      if (!p.persistent) break;
+      if (CL || !p.persistent) break;
       if (tid == 0) {
         DecWalk w = s_walk;
         DecSeg nx;
@@ -589,6 +664,12 @@ fwd_decode_kernel(const __grid_constant__ KParams p, const __grid_constant__ CUt
   }
 
   __syncthreads();
+  if (CL) {
+    cluster_barrier();  // every CTA's rows are in its slab
+    const int unit = blockIdx.x / p.num_splits;
+    cluster_merge<Tr>(p, smem_u32(smem_al + Tr::SLAB_OFF), smem_u32(s_lse), unit / he, unit % he, blockIdx.x % p.num_splits, tid);
+    cluster_barrier();  // nobody's shared memory goes while it is read
+  }
   if (s_abort) {
     for (int i = 0; i < 64; ++i) __nanosleep(2000);  // let copies in flight land before the CTA retires
     if (tid == 0 && p.status) atomicExch(p.status, 0x40000000 | (int)blockIdx.x);
