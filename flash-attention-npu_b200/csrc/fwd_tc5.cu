@@ -91,7 +91,7 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
   // scores of a row plus working set, the other roles need far fewer.
   if (warp < 8) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kRegsSoftmax));
-    softmax_loop<T, IN, CAP, Geo<HD>::kRows>(p, bar, tmem, p_smem, warp >> 2, warp & 3, lane);
+    softmax_loop<T, IN, CAP, HD>(p, bar, tmem, p_smem, warp >> 2, warp & 3, lane);
   } else if (warp < 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsCorr));
     correction_loop<T, IN, HD>(p, bar, tmem, warp & 3, lane);

@@ -114,7 +114,7 @@ __device__ __forceinline__ void chunk_softcap_fine(uint32_t (&a)[32], float mul,
   }
 }
 
-template <typename T, int IN, int CAP, int ROWS>
+template <typename T, int IN, int CAP, int HD>
 __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, uint32_t tmem, uint32_t p_smem, int t,
                                              int warp_in_wg, int lane) {
   volatile int* abort_flag = &bar->abort_flag;
@@ -135,7 +135,7 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
   TileWalk<IN> walk(bar);
   for (int n = walk.first(p); n < p.total_tiles; n = walk.next(p)) {
     TileInfo ti;
-    tile_info<ROWS>(p, tile_id<IN>(p, n), ti);
+    tile_info<Geo<HD>::kRows>(p, tile_id<IN>(p, n), ti);
     if (ti.row0[t] >= ti.q_len) continue;
     const int i = ti.row0[t] + row;
     if (!ti.has[t]) {  // no visible key for the whole sub-tile: O = 0, LSE = +inf
@@ -214,13 +214,17 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       uint64_t sum2[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) sum2[q] = pack_f32x2(0.f, 0.f);
-      uint32_t pk[16];
+      // P.V of the previous block must have read P_t before it is overwritten.  For 128 columns the wait stands behind half of
+      // the row's exponentials: b4 s4096 h32 causal 669 -> 661 us, full 1204 -> 1160 (three quarters: 673, 1200, P.V starts too
+      // late); for 64 and 256 columns behind a quarter (with half 1.5 % slower).
+      constexpr bool kHalfAhead = HD == 128;
+      uint32_t pk[16], pk1[16];
       chunk_exp<T, kPolyPairs>(sc[0], scale2, negms2, sum2, pk);
-      // P.V of the previous block must have read P_t before it is overwritten
+      if (kHalfAhead) chunk_exp<T, kPolyPairs>(sc[1], scale2, negms2, sum2, pk1);
       if (blk > 0 && !mbar_wait(bar_odone, (blk - 1) & 1, abort_flag, 42)) return;
       store_p_chunk(p_row, p_xor, 0, pk);
-      chunk_exp<T, kPolyPairs>(sc[1], scale2, negms2, sum2, pk);
-      store_p_chunk(p_row, p_xor, 1, pk);
+      if (!kHalfAhead) chunk_exp<T, kPolyPairs>(sc[1], scale2, negms2, sum2, pk1);
+      store_p_chunk(p_row, p_xor, 1, pk1);
       fence_proxy_async();  // generic-proxy stores -> visible to the MMA (async proxy)
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_addr(&bar->p_full[t][0]));  // first 64 keys of P are ready
