@@ -49,7 +49,7 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
       mbar_init(smem_addr(&bar->q_full[t]), 1);
       mbar_init(smem_addr(&bar->q_empty[t]), 1);
       mbar_init(smem_addr(&bar->s_full[t]), 1);
-      mbar_init(smem_addr(&bar->s_free[t]), 4);
+      mbar_init(smem_addr(&bar->s_free[t]), Geo<HD>::kWide ? 8 : 4);
       mbar_init(smem_addr(&bar->p_full[t][0]), 4);
       mbar_init(smem_addr(&bar->p_full[t][1]), 4);
       mbar_init(smem_addr(&bar->corr_ready[t]), 4);
@@ -64,6 +64,7 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
     }
     mbar_init(smem_addr(&bar->fix_req), 2);
     mbar_init(smem_addr(&bar->v_fixed), 1);
+    mbar_init(smem_addr(&bar->exchanged), 8);
     for (int s = 0; s < kQueue; ++s) {
       mbar_init(smem_addr(&bar->queue.full[s]), 1);
       mbar_init(smem_addr(&bar->queue.empty[s]), kQueueReaders);

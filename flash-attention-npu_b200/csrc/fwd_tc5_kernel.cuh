@@ -10,7 +10,7 @@
 // A operand) into the second MMA.
 //
 // CTA = 16 warps:  warps 0-3    softmax of query sub-tile 0 (128 rows, one thread per row)
-//                  warps 4-7    softmax of query sub-tile 1
+//                  warps 4-7    softmax of query sub-tile 1 (256-column tiles: the same rows as warps 0-3, keys 64-127)
 //                  warps 8-11   correction (rescale of O in TMEM when a row maximum moved) and
 //                               epilogue (O / l -> global) for both sub-tiles
 //                  warps 12-13  MMA issuers, one per sub-tile (one elected lane each)
@@ -37,6 +37,7 @@ constexpr int kBlockM = 128;          // rows of one query sub-tile
 constexpr int kTileM = 2 * kBlockM;   // rows of one CTA tile
 constexpr int kBlockN = 128;          // keys per KV block
 constexpr int kSlots = 3;             // ring of 32 KiB K / V buffers
+constexpr int kXchgCol = 128;  // TMEM columns of the exchange between warpgroups that share rows (S1's)
 constexpr int kThreads = 512;
 constexpr int kMmaWarp = 12 /* and 13: one per sub-tile */, kTmaWarp = 14;
 // Registers per thread after the roles have re-balanced them (setmaxnreg, one value per warpgroup).
@@ -59,7 +60,7 @@ static_assert(kSmemBytes <= 232448, "more than the 227 KiB a CTA can have");
 
 // Geometry by tile width HD (64, 128 or 256 columns; the head dim is at most HD).  Up to 128 a CTA tile is two
 // 128-row sub-tiles and a K / V tile fills one 32 KiB ring slot (its first half only for 64).  For 256 the 256 fp32
-// columns of O leave TMEM room for one sub-tile only: the CTA tile is 128 rows, Q takes both Q slots (64 KiB), the
+// columns of O leave TMEM room for one sub-tile only: the CTA tile is 128 rows (shared by the two softmax warpgroups), Q takes both Q slots (64 KiB), the
 // second P slot joins the ring, and the ring is two slots of 64 KiB.
 template <int HD>
 struct Geo {
@@ -197,6 +198,7 @@ struct Barriers {
   uint64_t o_free[2];      // correction -> MMA: the epilogue has read O_t
   uint64_t fix_req;        // MMA (both warps) -> warp 15: the last V tile of the CTA tile has landed and needs its tail cleared
   uint64_t v_fixed;        // warp 15 -> MMA (both warps): done
+  uint64_t exchanged;      // 256-column tiles: both softmax warpgroups have left their value in TMEM
   uint32_t tmem_base;
   int abort_flag;
   uint32_t fix_seen[2];    // tail repairs each issuing warp has been through (phase of fix_req / v_fixed)

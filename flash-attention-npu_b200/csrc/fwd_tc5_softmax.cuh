@@ -1,6 +1,7 @@
 // Softmax role and correction / epilogue role of the tcgen05 prefill kernel.
 //
-// Softmax: 128 threads per query sub-tile, one thread per query row (TMEM lane).  It restates the
+// Softmax: 128 threads per query sub-tile, one thread per query row (TMEM lane); 256-column tiles have one sub-tile and two
+// threads per row, 64 keys of a block each.  It restates the
 // arithmetic of the reference's OnlineSoftmax epilogue
 // (csrc/arch22/flash_attn_npu_v2/online_softmax.hpp:479-803) in the log2 domain:
 //   P = exp2(S * scale*log2e - m * scale*log2e), rounded to the input dtype before P.V.
@@ -115,12 +116,20 @@ __device__ __forceinline__ void chunk_softcap_fine(uint32_t (&a)[32], float mul,
 }
 
 template <typename T, int IN, int CAP, int HD>
-__device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, uint32_t tmem, uint32_t p_smem, int t,
+__device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, uint32_t tmem, uint32_t p_smem, int wg,
                                              int warp_in_wg, int lane) {
+  // With 256 columns there is one sub-tile, and one warpgroup by itself leaves the special-function unit idle for most of a
+  // block: both warpgroups share its rows.  b 2, s 2047, 16 / 8 heads, head dim 256, softcap 50: 100 -> 91 us; b 2, s 1777,
+  // 8 heads, forward and backward 190 -> 188.
+  constexpr bool kWide = Geo<HD>::kWide;
+  constexpr int kChunks = kWide ? 2 : 4;       // of 32 keys
+  const int t = kWide ? 0 : wg;                // sub-tile
+  const int chunk0 = kWide ? 2 * wg : 0;       // first chunk of this thread in a block
+  const bool lead = !kWide || wg == 0;         // writes the row's factors and statistics
   volatile int* abort_flag = &bar->abort_flag;
   const int row = warp_in_wg * 32 + lane;
   const uint32_t lane_addr = (uint32_t)(warp_in_wg * 32) << 16;
-  const uint32_t s_tmem = tmem + lane_addr + t * 128;
+  const uint32_t s_tmem = tmem + lane_addr + t * 128 + chunk0 * 32;
   uint32_t s_cnt = 0, cr_cnt = 0, st_cnt = 0;
   // this row of P_t: chunk kc (8 keys) of the row lives at  half(kc) + row * 128 + ((kc ^ row) & 7) * 16
   const uint32_t p_row = p_smem + t * kTileBytes + row * 128;
@@ -132,6 +141,26 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
   const float lse_scale = CAP ? 0.6931471805599453f : p.a.softmax_scale;  // running maximum -> natural log
   const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
 
+  // What the row's other thread has, through a TMEM column each.  Two pairs of columns in turn: a pair is written again only
+  // when the other side has been through the exchange in between, which it enters after it has read this one.
+  uint32_t x_cnt = 0;
+  auto exchange = [&](float v, float& other) -> bool {
+    const uint32_t col = tmem + lane_addr + kXchgCol + 2 * (x_cnt & 1);
+    tmem_st1(col + wg, __float_as_uint(v));
+    tmem_wait_st();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_addr(&bar->exchanged));
+    if (!mbar_wait(smem_addr(&bar->exchanged), x_cnt & 1, abort_flag, 49)) return false;
+    tc_fence_after();
+    ++x_cnt;
+    uint32_t r;
+    tmem_ld1(col + 1 - wg, r);
+    tmem_wait_ld();
+    other = __uint_as_float(r);
+    return true;
+  };
+
   TileWalk<IN> walk(bar);
   for (int n = walk.first(p); n < p.total_tiles; n = walk.next(p)) {
     TileInfo ti;
@@ -139,7 +168,7 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
     if (ti.row0[t] >= ti.q_len) continue;
     const int i = ti.row0[t] + row;
     if (!ti.has[t]) {  // no visible key for the whole sub-tile: O = 0, LSE = +inf
-      if (i < ti.q_len) {
+      if (lead && i < ti.q_len) {
         T* o_ptr = reinterpret_cast<T*>(p.a.o) + (int64_t)ti.bi * p.a.o_batch_stride +
                    (int64_t)(ti.q_row0 + i) * p.a.o_row_stride + (int64_t)ti.hh * p.a.o_head_stride;
         for (int c = 0; c < p.a.d; c += 8) *reinterpret_cast<uint4*>(o_ptr + c) = make_uint4(0, 0, 0, 0);
@@ -166,10 +195,10 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       const uint32_t blk = s_cnt;  // running number of this block (all tiles of this CTA)
       ++s_cnt;
       tc_fence_after();
-      // ---- all 128 scores of the row into registers (one TMEM round trip) ----
-      uint32_t sc[4][32];
+      // ---- the scores into registers (one TMEM round trip) ----
+      uint32_t sc[kChunks][32];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tmem_ld32(s_tmem + c * 32, sc[c]);
+      for (int c = 0; c < kChunks; ++c) tmem_ld32(s_tmem + c * 32, sc[c]);
       tmem_wait_ld();
       // the S columns are free: Q.K^T of the next block may overwrite them
       tc_fence_before();
@@ -177,18 +206,23 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       if (lane == 0) mbar_arrive(bar_sfree);
       if (CAP) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < kChunks; ++c) {
           if (CAP == kCapFine) chunk_softcap_fine(sc[c], p.softcap_mul, p.softcap_l2);
           else chunk_softcap(sc[c], p.softcap_mul, p.softcap_l2);
         }
       }
       if (need_mask) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) chunk_mask(sc[c], col0 + c * 32, lo, hi);
+        for (int c = 0; c < kChunks; ++c) chunk_mask(sc[c], col0 + (chunk0 + c) * 32, lo, hi);
       }
       float blk_max = chunk_max(sc[0], -INFINITY);
 #pragma unroll
-      for (int c = 1; c < 4; ++c) blk_max = chunk_max(sc[c], blk_max);
+      for (int c = 1; c < kChunks; ++c) blk_max = chunk_max(sc[c], blk_max);
+      if (kWide) {
+        float other;
+        if (!exchange(blk_max, other)) return;
+        blk_max = fmaxf(blk_max, other);
+      }
 
       float m_new = fmaxf(m_run, blk_max);
       // The running maximum follows every increase (P <= 1, and the row maximum has P = 1 exactly, like the
@@ -197,7 +231,7 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       if (kRescaleThreshold > 0.f && m_run != -INFINITY && (m_new - m_run) * scale_log2 <= kRescaleThreshold) m_new = m_run;
       const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
       const float corr = fast_exp2((m_run - m_use) * scale_log2);  // 0 when m_run = -inf
-      if (j > ti.jlo[t]) {
+      if (lead && j > ti.jlo[t]) {
         // The correction warps must have consumed the previous factors: this thread can be a whole
         // block ahead of them, and neither the factor array nor the barrier phase may be reused early.
         if (cr_cnt > 0 && !mbar_wait(bar_oready, (cr_cnt - 1) & 1, abort_flag, 47)) return;
@@ -222,22 +256,30 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       chunk_exp<T, kPolyPairs>(sc[0], scale2, negms2, sum2, pk);
       if (kHalfAhead) chunk_exp<T, kPolyPairs>(sc[1], scale2, negms2, sum2, pk1);
       if (blk > 0 && !mbar_wait(bar_odone, (blk - 1) & 1, abort_flag, 42)) return;
-      store_p_chunk(p_row, p_xor, 0, pk);
+      store_p_chunk(p_row, p_xor, chunk0, pk);
       if (!kHalfAhead) chunk_exp<T, kPolyPairs>(sc[1], scale2, negms2, sum2, pk1);
-      store_p_chunk(p_row, p_xor, 1, pk1);
+      store_p_chunk(p_row, p_xor, chunk0 + 1, pk1);
       fence_proxy_async();  // generic-proxy stores -> visible to the MMA (async proxy)
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_addr(&bar->p_full[t][0]));  // first 64 keys of P are ready
-      chunk_exp<T, kPolyPairs>(sc[2], scale2, negms2, sum2, pk);
-      store_p_chunk(p_row, p_xor, 2, pk);
-      chunk_exp<T, kPolyPairs>(sc[3], scale2, negms2, sum2, pk);
-      store_p_chunk(p_row, p_xor, 3, pk);
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_addr(&bar->p_full[t][1]));  // last 64 keys
+      if (lane == 0) mbar_arrive(smem_addr(&bar->p_full[t][kWide ? wg : 0]));  // the first (this warpgroup's) 64 keys of P are ready
+      if constexpr (!kWide) {
+        chunk_exp<T, kPolyPairs>(sc[2], scale2, negms2, sum2, pk);
+        store_p_chunk(p_row, p_xor, 2, pk);
+        chunk_exp<T, kPolyPairs>(sc[3], scale2, negms2, sum2, pk);
+        store_p_chunk(p_row, p_xor, 3, pk);
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_addr(&bar->p_full[t][1]));  // last 64 keys
+      }
       float s0, s1;
       unpack_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])), s0, s1);
       l_run = l_run * corr + (s0 + s1);
+    }
+    if (kWide) {
+      float other;
+      if (!exchange(l_run, other)) return;
+      l_run += other;
+      if (!lead) continue;
     }
     // 1 / l for the epilogue, LSE from here.  The previous tile's epilogue must have read its 1 / l
     // (a tile of a single block does not wait for anything else the epilogue does).
@@ -256,6 +298,24 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
 template <int HD>
 __device__ __forceinline__ void rescale_o(uint32_t o_tmem, float f) {
   const uint64_t f2 = pack_f32x2(f, f);
+  if constexpr (HD > 128) {  // (the 256-column instances spill with the form below)
+#pragma unroll 1
+    for (int c = 0; c < HD; c += 32) {
+      uint32_t a[32];
+      tmem_ld32(o_tmem + c, a);
+      tmem_wait_ld();
+#pragma unroll
+      for (int e = 0; e < 32; e += 2) {
+        float x0, x1;
+        unpack_f32x2(mul_f32x2(pack_f32x2(__uint_as_float(a[e]), __uint_as_float(a[e + 1])), f2), x0, x1);
+        a[e] = __float_as_uint(x0);
+        a[e + 1] = __float_as_uint(x1);
+      }
+      tmem_st32(o_tmem + c, a);
+    }
+    tmem_wait_st();
+    return;
+  }
   uint32_t a[32], b[32];
   tmem_ld32(o_tmem, a);
   tmem_ld32(o_tmem + 32, b);
