@@ -3,7 +3,9 @@
 // the same arithmetic as CombineScale (csrc/arch22/flash_attn_npu_v2/CombineScale.hpp:165-309).
 // An empty partial carries lse = -inf (weight 0, its O is never read).  A row whose every
 // partial is empty yields O = 0 and LSE = +inf (the API convention for a row without visible
-// keys, rescale_o.hpp:57) -- or -inf when the result is itself a partial.
+// keys, rescale_o.hpp:57) -- or -inf when the result is itself a partial.  A partial whose LSE is
+// NaN makes the row NaN; whether all are empty is therefore asked of the partials, not of the
+// maximum, which drops NaN.
 #pragma once
 
 #include "common.cuh"
@@ -41,7 +43,7 @@ __device__ __forceinline__ void merge_weights(int n, int lane, LoadLse lse_of, f
   m = l_mine;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  dead = (m == -INFINITY);
+  dead = __all_sync(0xffffffffu, l_mine == -INFINITY);
   tot = (!dead && lane < n) ? __expf(l_mine - m) : 0.f;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
@@ -133,9 +135,14 @@ __global__ void __launch_bounds__(kCombineWideWarps * 32) combine_wide_kernel(co
     return v;
   };
   float m = -INFINITY;
-  for (int i = tid; i < p.num_splits; i += kCombineWideWarps * 32) m = fmaxf(m, lp[(int64_t)i * p.lp_split_stride]);
+  int some = 0;
+  for (int i = tid; i < p.num_splits; i += kCombineWideWarps * 32) {
+    const float l = lp[(int64_t)i * p.lp_split_stride];
+    m = fmaxf(m, l);
+    some |= l != -INFINITY;
+  }
   m = block_reduce(m, [](float x, float y) { return fmaxf(x, y); });
-  const bool dead = m == -INFINITY;
+  const bool dead = __syncthreads_or(some) == 0;
   float tot = 0.f;
   if (!dead)
     for (int i = tid; i < p.num_splits; i += kCombineWideWarps * 32) tot += __expf(lp[(int64_t)i * p.lp_split_stride] - m);

@@ -46,6 +46,7 @@ __device__ __forceinline__ void cluster_merge(const KParams& p, uint32_t slab, u
     const int trow = c / (Tr::HD / 4), c4 = (c % (Tr::HD / 4)) * 4;
     const int i = trow / p.gp, head = hh * p.gp + (trow - i * p.gp);
     float l[kDecodeMaxCluster], m = -INFINITY, tot = 0.f;
+    bool dead = true;  // every part is empty (asked of the parts: the maximum of empty parts and NaN is -inf too)
     float4 x[kDecodeMaxCluster];
 #pragma unroll
     for (int k = 0; k < kDecodeMaxCluster; ++k) {
@@ -53,8 +54,10 @@ __device__ __forceinline__ void cluster_merge(const KParams& p, uint32_t slab, u
       x[k] = k < ns ? ld_cluster4(cluster_addr(slab + (trow * Tr::SLAB_LD + c4) * 4, k)) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
-    for (int k = 0; k < kDecodeMaxCluster; ++k) m = fmaxf(m, l[k]);
-    const bool dead = m == -INFINITY;
+    for (int k = 0; k < kDecodeMaxCluster; ++k) {
+      m = fmaxf(m, l[k]);
+      dead = dead && l[k] == -INFINITY;
+    }
 #pragma unroll
     for (int k = 0; k < kDecodeMaxCluster; ++k) tot += dead ? 0.f : __expf(l[k] - m);
     const float inv = dead ? 0.f : 1.f / tot;
@@ -587,8 +590,9 @@ fwd_decode_kernel(const __grid_constant__ KParams p, const __grid_constant__ CUt
                 const float2 x = ml[w * BM + trow];
                 l_all += x.y * fast_exp2(x.x - m_use);
               }
-              f_row[mt][hf] = (l_all > 0.f) ? fast_exp2(m_run[mt][hf] - m_use) / l_all : 0.f;
-              if (wn == 0 && t4 == 0) s_lse[trow] = (l_all > 0.f) ? (m_use + log2f(l_all)) * kLn2 : -INFINITY;
+              // Only a sum of exactly 0 means that the row saw no key: a NaN (from a NaN or infinite score) stays one.
+              f_row[mt][hf] = (l_all == 0.f) ? 0.f : fast_exp2(m_run[mt][hf] - m_use) / l_all;
+              if (wn == 0 && t4 == 0) s_lse[trow] = (l_all == 0.f) ? -INFINITY : (m_use + log2f(l_all)) * kLn2;
             }
           // slice 0 stores, slices 1 .. WN-1 add in turn: a fixed order, so the result does not depend on timing
 #pragma unroll 1

@@ -321,7 +321,8 @@ __global__ void __launch_bounds__(Tr::NTHREADS) fwd_mma_kernel(const __grid_cons
         const float2 x = ml[w * BM + trow];
         l_all += x.y * fast_exp2(x.x - m_use);
       }
-      const float f = (l_all > 0.f) ? fast_exp2(m_run[mt][hf] - m_use) / l_all : 0.f;
+      // only a sum of exactly 0 means that the row saw no key: a NaN stays one
+      const float f = (l_all == 0.f) ? 0.f : fast_exp2(m_run[mt][hf] - m_use) / l_all;
       float* dst = slab + (size_t)(wn * BM + trow) * Tr::SLAB_LD;
 #pragma unroll
       for (int dt = 0; dt < DT; ++dt)
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(Tr::NTHREADS) fwd_mma_kernel(const __grid_cons
       const float2 x = ml[w * BM + trow];
       l_all += x.y * fast_exp2(x.x - m_use);
     }
-    s_lse[trow] = (l_all > 0.f) ? (m_use + log2f(l_all)) * kLn2 : -INFINITY;
+    s_lse[trow] = (l_all == 0.f) ? -INFINITY : (m_use + log2f(l_all)) * kLn2;
   }
   __syncthreads();
   // one pass over (row, 4 columns)
