@@ -79,7 +79,6 @@ __device__ __forceinline__ void merge_store_lse(const fa_combine_params& p, int 
 // Up to 32 partials: one warp per output row.
 template <typename OutT>
 __global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const __grid_constant__ fa_combine_params p) {
-  grid_trigger();
   grid_wait();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * kCombineWarps + (threadIdx.x >> 5);
@@ -112,7 +111,6 @@ __global__ void __launch_bounds__(kCombineWarps * 32) combine_kernel(const __gri
 constexpr int kCombineWideWarps = 16;
 template <typename OutT>
 __global__ void __launch_bounds__(kCombineWideWarps * 32) combine_wide_kernel(const __grid_constant__ fa_combine_params p) {
-  grid_trigger();
   grid_wait();
   __shared__ float s_red[kCombineWideWarps];
   __shared__ float4 s_acc[kCombineWideWarps][32];

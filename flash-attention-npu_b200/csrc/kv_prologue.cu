@@ -19,7 +19,6 @@ struct PrologueTraits {
 template <typename T>
 __global__ void __launch_bounds__(256) kv_prologue_kernel(const __grid_constant__ KParams p, T* q_rot, int rot_per_token) {
   using Tr = PrologueTraits<T>;
-  grid_trigger();
   grid_wait();
   const int bi = blockIdx.y, unit = blockIdx.x, tid = threadIdx.x;
   const int l_cache = cache_len(p.a, bi, p.status);
