@@ -250,8 +250,10 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       for (int q = 0; q < 4; ++q) sum2[q] = pack_f32x2(0.f, 0.f);
       // P.V of the previous block must have read P_t before it is overwritten.  For 128 columns the wait stands behind half of
       // the row's exponentials: b4 s4096 h32 causal 669 -> 661 us, full 1204 -> 1160 (three quarters: 673, 1200, P.V starts too
-      // late); for 64 and 256 columns behind a quarter (with half 1.5 % slower).
-      constexpr bool kHalfAhead = HD == 128;
+      // late); elsewhere behind a quarter.  Half is slower for 64 and 256 columns (1.5 %), with softcap, whose scores are ready
+      // late by themselves (b2 s4096 h16 full 431 -> 444 us, b1 s1061 h16 causal 31.8 -> 32.4), and where no tile follows another
+      // (ragged input, fixed deal: 6 chunks of 705 rows against 1307 keys 32.4 -> 33.4, 5 of 135 rows 19.5 -> 19.8).
+      constexpr bool kHalfAhead = HD == 128 && CAP == kCapNone && IN != kRaggedFixed;
       uint32_t pk[16], pk1[16];
       chunk_exp<T, kPolyPairs>(sc[0], scale2, negms2, sum2, pk);
       if (kHalfAhead) chunk_exp<T, kPolyPairs>(sc[1], scale2, negms2, sum2, pk1);
