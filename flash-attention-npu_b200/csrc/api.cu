@@ -77,11 +77,13 @@ static bool few_tiles_long_range(const fa_fwd_params& a) {
   return keys >= 4096 && rows < 1024;
 }
 
+constexpr int kPlanClusterUnit = 256;  // fa_fwd_plan.config of a clustered decode call: the tile configuration + this x the cluster size
+
 struct Planned {
   fa_fwd_plan pl;
   KParams kp;
   int hd_pad;
-  int cluster = 0;  // decode: CTAs of a cluster that share a unit's keys instead of the plan's partials; 0: as planned
+  int cluster = 0;  // decode: CTAs of the cluster that shares a unit's keys; 0: no clusters
 };
 
 // `forced`: a plan made earlier for the same problem (fa_b200_plan_encode): its kernel family, tile configuration
@@ -197,9 +199,9 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
       }
       if (forced && forced->kernel == FA_KERNEL_DECODE) {
         DecodeConfigInfo t;
-        if (!decode_config_info(hd_pad, forced->config, &t) || t.block_m < rows_max)
+        dcfg = forced->config % kPlanClusterUnit;
+        if (!decode_config_info(hd_pad, dcfg, &t) || t.block_m < rows_max)
           return fail(FA_ERR_UNSUPPORTED, "the plan's tile configuration does not fit this problem");
-        dcfg = forced->config;
       }
       DecodeConfigInfo di;
       if (decode_config_info(hd_pad, dcfg, &di)) {
@@ -266,6 +268,7 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
   // sequence of 2048 keys and 8 kv heads ran on 8 CTAs: 36 -> 14 us with the merge), and for many units four, the most that equal
   // shares of near-equal units need.
   bool persistent = false;
+  const int forced_cluster = forced && forced->kernel == FA_KERNEL_DECODE ? forced->config / kPlanClusterUnit : 0;
   long long persist_grid = 0;
   int persist_slots = kMinPersistSlots;
   if (kernel_id == FA_KERNEL_DECODE && a.num_splits == 0 && !a.cu_seqlens_q && a.kv_total == 0 && !a.partial_out) {
@@ -301,7 +304,7 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
     }
     if (const char* e = std::getenv("FA_B200_DECODE_PERSISTENT"))  // tuning override: 0 off, 1 ragged ranges only, 2 wherever possible
       persistent = can_persist && (std::atoi(e) == 2 || (std::atoi(e) == 1 && !window_bound));
-    if (forced && forced->kernel == FA_KERNEL_DECODE && forced->num_splits > 1 && forced->blocks_per_split == 0) {
+    if (forced && forced->kernel == FA_KERNEL_DECODE && !forced_cluster && forced->num_splits > 1 && forced->blocks_per_split == 0) {
       if (!can_persist || forced->grid <= 0 || forced->num_splits < kMinPersistSlots)
         return fail(FA_ERR_UNSUPPORTED, "the plan's persistent decode schedule does not fit this problem");
       persistent = true;
@@ -312,7 +315,7 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
     }
     if (persistent) { ns = persist_slots; bps = 0; }
   }
-  if (forced && forced->kernel != FA_KERNEL_TCGEN05 && !persistent) {
+  if (forced && forced->kernel != FA_KERNEL_TCGEN05 && !persistent && !forced_cluster) {
     if (forced->num_splits < 1 || forced->blocks_per_split < 1 ||
         (long long)forced->num_splits * forced->blocks_per_split < max_blocks)
       return fail(FA_ERR_UNSUPPORTED, "the plan's KV splits do not cover this problem's key range");
@@ -329,11 +332,16 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
   }
 
   // Few units with short ranges run their key splits as one thread-block cluster each and merge them through shared memory
-  // (fwd_decode_kernel<., true>): no partials in memory, no merge launch.  The plan still says how the call would be shared out
-  // otherwise; splits that the caller or a plan asks for are kept.
-  out->cluster = 0;
-  if (kernel_id == FA_KERNEL_DECODE && cfg == 3 && m_blocks == 1 && a.num_splits == 0 && !a.cu_seqlens_q && a.kv_total == 0 &&
-      !a.partial_out && (!forced || persistent)) {
+  // (fwd_decode_kernel<., true>): no partials in memory, no merge launch.  A plan that was made earlier says itself whether its
+  // call runs so; splits that the caller or a tuning override asks for are kept.
+  const bool can_cluster = kernel_id == FA_KERNEL_DECODE && cfg == kDecodeClusterBase && m_blocks == 1 && a.num_splits == 0 &&
+                           !a.cu_seqlens_q && a.kv_total == 0 && !a.partial_out;
+  if (forced_cluster) {
+    if (!can_cluster || forced_cluster < 2 || forced_cluster > kDecodeMaxCluster)
+      return fail(FA_ERR_UNSUPPORTED, "the plan's clusters do not fit this problem");
+    out->cluster = forced_cluster;
+  } else if (can_cluster && !forced && !std::getenv("FA_B200_NUM_SPLITS") && !std::getenv("FA_B200_DECODE_PERSISTENT") &&
+             !std::getenv("FA_B200_DECODE_PERSISTENT_GRID")) {
     // Clusters of up to 8 CTAs, all resident at once; with one CTA per SM a GPC may not have room for its second cluster
     // of 8 (16 units of head dim 256, 128 CTAs: 17.4 us against 16.5 with a merge launch).
     const long long per_sm = std::max(1, (227 * 1024) / std::max(1, ci.smem_bytes));
@@ -352,22 +360,23 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
 
   fa_fwd_plan& pl = out->pl;
   pl.kernel = kernel_id;
-  pl.config = cfg;
+  pl.config = cfg + out->cluster * kPlanClusterUnit;
   pl.pack_gqa = pack;
   pl.block_m = ci.block_m;
   pl.block_n = ci.block_n;
   pl.m_blocks = m_blocks;
   pl.num_splits = ns;
   pl.blocks_per_split = bps;
-  pl.grid = persistent ? (int)persist_grid : (int)(base * ns);
+  pl.grid = out->cluster ? (int)(base * out->cluster) : persistent ? (int)persist_grid : (int)(base * ns);
   pl.threads = ci.threads;
   pl.smem_bytes = ci.smem_bytes;
   pl.is_causal = is_causal;
   pl.is_local = is_local;
   pl.window_left = wl;
   pl.window_right = wr;
-  pl.launches = ns > 1 && !out->cluster ? 2 : 1;
-  pl.workspace_bytes = ns > 1 ? (((size_t)ns * lse_elems * sizeof(float) + 15) & ~(size_t)15) + (size_t)ns * lse_elems * a.d * sizeof(float) : 0;
+  const bool partials = ns > 1 && !out->cluster;
+  pl.launches = partials ? 2 : 1;
+  pl.workspace_bytes = partials ? (((size_t)ns * lse_elems * sizeof(float) + 15) & ~(size_t)15) + (size_t)ns * lse_elems * a.d * sizeof(float) : 0;
   if (base * ns > 0x7fffffffLL) return fail(FA_ERR_UNSUPPORTED, "grid too large");
 
   KParams& kp = out->kp;
@@ -380,9 +389,9 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
   kp.gp = gp;
   kp.heads_eff = heads_eff;
   kp.m_blocks = m_blocks;
-  kp.num_splits = ns;
+  kp.num_splits = out->cluster ? out->cluster : ns;
   kp.blocks_per_split = bps;
-  kp.persistent = persistent ? 1 : 0;
+  kp.persistent = persistent && !out->cluster ? 1 : 0;
   kp.scale_log2 = a.softmax_scale * kLog2e;
   kp.lse_elems = lse_elems;
 
@@ -390,6 +399,7 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
   if (a.kernel != FA_KERNEL_MMA && a.kernel != FA_KERNEL_DECODE && !(a.kernel == FA_KERNEL_AUTO && few_tiles_long_range(a)) &&
       tc5_eligible(a, is_causal, is_local, wl_on_device)) {
     tc5_fill_plan(a, &pl);
+    out->cluster = 0;
   } else if (a.kernel == FA_KERNEL_TCGEN05) {
     return fail(FA_ERR_UNSUPPORTED, "the tcgen05 kernel does not cover this problem");
   }
@@ -442,8 +452,7 @@ static int run_fwd(const fa_fwd_params& a, Workspace& ws, cudaStream_t st, const
   int rc = make_plan(a, &P, forced);
   if (rc != FA_OK) return rc;
   if (a.total_q == 0 || a.seqlen_q == 0) return FA_OK;
-  if (P.pl.kernel != FA_KERNEL_DECODE) P.cluster = 0;
-  if (P.pl.workspace_bytes && !P.cluster) {
+  if (P.pl.workspace_bytes) {
     if (!ws.get(P.pl.workspace_bytes)) return fail(FA_ERR_WORKSPACE, "workspace missing or too small");
     if ((reinterpret_cast<uintptr_t>(ws.ptr) & 15) != 0) return fail(FA_ERR_WORKSPACE, "workspace must be 16-byte aligned");
   }
@@ -494,13 +503,7 @@ static int run_fwd(const fa_fwd_params& a, Workspace& ws, cudaStream_t st, const
     auto* launch = P.hd_pad == 64    ? (bf ? launch_decode_64_bf16 : launch_decode_64_fp16)
                    : P.hd_pad == 128 ? (bf ? launch_decode_128_bf16 : launch_decode_128_fp16)
                                      : (bf ? launch_decode_256_bf16 : launch_decode_256_fp16);
-    if (P.cluster) {
-      kp.num_splits = P.cluster;
-      kp.persistent = 0;
-      e = launch(kDecodeClusterConfig, kp, tm_k, tm_v, kp.heads_eff * a.b * P.cluster, st);
-    } else {
-      e = launch(P.pl.config, kp, tm_k, tm_v, P.pl.grid, st);
-    }
+    e = launch(P.cluster ? kDecodeClusterConfig : P.pl.config, kp, tm_k, tm_v, P.pl.grid, st);
   } else
   switch (P.hd_pad) {
     case 64: e = bf ? launch_mma_64_bf16(P.pl.config, kp, P.pl.grid, st) : launch_mma_64_fp16(P.pl.config, kp, P.pl.grid, st); break;

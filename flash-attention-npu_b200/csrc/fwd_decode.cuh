@@ -22,7 +22,8 @@ namespace fa {
 
 // Consumer warps form a WM x WN grid: WM splits the packed query rows (16 * MT rows per warp), WN
 // splits the keys of a stage.
-constexpr int kDecodeClusterConfig = -3;  // to the launchers: configuration 3, key splits as one thread-block cluster
+constexpr int kDecodeClusterBase = 3;     // the tile configuration (decode_configs.cuh) that is also built for clusters
+constexpr int kDecodeClusterConfig = -3;  // to the launchers: that configuration, key splits as one thread-block cluster
 constexpr int kDecodeMaxCluster = 8;      // the portable limit
 
 template <int HD_, typename T_, int MT_, int WM_, int WN_, int BN_, int ST_, int SR_ = 0>

@@ -124,11 +124,14 @@ typedef struct fa_fwd_params {
 
 typedef struct fa_fwd_plan {
   int32_t kernel;       /* enum fa_kernel_id actually chosen */
-  int32_t config;       /* tile configuration index inside that kernel family */
+  int32_t config;       /* tile configuration index inside that kernel family; decode kernel: + 256 x the CTAs of a cluster when
+                           the key splits of a unit (batch entry, packed head group) are the CTAs of one thread-block cluster */
   int32_t pack_gqa;     /* 1: the query heads of one kv head share a tile */
   int32_t block_m, block_n;
   int32_t m_blocks;
-  int32_t num_splits;   /* KV splits launched (1 = none) */
+  int32_t num_splits;   /* KV splits with partials in the workspace (1 = none); 0 blocks_per_split: most partials of a unit when
+                           resident CTAs share all blocks.  A clustered call launches neither: the two then say how it would
+                           be shared out without clusters */
   int32_t blocks_per_split;
   int32_t grid, threads, smem_bytes; /* grid: of the tcgen05 kernel's fixed deal; ragged input with more tiles than SMs launches a CTA per tile */
   int32_t is_causal, is_local, window_left, window_right; /* after host normalisation */

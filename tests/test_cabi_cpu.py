@@ -309,3 +309,36 @@ def test_plan_tcgen05_prefill_covers_head_dims_up_to_256_and_softcap():
     assert rc == 0 and pl.kernel == L.KERNEL_MMA
     rc, pl = _plan(dense(128, kernel=L.KERNEL_TCGEN05, sq=100))
     assert rc != 0  # forced, but the problem is not covered
+
+
+def _decode(b, h, hk, d, keys, **kw):
+    return _params(**{**dict(b=b, h=h, h_k=hk, d=d, seqlen_k=keys, total_q=b, seqused_k=256, causal=1, q_batch_stride=h * d, q_row_stride=h * d,
+                             q_head_stride=d, lse_batch_stride=h, lse_head_stride=1, k_batch_stride=keys * hk * d, k_row_stride=hk * d,
+                             k_head_stride=d, v_batch_stride=keys * hk * d, v_row_stride=hk * d, v_head_stride=d), **kw})
+
+
+def _clusters(pl):
+    return pl.config // 256 if pl.kernel == L.KERNEL_DECODE else 0
+
+
+@pytest.mark.parametrize("name,value", [("FA_B200_NUM_SPLITS", "3"), ("FA_B200_DECODE_PERSISTENT", "1"), ("FA_B200_DECODE_PERSISTENT_GRID", "100"),
+                                        ("FA_B200_DECODE_CLUSTER", "0")])
+def test_plan_of_a_clustered_call_says_what_is_launched(monkeypatch, name, value):
+    """One launch of units x cluster size CTAs and no workspace; the plan's bytes keep it, and the overrides of the other schedules replace it."""
+    p = _decode(1, 32, 8, 128, 2048)
+    rc, pl = _plan(p)
+    assert rc == 0 and pl.kernel == L.KERNEL_DECODE and pl.config % 256 == 3 and _clusters(pl) == 8
+    assert pl.grid == 8 * 8 and pl.launches == 1 and pl.workspace_bytes == 0
+    buf, kept = C.create_string_buffer(L.PLAN_BYTES), L.FwdPlan()
+    assert L.load().fa_b200_plan_encode(C.byref(p), buf, L.PLAN_BYTES) == 0 and L.load().fa_b200_plan_decode(buf, L.PLAN_BYTES, C.byref(kept)) == 0
+    assert bytes(kept) == bytes(pl)
+    for kw in (dict(num_splits=1), dict(num_splits=2), dict(partial_out=1)):
+        rc, other = _plan(_decode(1, 32, 8, 128, 2048, **kw))
+        assert rc == 0 and _clusters(other) == 0
+    monkeypatch.setenv(name, value)
+    rc, pl = _plan(p)
+    assert rc == 0 and _clusters(pl) == 0 and pl.launches == 2 and pl.workspace_bytes > 0
+    if name == "FA_B200_NUM_SPLITS":
+        assert pl.num_splits == 3 or pl.blocks_per_split == 0
+    if name == "FA_B200_DECODE_PERSISTENT_GRID":
+        assert pl.grid == 100

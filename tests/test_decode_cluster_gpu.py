@@ -58,3 +58,33 @@ def test_clustered_decode(dtype, d, b, hk, group, s_q, room, page, append, windo
         U.check_rules(out, lse, go, gl, tag=f"d {d} b {b}")
     assert L.load().fa_b200_launch_count() - n0 == 2  # no merge launch
     assert torch.equal(kc_g.cpu().view(torch.int16), kc_o.view(torch.int16)) and torch.equal(vc_g.cpu().view(torch.int16), vc_o.view(torch.int16))
+
+
+@pytest.mark.parametrize("b,hk,room,lens,window,cluster", [
+    (1, 8, 32768, [30000], 1024, True), (4, 8, 400, [400, 3, 250, 399], -1, True), (1, 8, 2048, [2000], -1, True),
+    (1, 8, 2048, [2000], -1, False), (4, 8, 400, [400, 3, 250, 399], -1, False), (3, 2, 600, [0, 0, 0], -1, True)])
+def test_a_plan_runs_what_it_says(monkeypatch, b, hk, room, lens, window, cluster):
+    """A planned call makes the plan's launches and gives the bits of the call that is planned on the spot, for plans with clusters and
+    for plans that were made without them."""
+    import ctypes as C
+    import flash_attn_npu_v3 as fa3
+    g = torch.Generator().manual_seed(room)
+    d, h = 128, 4 * hk
+    q, k, v = U.normal((b, 1, h, d), BF, g).cuda(), U.normal((b, room, hk, d), BF, g).cuda(), U.normal((b, room, hk, d), BF, g).cuda()
+    lens_g = torch.tensor(lens, dtype=torch.int32).cuda()
+    if not cluster:
+        monkeypatch.setenv("FA_B200_DECODE_CLUSTER", "0")
+    kw = dict(cache_seqlens=lens_g, causal=True, window_size=(window, -1), return_softmax_lse=True)
+    plan = fa3.get_scheduler_metadata(b, 1, room, h, hk, d, lens_g, qkv_dtype=BF, causal=True, window_size=(window, -1))
+    raw, pl = bytes(plan.cpu().numpy().tobytes()), L.FwdPlan()
+    L.check(L.load().fa_b200_plan_decode(raw, len(raw), C.byref(pl)))
+    want = fa3.flash_attn_with_kvcache(q, k, v, **kw)[:2]
+    monkeypatch.delenv("FA_B200_DECODE_CLUSTER", raising=False)
+    n0 = L.load().fa_b200_launch_count()
+    got = fa3.flash_attn_with_kvcache(q, k, v, scheduler_metadata=plan, **kw)[:2]
+    assert L.load().fa_b200_launch_count() - n0 == pl.launches
+    assert (pl.config // 256 > 1) == cluster
+    for x, y in zip(want, got):
+        assert torch.equal(x, y)
+    go, gl = OA.flash_attn_with_kvcache(q.cpu(), k.cpu(), v.cpu(), cache_seqlens=lens_g.cpu(), causal=True, window_size=(window, -1))
+    U.check_rules(got[0], got[1], go, gl, tag=f"planned {b} {room}")
