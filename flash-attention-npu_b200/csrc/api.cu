@@ -347,12 +347,19 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
     const long long per_sm = std::max(1, (227 * 1024) / std::max(1, ci.smem_bytes));
     int cs = kDecodeMaxCluster;
     while (cs > 1 && (cs > max_blocks || base * cs > (per_sm > 1 ? num_sm : cs > 2 ? num_sm / 2 : num_sm * 7 / 8))) cs >>= 1;
-    // Worth it while a call is bound by latencies and not by the chip's memory rate.  us a call, merge launch / cluster, 8 kv
-    // heads: one sequence of 512 .. 2048 .. 3072 keys 16.5 / 10.6, 14.1 / 10.9, 15.3 / 12.8, of 4096 14.1 / 14.7 (the other half
-    // of the chip is idle); two of 4096 19.2 / 16.8, four of 2048 19.8 / 16.9, eight of 1024 19.8 / 17.1, of 2048 23.7 / 25.3.
-    // Head dim 64: one sequence of 6144 15.1 / 13.6, of 8192 13.9 / 16.0; 256: one of 8192 30.0 / 27.3, of 12288 35.9 / 36.1.
-    // Several sequences may differ in length, and a cluster's share follows the longest: 512 keys a CTA.
-    const int most = a.b > 1 ? 512 : hd_pad == 64 ? 768 : hd_pad == 128 ? 384 : 1024;
+    // Worth it while a call is bound by latencies and not by what the clusters' few CTAs can stream, so the most keys a CTA may
+    // have follow the units: with few of them the other schedule has most of the chip to itself.  us a call in a CUDA graph with
+    // K / V from HBM, other schedule / clusters, 4 query heads per kv head, units x keys:
+    //   64 columns   1 x 6144 12.6 / 12.5, 2 x 6144 13.5 / 13.0, 16 x 6144 17.7 / 14.8 (back to back 15.1 / 12.6 for one unit)
+    //   128 columns  1 x 3072 13.1 / 11.4, 2 x 4096 13.2 / 13.8, 4 x 4096 (lengths 512 - 4096) 13.7 / 13.7, 8 x 4096 15.5 / 14.3,
+    //                16 x 4096 18.6 / 15.7
+    //   256 columns  1 x 3584 18.4 / 15.8, 1 x 4096 16.8 / 16.9, 1 x 8192 17.9 / 25.5, 4 x 8192 21.9 / 26.0, 8 x 8192 30.0 / 26.5;
+    //                clusters of 2: 32 x 1024 22.5 / 18.0, 32 x 2048 (head dim 192) 26.5 / 26.5
+    // A plain launch (ranges that the other schedule does not cut) loses to clusters at every size down to 128 keys: 8 units of
+    // 384 keys 64 columns 0.94 x, 128 columns 0.73 x.  Several sequences may differ in length, and a cluster's share follows the
+    // longest: measured with lengths down to an eighth up to 512 keys a CTA (0.6 - 0.95 x).
+    int most = hd_pad == 64 ? (base < 2 ? 640 : 768) : hd_pad == 128 ? (base < 8 ? 384 : 512) : base < 8 ? 448 : cs == 2 ? 768 : 1024;
+    if (a.b > 1) most = std::min(most, 512);
     bool use = cs > 1 && ceil_div(max_blocks, cs) * ci.block_n <= most;
     if (const char* e = std::getenv("FA_B200_DECODE_CLUSTER")) use = cs > 1 && std::atoi(e) != 0;  // tuning override
     if (use) out->cluster = cs;

@@ -342,3 +342,16 @@ def test_plan_of_a_clustered_call_says_what_is_launched(monkeypatch, name, value
         assert pl.num_splits == 3 or pl.blocks_per_split == 0
     if name == "FA_B200_DECODE_PERSISTENT_GRID":
         assert pl.grid == 100
+
+
+@pytest.mark.parametrize("b,hk,d,keys,clusters", [
+    (1, 1, 64, 5120, 8), (1, 1, 64, 6144, 0), (1, 2, 64, 6144, 8), (8, 1, 64, 4096, 8), (8, 1, 64, 4224, 0),
+    (1, 1, 128, 3072, 8), (1, 1, 128, 3136, 0), (2, 1, 128, 4096, 0), (1, 2, 128, 4096, 0), (8, 1, 128, 4096, 8), (1, 8, 128, 4096, 8), (8, 1, 128, 4160, 0),
+    (1, 1, 256, 3584, 8), (1, 1, 256, 8192, 0), (4, 1, 256, 4096, 0), (1, 4, 256, 8192, 0), (1, 8, 256, 8192, 8), (8, 1, 256, 8192, 0),
+    (1, 32, 256, 1024, 2), (1, 32, 256, 2048, 0), (3, 2, 96, 1, 0), (3, 2, 96, 100, 2), (200, 8, 128, 512, 0)])
+def test_clusters_follow_the_units_and_the_keys(b, hk, d, keys, clusters):
+    """Both sides of the line for few and many units (sequences x kv heads), whichever of the two they are."""
+    rc, pl = _plan(_decode(b, 4 * hk, hk, d, keys))
+    assert rc == 0 and pl.kernel == L.KERNEL_DECODE and _clusters(pl) == clusters
+    if clusters:
+        assert pl.grid == b * hk * clusters and pl.launches == 1
