@@ -13,12 +13,32 @@
 //   5   17-32 rows, long key ranges or persistent launches.  128: one CTA of 2 x 4 warps, 128-key stages; 64: two such
 //       CTAs; 256: one CTA of 2 x 2 warps and five 32-key stages (the fp32 merge slab of 32 rows takes 33 KiB)
 //   11  128 only: 17-32 rows, short key ranges (a sliding window): two resident CTAs of 2 x 2 warps, slab over the ring
-// Configuration 3 is built a second time with the key splits of a unit in one thread-block cluster (kDecodeClusterConfig).
+// Configuration 3 (kDecodeClusterBase) is built a second time with the key splits of a unit in one thread-block cluster
+// (kDecodeClusterConfig).
 #define FA_DECODE_CONFIGS_64(X) X(3, 1, 1, 4, 128, 3, 0) X(5, 1, 2, 4, 128, 3, 0)
 #define FA_DECODE_CONFIGS_128(X) X(3, 1, 1, 4, 64, 3, 0) X(5, 1, 2, 4, 128, 3, 0) X(11, 1, 2, 2, 64, 3, 1)
 #define FA_DECODE_CONFIGS_256(X) X(3, 1, 1, 4, 64, 3, 0) X(5, 1, 2, 2, 32, 5, 0)
 
 namespace fa {
+
+// The traits of configuration I, as listed above (the planner and the TMA boxes read the same list).
+template <int HD, typename T, int I>
+struct DecConfig;
+#define FA_X(I_, MT_, WM_, WN_, BN_, ST_, SR_)                              \
+  template <typename T>                                                     \
+  struct DecConfig<FA_HD_, T, I_> {                                         \
+    using Tr = DecTraits<FA_HD_, T, MT_, WM_, WN_, BN_, ST_, SR_>;          \
+  };
+#define FA_HD_ 64
+FA_DECODE_CONFIGS_64(FA_X)
+#undef FA_HD_
+#define FA_HD_ 128
+FA_DECODE_CONFIGS_128(FA_X)
+#undef FA_HD_
+#define FA_HD_ 256
+FA_DECODE_CONFIGS_256(FA_X)
+#undef FA_HD_
+#undef FA_X
 
 struct DecodeConfigInfo {
   int block_m, block_n, threads, smem_bytes;

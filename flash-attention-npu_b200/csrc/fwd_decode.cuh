@@ -65,10 +65,6 @@ struct DecTraits {
   static_assert(NW % 16 == 0, "each consumer warp needs a multiple of 16 keys");
 };
 
-// Configuration 3 (decode_configs.cuh), the one that also runs as clusters.
-template <int HD, typename T>
-using DecClusterTraits = DecTraits<HD, T, 1, 1, 4, HD == 64 ? 128 : 64, 3, 0>;
-
 // Address of 16-byte chunk `ch` (0 .. HD / 8 - 1) of row `row` in a K / V tile laid out by TMA boxes of
 // 64 columns with the 128-byte swizzle (chunk index XOR row % 8 inside each 128-byte row).
 template <class Tr>
