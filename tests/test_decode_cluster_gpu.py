@@ -6,6 +6,7 @@ import torch
 
 import parity_util as U
 from flash_b200 import lib as L
+from flash_b200 import ops
 from oracle import api as OA
 
 pytestmark = pytest.mark.gpu
@@ -26,14 +27,14 @@ def test_splits_that_are_asked_for_are_kept():
         U.check_rules(out, lse, go, gl, tag=f"splits {splits}")
 
 
-@pytest.mark.parametrize("dtype,d,b,hk,group,s_q,room,page,append,window,softcap", [
-    (BF, 128, 1, 8, 4, 1, 2048, 0, False, -1, 0.0),     # clusters of 8
-    (FP, 64, 3, 4, 8, 2, 700, 128, True, -1, 0.0),      # 16 rows; sequences with fewer blocks than CTAs
-    (BF, 256, 5, 6, 2, 1, 1000, 256, True, 300, 0.0),   # clusters of 2, a window
-    (BF, 96, 16, 4, 1, 3, 513, 0, False, -1, 30.0),     # clusters of 2
-    (FP, 136, 4, 2, 4, 4, 130, 128, False, 40, 0.0),    # a range of three key blocks
-    (BF, 128, 2, 2, 16, 1, 129, 0, True, -1, 0.0)])
-def test_clustered_decode(dtype, d, b, hk, group, s_q, room, page, append, window, softcap):
+@pytest.mark.parametrize("dtype,d,b,hk,group,s_q,room,page,append,window,softcap,cluster", [
+    (BF, 128, 1, 8, 4, 1, 2048, 0, False, -1, 0.0, 8),
+    (FP, 64, 3, 4, 8, 2, 700, 128, True, -1, 0.0, 4),      # 16 rows; sequences with fewer blocks than CTAs
+    (BF, 256, 5, 6, 2, 1, 1000, 256, True, 300, 0.0, 2),   # a window
+    (BF, 96, 16, 4, 1, 3, 513, 0, False, -1, 30.0, 2),
+    (FP, 136, 4, 2, 4, 4, 130, 128, False, 40, 0.0, 2),    # a range of two key blocks
+    (BF, 128, 2, 2, 16, 1, 129, 0, True, -1, 0.0, 2)])
+def test_clustered_decode(dtype, d, b, hk, group, s_q, room, page, append, window, softcap, cluster):
     import flash_attn_npu_v2 as fa2
     g = torch.Generator().manual_seed(d * 10 + b)
     new = s_q if append else 0
@@ -51,6 +52,9 @@ def test_clustered_decode(dtype, d, b, hk, group, s_q, room, page, append, windo
     kc_o, vc_o, kc_g, vc_g = kc.clone(), vc.clone(), kc.cuda(), vc.cuda()
     kw = dict(causal=True, window_size=(window, -1), softcap=softcap)
     go, gl = OA.flash_attn_with_kvcache(q, kc_o, vc_o, kn, vn, cache_seqlens=lens, block_table=bt, **kw)
+    pl = ops.attention_forward(q.cuda(), kc.cuda(), vc.cuda(), k_new=dev(kn), v_new=dev(vn), seqused_k=lens.cuda(), block_table=dev(bt),
+                               causal=True, window_left=window, softcap=softcap, return_plan=True)[2]
+    assert pl.kernel == L.KERNEL_DECODE and pl.config == 3 + 256 * cluster and pl.grid == b * hk * cluster
     n0 = L.load().fa_b200_launch_count()
     for _ in range(2):  # the appended rows are written again with the same values
         out, lse = fa2.flash_attn_with_kvcache(q.cuda(), kc_g, vc_g, dev(kn), dev(vn), cache_seqlens=lens.cuda(), block_table=dev(bt),

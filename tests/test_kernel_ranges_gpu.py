@@ -300,3 +300,79 @@ def test_backward_of_many_short_sequences(dtype, d, causal):
     ops.attention_backward(dout.cuda(), q.cuda(), k.cuda(), v.cuda(), out, lse, dq=grads[0], dk=grads[1], dv=grads[2], **kw)
     _check_gradients(grads, OB.attention_varlen_backward(q, k, v, dout, lse.cpu(), cu, cu, softmax_scale=d ** -0.5, causal=causal,
                                                          window=(-1, -1)))
+
+
+SCHEDULES = {"plain": (dict(num_splits=1), 1, 1), "splits": (dict(num_splits=2), 2, 2), "shared": (dict(), 2, 5)}  # arguments, launches, least splits
+
+
+@pytest.mark.parametrize("schedule", SCHEDULES)
+@pytest.mark.parametrize("rows", [1, 16])
+@pytest.mark.parametrize("d", [64, 72, 96, 128, 136, 192, 256])
+def test_decode_kernel_without_clusters(monkeypatch, d, rows, schedule):
+    """Up to 16 packed rows on one CTA per unit, on key splits with partials and on equal shares of all blocks; new tokens appended
+    with rotary; lengths around the key blocks' edges."""
+    monkeypatch.setenv("FA_B200_DECODE_CLUSTER", "0")
+    g = torch.Generator().manual_seed(d * 100 + rows)
+    dtype = BF if rows % 2 else FP
+    hk, group, s_q = 2, {1: 1, 16: 8}[rows], {1: 1, 16: 2}[rows]
+    new, room = s_q, 1300
+    lens = torch.tensor([0, 1, 127, 128, 700, room - new], dtype=torch.int32)
+    b, rotary = lens.numel(), d // 16 * 16
+    q, (kc, vc, _) = U.normal((b, s_q, hk * group, d), dtype, g), _cache(g, dtype, b, room, hk, d, 0)
+    k, v = U.normal((b, new, hk, d), dtype, g), U.normal((b, new, hk, d), dtype, g)
+    cos, sin = U.rotary_tables(room, rotary, dtype)
+    kw, launches, least = SCHEDULES[schedule]
+    kc_g, vc_g = kc.cuda(), vc.cuda()
+    n0 = L.load().fa_b200_launch_count()
+    out, lse, pl = ops.attention_forward(q.cuda(), kc_g, vc_g, k_new=k.cuda(), v_new=v.cuda(), seqused_k=lens.cuda(), rotary_cos=cos.cuda(),
+                                         rotary_sin=sin.cuda(), rotary_interleaved=False, causal=True, softmax_scale=d ** -0.5, return_plan=True, **kw)
+    assert L.load().fa_b200_launch_count() - n0 == launches == pl.launches
+    assert pl.kernel == L.KERNEL_DECODE and pl.config == 3 and pl.num_splits >= least and (pl.blocks_per_split == 0) == (schedule == "shared")
+    go, gl = OA.flash_attn_with_kvcache(q, kc, vc, k, v, rotary_cos=cos, rotary_sin=sin, cache_seqlens=lens, causal=True,
+                                        rotary_interleaved=False)  # appends to kc, vc
+    assert torch.equal(kc_g.cpu().view(torch.int16), kc.view(torch.int16)) and torch.equal(vc_g.cpu().view(torch.int16), vc.view(torch.int16))
+    U.check_rules(out, lse, go, gl, tag=f"d {d} rows {rows} {schedule}")
+
+
+@pytest.mark.parametrize("schedule", SCHEDULES)
+def test_alibi_without_clusters(monkeypatch, schedule):
+    monkeypatch.setenv("FA_B200_DECODE_CLUSTER", "0")
+    g = torch.Generator().manual_seed(5)
+    b, h, hk, d, room = 3, 6, 3, 128, 1300
+    q, kc, vc = U.normal((b, 2, h, d), FP, g), U.normal((5, room, hk, d), FP, g), U.normal((5, room, hk, d), FP, g)
+    lens, idx = torch.tensor([10, 1250, 640], dtype=torch.int32), torch.tensor([4, 0, 2], dtype=torch.int32)
+    slopes = torch.rand(b, h, generator=g) * 0.3
+    kw, launches, _ = SCHEDULES[schedule]
+    for causal in (False, True):
+        out, lse, pl = ops.attention_forward(q.cuda(), kc.cuda(), vc.cuda(), seqused_k=lens.cuda(), cache_batch_idx=idx.cuda(), causal=causal,
+                                             alibi_slopes=slopes.cuda(), softmax_scale=d ** -0.5, return_plan=True, **kw)
+        assert pl.kernel == L.KERNEL_DECODE and pl.config == 3 and pl.launches == launches
+        go, gl = OA.flash_attn_with_kvcache(q, kc, vc, cache_seqlens=lens, cache_batch_idx=idx, causal=causal, alibi_slopes=slopes)
+        U.check_rules(out, lse, go, gl, tag=f"alibi {schedule}")
+
+
+@pytest.mark.parametrize("b,hk,d,keys", [(1, 8, 128, 4500), (1, 8, 128, 2048), (3, 4, 128, 512)])
+def test_short_sequences_are_cut_over_the_grid_without_clusters(monkeypatch, b, hk, d, keys):
+    """Partials and a merge where clusters are switched off, up to and behind the range that they take."""
+    monkeypatch.setenv("FA_B200_DECODE_CLUSTER", "0")
+    n0 = L.load().fa_b200_launch_count()
+    test_few_sequences_are_cut_over_the_grid(b, hk, d, keys)
+    assert L.load().fa_b200_launch_count() - n0 == 2
+
+
+@pytest.mark.parametrize("d,h", [(128, 32), (192, 24)])
+def test_backward_item_order_of_streams_beyond_l2(d, h):
+    """The causal backward takes a pair at a time when the streamed tensors exceed 96 MB, and the blocks of all pairs together below:
+    a head's gradients are the same to the bit."""
+    g = torch.Generator().manual_seed(d)
+    b, s, part = 1, 8192, 8
+    assert 4 * b * s * h * d > 96 << 20 >= 4 * b * s * part * d
+    q, k, v, dout = (t.cuda() for t in _backward_inputs(g, BF, (b, s), (b, s), h, h, d))
+    kw = dict(softmax_scale=d ** -0.5, causal=True)
+    out, lse = ops.attention_forward(q, k, v, **kw)
+    grads = ops.attention_backward(dout, q, k, v, out, lse, **kw)
+    for h0 in range(0, h, part):
+        at = [t[:, :, h0:h0 + part].contiguous() for t in (dout, q, k, v, out)]
+        some = ops.attention_backward(*at, lse[:, h0:h0 + part].reshape(-1).view(b, part, s), **kw)
+        for all_heads, x in zip(grads, some):
+            assert torch.equal(all_heads[:, :, h0:h0 + part], x), h0
