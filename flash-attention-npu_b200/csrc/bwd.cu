@@ -20,11 +20,14 @@ void count_launches(int n);                      // api.cu: fa_b200_launch_count
 static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 // Pairs per chunk of the work-item order (item_place in tile_order.cuh): all of them when what they stream (two 16-bit
-// tensors of `rows` rows and `heads` heads) stays in L2 together, otherwise one (the 4 K causal case, 268 MB, in chunks of ten
-// pairs: dK / dV kernel 917 -> 1017 us).  Only a causal mask makes the blocks of a pair unequal; without one a pair at a time.
-static int bwd_chunk(bool causal, int pairs, int64_t rows, int heads, int d) {
-  constexpr int64_t kL2Budget = 96ll << 20;
-  return causal && 4 * rows * heads * d <= kL2Budget ? pairs : 1;
+// tensors of `rows` rows and `heads` heads) stays in L2 together, otherwise one.  Forward and backward, all pairs against one
+// at a time: 14 - 60 MB 0.89 - 0.98 x, 64 - 88 MB 0.98 - 1.00 x, 92 - 96 MB 0.99 - 1.035 x (b 24, s 512, 16 heads, d 128: 298
+// -> 309 us), 104 - 114 MB 1.01 - 1.06 x; the 4 K causal case, 268 MB, in chunks of ten pairs: dK / dV kernel 917 -> 1017 us.
+// With grouped heads the dK / dV items are fewer and longer, and balance is worth more: 96 MB 1306 -> 1252 us (b 3, s 4096, 32 / 8
+// heads, d 64).  Only a causal mask makes the blocks of a pair unequal; without one a pair at a time.
+static int bwd_chunk(bool causal, int pairs, int64_t rows, int heads, int d, bool grouped) {
+  const int64_t budget = (grouped ? 96ll : 88ll) << 20;
+  return causal && 4 * rows * heads * d <= budget ? pairs : 1;
 }
 
 template <int HD, typename T>
@@ -122,8 +125,8 @@ int fa_b200_bwd(const fa_bwd_params* a, void* workspace, size_t workspace_bytes,
   p.softcap = a->softcap;
   {
     const int64_t k_rows = varlen ? a->total_k : (int64_t)a->b * a->seqlen_k;
-    p.chunk_kv = bwd_chunk(p.is_causal, a->h_k * a->b, rows, a->h, a->d);
-    p.chunk_q = bwd_chunk(p.is_causal, a->h * a->b, k_rows, a->h_k, a->d);
+    p.chunk_kv = bwd_chunk(p.is_causal, a->h_k * a->b, rows, a->h, a->d, a->h > a->h_k);
+    p.chunk_q = bwd_chunk(p.is_causal, a->h * a->b, k_rows, a->h_k, a->d, a->h > a->h_k);
   }
   const size_t acc_bytes = bwd_accum_bytes(a, rows);
   p.dq_accum = reinterpret_cast<float*>(workspace);
