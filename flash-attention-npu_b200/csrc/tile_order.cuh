@@ -45,13 +45,13 @@ FA_TILE_HD bool tile_locate(TileCursor& c, const Levels& lv, int heads_all, int 
   return true;
 }
 
-// Order of the backward's work items, shared with a host test too.  An item is a block of 128 keys or rows of a (batch entry, head) pair.  Items near one another
-// should stream the same tiles (from L2), which asks for a pair's blocks to be neighbours; but under a causal mask a pair's
+// Order of the backward's work items, shared with a host test too.  An item is a block of 128 keys or rows of a (batch entry,
+// head) pair.  Items near one another should stream the same tiles (from L2), which asks for a pair's blocks to be neighbours; but under a causal mask a pair's
 // blocks differ by up to the length of the sequence, and a launch that ends on the heavy blocks of its last pair leaves most
 // CTAs idle meanwhile.  So the pairs are cut into chunks, and a chunk runs block 0 of all its pairs, then block 1, and so on
-// (bwd_chunk in bwd.cu; a chunk of one pair is the plain order).   Without the chunks 12 packed
-// sequences of 37 - 2999 rows (16 heads of 4 groups, head dim 64) took 711 us forward and backward, with them 677; b 2, s 1777,
-// 8 heads, head dim 256 (bwd_wide_kernel): backward kernel 175 -> 148 us.
+// (bwd_chunk in bwd.cu; a chunk of one pair is the plain order).  One pair at a time / all pairs together, forward and
+// backward: 12 packed sequences of 37 - 2999 rows (16 heads of 4 groups, head dim 64) 635 / 607 us; b 2, s 1777, 8 heads, head
+// dim 256 (bwd_wide_kernel) 208 / 192 us.
 struct ItemPlace {
   int pair, block;
 };
