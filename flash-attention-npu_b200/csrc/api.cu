@@ -399,6 +399,7 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
   kp.num_splits = out->cluster ? out->cluster : ns;
   kp.blocks_per_split = bps;
   kp.persistent = persistent && !out->cluster ? 1 : 0;
+  kp.overlap = pl.grid <= num_sm ? 1 : 0;
   kp.scale_log2 = a.softmax_scale * kLog2e;
   kp.lse_elems = lse_elems;
 

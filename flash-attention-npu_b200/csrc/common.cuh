@@ -25,6 +25,7 @@ struct KParams {
   int32_t m_blocks;
   int32_t num_splits, blocks_per_split;
   int32_t persistent;  // decode kernel: persistent CTAs with equal shares of the KV blocks; num_splits = partial slots
+  int32_t overlap;     // mma.sync kernel: launched so that it starts under the end of the kernel in front (launch_dependent)
   float scale_log2;   // softmax_scale * log2(e)   (softcap: log2(e) only, see kernel)
   float* o_partial;   // [split][lse_index][d] fp32 (num_splits > 1)
   float* lse_partial; // [split][lse_index]
@@ -46,8 +47,10 @@ cudaError_t allow_smem(const void* kernel, int bytes);
 // three kernels hold their SMs' shared memory while they wait.  131 drawn decode calls of 8 - 30 us against the ordinary
 // launch: back to back 7.5 % faster, in a CUDA graph 1.2 % (worst call 2.3 % slower); with both triggers in front 5 % faster,
 // in a graph 0.3 % slower (worst 8.6 %).
-// The mma.sync and tcgen05 kernels keep the ordinary launch: one chunk of 128 rows, 8 heads, 2404 keys (mma.sync) 57.4 -> 61.5
-// us, prefill with softcap, head dim 256 (tcgen05) 101.6 -> 109, chunked prefill 499 -> 504.
+// The mma.sync kernel is launched so where its grid has no more CTAs than the GPU has SMs (KParams::overlap), so that the next
+// kernel's fit beside them: 20 calls of 16 - 128 CTAs 0.83 - 1.00 x back to back, 0.97 - 1.00 x in a graph; 8 calls of 192 - 880
+// CTAs 0.94 - 1.00 x and 0.98 - 1.07 x.  The tcgen05 kernels keep the ordinary launch: prefill with softcap, head dim 256, 101.6
+// -> 109 us, chunked prefill 499 -> 504.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 template <typename... Params, typename... Args>

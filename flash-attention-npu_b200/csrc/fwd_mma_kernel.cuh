@@ -13,7 +13,8 @@ __global__ void __launch_bounds__(Tr::NTHREADS) fwd_mma_kernel(const __grid_cons
   __shared__ int s_red[32];
   __shared__ float s_lse[Tr::BM];
 
-  grid_trigger();  // a merge kernel queued behind this one may start launching its CTAs now (they wait for this grid to complete)
+  grid_wait();
+  grid_trigger();  // a kernel queued behind this one may start launching its CTAs now (they wait for this grid to complete)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp / Tr::WN, wn = warp % Tr::WN;
   const int g8 = lane >> 2, t4 = lane & 3;
