@@ -255,7 +255,9 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
     long long want = (per_sm * num_sm + base - 1) / base;
     ns = (int)std::max(1LL, std::min<long long>(want, max_blocks / 8));
   }
+  bool overridden = false;  // a tuning override asks for a schedule without clusters
   if (const char* e = std::getenv("FA_B200_NUM_SPLITS")) {  // tuning override of the split heuristic
+    overridden = true;
     if (a.num_splits == 0) ns = std::max(1, std::min(std::atoi(e), max_blocks));
   }
   int bps = ceil_div(max_blocks, ns);
@@ -275,7 +277,10 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
     const bool window_bound = is_local && wl >= 0 && range < max_k_bound;
     const long long resident = std::max(1, (227 * 1024) / std::max(1, ci.smem_bytes));
     persist_grid = (long long)num_sm * resident;
-    if (const char* e = std::getenv("FA_B200_DECODE_PERSISTENT_GRID")) persist_grid = std::max(1, std::atoi(e));  // tuning override
+    if (const char* e = std::getenv("FA_B200_DECODE_PERSISTENT_GRID")) {  // tuning override
+      overridden = true;
+      persist_grid = std::max(1, std::atoi(e));
+    }
     // (a unit cut into grid / base shares touches up to two CTAs more than whole shares.)  A share is two blocks at
     // least: the merge reads every slot (one sequence, one kv head, 1560 keys: 298 slots 28.7 us, 14 slots 18).
     if (persist_grid / base > 3)
@@ -302,8 +307,10 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
       const double shared = (double)base * (max_blocks + fixed) / persist_grid + fixed;
       persistent = waves >= 2 && a.d >= 128 && shared < 0.85 * plain;
     }
-    if (const char* e = std::getenv("FA_B200_DECODE_PERSISTENT"))  // tuning override: 0 off, 1 ragged ranges only, 2 wherever possible
+    if (const char* e = std::getenv("FA_B200_DECODE_PERSISTENT")) {  // tuning override: 0 off, 1 ragged ranges only, 2 wherever possible
+      overridden = true;
       persistent = can_persist && (std::atoi(e) == 2 || (std::atoi(e) == 1 && !window_bound));
+    }
     if (forced && forced->kernel == FA_KERNEL_DECODE && !forced_cluster && forced->num_splits > 1 && forced->blocks_per_split == 0) {
       if (!can_persist || forced->grid <= 0 || forced->num_splits < kMinPersistSlots)
         return fail(FA_ERR_UNSUPPORTED, "the plan's persistent decode schedule does not fit this problem");
@@ -340,8 +347,7 @@ static int make_plan(const fa_fwd_params& a_in, Planned* out, const fa_fwd_plan*
     if (!can_cluster || forced_cluster < 2 || forced_cluster > kDecodeMaxCluster)
       return fail(FA_ERR_UNSUPPORTED, "the plan's clusters do not fit this problem");
     out->cluster = forced_cluster;
-  } else if (can_cluster && !forced && !std::getenv("FA_B200_NUM_SPLITS") && !std::getenv("FA_B200_DECODE_PERSISTENT") &&
-             !std::getenv("FA_B200_DECODE_PERSISTENT_GRID")) {
+  } else if (can_cluster && !forced && !overridden) {
     // Clusters of up to 8 CTAs, all resident at once; with one CTA per SM a GPC may not have room for its second cluster
     // of 8 (16 units of head dim 256, 128 CTAs: 17.4 us against 16.5 with a merge launch).
     const long long per_sm = std::max(1, (227 * 1024) / std::max(1, ci.smem_bytes));
