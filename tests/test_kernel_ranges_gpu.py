@@ -376,3 +376,40 @@ def test_backward_item_order_of_streams_beyond_l2(d, h):
         some = ops.attention_backward(*at, lse[:, h0:h0 + part].reshape(-1).view(b, part, s), **kw)
         for all_heads, x in zip(grads, some):
             assert torch.equal(all_heads[:, :, h0:h0 + part], x), h0
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+def test_calls_that_start_under_one_another(d):
+    """Kernels that are launched to start under the end of the one in front: a chain in which every call reads what the call before
+    wrote (its output as q, its keys in the cache) gives the bits of the same chain with a synchronisation behind every call, back to
+    back and in a CUDA graph."""
+    import flash_attn_npu_v2 as fa2
+    g = torch.Generator().manual_seed(d)
+    b, s, h, hk, room = 2, 100, 8, 2, 6000  # 100 rows: the mma.sync kernel, 32 CTAs; the caches: equal shares and key splits
+    q0, k0, v0 = (U.normal((b, s, n, d), BF, g).cuda() for n in (h, hk, hk))
+    kc0, vc0 = (U.normal((b, room, hk, d), BF, g).cuda() for _ in range(2))
+    lens, short = (torch.tensor(t, dtype=torch.int32).cuda() for t in ([5900, 3000], [300, 20]))
+
+    def chain(sync):
+        wait = torch.cuda.synchronize if sync else (lambda: None)
+        kc, vc, x, seen = kc0.clone(), vc0.clone(), q0, []
+        for n in range(6):
+            x = fa2.flash_attn_func(x, k0, v0, causal=True); wait()
+            row = x[:, n:n + 1].contiguous()
+            new = row[:, :, ::4].contiguous()
+            row = fa2.flash_attn_with_kvcache(row, kc, vc, new, new, cache_seqlens=lens + n, causal=True); wait()           # appends
+            row = fa2.flash_attn_with_kvcache(row, kc, vc, cache_seqlens=lens + n + 1, causal=True, num_splits=3); wait()
+            row = fa2.flash_attn_with_kvcache(row, kc[:, :512], vc[:, :512], cache_seqlens=short, causal=True); wait()      # clusters
+            x = x + row
+            seen.append(row)
+        return [x, kc, vc] + seen
+
+    want = [t.clone() for t in chain(True)]
+    for got in (chain(False), chain(False)):
+        assert all(torch.equal(a, c) for a, c in zip(want, got))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(False)
+    for _ in range(3):
+        graph.replay()
+        assert all(torch.equal(a, c) for a, c in zip(want, got))
