@@ -88,6 +88,7 @@ struct Tc5Params {
   int32_t total_tiles;
   float scale_log2;
   float softcap_mul, softcap_l2;  // softcap: scores become softcap_l2 * tanh(s * softcap_mul) in the log2 domain (scale / softcap, softcap * log2 e)
+  int32_t o_sectors;         // rows of O start on 32-byte boundaries and are whole 32-byte sectors long
   int32_t chunk_bh;          // (batch, head) pairs per L2 chunk of the tile order (static_tile)
   int32_t chunk_heads;       // ragged input: query heads per L2 chunk (TileDraw)
   // 1: the rows behind the last key of a sequence hold foreign data (the unused tail of a KV cache or of a page,

@@ -347,6 +347,27 @@ __device__ __forceinline__ void rescale_o(uint32_t o_tmem, float f) {
   tmem_wait_st();
 }
 
+// 64 columns of a row of O, of which the first n_cols exist (head dims between the tile widths: the tiles' other columns are the
+// zeros that the TMA unit fills in).  A warp's store touches 32 rows, a line each, and the load / store unit takes them one by
+// one, whether 16 or 32 bytes go there: with 16 a CTA tile's epilogue held the correction warps, and through them the next tile's
+// first P.V, for some 4000 cycles.  SECTORS stores whole 32-byte sectors, where the rows allow it (o_sectors); 16 / 32 bytes:
+// 12 x 148 heads of 256 rows, head dim 64 102.4 / 95.4 us, head dim 128 127 / 107, of 128 rows, head dim 256 100 / 86;
+// b 4, s 2048, 16 heads, head dim 256, causal 151 / 147; 4 K causal, head dim 128, no difference.
+template <bool SECTORS, typename T>
+__device__ __forceinline__ void store_cols(T* dst, const uint32_t (&w)[32], int n_cols) {
+#pragma unroll
+  for (int c = 0; c < 32; c += SECTORS ? 8 : 4) {
+    if (2 * c >= n_cols) continue;
+    if (SECTORS) {
+      asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(dst + 2 * c), "r"(w[c]), "r"(w[c + 1]), "r"(w[c + 2]),
+                   "r"(w[c + 3]), "r"(w[c + 4]), "r"(w[c + 5]), "r"(w[c + 6]), "r"(w[c + 7])
+                   : "memory");
+    } else {  // written once, read by nobody here: streaming
+      __stcs(reinterpret_cast<uint4*>(dst + 2 * c), make_uint4(w[c], w[c + 1], w[c + 2], w[c + 3]));
+    }
+  }
+}
+
 template <typename T, int IN, int HD>
 __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* bar, uint32_t tmem, int warp_in_wg,
                                                 int lane) {
@@ -394,42 +415,28 @@ __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* ba
       T* o_ptr = reinterpret_cast<T*>(p.a.o) + (int64_t)ti.bi * p.a.o_batch_stride +
                  (int64_t)(ti.q_row0 + i) * p.a.o_row_stride + (int64_t)ti.hh * p.a.o_head_stride;
       const uint32_t o_tmem = tmem + lane_addr + 256 + t * 128;
-      uint32_t a[32], b[32];
-      tmem_ld32(o_tmem, a);
-      tmem_ld32(o_tmem + 32, b);
 #pragma unroll
       for (int half = 0; half < HD / 64; ++half) {
+        uint32_t a[32], b[32];
+        tmem_ld32(o_tmem + half * 64, a);
+        tmem_ld32(o_tmem + half * 64 + 32, b);
         tmem_wait_ld();
-        if (row_valid) {
-#pragma unroll
-          for (int e = 0; e < 32; e += 8) {
-            uint4 w;
-            w.x = pack2<T>(__uint_as_float(a[e]) * inv, __uint_as_float(a[e + 1]) * inv);
-            w.y = pack2<T>(__uint_as_float(a[e + 2]) * inv, __uint_as_float(a[e + 3]) * inv);
-            w.z = pack2<T>(__uint_as_float(a[e + 4]) * inv, __uint_as_float(a[e + 5]) * inv);
-            w.w = pack2<T>(__uint_as_float(a[e + 6]) * inv, __uint_as_float(a[e + 7]) * inv);
-            // written once, read by nobody here: streaming.  Head dims between the two tile widths: the tiles' columns
-            // beyond the head dim are the zeros the TMA unit fills in, and are not stored.
-            if (half * 64 + e < d_cols) __stcs(reinterpret_cast<uint4*>(o_ptr + half * 64 + e), w);
-          }
-#pragma unroll
-          for (int e = 0; e < 32; e += 8) {
-            uint4 w;
-            w.x = pack2<T>(__uint_as_float(b[e]) * inv, __uint_as_float(b[e + 1]) * inv);
-            w.y = pack2<T>(__uint_as_float(b[e + 2]) * inv, __uint_as_float(b[e + 3]) * inv);
-            w.z = pack2<T>(__uint_as_float(b[e + 4]) * inv, __uint_as_float(b[e + 5]) * inv);
-            w.w = pack2<T>(__uint_as_float(b[e + 6]) * inv, __uint_as_float(b[e + 7]) * inv);
-            if (half * 64 + 32 + e < d_cols) __stcs(reinterpret_cast<uint4*>(o_ptr + half * 64 + 32 + e), w);
-          }
+        if (half + 1 == HD / 64) {  // all of O has been read: P.V of the next tile may overwrite it under the last stores
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_addr(&bar->o_free[t]));
         }
-        if (half + 1 < HD / 64) {
-          tmem_ld32(o_tmem + (half + 1) * 64, a);
-          tmem_ld32(o_tmem + (half + 1) * 64 + 32, b);
+        uint32_t w[32];
+#pragma unroll
+        for (int e = 0; e < 32; e += 2) {
+          w[e >> 1] = pack2<T>(__uint_as_float(a[e]) * inv, __uint_as_float(a[e + 1]) * inv);
+          w[16 + (e >> 1)] = pack2<T>(__uint_as_float(b[e]) * inv, __uint_as_float(b[e + 1]) * inv);
+        }
+        if (row_valid) {
+          if (p.o_sectors) store_cols<true>(o_ptr + half * 64, w, d_cols - half * 64);
+          else store_cols<false>(o_ptr + half * 64, w, d_cols - half * 64);
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_addr(&bar->o_free[t]));
     }
   }
 }

@@ -26,3 +26,22 @@ def test_two_threads_per_row(dtype, d, b, s_q, s_k, h, hk, causal, window, softc
     assert pl.kernel == L.KERNEL_TCGEN05 and pl.block_m == 128
     go, gl = OA.flash_attn_func(q, k, v, causal=causal, window_size=window, softcap=softcap)
     U.check_rules(out, lse, go, gl, tag=f"d {d} {s_q} x {s_k}")
+
+
+@pytest.mark.parametrize("d", [64, 72, 128, 200, 256])
+@pytest.mark.parametrize("where", ["rows", "base", "batch"])
+def test_output_rows_off_the_sector_boundary(d, where):
+    """Output rows that do not start on 32-byte boundaries (or are no whole sectors long) give the same bits, and what lies around
+    them stays as it was."""
+    g = torch.Generator().manual_seed(d)
+    b, n, h = 2, 300, 3
+    q, k, v = (U.normal((b, n, h, d), BF, g).cuda() for _ in range(3))
+    want, _ = ops.attention_forward(q, k, v, softmax_scale=d ** -0.5, causal=True)
+    pad = {"rows": 8, "base": 16, "batch": 16}[where]  # elements behind each row
+    buf = torch.full((b * n * h * (d + pad) + 64,), 7.0, dtype=BF, device="cuda")
+    first, per = (8, n * h * (d + pad)) if where == "base" else (0, n * h * (d + pad) + (8 if where == "batch" else 0))
+    view = buf.as_strided((b, n, h, d), (per, h * (d + pad), d + pad, 1), first)
+    out, _, pl = ops.attention_forward(q, k, v, softmax_scale=d ** -0.5, causal=True, out=view, return_plan=True)
+    assert pl.kernel == L.KERNEL_TCGEN05 and torch.equal(out, want)
+    view.fill_(7.0)
+    assert bool((buf == 7.0).all())
