@@ -52,10 +52,10 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
       mbar_init(smem_addr(&bar->s_free[t]), Geo<HD>::kWide ? 8 : 4);
       mbar_init(smem_addr(&bar->p_full[t][0]), 4);
       mbar_init(smem_addr(&bar->p_full[t][1]), 4);
-      mbar_init(smem_addr(&bar->corr_ready[t]), 4);
+      mbar_init(smem_addr(&bar->corr_ready[t][0]), 4);
+      mbar_init(smem_addr(&bar->corr_ready[t][1]), 4);
       mbar_init(smem_addr(&bar->o_ready[t]), 4);
       mbar_init(smem_addr(&bar->o_done[t]), 1);
-      mbar_init(smem_addr(&bar->stats_ready[t]), 4);
       mbar_init(smem_addr(&bar->o_free[t]), 4);
     }
     for (int s = 0; s < kSlots; ++s) {

@@ -192,10 +192,14 @@ struct Barriers {
   // softmax -> MMA: half h (64 keys) of P_t is in shared memory.  One barrier per half: a waiter must
   // never fall two phases behind a barrier, which two arrivals per block on one barrier would allow.
   uint64_t p_full[2][2];
-  uint64_t corr_ready[2];  // softmax -> correction: rescale factors of block j are in shared memory
+  // softmax -> correction: what the sub-tile's next event hands over is in corr (rescale factors of a block, or 1 / l at the end
+  // of a tile).  Events alternate between two barriers and two rows of corr, so that the softmax warps never wait for a row:
+  // event c - 2 has been read by then.  Before event c of block n (or behind the last block n) a softmax warp has seen P.V of block
+  // n - 2 (n - 1) complete, which was issued after every correction warp had read its factors, or, for the first block of a
+  // tile, the 1 / l of the tile before.
+  uint64_t corr_ready[2][2];
   uint64_t o_ready[2];     // correction -> MMA: O_t has been rescaled, P.V of block j may accumulate
   uint64_t o_done[2];      // MMA -> correction, softmax: P.V of a block has completed (O_t updated, P_t read)
-  uint64_t stats_ready[2]; // softmax -> correction: 1 / l of the tile's rows is in shared memory
   uint64_t o_free[2];      // correction -> MMA: the epilogue has read O_t
   uint64_t fix_req;        // MMA (both warps) -> warp 15: the last V tile of the CTA tile has landed and needs its tail cleared
   uint64_t v_fixed;        // warp 15 -> MMA (both warps): done
@@ -204,8 +208,7 @@ struct Barriers {
   int abort_flag;
   uint32_t fix_seen[2];    // tail repairs each issuing warp has been through (phase of fix_req / v_fixed)
   uint32_t fix_slot;       // ring slot of the V tile to repair
-  float corr[2][kBlockM];
-  float row_inv[2][kBlockM];
+  float corr[2][2][kBlockM];  // [sub-tile][event & 1]
   TileQueue queue;
 };
 static_assert(sizeof(Barriers) <= kBarBytes, "barrier block does not fit");

@@ -1,5 +1,10 @@
 // Softmax role and correction / epilogue role of the tcgen05 prefill kernel.
 //
+// The softmax warps are the kernel's slowest chain: two of them share a scheduler, and next to 2050 cycles of exponentials for a
+// block of both sub-tiles a block took them 3700.  So whatever they do once a block counts: the mask's range as two compares, no
+// wait for the correction warps (corr_ready), arrivals without a branch, one instruction per address of P, the maximum as a tree.
+// 4 K causal, b 4, 32 heads, head dim 64 510 -> 468 us, head dim 128 674 -> 647 under the power cap.
+//
 // Softmax: 128 threads per query sub-tile, one thread per query row (TMEM lane); 256-column tiles have one sub-tile and two
 // threads per row, 64 keys of a block each.  It restates the
 // arithmetic of the reference's OnlineSoftmax epilogue
@@ -23,16 +28,14 @@
 namespace fa {
 namespace tc5 {
 
+// Maximum of m and 32 scores, as a tree (a few chains of three-operand maxima take twice as long as their 16 instructions issue).
 __device__ __forceinline__ float chunk_max(const uint32_t (&a)[32], float m) {
-  float m0 = m, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
+  float r[11];
 #pragma unroll
-  for (int e = 0; e < 32; e += 8) {
-    m0 = max3(m0, __uint_as_float(a[e]), __uint_as_float(a[e + 1]));
-    m1 = max3(m1, __uint_as_float(a[e + 2]), __uint_as_float(a[e + 3]));
-    m2 = max3(m2, __uint_as_float(a[e + 4]), __uint_as_float(a[e + 5]));
-    m3 = max3(m3, __uint_as_float(a[e + 6]), __uint_as_float(a[e + 7]));
-  }
-  return fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+  for (int e = 0; e < 10; ++e) r[e] = max3(__uint_as_float(a[3 * e]), __uint_as_float(a[3 * e + 1]), __uint_as_float(a[3 * e + 2]));
+  r[10] = max3(__uint_as_float(a[30]), __uint_as_float(a[31]), m);
+  const float x = max3(r[0], r[1], r[2]), y = max3(r[3], r[4], r[5]), z = max3(r[6], r[7], r[8]);
+  return max3(max3(x, y, z), r[9], r[10]);
 }
 
 // Columns outside [lo, hi] become -inf.  The valid columns of the chunk form one bit mask, so an
@@ -92,12 +95,13 @@ __device__ __forceinline__ void chunk_exp(const uint32_t (&a)[32], uint64_t scal
   }
 }
 
-// 32 keys of P (16 packed pairs = four 16-byte chunks) of one row into the swizzled A-operand tile.
-__device__ __forceinline__ void store_p_chunk(uint32_t p_row, uint32_t p_xor, int c, const uint32_t (&pk)[16]) {
+// 32 keys of P (16 packed pairs = four 16-byte chunks) of one row into the swizzled A-operand tile: 16-byte chunk kc of a row lies
+// at  half(kc) + row * 128 + ((kc ^ row) & 7) * 16.  p_row holds chunk 0, so a chunk's address is one exclusive-or away.
+__device__ __forceinline__ void store_p_chunk(uint32_t p_row, int c, const uint32_t (&pk)[16]) {
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const uint32_t kc = (uint32_t)(c * 4 + q);
-    const uint32_t addr = p_row + (kc >> 3) * kHalfBytes + (((kc & 7) ^ p_xor) << 4);
+    const uint32_t addr = (p_row ^ ((kc & 7) << 4)) + (kc >> 3) * kHalfBytes;
     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(addr), "r"(pk[4 * q]), "r"(pk[4 * q + 1]),
                  "r"(pk[4 * q + 2]), "r"(pk[4 * q + 3])
                  : "memory");
@@ -130,12 +134,9 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
   const int row = warp_in_wg * 32 + lane;
   const uint32_t lane_addr = (uint32_t)(warp_in_wg * 32) << 16;
   const uint32_t s_tmem = tmem + lane_addr + t * 128 + chunk0 * 32;
-  uint32_t s_cnt = 0, cr_cnt = 0, st_cnt = 0;
-  // this row of P_t: chunk kc (8 keys) of the row lives at  half(kc) + row * 128 + ((kc ^ row) & 7) * 16
-  const uint32_t p_row = p_smem + t * kTileBytes + row * 128;
-  const uint32_t p_xor = (uint32_t)(row & 7);
+  uint32_t s_cnt = 0, ev_cnt = 0;  // blocks, events (corr_ready) so far
+  const uint32_t p_row = p_smem + t * kTileBytes + row * 128 + ((row & 7) << 4);
   const uint32_t bar_sfree = smem_addr(&bar->s_free[t]), bar_odone = smem_addr(&bar->o_done[t]);
-  const uint32_t bar_oready = smem_addr(&bar->o_ready[t]), bar_ofree = smem_addr(&bar->o_free[t]);
   // with softcap the scores are in the log2 domain once they have been capped: the scale is part of the cap
   const float scale_log2 = CAP ? 1.f : p.scale_log2;
   const float lse_scale = CAP ? 0.6931471805599453f : p.a.softmax_scale;  // running maximum -> natural log
@@ -150,7 +151,7 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
     tmem_wait_st();
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_addr(&bar->exchanged));
+    mbar_arrive_lane0(smem_addr(&bar->exchanged), lane);
     if (!mbar_wait(smem_addr(&bar->exchanged), x_cnt & 1, abort_flag, 49)) return false;
     tc_fence_after();
     ++x_cnt;
@@ -184,12 +185,14 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
     }
     const int i_min = ti.row0[t], i_max = min(ti.q_len, ti.row0[t] + kBlockM) - 1;
     float m_run = -INFINITY, l_run = 0.f;
+    // blocks [full_lo, full_hi) need no mask
+    int full_lo = 0, full_hi = ti.k_len / kBlockN;
+    if (p.is_causal || p.is_local) full_hi = min(full_hi, max(0, i_min + ti.koff + (p.is_local ? p.wr : 0) + 1) / kBlockN);
+    if (p.is_local) full_lo = ceil_div(max(0, i_max + ti.koff - p.wl), kBlockN);
 
     for (int j = ti.jlo[t]; j < ti.jhi[t]; ++j) {
       const int col0 = j * kBlockN;
-      bool need_mask = col0 + kBlockN > ti.k_len;
-      if (p.is_causal || p.is_local) need_mask = need_mask || (col0 + kBlockN - 1 > i_min + ti.koff + (p.is_local ? p.wr : 0));
-      if (p.is_local) need_mask = need_mask || (col0 < i_max + ti.koff - p.wl);
+      const bool need_mask = j < full_lo || j >= full_hi;
 
       if (!mbar_wait(smem_addr(&bar->s_full[t]), s_cnt & 1, abort_flag, 41)) return;
       const uint32_t blk = s_cnt;  // running number of this block (all tiles of this CTA)
@@ -203,7 +206,7 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       // the S columns are free: Q.K^T of the next block may overwrite them
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_sfree);
+      mbar_arrive_lane0(bar_sfree, lane);
       if (CAP) {
 #pragma unroll
         for (int c = 0; c < kChunks; ++c) {
@@ -232,13 +235,10 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
       const float corr = fast_exp2((m_run - m_use) * scale_log2);  // 0 when m_run = -inf
       if (lead && j > ti.jlo[t]) {
-        // The correction warps must have consumed the previous factors: this thread can be a whole
-        // block ahead of them, and neither the factor array nor the barrier phase may be reused early.
-        if (cr_cnt > 0 && !mbar_wait(bar_oready, (cr_cnt - 1) & 1, abort_flag, 47)) return;
-        ++cr_cnt;
-        bar->corr[t][row] = (m_new != m_run) ? corr : 1.f;
+        bar->corr[t][ev_cnt & 1][row] = (m_new != m_run) ? corr : 1.f;
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&bar->corr_ready[t]));
+        mbar_arrive_lane0(smem_addr(&bar->corr_ready[t][ev_cnt & 1]), lane);
+        ++ev_cnt;
       }
       m_run = m_new;
       const float neg_ms = -m_use * scale_log2;
@@ -258,20 +258,20 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       chunk_exp<T, kPolyPairs>(sc[0], scale2, negms2, sum2, pk);
       if (kHalfAhead) chunk_exp<T, kPolyPairs>(sc[1], scale2, negms2, sum2, pk1);
       if (blk > 0 && !mbar_wait(bar_odone, (blk - 1) & 1, abort_flag, 42)) return;
-      store_p_chunk(p_row, p_xor, chunk0, pk);
+      store_p_chunk(p_row, chunk0, pk);
       if (!kHalfAhead) chunk_exp<T, kPolyPairs>(sc[1], scale2, negms2, sum2, pk1);
-      store_p_chunk(p_row, p_xor, chunk0 + 1, pk1);
+      store_p_chunk(p_row, chunk0 + 1, pk1);
       fence_proxy_async();  // generic-proxy stores -> visible to the MMA (async proxy)
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_addr(&bar->p_full[t][kWide ? wg : 0]));  // the first (this warpgroup's) 64 keys of P are ready
+      mbar_arrive_lane0(smem_addr(&bar->p_full[t][kWide ? wg : 0]), lane);  // the first (this warpgroup's) 64 keys of P are ready
       if constexpr (!kWide) {
         chunk_exp<T, kPolyPairs>(sc[2], scale2, negms2, sum2, pk);
-        store_p_chunk(p_row, p_xor, 2, pk);
+        store_p_chunk(p_row, 2, pk);
         chunk_exp<T, kPolyPairs>(sc[3], scale2, negms2, sum2, pk);
-        store_p_chunk(p_row, p_xor, 3, pk);
+        store_p_chunk(p_row, 3, pk);
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&bar->p_full[t][1]));  // last 64 keys
+        mbar_arrive_lane0(smem_addr(&bar->p_full[t][1]), lane);  // last 64 keys
       }
       float s0, s1;
       unpack_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])), s0, s1);
@@ -283,13 +283,11 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       l_run += other;
       if (!lead) continue;
     }
-    // 1 / l for the epilogue, LSE from here.  The previous tile's epilogue must have read its 1 / l
-    // (a tile of a single block does not wait for anything else the epilogue does).
-    if (st_cnt > 0 && !mbar_wait(bar_ofree, (st_cnt - 1) & 1, abort_flag, 48)) return;
-    ++st_cnt;
-    bar->row_inv[t][row] = l_run > 0.f ? 1.f / l_run : 0.f;
+    // 1 / l for the epilogue, LSE from here
+    bar->corr[t][ev_cnt & 1][row] = l_run > 0.f ? 1.f / l_run : 0.f;
     __syncwarp();
-    if (lane == 0) mbar_arrive(smem_addr(&bar->stats_ready[t]));
+    mbar_arrive_lane0(smem_addr(&bar->corr_ready[t][ev_cnt & 1]), lane);
+    ++ev_cnt;
     if (i < ti.q_len)
       p.a.lse[(int64_t)ti.bi * p.a.lse_batch_stride + (int64_t)ti.hh * p.a.lse_head_stride + ti.q_row0 + i] =
           l_run > 0.f ? (m_run * lse_scale + __logf(l_run)) : INFINITY;
@@ -374,7 +372,7 @@ __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* ba
   volatile int* abort_flag = &bar->abort_flag;
   const int row = warp_in_wg * 32 + lane;
   const uint32_t lane_addr = (uint32_t)(warp_in_wg * 32) << 16;
-  uint32_t cr_cnt[2] = {0, 0}, od_cnt[2] = {0, 0}, st_cnt[2] = {0, 0};
+  uint32_t ev_cnt[2] = {0, 0}, od_cnt[2] = {0, 0};
   const int d_cols = p.a.d;
 
   TileWalk<IN> walk(bar);
@@ -386,9 +384,9 @@ __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* ba
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         if (!(ti.has[t] && j > ti.jlo[t] && j < ti.jhi[t])) continue;
-        if (!mbar_wait(smem_addr(&bar->corr_ready[t]), cr_cnt[t] & 1, abort_flag, 43)) return;
-        ++cr_cnt[t];
-        const float f = bar->corr[t][row];
+        if (!mbar_wait(smem_addr(&bar->corr_ready[t][ev_cnt[t] & 1]), (ev_cnt[t] >> 1) & 1, abort_flag, 43)) return;
+        const float f = bar->corr[t][ev_cnt[t] & 1][row];
+        ++ev_cnt[t];
         if (!mbar_wait(smem_addr(&bar->o_done[t]), od_cnt[t] & 1, abort_flag, 44)) return;  // P.V of block j-1 done
         ++od_cnt[t];
         if (__any_sync(0xffffffffu, f != 1.f)) {
@@ -397,16 +395,16 @@ __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* ba
           tc_fence_before();
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&bar->o_ready[t]));
+        mbar_arrive_lane0(smem_addr(&bar->o_ready[t]), lane);
       }
     }
     // ---- epilogue of both sub-tiles ----
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       if (!ti.has[t]) continue;
-      if (!mbar_wait(smem_addr(&bar->stats_ready[t]), st_cnt[t] & 1, abort_flag, 45)) return;
-      ++st_cnt[t];
-      const float inv = bar->row_inv[t][row];
+      if (!mbar_wait(smem_addr(&bar->corr_ready[t][ev_cnt[t] & 1]), (ev_cnt[t] >> 1) & 1, abort_flag, 45)) return;
+      const float inv = bar->corr[t][ev_cnt[t] & 1][row];
+      ++ev_cnt[t];
       if (!mbar_wait(smem_addr(&bar->o_done[t]), od_cnt[t] & 1, abort_flag, 46)) return;  // last P.V done
       ++od_cnt[t];
       tc_fence_after();
@@ -424,7 +422,7 @@ __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* ba
         if (half + 1 == HD / 64) {  // all of O has been read: P.V of the next tile may overwrite it under the last stores
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_addr(&bar->o_free[t]));
+          mbar_arrive_lane0(smem_addr(&bar->o_free[t]), lane);
         }
         uint32_t w[32];
 #pragma unroll
