@@ -269,6 +269,12 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
     else if (per_m * kv_bytes_per_pair <= l2_budget || chunk * kv_bytes_per_pair > l2_budget) chunk = per_m;
     if (chunk <= 0 || chunk > per_m) chunk = per_m;
     p.chunk_bh = (int)chunk;
+    p.by_h.set(a.h);
+    p.by_group.set(p.group);
+    p.by_m_tiles.set(p.m_tiles);
+    p.by_chunk.set((int)(chunk * p.m_tiles));
+    p.by_pairs.set((int)chunk);
+    p.by_last_pairs.set(chunk > 0 ? (int)(per_m % chunk) : 0);
     // Ragged input: as many heads as keep their K / V in L2, whole groups; all heads when one group's do not fit.
     const long long kv_rows = a.cu_seqlens_k ? a.total_k : (long long)a.b * a.seqlen_k;
     const long long kv_heads = l2_budget / std::max(1LL, kv_rows * a.d * 4);

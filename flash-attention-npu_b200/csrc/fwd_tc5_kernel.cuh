@@ -86,6 +86,8 @@ struct Tc5Params {
   int32_t group;    // h / h_k
   int32_t m_tiles;  // ceil(max seqlen_q / 256)
   int32_t total_tiles;
+  FastDiv by_h, by_group, by_m_tiles;             // h, group, m_tiles
+  FastDiv by_chunk, by_pairs, by_last_pairs;      // tiles of an L2 chunk, its pairs, the pairs of the last chunk (static_tile)
   float scale_log2;
   float softcap_mul, softcap_l2;  // softcap: scores become softcap_l2 * tanh(s * softcap_mul) in the log2 domain (scale / softcap, softcap * log2 e)
   int32_t o_sectors;         // rows of O start on 32-byte boundaries and are whole 32-byte sectors long
@@ -119,10 +121,11 @@ struct TileId {
 __device__ __forceinline__ TileId static_tile(const Tc5Params& p, int n) {
   const int per_m = p.a.b * p.a.h;
   const int per_chunk = p.chunk_bh * p.m_tiles;
-  const int ck = n / per_chunk, r = n - ck * per_chunk;
+  const int ck = p.by_chunk.div(n), r = n - ck * per_chunk;
   const int cnt = min(p.chunk_bh, per_m - ck * p.chunk_bh);  // pairs in this chunk (the last one may be short)
-  const int rem = ck * p.chunk_bh + r % cnt;
-  return {rem / p.a.h, rem % p.a.h, p.m_tiles - 1 - r / cnt};  // heavy (late, causal) tiles first
+  const int level = cnt == p.chunk_bh ? p.by_pairs.div(r) : p.by_last_pairs.div(r);
+  const int rem = ck * p.chunk_bh + r - level * cnt, bi = p.by_h.div(rem);
+  return {bi, rem - bi * p.a.h, p.m_tiles - 1 - level};  // heavy (late, causal) tiles first
 }
 
 __device__ __forceinline__ int q_length(const Tc5Params& p, int bi) {
@@ -135,12 +138,48 @@ __device__ __forceinline__ int k_length(const Tc5Params& p, int bi) {
   return p.a.cu_seqlens_k ? p.a.cu_seqlens_k[bi + 1] - p.a.cu_seqlens_k[bi] : p.a.seqlen_k;
 }
 
+// The key blocks [jlo, jhi) that the rows of a sub-tile see, which starts at row row0 (of the sequence); none: jlo = jhi.
+__device__ __forceinline__ void block_range(const Tc5Params& p, int row0, int q_len, int k_len, int& jlo, int& jhi) {
+  jlo = jhi = 0;
+  if (row0 >= q_len) return;
+  const int koff = k_len - q_len, i_max = min(q_len, row0 + kBlockM) - 1;
+  int j_lo = 0, j_hi = k_len;
+  if (p.is_causal) j_hi = min(k_len, i_max + koff + 1);
+  if (p.is_local) {
+    j_hi = min(k_len, i_max + koff + p.wr + 1);
+    j_lo = max(0, row0 + koff - p.wl);
+  }
+  if (j_hi > j_lo) {
+    jlo = j_lo / kBlockN;
+    jhi = ceil_div(j_hi, kBlockN);
+  }
+}
+
+// What a softmax warp needs of a tile: its own sub-tile.
+struct SubTile {
+  int bi, hh, q_row0, q_len, k_len, koff;
+  int row0, jlo, jhi;
+};
+template <int ROWS>
+__device__ __forceinline__ SubTile sub_tile(const Tc5Params& p, const TileId id, int t) {
+  SubTile s;
+  s.bi = id.bi;
+  s.hh = id.hh;
+  s.q_row0 = p.a.cu_seqlens_q ? p.a.cu_seqlens_q[id.bi] : 0;
+  s.q_len = q_length(p, id.bi);
+  s.k_len = k_length(p, id.bi);
+  s.koff = s.k_len - s.q_len;
+  s.row0 = id.mt * ROWS + t * kBlockM;
+  block_range(p, s.row0, s.q_len, s.k_len, s.jlo, s.jhi);
+  return s;
+}
+
 template <int ROWS>  // query rows of a CTA tile: 256 (two sub-tiles) or 128 (sub-tile 0 only)
 __device__ __forceinline__ void tile_info(const Tc5Params& p, const TileId id, TileInfo& ti) {
   const int mt = id.mt;
   ti.bi = id.bi;
   ti.hh = id.hh;
-  ti.hk = ti.hh / p.group;
+  ti.hk = p.by_group.div(ti.hh);
   ti.q_row0 = p.a.cu_seqlens_q ? p.a.cu_seqlens_q[ti.bi] : 0;
   ti.q_len = q_length(p, ti.bi);
   ti.k_row0 = p.a.cu_seqlens_k ? p.a.cu_seqlens_k[ti.bi] : 0;
@@ -153,23 +192,11 @@ __device__ __forceinline__ void tile_info(const Tc5Params& p, const TileId id, T
   for (int t = 0; t < 2; ++t) {
     const int r0 = (ROWS == kBlockM && t == 1) ? 0x3fffffff : mt * ROWS + t * kBlockM;  // no second sub-tile in 128-row tiles
     ti.row0[t] = r0;
-    ti.jlo[t] = ti.jhi[t] = 0;
-    ti.has[t] = false;
-    if (r0 < ti.q_len) {
-      const int i_min = r0, i_max = min(ti.q_len, r0 + kBlockM) - 1;
-      int j_lo = 0, j_hi = ti.k_len;
-      if (p.is_causal) j_hi = min(ti.k_len, i_max + ti.koff + 1);
-      if (p.is_local) {
-        j_hi = min(ti.k_len, i_max + ti.koff + p.wr + 1);
-        j_lo = max(0, i_min + ti.koff - p.wl);
-      }
-      if (j_hi > j_lo) {
-        ti.jlo[t] = j_lo / kBlockN;
-        ti.jhi[t] = ceil_div(j_hi, kBlockN);
-        ti.has[t] = true;
-        ti.ulo = min(ti.ulo, ti.jlo[t]);
-        ti.uhi = max(ti.uhi, ti.jhi[t]);
-      }
+    block_range(p, r0, ti.q_len, ti.k_len, ti.jlo[t], ti.jhi[t]);
+    ti.has[t] = ti.jhi[t] > ti.jlo[t];
+    if (ti.has[t]) {
+      ti.ulo = min(ti.ulo, ti.jlo[t]);
+      ti.uhi = max(ti.uhi, ti.jhi[t]);
     }
   }
   if (ti.uhi == 0) ti.ulo = 0;
@@ -261,8 +288,8 @@ using TileWalk = typename std::conditional<IN == kRaggedDraw, QueueWalk, StaticW
 template <int IN>
 __device__ __forceinline__ TileId tile_id(const Tc5Params& p, int n) {
   if (IN != kRaggedDraw) return static_tile(p, n);
-  const int pair = n / p.m_tiles;
-  return {pair / p.a.h, pair % p.a.h, n % p.m_tiles};
+  const int pair = p.by_m_tiles.div(n), bi = p.by_h.div(pair);
+  return {bi, pair - bi * p.a.h, n - pair * p.m_tiles};
 }
 
 // The producer's side.  Position n (a CTA index) -> tile: the heads are cut into chunks whose K / V stay in L2 together;

@@ -164,11 +164,10 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
 
   TileWalk<IN> walk(bar);
   for (int n = walk.first(p); n < p.total_tiles; n = walk.next(p)) {
-    TileInfo ti;
-    tile_info<Geo<HD>::kRows>(p, tile_id<IN>(p, n), ti);
-    if (ti.row0[t] >= ti.q_len) continue;
-    const int i = ti.row0[t] + row;
-    if (!ti.has[t]) {  // no visible key for the whole sub-tile: O = 0, LSE = +inf
+    const SubTile ti = sub_tile<Geo<HD>::kRows>(p, tile_id<IN>(p, n), t);
+    if (ti.row0 >= ti.q_len) continue;
+    const int i = ti.row0 + row;
+    if (ti.jhi <= ti.jlo) {  // no visible key for the whole sub-tile: O = 0, LSE = +inf
       if (lead && i < ti.q_len) {
         T* o_ptr = reinterpret_cast<T*>(p.a.o) + (int64_t)ti.bi * p.a.o_batch_stride +
                    (int64_t)(ti.q_row0 + i) * p.a.o_row_stride + (int64_t)ti.hh * p.a.o_head_stride;
@@ -183,14 +182,14 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       hi = min(hi, i + ti.koff + p.wr);
       lo = max(0, i + ti.koff - p.wl);
     }
-    const int i_min = ti.row0[t], i_max = min(ti.q_len, ti.row0[t] + kBlockM) - 1;
+    const int i_min = ti.row0, i_max = min(ti.q_len, ti.row0 + kBlockM) - 1;
     float m_run = -INFINITY, l_run = 0.f;
     // blocks [full_lo, full_hi) need no mask
     int full_lo = 0, full_hi = ti.k_len / kBlockN;
     if (p.is_causal || p.is_local) full_hi = min(full_hi, max(0, i_min + ti.koff + (p.is_local ? p.wr : 0) + 1) / kBlockN);
     if (p.is_local) full_lo = ceil_div(max(0, i_max + ti.koff - p.wl), kBlockN);
 
-    for (int j = ti.jlo[t]; j < ti.jhi[t]; ++j) {
+    for (int j = ti.jlo; j < ti.jhi; ++j) {
       const int col0 = j * kBlockN;
       const bool need_mask = j < full_lo || j >= full_hi;
 
@@ -234,7 +233,7 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       if (kRescaleThreshold > 0.f && m_run != -INFINITY && (m_new - m_run) * scale_log2 <= kRescaleThreshold) m_new = m_run;
       const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
       const float corr = fast_exp2((m_run - m_use) * scale_log2);  // 0 when m_run = -inf
-      if (lead && j > ti.jlo[t]) {
+      if (lead && j > ti.jlo) {
         bar->corr[t][ev_cnt & 1][row] = (m_new != m_run) ? corr : 1.f;
         __syncwarp();
         mbar_arrive_lane0(smem_addr(&bar->corr_ready[t][ev_cnt & 1]), lane);

@@ -12,7 +12,27 @@
 #define FA_TILE_HD inline
 #endif
 
+#include <stdint.h>
+
 namespace fa {
+
+// n / d for 0 <= n < 2^31 as a multiplication: mul = ceil(2^(31 + s) / d) with 2^s >= d exceeds 2^(31 + s) / d by less than
+// 2^s / d, so the quotient is off by less than n / 2^31 / d < 1 / d and its whole part is exact.  Every role of the prefill kernel
+// finds its tile by itself, four or five divisions by run-time values, of some 100 cycles each as the compiler does them.
+struct FastDiv {
+  uint32_t mul, shift;  // mul 0: d = 1
+  void set(int d) {
+    mul = shift = 0;
+    if (d <= 1) return;
+    uint32_t s = 1;
+    while ((1ull << s) < (uint64_t)d) ++s;
+    mul = (uint32_t)(((1ull << (31 + s)) + (uint32_t)d - 1) / (uint32_t)d);
+    shift = s - 1;
+  }
+  FA_TILE_HD int div(int n) const {
+    return mul ? (int)(((uint64_t)(uint32_t)n * mul) >> 32 >> shift) : n;
+  }
+};
 
 // Levels must offer:  int live (tiles of one head over all batch entries), int top (highest level that holds a tile),
 // int count(level) (batch entries with a tile in it).

@@ -70,3 +70,36 @@ def test_every_tile_has_one_position_in_any_order(tmp_path):
     subprocess.run(["g++", "-O1", "-std=c++17", "-fsanitize=undefined", "-fno-sanitize-recover", "-I", CSRC, str(src), "-o", str(exe)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+DIVISION = r"""
+#include <cstdio>
+#include <random>
+#include "tile_order.cuh"
+int main() {
+  std::mt19937 rng(3);
+  std::uniform_int_distribution<int> any(0, 0x7fffffff);
+  for (int k = 0; k < 4000; ++k) {
+    const int d = k < 2000 ? k + 1 : k < 2060 ? (k % 2 ? (1 << (k - 2000) / 2) : 0x7fffffff - (k - 2000)) : any(rng) >> (k % 31);
+    fa::FastDiv f;
+    f.set(d);
+    if (d < 1) continue;
+    for (int i = 0; i < 400; ++i) {
+      long long n = i < 4 ? i : i < 8 ? 0x7fffffffLL - (i - 4) : (long long)d * (any(rng) / d) + (i % 3) - 1;
+      if (n < 0 || n > 0x7fffffffLL) n = any(rng);
+      if (f.div((int)n) != (int)n / d) { std::printf("%lld / %d: %d\n", n, d, f.div((int)n)); return 1; }
+    }
+  }
+  return 0;
+}
+"""
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="no host compiler")
+def test_division_by_multiplication(tmp_path):
+    """Every divisor up to 2000, powers of two, the largest and random ones; dividends at multiples and one beside them."""
+    src, exe = tmp_path / "div.cpp", tmp_path / "div"
+    src.write_text(DIVISION)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fsanitize=undefined", "-fno-sanitize-recover", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
