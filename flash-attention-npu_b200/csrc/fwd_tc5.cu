@@ -35,7 +35,7 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
     return;
   }
   const uint32_t q_smem = base;
-  const uint32_t p_smem = base + 2 * kTileBytes;
+  const uint32_t p_smem = base + Geo<HD>::kPOff;
   const uint32_t kv_smem = base + Geo<HD>::kRingOff;
   Barriers* bar = reinterpret_cast<Barriers*>(smem + 4 * kTileBytes + kSlots * kTileBytes);
 
@@ -50,15 +50,14 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
       mbar_init(smem_addr(&bar->q_empty[t]), 1);
       mbar_init(smem_addr(&bar->s_full[t]), 1);
       mbar_init(smem_addr(&bar->s_free[t]), Geo<HD>::kWide ? 8 : 4);
-      mbar_init(smem_addr(&bar->p_full[t][0]), 4);
-      mbar_init(smem_addr(&bar->p_full[t][1]), 4);
+      for (int c = 0; c < 4; ++c) mbar_init(smem_addr(&bar->p_full[t][c >> 1][c & 1]), 4);
       mbar_init(smem_addr(&bar->corr_ready[t][0]), 4);
       mbar_init(smem_addr(&bar->corr_ready[t][1]), 4);
       mbar_init(smem_addr(&bar->o_ready[t]), 4);
       mbar_init(smem_addr(&bar->o_done[t]), 1);
       mbar_init(smem_addr(&bar->o_free[t]), 4);
     }
-    for (int s = 0; s < kSlots; ++s) {
+    for (int s = 0; s < kMaxSlots; ++s) {
       mbar_init(smem_addr(&bar->kv_full[s]), 1);
       mbar_init(smem_addr(&bar->kv_empty[s]), 2);
     }

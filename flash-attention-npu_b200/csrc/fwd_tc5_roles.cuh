@@ -59,7 +59,7 @@ __device__ __forceinline__ void producer_loop(const Tc5Params& p, const CUtensor
         mbar_arrive_expect_tx(full, G::kHalves * kHalfBytes);
 #pragma unroll
         for (int hf = 0; hf < G::kHalves; ++hf)
-          tma_load_4d_hint(q_smem + t * kTileBytes + hf * kHalfBytes, tm_q, full, 64 * hf, ti.hh, row, bq, q_policy);
+          tma_load_4d_hint(q_smem + t * G::kQStep + hf * kHalfBytes, tm_q, full, 64 * hf, ti.hh, row, bq, q_policy);
       }
       __syncwarp();
     }
@@ -164,15 +164,15 @@ __device__ __forceinline__ void mma_loop(const Tc5Params& p, Barriers* bar, uint
   RingPos<G::kRing> ring;
   uint32_t q_cnt = 0, qk_cnt = 0, p_cnt = 0, ofree_cnt = 0, oready_cnt = 0;
   // Descriptor bases are built once; inside the loops a descriptor is base + a small constant.
-  const uint64_t q_desc = make_smem_desc(q_smem + t * kTileBytes, 16, 1024);
-  const uint64_t p_desc = make_smem_desc(p_smem + t * kTileBytes, 16, 1024);
+  const uint64_t q_desc = make_smem_desc(q_smem + t * G::kQStep, 16, 1024);
+  const uint64_t p_desc0 = make_smem_desc(p_smem + t * G::kPBufs * kTileBytes, 16, 1024);
   const uint64_t k_desc0 = make_smem_desc(kv_smem, 16, 1024);          // K-major operand (K)
   const uint64_t v_desc0 = make_smem_desc(kv_smem, kHalfBytes, 1024);  // N-contiguous operand (V)
   constexpr uint64_t kSlotStep = G::kSlotBytes >> 4;
   // K-major operands: 16 columns per k-step = 32 bytes inside the 128-byte swizzle span
   auto k_off = [](int ks) { return (uint64_t)(((ks >> 2) * kHalfBytes + (ks & 3) * 32) >> 4); };
   const uint32_t s_tmem = tmem + t * 128, o_tmem = tmem + 256 + t * 128;
-  const uint32_t bar_pfull0 = smem_addr(&bar->p_full[t][0]), bar_pfull1 = smem_addr(&bar->p_full[t][1]);
+  const uint32_t bar_pfull = smem_addr(&bar->p_full[t][0][0]);
   const uint32_t bar_ofree = smem_addr(&bar->o_free[t]), bar_oready = smem_addr(&bar->o_ready[t]);
   const uint32_t bar_odone = smem_addr(&bar->o_done[t]), bar_sfull = smem_addr(&bar->s_full[t]);
   const uint32_t bar_sfree = smem_addr(&bar->s_free[t]);
@@ -250,7 +250,9 @@ __device__ __forceinline__ void mma_loop(const Tc5Params& p, Barriers* bar, uint
       if (!mbar_wait(bar_kvfull0 + slot * 8, par, abort_flag, 18)) return false;
       if (FIX && j == fix_j && !tail_fix(slot)) return false;
       const uint64_t v_desc = v_desc0 + slot * kSlotStep;
-      if (!mbar_wait(bar_pfull0, p_cnt & 1, abort_flag, 19)) return false;  // first 64 keys of P
+      const uint32_t buf = p_cnt % G::kPBufs, p_par = (p_cnt / G::kPBufs) & 1;
+      const uint64_t p_desc = p_desc0 + buf * (uint64_t)(kTileBytes >> 4);
+      if (!mbar_wait(bar_pfull + 16 * buf, p_par, abort_flag, 19)) return false;  // first 64 keys of P
       tc_fence_after();
       if (elect_one()) {
         if (first_pv) mma_ss_c<false>(o_tmem, p_desc, v_desc, idesc_pv);
@@ -258,7 +260,7 @@ __device__ __forceinline__ void mma_loop(const Tc5Params& p, Barriers* bar, uint
 #pragma unroll
         for (int ks = 1; ks < 4; ++ks) mma_ss_c<true>(o_tmem, p_desc + k_off(ks), v_desc + (uint64_t)(ks * (2048 >> 4)), idesc_pv);
       }
-      if (!mbar_wait(bar_pfull1, p_cnt & 1, abort_flag, 20)) return false;  // last 64 keys
+      if (!mbar_wait(bar_pfull + 16 * buf + 8, p_par, abort_flag, 20)) return false;  // last 64 keys
       tc_fence_after();
       const bool other = j >= jlo_o && j < jhi_o;
       if (elect_one()) {

@@ -135,7 +135,8 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
   const uint32_t lane_addr = (uint32_t)(warp_in_wg * 32) << 16;
   const uint32_t s_tmem = tmem + lane_addr + t * 128 + chunk0 * 32;
   uint32_t s_cnt = 0, ev_cnt = 0;  // blocks, events (corr_ready) so far
-  const uint32_t p_row = p_smem + t * kTileBytes + row * 128 + ((row & 7) << 4);
+  constexpr int kPBufs = Geo<HD>::kPBufs;
+  const uint32_t p_row0 = p_smem + t * kPBufs * kTileBytes + row * 128 + ((row & 7) << 4);
   const uint32_t bar_sfree = smem_addr(&bar->s_free[t]), bar_odone = smem_addr(&bar->o_done[t]);
   // with softcap the scores are in the log2 domain once they have been capped: the scale is part of the cap
   const float scale_log2 = CAP ? 1.f : p.scale_log2;
@@ -253,16 +254,17 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       // late by themselves (b2 s4096 h16 full 431 -> 444 us, b1 s1061 h16 causal 31.8 -> 32.4), and where no tile follows another
       // (ragged input, fixed deal: 6 chunks of 705 rows against 1307 keys 32.4 -> 33.4, 5 of 135 rows 19.5 -> 19.8).
       constexpr bool kHalfAhead = HD == 128 && CAP == kCapNone && IN != kRaggedFixed;
+      const uint32_t buf = blk % kPBufs, p_row = p_row0 + buf * kTileBytes;
       uint32_t pk[16], pk1[16];
       chunk_exp<T, kPolyPairs>(sc[0], scale2, negms2, sum2, pk);
       if (kHalfAhead) chunk_exp<T, kPolyPairs>(sc[1], scale2, negms2, sum2, pk1);
-      if (blk > 0 && !mbar_wait(bar_odone, (blk - 1) & 1, abort_flag, 42)) return;
+      if (kPBufs == 1 && blk > 0 && !mbar_wait(bar_odone, (blk - 1) & 1, abort_flag, 42)) return;
       store_p_chunk(p_row, chunk0, pk);
       if (!kHalfAhead) chunk_exp<T, kPolyPairs>(sc[1], scale2, negms2, sum2, pk1);
       store_p_chunk(p_row, chunk0 + 1, pk1);
       fence_proxy_async();  // generic-proxy stores -> visible to the MMA (async proxy)
       __syncwarp();
-      mbar_arrive_lane0(smem_addr(&bar->p_full[t][kWide ? wg : 0]), lane);  // the first (this warpgroup's) 64 keys of P are ready
+      mbar_arrive_lane0(smem_addr(&bar->p_full[t][buf][kWide ? wg : 0]), lane);  // the first (this warpgroup's) 64 keys of P are ready
       if constexpr (!kWide) {
         chunk_exp<T, kPolyPairs>(sc[2], scale2, negms2, sum2, pk);
         store_p_chunk(p_row, 2, pk);
@@ -270,7 +272,9 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
         store_p_chunk(p_row, 3, pk);
         fence_proxy_async();
         __syncwarp();
-        mbar_arrive_lane0(smem_addr(&bar->p_full[t][1]), lane);  // last 64 keys
+        // for the event behind the tile's last block (corr_ready)
+        if (kPBufs > 1 && j == ti.jhi - 1 && blk > 0 && !mbar_wait(bar_odone, (blk - 1) & 1, abort_flag, 42)) return;
+        mbar_arrive_lane0(smem_addr(&bar->p_full[t][buf][1]), lane);  // last 64 keys
       }
       float s0, s1;
       unpack_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])), s0, s1);
