@@ -39,6 +39,7 @@ struct BwdParams {
   int32_t b, seqlen_q, seqlen_k, h, h_k, d, d_pad, total_q;
   int32_t is_causal, is_local, wl, wr;
   float softmax_scale, scale_log2;
+  int32_t dq_sectors, dk_sectors, dv_sectors;  // rows start on 32-byte boundaries and are whole 32-byte sectors long
   int32_t chunk_kv, chunk_q;  // tcgen05 kernels: (batch entry, kv head) / (batch entry, head) pairs per chunk of the work-item order (item_place)
   float softcap;  // 0 = off; scores become softcap * tanh(S * scale / softcap) (tests/fa_small_op_golden.py:80-89,124-125)
 };

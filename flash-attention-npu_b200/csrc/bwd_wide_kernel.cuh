@@ -547,8 +547,9 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_addr(&bar->acc_free));
         if (row_ok) {
-          store_slice<T>(out, a0, p.d - 64 * q4);
-          store_slice<T>(out + 32, a1r, p.d - 64 * q4 - 32);
+          const bool sectors = w.kind == kWideDQ ? p.dq_sectors : w.kind == kWideDK ? p.dk_sectors : p.dv_sectors;
+          store_slice<T>(out, a0, p.d - 64 * q4, sectors);
+          store_slice<T>(out + 32, a1r, p.d - 64 * q4 - 32, sectors);
         }
       } else if (lane == 0) {
         mbar_arrive(smem_addr(&bar->acc_free));

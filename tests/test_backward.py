@@ -307,3 +307,26 @@ def test_tcgen05_backward_refuses_what_it_does_not_cover():
     ops.attention_backward(dout, q, k, v, out, lse, softmax_scale=d ** -0.5)  # the other kernel takes it
     with pytest.raises(RuntimeError, match="kernel must be"):
         ops.attention_backward(dout, q, k, v, out, lse, softmax_scale=d ** -0.5, kernel=7)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [64, 72, 128, 192, 256])
+@pytest.mark.parametrize("where", ["rows", "base"])
+def test_gradient_rows_off_the_sector_boundary(d, where):
+    """Gradient rows that do not start on 32-byte boundaries (or are no whole sectors long) get the same bits, and what lies around
+    them stays as it was."""
+    from flash_b200 import ops
+    g = torch.Generator().manual_seed(d)
+    b, n, h = 2, 200, 2
+    q, k, v, dout = (torch.randn(b, n, h, d, generator=g).to(torch.bfloat16).cuda() for _ in range(4))
+    kw = dict(softmax_scale=d ** -0.5, causal=True)
+    out, lse = ops.attention_forward(q, k, v, **kw)
+    want = ops.attention_backward(dout, q, k, v, out, lse, **kw)
+    pad, first = (8, 0) if where == "rows" else (16, 8)
+    bufs = [torch.full((b * n * h * (d + pad) + 64,), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+    views = [x.as_strided((b, n, h, d), (n * h * (d + pad), h * (d + pad), d + pad, 1), first) for x in bufs]
+    ops.attention_backward(dout, q, k, v, out, lse, dq=views[0], dk=views[1], dv=views[2], **kw)
+    for buf, view, x in zip(bufs, views, want):
+        assert torch.equal(view, x)
+        view.fill_(7.0)
+        assert bool((buf == 7.0).all())
