@@ -50,12 +50,16 @@ int bwd_tc5_launch(const BwdParams& p, const fa_bwd_params& a, cudaStream_t st, 
   // the two work-item counters: the first 16 bytes of the workspace, cleared by the kernel in front (bwd_delta_kernel)
   int32_t* counters = reinterpret_cast<int32_t*>(p.dq_accum);
   cudaError_t e = cudaSuccess;
-  auto launch = [&](auto kern, dim3 grid, const CUtensorMap& mq, const CUtensorMap& mdo, int32_t* counter) {
+  auto launch = [&](auto kern, dim3 grid, const CUtensorMap& mq, const CUtensorMap& mdo, int32_t* counter, bool overlap) {
     if (e != cudaSuccess) return;
     e = allow_smem(reinterpret_cast<const void*>(kern), kSmemBytes);
     if (e == cudaSuccess) {
-      kern<<<grid, kThreads, kSmemBytes, st>>>(p, mq, mdo, tk, tv, status, counter);
-      e = cudaGetLastError();
+      if (overlap) {
+        e = launch_dependent(kern, grid, kThreads, kSmemBytes, st, p, mq, mdo, tk, tv, status, counter);
+      } else {
+        kern<<<grid, kThreads, kSmemBytes, st>>>(p, mq, mdo, tk, tv, status, counter);
+        e = cudaGetLastError();
+      }
     }
   };
   auto both = [&](auto t_tag, auto fmt_tag, auto cap_tag, auto hd_tag) {  // tags: compile-time choices as types
@@ -63,8 +67,10 @@ int bwd_tc5_launch(const BwdParams& p, const fa_bwd_params& a, cudaStream_t st, 
     constexpr uint32_t F = decltype(fmt_tag)::value;
     constexpr bool C = decltype(cap_tag)::value;
     constexpr int HD = decltype(hd_tag)::value;
-    launch(bwd_dkv_kernel<T, F, C, HD>, grid_kv, tq_u, tdo_u, counters);
-    launch(bwd_dq_kernel<T, F, C, HD>, grid_q, tq, tdo, counters + 1);
+    launch(bwd_dkv_kernel<T, F, C, HD>, grid_kv, tq_u, tdo_u, counters, false);
+    // nothing that the dK / dV kernel reads is written by the dQ kernel, unless a caller has dQ written over an input
+    const bool apart = a.dq != a.q && a.dq != a.dout && a.dq != a.k && a.dq != a.v;
+    launch(bwd_dq_kernel<T, F, C, HD>, grid_q, tq, tdo, counters + 1, apart);
   };
   auto by_hd = [&](auto t_tag, auto fmt_tag, auto cap_tag) {
     if (a.d <= 64) both(t_tag, fmt_tag, cap_tag, std::integral_constant<int, 64>{});

@@ -49,7 +49,8 @@ cudaError_t allow_smem(const void* kernel, int bytes);
 // in a graph 0.3 % slower (worst 8.6 %).
 // The mma.sync kernel is launched so where its grid has no more CTAs than the GPU has SMs (KParams::overlap), so that the next
 // kernel's fit beside them: 20 calls of 16 - 128 CTAs 0.83 - 1.00 x back to back, 0.97 - 1.00 x in a graph; 8 calls of 192 - 880
-// CTAs 0.94 - 1.00 x and 0.98 - 1.07 x.  The tcgen05 kernels keep the ordinary launch: prefill with softcap, head dim 256, 101.6
+// CTAs 0.94 - 1.00 x and 0.98 - 1.07 x.  The tcgen05 kernels keep the ordinary launch (but for bwd_dq_kernel, which does not depend
+// on the kernel in front and waits for it at its end): prefill with softcap, head dim 256, 101.6
 // -> 109 us, chunked prefill 499 -> 504.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
