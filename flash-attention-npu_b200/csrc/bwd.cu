@@ -131,8 +131,13 @@ int fa_b200_bwd(const fa_bwd_params* a, void* workspace, size_t workspace_bytes,
   p.softcap = a->softcap;
   {
     const int64_t k_rows = varlen ? a->total_k : (int64_t)a->b * a->seqlen_k;
-    p.chunk_kv = bwd_chunk(p.is_causal, a->h_k * a->b, rows, a->h, a->d, a->h > a->h_k);
-    p.chunk_q = bwd_chunk(p.is_causal, a->h * a->b, k_rows, a->h_k, a->d, a->h > a->h_k);
+    const int kv_pairs = a->h_k * a->b, q_pairs = a->h * a->b;
+    p.kv_items.set((a->seqlen_k + kBwdItem - 1) / kBwdItem, kv_pairs, bwd_chunk(p.is_causal, kv_pairs, rows, a->h, a->d, a->h > a->h_k));
+    p.q_items.set((a->seqlen_q + kBwdItem - 1) / kBwdItem, q_pairs, bwd_chunk(p.is_causal, q_pairs, k_rows, a->h_k, a->d, a->h > a->h_k));
+    p.group = a->h / a->h_k;
+    p.by_group.set(p.group);
+    p.by_h_k.set(a->h_k);
+    p.by_h.set(a->h);
   }
   const size_t acc_bytes = bwd_accum_bytes(a, rows);
   p.dq_accum = reinterpret_cast<float*>(workspace);

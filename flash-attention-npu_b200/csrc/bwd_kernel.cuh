@@ -17,6 +17,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "tile_order.cuh"
 
 namespace fa {
 
@@ -40,11 +41,15 @@ struct BwdParams {
   int32_t is_causal, is_local, wl, wr;
   float softmax_scale, scale_log2;
   int32_t dq_sectors, dk_sectors, dv_sectors;  // rows start on 32-byte boundaries and are whole 32-byte sectors long
-  int32_t chunk_kv, chunk_q;  // tcgen05 kernels: (batch entry, kv head) / (batch entry, head) pairs per chunk of the work-item order (item_place)
+  // tcgen05 kernels: order of the work items over (batch entry, kv head) / (batch entry, head) pairs, and divisions by h / h_k, h_k, h
+  ItemOrder kv_items, q_items;
+  int32_t group;
+  FastDiv by_group, by_h_k, by_h;
   float softcap;  // 0 = off; scores become softcap * tanh(S * scale / softcap) (tests/fa_small_op_golden.py:80-89,124-125)
 };
 
 constexpr int kBwdBM = 64, kBwdBN = 64, kBwdThreads = 128;
+constexpr int kBwdItem = 128;  // keys or rows of a work item of the tcgen05 kernels
 
 template <int HD>
 struct BwdSmem {

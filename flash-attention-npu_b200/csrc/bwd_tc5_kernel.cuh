@@ -43,12 +43,17 @@ namespace btc5 {
 
 using namespace tc5;
 
-constexpr int kBlk = 128;                 // rows of a query block = keys of a key block
+constexpr int kBlk = kBwdItem;            // rows of a query block = keys of a key block
 constexpr int kHalfBytes = kBlk * 128;    // one 64-column half of a [128 x 128] 16-bit tile (128-byte rows)
 constexpr int kTileBytes = 2 * kHalfBytes;
 constexpr int kEwWarps = 16, kMmaWarp = 16 /* .. 18 */, kTmaWarp = 19;
 constexpr int kThreads = 20 * 32;
 constexpr int kBarBytes = 3072;
+// Sets of resident tiles: with 64 columns there is room for those of the next item beside this one's, so that they are loaded under
+// its last units.  (Together with the items' divisions by multiplication: 12 packed sequences of 37 - 2999 rows, 16 / 4 heads, head
+// dim 64, backward 362 -> 353 us.)
+template <int HD>
+constexpr int kSets = HD == 64 ? 2 : 1;
 constexpr int kDqSlots = 5, kDqKSlots = 3;  // rings of bwd_dq_kernel: three K tiles (slots 0-2), two V tiles (slots 3-4)
 constexpr int kSmemBytes = 7 * kTileBytes + kBarBytes;   // dQ: 2 resident tiles + 5 ring tiles; dK / dV: 2 + 4 stages of 32 KiB (6 tiles' worth)
 static_assert(kSmemBytes <= 232448, "more than the 227 KiB a CTA can have");
@@ -133,7 +138,7 @@ __device__ __forceinline__ void ew_pair(const bool poly, uint32_t s0, uint32_t s
 // published: the producer warp writes their zeros itself.  The ring needs no "empty" barrier: the producer publishes item
 // n + 1 after the last S of item n - 1, and with items of one block or unit that S has waited for the elementwise warps in
 // item n - 2 or n - 3 and those for the accumulating issuer one item behind; so it is at most five items ahead of any
-// other role, and the ring has eight slots.
+// other role, with two sets of resident tiles (kSets) six, and the ring has eight slots.
 constexpr int kQueue = 8;
 struct ItemQueue {
   uint64_t full[kQueue];
@@ -269,7 +274,7 @@ constexpr int kUnitTile = 2 * kUnitHalf;     // 16 KiB
 constexpr int kStages = 4;                   // ring stages, each Q (16 KiB) then dO (16 KiB)
 
 struct BarA {
-  uint64_t kv_full, kv_empty;  // K / V of the item have landed; the item's last S^T / dP^T have read them
+  uint64_t kv_full[2], kv_empty[2];  // per set: K / V of the item have landed; the item's last S^T / dP^T have read them
   uint64_t qdo_full[kStages], qdo_empty[kStages];
   uint64_t st_full[2];   // MMA -> elementwise: S^T and dP^T of the buffer are in TMEM
   uint64_t pds_full[2];  // elementwise -> MMA: P^T and dS^T of the buffer are in TMEM
@@ -293,10 +298,9 @@ struct ItemA {
 };
 __device__ __forceinline__ ItemA item_a(const BwdParams& p, int t) {
   ItemA w;
-  const int n_kblocks = ceil_div(p.seqlen_k, kBlk);
-  const ItemPlace at = item_place(t, n_kblocks, p.h_k * p.b, p.chunk_kv);
-  w.hk = at.pair % p.h_k;
-  w.bi = at.pair / p.h_k;
+  const ItemPlace at = p.kv_items.place(t);
+  w.bi = p.by_h_k.div(at.pair);
+  w.hk = at.pair - w.bi * p.h_k;
   w.sq = seq_info(p, w.bi);
   w.key0 = at.block * kBlk;
   w.live = w.key0 < w.sq.k_len;
@@ -308,7 +312,7 @@ __device__ __forceinline__ ItemA item_a(const BwdParams& p, int t) {
     const int i_hi = w.sq.wl >= 0 ? min(w.sq.q_len - 1, k1 - w.sq.koff + w.sq.wl) : w.sq.q_len - 1;  // inclusive
     w.u_lo = i_lo / kUnit;
     w.nu = i_hi >= i_lo ? i_hi / kUnit + 1 - w.u_lo : 0;
-    w.iters = w.nu * (p.h / p.h_k);
+    w.iters = w.nu * p.group;
   }
   return w;
 }
@@ -327,13 +331,16 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
     if (tid == 0) atomicExch(status, 0x20000000);
     return;
   }
-  const int group = p.h / p.h_k;
-  const int n_items = ceil_div(p.seqlen_k, kBlk) * p.h_k * p.b;
-  const uint32_t k_smem = base, v_smem = base + kTileBytes, ring = base + 2 * kTileBytes;  // stage s: Q at ring + s * 32 KiB, dO behind it
+  const int group = p.group;
+  const int n_items = p.kv_items.blocks * p.kv_items.pairs;
+  // 64 columns: set s has K at s * 32 KiB, V 16 KiB on
+  const uint32_t k_smem = base, v_smem = base + kTileBytes / kSets<HD>, ring = base + 2 * kTileBytes;  // stage s: Q at ring + s * 32 KiB, dO behind it
   BarA* bar = reinterpret_cast<BarA*>(smem + 7 * kTileBytes);
   if (tid == 0) {
-    mbar_init(smem_addr(&bar->kv_full), 1);
-    mbar_init(smem_addr(&bar->kv_empty), 2);        // one commit per issuing warp
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_addr(&bar->kv_full[s]), 1);
+      mbar_init(smem_addr(&bar->kv_empty[s]), 2);  // one commit per issuing warp
+    }
     for (int s = 0; s < kStages; ++s) {
       mbar_init(smem_addr(&bar->qdo_full[s]), 1);
       mbar_init(smem_addr(&bar->qdo_empty[s]), 2);
@@ -395,14 +402,15 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
         continue;
       }
       queue_publish(&bar->queue, wi, t, lane);
-      if (!mbar_wait(smem_addr(&bar->kv_empty), (wi & 1) ^ 1, abort_flag, 60)) break;
+      const uint32_t set = wi % kSets<HD>, at = set * kTileBytes;
+      if (!mbar_wait(smem_addr(&bar->kv_empty[set]), ((wi / kSets<HD>) & 1) ^ 1, abort_flag, 60)) break;
       if (elect_one()) {
-        const uint32_t full = smem_addr(&bar->kv_full);
+        const uint32_t full = smem_addr(&bar->kv_full[set]);
         mbar_arrive_expect_tx(full, 2 * (HD / 64) * kHalfBytes);
-        tma_load_4d(k_smem, &tm_k, full, 0, w.hk, sq.k_row0 + w.key0, sq.bq);
-        if (HD > 64) tma_load_4d(k_smem + kHalfBytes, &tm_k, full, 64, w.hk, sq.k_row0 + w.key0, sq.bq);
-        tma_load_4d(v_smem, &tm_v, full, 0, w.hk, sq.k_row0 + w.key0, sq.bq);
-        if (HD > 64) tma_load_4d(v_smem + kHalfBytes, &tm_v, full, 64, w.hk, sq.k_row0 + w.key0, sq.bq);
+        tma_load_4d(k_smem + at, &tm_k, full, 0, w.hk, sq.k_row0 + w.key0, sq.bq);
+        if (HD > 64) tma_load_4d(k_smem + at + kHalfBytes, &tm_k, full, 64, w.hk, sq.k_row0 + w.key0, sq.bq);
+        tma_load_4d(v_smem + at, &tm_v, full, 0, w.hk, sq.k_row0 + w.key0, sq.bq);
+        if (HD > 64) tma_load_4d(v_smem + at + kHalfBytes, &tm_v, full, 64, w.hk, sq.k_row0 + w.key0, sq.bq);
       }
       __syncwarp();
       int head = w.hk * group, u = 0;
@@ -438,7 +446,7 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
     const int r = warp - kMmaWarp;
     constexpr uint32_t idesc_st = make_idesc(AB_FMT, kBlk, kUnit, 0);  // [128 keys] x [64 rows], both operands K-major
     constexpr uint32_t idesc_acc = make_idesc(AB_FMT, kBlk, HD, 1);    // [128 keys] x [head dim], B N-contiguous
-    const uint64_t a_desc = make_smem_desc(r ? v_smem : k_smem, 16, 1024);                    // K (S^T = K Q^T) or V (dP^T = V dO^T)
+    const uint64_t a_desc0 = make_smem_desc(r ? v_smem : k_smem, 16, 1024);                   // K (S^T = K Q^T) or V (dP^T = V dO^T)
     const uint64_t b_desc0 = make_smem_desc(ring + (r ? kUnitTile : 0), 16, 1024);            // Q or dO of stage 0, K-major
     const uint64_t b_nd0 = make_smem_desc(ring + (r ? 0 : kUnitTile), kUnitHalf, 1024);       // dO (dV += P^T dO) or Q (dK += dS^T Q), N-contiguous
     constexpr uint64_t kStageStep = (2 * kUnitTile) >> 4;
@@ -447,13 +455,16 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
     const uint32_t acc_tmem = tmem + 256 + 128 * r;
     const uint32_t bar_stfull0 = smem_addr(&bar->st_full[0]), bar_pds0 = smem_addr(&bar->pds_full[0]);
     const uint32_t bar_full0 = smem_addr(&bar->qdo_full[0]), bar_empty0 = smem_addr(&bar->qdo_empty[0]);
-    const uint32_t bar_kvempty = smem_addr(&bar->kv_empty), bar_accdone = smem_addr(&bar->acc_done);
+    const uint32_t bar_accdone = smem_addr(&bar->acc_done);
     bool ok = true;
     while (ok) {
       const int t = queue_get(&bar->queue, wi, abort_flag);
       if (t < 0) break;
       const ItemA w = item_a(p, t);
       const int iters = w.iters;
+      const uint32_t set = wi % kSets<HD>;
+      const uint64_t a_desc = a_desc0 + set * (uint64_t)(kTileBytes >> 4);
+      const uint32_t bar_kvempty = smem_addr(&bar->kv_empty[set]);
       // rows of the sequence from a unit's first row on: below kUnit in the unit that runs past it (packed input only)
       const int left_first = p.cu_seqlens_q ? w.sq.q_len - w.u_lo * kUnit : 0x40000000, left_last = left_first - (w.nu - 1) * kUnit;
       int left = left_first;
@@ -477,7 +488,7 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
         __syncwarp();
         return true;
       };
-      if (!mbar_wait(smem_addr(&bar->kv_full), wi & 1, abort_flag, 62)) break;
+      if (!mbar_wait(smem_addr(&bar->kv_full[set]), (wi / kSets<HD>) & 1, abort_flag, 62)) break;
       if (!issue_st(0)) break;
       for (int u = 0; u < iters; ++u) {
         if (u + 1 < iters && !issue_st(u + 1)) { ok = false; break; }
@@ -552,9 +563,11 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
       // query rows that see this key
       const int vis_lo = sq.wr >= 0 ? jk - sq.koff - sq.wr : -0x40000000;
       const int vis_hi = jk < sq.k_len ? (sq.wl >= 0 ? jk - sq.koff + sq.wl : 0x40000000) : -0x40000001;
-      for (int u = (int)((grp - gu) & 1u); u < w.iters; u += 2) {  // the units whose running number has this group's parity
+      int um = (int)((grp - gu) & 1u);  // u modulo w.nu: the unit of its query head
+      for (int u = um; u < w.iters; u += 2, um += 2) {  // the units whose running number has this group's parity
+        while (um >= w.nu) um -= w.nu;
         const uint32_t g = gu + u;
-        const int s = g % kStages, r0 = (w.u_lo + u % w.nu) * kUnit, i0 = r0 + 32 * q2;
+        const int s = g % kStages, r0 = (w.u_lo + um) * kUnit, i0 = r0 + 32 * q2;
         if (!mbar_wait(smem_addr(&bar->qdo_full[s]), (g / kStages) & 1, abort_flag, 65)) { ok = false; break; }  // LSE / D of the stage
         if (!mbar_wait(smem_addr(&bar->st_full[grp]), (g >> 1) & 1, abort_flag, 66)) { ok = false; break; }
         tc_fence_after();
@@ -611,7 +624,7 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
 // and D of their own row from global memory instead.  The issuers release qdo_empty and kv_empty themselves; the dQ
 // issuer's commit is one of the two that release a K tile.
 struct BarB {
-  uint64_t qdo_full, qdo_empty;  // Q / dO of the item have landed; the item's last S / dP have read them
+  uint64_t qdo_full[2], qdo_empty[2];  // per set: Q / dO of the item have landed; the item's last S / dP have read them
   uint64_t kv_full[kDqSlots], kv_empty[kDqSlots];
   uint64_t s_full;    // MMA -> elementwise: S and dP are in TMEM
   uint64_t s_free;    // elementwise -> MMA: S and dP are in registers
@@ -634,13 +647,12 @@ struct ItemB {
 };
 __device__ __forceinline__ ItemB item_b(const BwdParams& p, int t) {
   ItemB w;
-  const int m_blocks = ceil_div(p.seqlen_q, kBlk);
-  const ItemPlace at = item_place(t, m_blocks, p.h * p.b, p.chunk_q);
-  w.head = at.pair % p.h;
-  w.bi = at.pair / p.h;
-  w.hk = w.head / (p.h / p.h_k);
+  const ItemPlace at = p.q_items.place(t);
+  w.bi = p.by_h.div(at.pair);
+  w.head = at.pair - w.bi * p.h;
+  w.hk = p.by_group.div(w.head);
   w.sq = seq_info(p, w.bi);
-  w.row0 = (m_blocks - 1 - at.block) * kBlk;
+  w.row0 = (p.q_items.blocks - 1 - at.block) * kBlk;
   w.live = w.row0 < w.sq.q_len;
   w.j_lo = w.iters = 0;
   if (w.live) {
@@ -667,12 +679,14 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
     if (tid == 0) atomicExch(status, 0x20000000);
     return;
   }
-  const int n_items = ceil_div(p.seqlen_q, kBlk) * p.h * p.b;
-  const uint32_t q_smem = base, do_smem = base + kTileBytes, ring = base + 2 * kTileBytes;
+  const int n_items = p.q_items.blocks * p.q_items.pairs;
+  const uint32_t q_smem = base, do_smem = base + kTileBytes / kSets<HD>, ring = base + 2 * kTileBytes;  // (sets as in bwd_dkv_kernel)
   BarB* bar = reinterpret_cast<BarB*>(smem + 7 * kTileBytes);
   if (tid == 0) {
-    mbar_init(smem_addr(&bar->qdo_full), 1);
-    mbar_init(smem_addr(&bar->qdo_empty), 2);      // the S and the dP issuer
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_addr(&bar->qdo_full[s]), 1);
+      mbar_init(smem_addr(&bar->qdo_empty[s]), 2);  // the S and the dP issuer
+    }
     for (int s = 0; s < kDqSlots; ++s) {
       mbar_init(smem_addr(&bar->kv_full[s]), 1);
       mbar_init(smem_addr(&bar->kv_empty[s]), 2);  // K: the S and the dQ issuer; V: the dP issuer, twice
@@ -725,14 +739,15 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
         continue;
       }
       queue_publish(&bar->queue, wi, t, lane);
-      if (!mbar_wait(smem_addr(&bar->qdo_empty), (wi & 1) ^ 1, abort_flag, 70)) break;
+      const uint32_t set = wi % kSets<HD>, at = set * kTileBytes;
+      if (!mbar_wait(smem_addr(&bar->qdo_empty[set]), ((wi / kSets<HD>) & 1) ^ 1, abort_flag, 70)) break;
       if (elect_one()) {
-        const uint32_t full = smem_addr(&bar->qdo_full);
+        const uint32_t full = smem_addr(&bar->qdo_full[set]);
         mbar_arrive_expect_tx(full, 2 * (HD / 64) * kHalfBytes);
-        tma_load_4d(q_smem, &tm_q, full, 0, w.head, sq.q_row0 + w.row0, sq.bq);
-        if (HD > 64) tma_load_4d(q_smem + kHalfBytes, &tm_q, full, 64, w.head, sq.q_row0 + w.row0, sq.bq);
-        tma_load_4d(do_smem, &tm_do, full, 0, w.head, sq.q_row0 + w.row0, sq.bq);
-        if (HD > 64) tma_load_4d(do_smem + kHalfBytes, &tm_do, full, 64, w.head, sq.q_row0 + w.row0, sq.bq);
+        tma_load_4d(q_smem + at, &tm_q, full, 0, w.head, sq.q_row0 + w.row0, sq.bq);
+        if (HD > 64) tma_load_4d(q_smem + at + kHalfBytes, &tm_q, full, 64, w.head, sq.q_row0 + w.row0, sq.bq);
+        tma_load_4d(do_smem + at, &tm_do, full, 0, w.head, sq.q_row0 + w.row0, sq.bq);
+        if (HD > 64) tma_load_4d(do_smem + at + kHalfBytes, &tm_do, full, 64, w.head, sq.q_row0 + w.row0, sq.bq);
       }
       __syncwarp();
       // K(j) lives in slot j % 3 and is held until dQ += dS K of its block has run; V(j) in slot 3 + j % 2 until dP has
@@ -760,19 +775,21 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
     // ------------------------------------------------------------------ MMA issuers 0 / 1: S = Q K^T / dP = dO V^T
     const int r = warp - kMmaWarp;
     constexpr uint32_t idesc_kk = make_idesc(AB_FMT, kBlk, kBlk, 0);
-    const uint64_t a_desc = make_smem_desc(r ? do_smem : q_smem, 16, 1024);
+    const uint64_t a_desc0 = make_smem_desc(r ? do_smem : q_smem, 16, 1024);
     const uint64_t ring_kd = make_smem_desc(ring, 16, 1024);
     constexpr uint64_t kSlotStep = kTileBytes >> 4;
     const uint32_t bar_full0 = smem_addr(&bar->kv_full[0]), bar_empty0 = smem_addr(&bar->kv_empty[0]);
     const uint32_t bar_sfull = smem_addr(&bar->s_full), bar_sfree = smem_addr(&bar->s_free);
-    const uint32_t bar_qdoempty = smem_addr(&bar->qdo_empty);
     const uint32_t d_tmem = tmem + 128 * r;
     bool ok = true;
     while (ok) {
       const int t = queue_get(&bar->queue, wi, abort_flag);
       if (t < 0) break;
       const ItemB w = item_b(p, t);
-      if (!mbar_wait(smem_addr(&bar->qdo_full), wi & 1, abort_flag, 73)) break;
+      const uint32_t set = wi % kSets<HD>;
+      const uint64_t a_desc = a_desc0 + set * (uint64_t)(kTileBytes >> 4);
+      const uint32_t bar_qdoempty = smem_addr(&bar->qdo_empty[set]);
+      if (!mbar_wait(smem_addr(&bar->qdo_full[set]), (wi / kSets<HD>) & 1, abort_flag, 73)) break;
       for (int it = 0; it < w.iters; ++it) {
         const uint32_t g = gj + it;
         const uint32_t slot = r ? kDqKSlots + (g & 1) : g % kDqKSlots;  // V(g) or K(g)

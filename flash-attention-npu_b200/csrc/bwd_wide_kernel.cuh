@@ -88,14 +88,14 @@ struct ItemW {
 // item_place, the heaviest block under a causal mask first.
 __device__ __forceinline__ ItemW item_w(const BwdParams& p, int t) {
   ItemW w;
-  const int n_kblocks = ceil_div(p.seqlen_k, kBlk), n_kv = n_kblocks * p.h_k * p.b;
+  const int n_kv = p.kv_items.blocks * p.kv_items.pairs;
   w.u_lo = w.nu = w.iters = 0;
   if (t < 2 * n_kv) {
     w.kind = t < n_kv ? kWideDK : kWideDV;
     if (t >= n_kv) t -= n_kv;
-    const ItemPlace at = item_place(t, n_kblocks, p.h_k * p.b, p.chunk_kv);
-    w.hk = at.pair % p.h_k;
-    w.bi = at.pair / p.h_k;
+    const ItemPlace at = p.kv_items.place(t);
+    w.bi = p.by_h_k.div(at.pair);
+    w.hk = at.pair - w.bi * p.h_k;
     w.head = 0;
     w.sq = seq_info(p, w.bi);
     w.row0 = at.block * kBlk;
@@ -106,18 +106,17 @@ __device__ __forceinline__ ItemW item_w(const BwdParams& p, int t) {
       const int i_hi = w.sq.wl >= 0 ? min(w.sq.q_len - 1, k1 - w.sq.koff + w.sq.wl) : w.sq.q_len - 1;
       w.u_lo = i_lo / kUnit;
       w.nu = i_hi >= i_lo ? i_hi / kUnit + 1 - w.u_lo : 0;
-      w.iters = w.nu * (p.h / p.h_k);
+      w.iters = w.nu * p.group;
     }
   } else {
     w.kind = kWideDQ;
     t -= 2 * n_kv;
-    const int m_blocks = ceil_div(p.seqlen_q, kBlk);
-    const ItemPlace at = item_place(t, m_blocks, p.h * p.b, p.chunk_q);
-    w.head = at.pair % p.h;
-    w.bi = at.pair / p.h;
-    w.hk = w.head / (p.h / p.h_k);
+    const ItemPlace at = p.q_items.place(t);
+    w.bi = p.by_h.div(at.pair);
+    w.head = at.pair - w.bi * p.h;
+    w.hk = p.by_group.div(w.head);
     w.sq = seq_info(p, w.bi);
-    w.row0 = (m_blocks - 1 - at.block) * kBlk;
+    w.row0 = (p.q_items.blocks - 1 - at.block) * kBlk;
     w.live = w.row0 < w.sq.q_len;
     if (w.live) {  // keys that at least one row of the block sees
       const int r1 = min(w.sq.q_len, w.row0 + kBlk) - 1;
@@ -199,8 +198,8 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
     if (tid == 0) atomicExch(status, 0x20000000);
     return;
   }
-  const int group = p.h / p.h_k;
-  const int n_items = 2 * ceil_div(p.seqlen_k, kBlk) * p.h_k * p.b + ceil_div(p.seqlen_q, kBlk) * p.h * p.b;
+  const int group = p.group;
+  const int n_items = 2 * p.kv_items.blocks * p.kv_items.pairs + p.q_items.blocks * p.q_items.pairs;
   BarW<HD>* bar = reinterpret_cast<BarW<HD>*>(smem + G::kBarOff);
   if (tid == 0) {
     mbar_init(smem_addr(&bar->a_full), 1);
@@ -504,9 +503,11 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
         hi = row_ok ? (sq.wl >= 0 ? j - sq.koff + sq.wl : 0x40000000) : -0x40000001;
       }
       const uint64_t nl_row = pack_f32x2(nl1, nl1), nd_row = pack_f32x2(nd1, nd1);
-      for (int u = (int)((grp - gu) & 1u); u < w.iters; u += 2) {  // the units whose running number has this group's parity
+      int um = (int)((grp - gu) & 1u);  // u modulo w.nu: the unit of its head
+      for (int u = um; u < w.iters; u += 2, um += 2) {  // the units whose running number has this group's parity
+        while (um >= w.nu) um -= w.nu;
         const uint32_t g = gu + u;
-        const int st = g % G::kStats, c0 = (w.u_lo + u % w.nu) * kUnit;
+        const int st = g % G::kStats, c0 = (w.u_lo + um) * kUnit;
         if (!is_q && !mbar_wait(smem_addr(&bar->stat_full[st]), (g / G::kStats) & 1, abort_flag, 72)) { ok = false; break; }
         if (!mbar_wait(smem_addr(&bar->st_full[grp]), (g >> 1) & 1, abort_flag, 73)) { ok = false; break; }
         tc_fence_after();

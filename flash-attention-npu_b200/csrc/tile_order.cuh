@@ -75,11 +75,28 @@ FA_TILE_HD bool tile_locate(TileCursor& c, const Levels& lv, int heads_all, int 
 struct ItemPlace {
   int pair, block;
 };
-FA_TILE_HD ItemPlace item_place(int t, int blocks, int pairs, int chunk) {
-  const int ck = t / (chunk * blocks), r = t - ck * chunk * blocks, first = ck * chunk;
-  const int cnt = chunk < pairs - first ? chunk : pairs - first;  // pairs in this chunk (the last one may be short)
-  const int nb = r / cnt;
-  return {first + r - nb * cnt, nb};
+struct ItemOrder {
+  int blocks, pairs, chunk;
+  FastDiv by_chunk_items, by_chunk, by_last;  // items of a chunk, its pairs, the pairs of the last chunk (if that is short)
+  void set(int blocks_, int pairs_, int chunk_) {
+    blocks = blocks_;
+    pairs = pairs_;
+    chunk = chunk_;
+    by_chunk_items.set(chunk * blocks);
+    by_chunk.set(chunk);
+    by_last.set(chunk > 0 ? pairs % chunk : 0);
+  }
+  FA_TILE_HD ItemPlace place(int t) const {
+    const int ck = by_chunk_items.div(t), r = t - ck * chunk * blocks, first = ck * chunk;
+    const int cnt = chunk < pairs - first ? chunk : pairs - first;  // pairs in this chunk (the last one may be short)
+    const int nb = cnt == chunk ? by_chunk.div(r) : by_last.div(r);
+    return {first + r - nb * cnt, nb};
+  }
+};
+inline ItemPlace item_place(int t, int blocks, int pairs, int chunk) {
+  ItemOrder o;
+  o.set(blocks, pairs, chunk);
+  return o.place(t);
 }
 
 }  // namespace fa
