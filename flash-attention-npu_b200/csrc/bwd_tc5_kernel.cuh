@@ -856,11 +856,28 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
     const float a1 = SOFTCAP ? p.softmax_scale / p.softcap : p.scale_log2, cap1 = p.softcap * kLog2e;
     const uint64_t sl2 = pack_f32x2(a1, a1), cap2 = pack_f32x2(cap1, cap1), sc2 = pack_f32x2(p.softmax_scale, p.softmax_scale);
+    // Item number k and its row's LSE and D (rows beyond the sequence: P = 0).  An item's are asked for before the wait for the dQ of
+    // the item before, which hides the loads and the item's arithmetic, some 1300
+    // cycles: 12 packed sequences of 37 - 2999 rows, 16 / 4 heads, head dim 64, backward 352 -> 341 us; 4 K causal, b 4, 32 heads, head dim
+    // 128 1566 -> 1551.
+    auto fetch = [&](uint32_t k, ItemB& w, float& lse, float& delta) -> bool {
+      const int t = queue_get(&bar->queue, k, abort_flag);
+      if (t < 0) return false;
+      w = item_b(p, t);
+      lse = INFINITY;
+      delta = 0.f;
+      if (w.row0 + r < w.sq.q_len) {
+        const int64_t li = (int64_t)w.sq.bq * p.lse_batch_stride + (int64_t)w.head * p.lse_head_stride + w.sq.q_row0 + w.row0 + r;
+        lse = p.lse[li];
+        delta = p.delta[li];
+      }
+      return true;
+    };
     bool ok = true;
-    while (ok) {
-      const int t = queue_get(&bar->queue, wi, abort_flag);
-      if (t < 0) break;
-      const ItemB w = item_b(p, t);
+    ItemB w;
+    float lse, delta;
+    bool more = fetch(0, w, lse, delta);
+    while (ok && more) {
       const SeqInfo& sq = w.sq;
       const int row0 = w.row0, i = row0 + r;
       T* dq_row = reinterpret_cast<T*>(p.dq) + (int64_t)sq.bq * p.dq_batch_stride + (int64_t)(sq.q_row0 + i) * p.dq_row_stride +
@@ -868,12 +885,7 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
       int hi = sq.k_len - 1, lo = 0;
       if (sq.wr >= 0) hi = min(hi, i + sq.koff + sq.wr);
       if (sq.wl >= 0) lo = max(0, i + sq.koff - sq.wl);
-      float nl = -INFINITY, nd = 0.f;  // -LSE * log2(e) and -D * scale; rows beyond the sequence: P = 0
-      if (i < sq.q_len) {
-        const int64_t li = (int64_t)sq.bq * p.lse_batch_stride + (int64_t)w.head * p.lse_head_stride + sq.q_row0 + i;
-        nl = -p.lse[li] * kLog2e;
-        nd = -p.delta[li] * p.softmax_scale;
-      }
+      const float nl = -lse * kLog2e, nd = -delta * p.softmax_scale;
       const uint64_t nlse2 = pack_f32x2(nl, nl), ndls2 = pack_f32x2(nd, nd);
       const int i_max = min(sq.q_len, row0 + kBlk) - 1;
       for (int it = 0; it < w.iters; ++it) {
@@ -913,6 +925,9 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
       }
       if (!ok) break;
       // ---- epilogue: the accumulator is handed back once it is in registers
+      const int n_cols = i < sq.q_len ? p.d - 32 * q4 : 0;
+      gj += w.iters;
+      more = fetch(wi + 1, w, lse, delta);
       if (!mbar_wait(smem_addr(&bar->acc_done), wi & 1, abort_flag, 80)) break;
       tc_fence_after();
       uint32_t a[32];
@@ -921,9 +936,8 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_addr(&bar->acc_free));
-      if (i < sq.q_len) store_slice<T>(dq_row, a, p.d - 32 * q4, p.dq_sectors);
+      store_slice<T>(dq_row, a, n_cols, p.dq_sectors);
       ++wi;
-      gj += w.iters;
     }
   }
 
