@@ -581,7 +581,7 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&bar->pds_full[grp]));
+        mbar_arrive_lane0(smem_addr(&bar->pds_full[grp]), lane);
       }
       if (!ok) break;
       // ---- epilogue: dV, dK of this key, 32 columns of the head dim; the accumulators are handed back once they are in
@@ -594,7 +594,7 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_addr(&bar->acc_free));
+      mbar_arrive_lane0(smem_addr(&bar->acc_free), lane);
       if (jk < sq.k_len) {
         store_slice<T>(dv_row, av, p.d - 32 * q4, p.dv_sectors);
         store_slice<T>(dk_row, ak, p.d - 32 * q4, p.dk_sectors);
@@ -689,7 +689,7 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
     }
     for (int s = 0; s < kDqSlots; ++s) {
       mbar_init(smem_addr(&bar->kv_full[s]), 1);
-      mbar_init(smem_addr(&bar->kv_empty[s]), 2);  // K: the S and the dQ issuer; V: the dP issuer, twice
+      mbar_init(smem_addr(&bar->kv_empty[s]), s < kDqKSlots ? 2 : 1);  // K: the S and the dQ issuer; V: the dP issuer
     }
     mbar_init(smem_addr(&bar->s_full), 2);           // S and dP
     mbar_init(smem_addr(&bar->s_free), kEwWarps);
@@ -807,7 +807,6 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
           for (int ks = 1; ks < HD / 16; ++ks) mma_ss_c<true>(d_tmem, a_desc + kmaj_off(ks), b_desc + kmaj_off(ks), idesc_kk);
           mma_commit(bar_sfull);
           mma_commit(bar_empty0 + 8 * slot);
-          if (r) mma_commit(bar_empty0 + 8 * slot);        // nobody else reads the V tile
           if (it == w.iters - 1) mma_commit(bar_qdoempty);   // the item's last reader of Q / dO
         }
         __syncwarp();
@@ -898,7 +897,7 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&bar->s_free));  // the products of the next block may overwrite S and dP
+        mbar_arrive_lane0(smem_addr(&bar->s_free), lane);  // the products of the next block may overwrite S and dP
         const int c0 = (w.j_lo + it) * kBlk;
         // does any (row of the block, key of the block) pair fall outside the mask?  (the same answer in every thread)
         bool need_mask = c0 + kBlk > sq.k_len;
@@ -921,7 +920,7 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&bar->ds_full));
+        mbar_arrive_lane0(smem_addr(&bar->ds_full), lane);
       }
       if (!ok) break;
       // ---- epilogue: the accumulator is handed back once it is in registers
@@ -935,7 +934,7 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_addr(&bar->acc_free));
+      mbar_arrive_lane0(smem_addr(&bar->acc_free), lane);
       store_slice<T>(dq_row, a, n_cols, p.dq_sectors);
       ++wi;
     }

@@ -533,7 +533,7 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&bar->pds_full[grp]));
+        mbar_arrive_lane0(smem_addr(&bar->pds_full[grp]), lane);
       }
       if (!ok) break;
       // ---- epilogue: 64 columns of this row; the accumulator is handed back once it is in registers
@@ -546,7 +546,7 @@ bwd_wide_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ Wid
         tmem_wait_ld();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&bar->acc_free));
+        mbar_arrive_lane0(smem_addr(&bar->acc_free), lane);
         if (row_ok) {
           const bool sectors = w.kind == kWideDQ ? p.dq_sectors : w.kind == kWideDK ? p.dk_sectors : p.dv_sectors;
           store_slice<T>(out, a0, p.d - 64 * q4, sectors);
