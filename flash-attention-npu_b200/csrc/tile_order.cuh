@@ -24,8 +24,7 @@ struct FastDiv {
   void set(int d) {
     mul = shift = 0;
     if (d <= 1) return;
-    uint32_t s = 1;
-    while ((1ull << s) < (uint64_t)d) ++s;
+    const uint32_t s = 32 - (uint32_t)__builtin_clz((uint32_t)d - 1);  // (six to nine of these a call: no loop)
     mul = (uint32_t)(((1ull << (31 + s)) + (uint32_t)d - 1) / (uint32_t)d);
     shift = s - 1;
   }
