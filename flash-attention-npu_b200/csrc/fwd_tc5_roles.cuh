@@ -29,7 +29,7 @@ struct RingPos {
 // pages hold whole 128-key blocks, the page of a block comes from the block table (the warp keeps
 // 32 consecutive entries in registers, one per lane).
 // ---------------------------------------------------------------------------------------------
-// HD (64 or 128) is the head dim: with 64 a Q / K / V tile is the first 64-column half of its 32 KiB slot only.
+// HD is the tile width; with 64 a tile has one 64-column half and a ring slot of 16 KiB (Geo).
 template <int IN, int HD>
 __device__ __forceinline__ void producer_loop(const Tc5Params& p, const CUtensorMap* tm_q, const CUtensorMap* tm_k,
                                               const CUtensorMap* tm_v, Barriers* bar, uint32_t q_smem, uint32_t kv_smem) {
