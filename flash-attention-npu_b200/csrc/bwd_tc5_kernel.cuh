@@ -677,6 +677,7 @@ bwd_dq_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUten
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   if ((base & 1023u) != 0) {
     if (tid == 0) atomicExch(status, 0x20000000);
+    grid_wait();
     return;
   }
   const int n_items = p.q_items.blocks * p.q_items.pairs;

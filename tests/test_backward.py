@@ -330,3 +330,36 @@ def test_gradient_rows_off_the_sector_boundary(d, where):
         assert torch.equal(view, x)
         view.fill_(7.0)
         assert bool((buf == 7.0).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d,s,h", [(64, 130, 1), (64, 700, 30), (128, 128, 2), (128, 1100, 20)])
+def test_what_follows_the_backward_follows_both_kernels(d, s, h):
+    """The dQ kernel starts beside the dK / dV kernel: fewer work items than SMs, and more.  Inputs are overwritten right behind the
+    call, in stream order; the same through a captured graph."""
+    from flash_b200 import ops
+    g = torch.Generator().manual_seed(s)
+    q, k, v, dout = (torch.randn(1, s, h, d, generator=g).to(torch.bfloat16).cuda() for _ in range(4))
+    kw = dict(softmax_scale=d ** -0.5, causal=True)
+    out, lse = ops.attention_forward(q, k, v, **kw)
+    want = ops.attention_backward(dout, q, k, v, out, lse, **kw)
+    torch.cuda.synchronize()
+    for _ in range(20):
+        x = [t.clone() for t in (dout, q, k, v)]
+        got = ops.attention_backward(*x, out, lse, **kw)
+        for t in x:
+            t.fill_(float("nan"))
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
+    x = [t.clone() for t in (dout, q, k, v)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = ops.attention_backward(*x, out, lse, **kw)
+        for t in x:
+            t.fill_(float("nan"))
+    for _ in range(3):
+        for t, src in zip(x, (dout, q, k, v)):
+            t.copy_(src)
+        graph.replay()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
