@@ -413,3 +413,20 @@ def test_calls_that_start_under_one_another(d):
     for _ in range(3):
         graph.replay()
         assert all(torch.equal(a, c) for a, c in zip(want, got))
+
+
+@pytest.mark.parametrize("s_q,s_k,causal,window", [
+    (128, 1, False, (-1, -1)), (128, 128, True, (-1, -1)), (129, 129, True, (-1, -1)), (256, 256, False, (-1, -1)),
+    (257, 385, True, (-1, -1)), (300, 200, True, (-1, -1)),  # rows that see no key
+    (513, 513, True, (100, 0)), (400, 640, False, (200, 130))])
+def test_two_p_buffers_over_many_tiles(s_q, s_k, causal, window):
+    """Head dim 64: tiles of one, two and more key blocks, sub-tiles of unequal length, one tile after another on every SM (two P
+    buffers, and factors that alternate between two rows across tiles)."""
+    g = torch.Generator().manual_seed(s_q + s_k)
+    b, h, hk = 5, 64, 4
+    q, k, v = U.normal((b, s_q, h, 64), FP, g), U.normal((b, s_k, hk, 64), FP, g), U.normal((b, s_k, hk, 64), FP, g)
+    out, lse, pl = ops.attention_forward(q.cuda(), k.cuda(), v.cuda(), softmax_scale=0.125, causal=causal, window_left=window[0],
+                                         window_right=window[1], return_plan=True)
+    assert pl.kernel == L.KERNEL_TCGEN05 and b * h > 2 * 148
+    go, gl = OA.flash_attn_func(q, k, v, causal=causal, window_size=window)
+    U.check_rules(out, lse, go, gl, tag=f"{s_q} x {s_k}")
