@@ -59,7 +59,7 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
     }
     for (int s = 0; s < kMaxSlots; ++s) {
       mbar_init(smem_addr(&bar->kv_full[s]), 1);
-      mbar_init(smem_addr(&bar->kv_empty[s]), 2);
+      mbar_init(smem_addr(&bar->kv_empty[s]), Geo<HD>::kWide ? 1 : 2);  // the issuing warps that read the tile
     }
     mbar_init(smem_addr(&bar->fix_req), 2);
     mbar_init(smem_addr(&bar->v_fixed), 1);
