@@ -54,7 +54,8 @@ fwd_tc5_kernel(const __grid_constant__ Tc5Params p, const __grid_constant__ CUte
       mbar_init(smem_addr(&bar->corr_ready[t][0]), 4);
       mbar_init(smem_addr(&bar->corr_ready[t][1]), 4);
       mbar_init(smem_addr(&bar->o_ready[t]), 4);
-      mbar_init(smem_addr(&bar->o_done[t]), 1);
+      mbar_init(smem_addr(&bar->o_done[t][0]), 1);
+      mbar_init(smem_addr(&bar->o_done[t][1]), 1);
       mbar_init(smem_addr(&bar->o_free[t]), 4);
     }
     for (int s = 0; s < kMaxSlots; ++s) {

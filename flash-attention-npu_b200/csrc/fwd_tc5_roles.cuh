@@ -185,7 +185,7 @@ __device__ __forceinline__ void mma_loop(const Tc5Params& p, Barriers* bar, uint
   const uint32_t s_tmem = tmem + t * 128, o_tmem = tmem + 256 + t * 128;
   const uint32_t bar_pfull = smem_addr(&bar->p_full[t][0][0]);
   const uint32_t bar_ofree = smem_addr(&bar->o_free[t]), bar_oready = smem_addr(&bar->o_ready[t]);
-  const uint32_t bar_odone = smem_addr(&bar->o_done[t]), bar_sfull = smem_addr(&bar->s_full[t]);
+  const uint32_t bar_odone = smem_addr(&bar->o_done[t][0]), bar_sfull = smem_addr(&bar->s_full[t]);
   const uint32_t bar_sfree = smem_addr(&bar->s_free[t]);
   const uint32_t bar_kvfull0 = smem_addr(&bar->kv_full[0]), bar_kvempty0 = smem_addr(&bar->kv_empty[0]);
   const int o = 1 - t;
@@ -277,7 +277,7 @@ __device__ __forceinline__ void mma_loop(const Tc5Params& p, Barriers* bar, uint
       if (elect_one()) {
 #pragma unroll
         for (int ks = 4; ks < 8; ++ks) mma_ss_c<true>(o_tmem, p_desc + k_off(ks), v_desc + (uint64_t)(ks * (2048 >> 4)), idesc_pv);
-        mma_commit(bar_odone);
+        mma_commit(bar_odone + 8 * buf);
         mma_commit(bar_kvempty0 + slot * 8);
         if (!G::kWide && !other) mma_commit(bar_kvempty0 + slot * 8);
       }

@@ -137,7 +137,7 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
   uint32_t s_cnt = 0, ev_cnt = 0;  // blocks, events (corr_ready) so far
   constexpr int kPBufs = Geo<HD>::kPBufs;
   const uint32_t p_row0 = p_smem + t * kPBufs * kTileBytes + row * 128 + ((row & 7) << 4);
-  const uint32_t bar_sfree = smem_addr(&bar->s_free[t]), bar_odone = smem_addr(&bar->o_done[t]);
+  const uint32_t bar_sfree = smem_addr(&bar->s_free[t]), bar_odone = smem_addr(&bar->o_done[t][0]);
   // with softcap the scores are in the log2 domain once they have been capped: the scale is part of the cap
   const float scale_log2 = CAP ? 1.f : p.scale_log2;
   const float lse_scale = CAP ? 0.6931471805599453f : p.a.softmax_scale;  // running maximum -> natural log
@@ -272,8 +272,6 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
         store_p_chunk(p_row, 3, pk);
         fence_proxy_async();
         __syncwarp();
-        // for the event behind the tile's last block (corr_ready)
-        if (kPBufs > 1 && j == ti.jhi - 1 && blk > 0 && !mbar_wait(bar_odone, (blk - 1) & 1, abort_flag, 42)) return;
         mbar_arrive_lane0(smem_addr(&bar->p_full[t][buf][1]), lane);  // last 64 keys
       }
       float s0, s1;
@@ -286,7 +284,8 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
       l_run += other;
       if (!lead) continue;
     }
-    // 1 / l for the epilogue, LSE from here
+    // 1 / l for the epilogue, LSE from here.  The event behind the tile's last block n waits for P.V of block n - 1 (corr_ready).
+    if (kPBufs > 1 && s_cnt > 1 && !mbar_wait(bar_odone + 8 * (s_cnt % kPBufs), ((s_cnt - 2) / kPBufs) & 1, abort_flag, 42)) return;
     bar->corr[t][ev_cnt & 1][row] = l_run > 0.f ? 1.f / l_run : 0.f;
     __syncwarp();
     mbar_arrive_lane0(smem_addr(&bar->corr_ready[t][ev_cnt & 1]), lane);
@@ -376,6 +375,7 @@ __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* ba
   const int row = warp_in_wg * 32 + lane;
   const uint32_t lane_addr = (uint32_t)(warp_in_wg * 32) << 16;
   uint32_t ev_cnt[2] = {0, 0}, od_cnt[2] = {0, 0};
+  constexpr uint32_t kPBufs = Geo<HD>::kPBufs;
   const int d_cols = p.a.d;
 
   TileWalk<IN> walk(bar);
@@ -390,7 +390,7 @@ __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* ba
         if (!mbar_wait(smem_addr(&bar->corr_ready[t][ev_cnt[t] & 1]), (ev_cnt[t] >> 1) & 1, abort_flag, 43)) return;
         const float f = bar->corr[t][ev_cnt[t] & 1][row];
         ++ev_cnt[t];
-        if (!mbar_wait(smem_addr(&bar->o_done[t]), od_cnt[t] & 1, abort_flag, 44)) return;  // P.V of block j-1 done
+        if (!mbar_wait(smem_addr(&bar->o_done[t][od_cnt[t] % kPBufs]), (od_cnt[t] / kPBufs) & 1, abort_flag, 44)) return;  // P.V of block j-1 done
         ++od_cnt[t];
         if (__any_sync(0xffffffffu, f != 1.f)) {
           tc_fence_after();
@@ -408,7 +408,7 @@ __device__ __forceinline__ void correction_loop(const Tc5Params& p, Barriers* ba
       if (!mbar_wait(smem_addr(&bar->corr_ready[t][ev_cnt[t] & 1]), (ev_cnt[t] >> 1) & 1, abort_flag, 45)) return;
       const float inv = bar->corr[t][ev_cnt[t] & 1][row];
       ++ev_cnt[t];
-      if (!mbar_wait(smem_addr(&bar->o_done[t]), od_cnt[t] & 1, abort_flag, 46)) return;  // last P.V done
+      if (!mbar_wait(smem_addr(&bar->o_done[t][od_cnt[t] % kPBufs]), (od_cnt[t] / kPBufs) & 1, abort_flag, 46)) return;  // last P.V done
       ++od_cnt[t];
       tc_fence_after();
       const int i = ti.row0[t] + row;

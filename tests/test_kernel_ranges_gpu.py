@@ -418,10 +418,12 @@ def test_calls_that_start_under_one_another(d):
 @pytest.mark.parametrize("s_q,s_k,causal,window", [
     (128, 1, False, (-1, -1)), (128, 128, True, (-1, -1)), (129, 129, True, (-1, -1)), (256, 256, False, (-1, -1)),
     (257, 385, True, (-1, -1)), (300, 200, True, (-1, -1)),  # rows that see no key
-    (513, 513, True, (100, 0)), (400, 640, False, (200, 130))])
+    (513, 513, True, (100, 0)), (400, 640, False, (200, 130)),
+    (256, 1500, False, (-1, -1)), (700, 1100, True, (-1, -1))])  # many blocks between two tiles' last ones
 def test_two_p_buffers_over_many_tiles(s_q, s_k, causal, window):
     """Head dim 64: tiles of one, two and more key blocks, sub-tiles of unequal length, one tile after another on every SM (two P
-    buffers, and factors that alternate between two rows across tiles)."""
+    buffers with a barrier each for the P.V that has read them, and factors that alternate between two rows across tiles; the
+    softmax warps look at one phase of those barriers a tile, the more the blocks the more pass unseen)."""
     g = torch.Generator().manual_seed(s_q + s_k)
     b, h, hk = 5, 64, 4
     q, k, v = U.normal((b, s_q, h, 64), FP, g), U.normal((b, s_k, hk, 64), FP, g), U.normal((b, s_k, hk, 64), FP, g)
