@@ -290,9 +290,11 @@ __device__ __forceinline__ void softmax_loop(const Tc5Params& p, Barriers* bar, 
     __syncwarp();
     mbar_arrive_lane0(smem_addr(&bar->corr_ready[t][ev_cnt & 1]), lane);
     ++ev_cnt;
+    // m_run * lse_scale + ln l.  Which product is fused into the sum is written out: both factors are constants with softcap, the
+    // compiler's choice changed with the code around it, and a backward that reads the LSE gets other bits then.
+    const float lse = CAP ? fmaf(__log2f(l_run), 0.6931471805599453f, __fmul_rn(m_run, lse_scale)) : fmaf(m_run, lse_scale, __logf(l_run));
     if (i < ti.q_len)
-      p.a.lse[(int64_t)ti.bi * p.a.lse_batch_stride + (int64_t)ti.hh * p.a.lse_head_stride + ti.q_row0 + i] =
-          l_run > 0.f ? (m_run * lse_scale + __logf(l_run)) : INFINITY;
+      p.a.lse[(int64_t)ti.bi * p.a.lse_batch_stride + (int64_t)ti.hh * p.a.lse_head_stride + ti.q_row0 + i] = l_run > 0.f ? lse : INFINITY;
   }
 }
 
