@@ -234,7 +234,7 @@ struct Barriers {
   // the phase before, block n - 3's, is over (the correction warps waited for it before they let P.V of block n - 2 be issued),
   // and the phase behind, block n + 1's, cannot end before the warp has delivered its P.  (The wait lies behind that warp's last
   // arrival for block n; with one barrier for both buffers it had to lie in front of it: b 4, s 4096, 32 heads, head dim 64, full
-  // 763 -> 728 us, causal 445 -> 423, 12 packed sequences of 37 - 2999 rows, 16 / 4 heads, 181 -> 183.)
+  // 763 -> 728 us, causal 445 -> 423.)
   uint64_t corr_ready[2][2];
   uint64_t o_ready[2];     // correction -> MMA: O_t has been rescaled, P.V of block j may accumulate
   uint64_t o_done[2][2];   // MMA -> correction, softmax: P.V of a block has completed (O_t updated, P_t read); [sub-tile][P buffer]

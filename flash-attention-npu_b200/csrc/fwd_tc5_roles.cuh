@@ -8,25 +8,19 @@ namespace tc5 {
 
 // Both single-thread roles walk the K / V tiles of a CTA tile in the order the tensor pipe needs them:
 //   K_lo | K_lo+1 V_lo | K_lo+2 V_lo+1 | ... | V_hi-1
-// (Q.K^T of block j+1 is issued before P.V of block j).  Ring slot and parity follow from a running count.
+// (Q.K^T of block j+1 is issued before P.V of block j).  Ring slot and parity advance tile by tile.
 // (Carrying the order across tile boundaries -- Q.K^T of the next tile's first block before P.V of this tile's last
 // one -- lets one sub-tile run a block ahead of the other, and then the two need four K / V tiles at a time where the
-// ring has three: measured 8 % slower on causal 4K.)
+// ring of 128 columns has three: measured 8 % slower there on causal 4K.)
 template <int SLOTS>
 struct RingPos {
-  uint32_t cnt = 0, phase = 0;  // four slots: a running count; otherwise slot and phase, two instructions less on the issuing warps' path
+  uint32_t at = 0, phase = 0;
   __device__ __forceinline__ void next(uint32_t& slot, uint32_t& par) {
-    if (SLOTS == 4) {
-      slot = cnt % SLOTS;
-      par = (cnt / SLOTS) & 1;
-      ++cnt;
-    } else {
-      slot = cnt;
-      par = phase;
-      if (++cnt == SLOTS) {
-        cnt = 0;
-        phase ^= 1;
-      }
+    slot = at;
+    par = phase;
+    if (++at == SLOTS) {
+      at = 0;
+      phase ^= 1;
     }
   }
 };
