@@ -112,12 +112,9 @@ int fa_b200_bwd(const fa_bwd_params* a, void* workspace, size_t workspace_bytes,
   p.b = a->b; p.seqlen_q = a->seqlen_q; p.seqlen_k = a->seqlen_k; p.h = a->h; p.h_k = a->h_k; p.d = a->d;
   p.d_pad = a->d <= 64 ? 64 : (a->d <= 128 ? 128 : 256);
   p.total_q = (int32_t)rows;
-  auto sectors = [&](const void* ptr, int64_t row, int64_t head, int64_t batch) {
-    return (reinterpret_cast<uintptr_t>(ptr) % 32 == 0 && a->d % 16 == 0 && row % 16 == 0 && head % 16 == 0 && (a->b == 1 || batch % 16 == 0)) ? 1 : 0;
-  };
-  p.dq_sectors = sectors(p.dq, p.dq_row_stride, p.dq_head_stride, p.dq_batch_stride);
-  p.dk_sectors = sectors(p.dk, p.dk_row_stride, p.dk_head_stride, p.dk_batch_stride);
-  p.dv_sectors = sectors(p.dv, p.dv_row_stride, p.dv_head_stride, p.dv_batch_stride);
+  p.dq_sectors = whole_sectors(p.dq, p.d, p.b, p.dq_row_stride, p.dq_head_stride, p.dq_batch_stride);
+  p.dk_sectors = whole_sectors(p.dk, p.d, p.b, p.dk_row_stride, p.dk_head_stride, p.dk_batch_stride);
+  p.dv_sectors = whole_sectors(p.dv, p.d, p.b, p.dv_row_stride, p.dv_head_stride, p.dv_batch_stride);
   // window normalisation of the golden (tests/fa_small_op_golden.py:21-33; the same rule as the forward's host code)
   int wl = a->window_left, wr = a->window_right;
   if (wl >= a->seqlen_k - 1) wl = -1;

@@ -218,9 +218,7 @@ __device__ __forceinline__ void store_slice(T* dst, const uint32_t (&a)[32], int
 #pragma unroll
     for (int e = 0; e < 16; e += 8) {
       if (2 * e >= n_cols) break;
-      asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(dst + 2 * e), "r"(w[e]), "r"(w[e + 1]), "r"(w[e + 2]),
-                   "r"(w[e + 3]), "r"(w[e + 4]), "r"(w[e + 5]), "r"(w[e + 6]), "r"(w[e + 7])
-                   : "memory");
+      store_sector(dst + 2 * e, w, e);
     }
     return;
   }

@@ -37,6 +37,20 @@ struct KParams {
 // call would pay on every launch (fwd_tc5.cu).
 cudaError_t allow_smem(const void* kernel, int bytes);
 
+// ---- stores of whole 32-byte sectors ----
+// Do all rows of a 16-bit tensor of head dim d start on 32-byte boundaries, and are they whole sectors long?  (strides in elements)
+inline bool whole_sectors(const void* ptr, int d, int b, int64_t row_stride, int64_t head_stride, int64_t batch_stride) {
+  return reinterpret_cast<uintptr_t>(ptr) % 32 == 0 && d % 16 == 0 && row_stride % 16 == 0 && head_stride % 16 == 0 &&
+         (b == 1 || batch_stride % 16 == 0);
+}
+// The eight registers w[c ..] to a 32-byte boundary.
+template <int N>
+__device__ __forceinline__ void store_sector(void* dst, const uint32_t (&w)[N], int c) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(dst), "r"(w[c]), "r"(w[c + 1]), "r"(w[c + 2]), "r"(w[c + 3]),
+               "r"(w[c + 4]), "r"(w[c + 5]), "r"(w[c + 6]), "r"(w[c + 7])
+               : "memory");
+}
+
 // ---- programmatic dependent launch ----
 // The decode kernels and the merges are launched so that the launch and the start of their CTAs lie under the end of the
 // kernel in front of them on the stream (launch_dependent).  Such a kernel must call grid_wait() in every CTA before it reads

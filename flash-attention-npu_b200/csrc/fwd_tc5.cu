@@ -253,8 +253,7 @@ int tc5_launch(const fa_fwd_params& a, const fa_fwd_plan& pl, cudaStream_t st, s
     p.softcap_mul = a.softmax_scale / a.softcap;
     p.softcap_l2 = a.softcap * kLog2e;
   }
-  p.o_sectors = (reinterpret_cast<uintptr_t>(a.o) % 32 == 0 && a.d % 16 == 0 && a.o_row_stride % 16 == 0 && a.o_head_stride % 16 == 0 &&
-                 (a.b == 1 || a.o_batch_stride % 16 == 0)) ? 1 : 0;
+  p.o_sectors = whole_sectors(a.o, a.d, a.b, a.o_row_stride, a.o_head_stride, a.o_batch_stride);
   p.fix_tail = (a.seqused_k || a.cu_seqlens_k) ? 1 : 0;
   {
     // L2 chunks of the tile order (tile_info).  A chunk is 2 * grid / gcd(2 * grid, m_tiles) pairs: a whole

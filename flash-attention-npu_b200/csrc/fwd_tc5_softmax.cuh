@@ -361,9 +361,7 @@ __device__ __forceinline__ void store_cols(T* dst, const uint32_t (&w)[32], int 
   for (int c = 0; c < 32; c += SECTORS ? 8 : 4) {
     if (2 * c >= n_cols) continue;
     if (SECTORS) {
-      asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(dst + 2 * c), "r"(w[c]), "r"(w[c + 1]), "r"(w[c + 2]),
-                   "r"(w[c + 3]), "r"(w[c + 4]), "r"(w[c + 5]), "r"(w[c + 6]), "r"(w[c + 7])
-                   : "memory");
+      store_sector(dst + 2 * c, w, c);
     } else {  // written once, read by nobody here: streaming
       __stcs(reinterpret_cast<uint4*>(dst + 2 * c), make_uint4(w[c], w[c + 1], w[c + 2], w[c + 3]));
     }
