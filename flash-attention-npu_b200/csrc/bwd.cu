@@ -19,7 +19,7 @@ void count_launches(int n);                      // api.cu: fa_b200_launch_count
 
 static size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
-// Pairs per chunk of the work-item order (item_place in tile_order.cuh): all of them when what they stream (two 16-bit
+// Pairs per chunk of the work-item order (ItemOrder in tile_order.cuh): all of them when what they stream (two 16-bit
 // tensors of `rows` rows and `heads` heads) stays in L2 together, otherwise one.  Forward and backward, all pairs against one
 // at a time: 14 - 60 MB 0.89 - 0.98 x, 64 - 88 MB 0.98 - 1.00 x, 92 - 96 MB 0.99 - 1.035 x (b 24, s 512, 16 heads, d 128: 298
 // -> 309 us), 104 - 114 MB 1.01 - 1.06 x; the 4 K causal case, 268 MB, in chunks of ten pairs: dK / dV kernel 917 -> 1017 us.

@@ -85,7 +85,7 @@ struct ItemW {
   bool live;                                      // false: the sequence has no such rows
 };
 // Items: all dK, then all dV, then all dQ (with grouped heads the smallest ones come last).  Inside a kind in the order of
-// item_place, the heaviest block under a causal mask first.
+// ItemOrder, the heaviest block under a causal mask first.
 __device__ __forceinline__ ItemW item_w(const BwdParams& p, int t) {
   ItemW w;
   const int n_kv = p.kv_items.blocks * p.kv_items.pairs;

@@ -92,10 +92,5 @@ struct ItemOrder {
     return {first + r - nb * cnt, nb};
   }
 };
-inline ItemPlace item_place(int t, int blocks, int pairs, int chunk) {
-  ItemOrder o;
-  o.set(blocks, pairs, chunk);
-  return o.place(t);
-}
 
 }  // namespace fa

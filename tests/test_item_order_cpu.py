@@ -1,4 +1,4 @@
-"""CPU: the order of the backward's work items (item_place in csrc/tile_order.cuh) gives every (pair, block) exactly one number,
+"""CPU: the order of the backward's work items (ItemOrder in csrc/tile_order.cuh, which the kernels call) gives every (pair, block) exactly one number,
 for chunks of one pair, of all pairs and in between."""
 import os
 import shutil
@@ -17,10 +17,12 @@ int main() {
     for (int blocks : {1, 2, 24})
       for (int chunk : {1, 2, 5, pairs}) {
         if (chunk > pairs) continue;
+        fa::ItemOrder order;
+        order.set(blocks, pairs, chunk);
         std::set<std::pair<int, int>> seen;
         int last_chunk = 0, last_block = 0;
         for (int t = 0; t < pairs * blocks; ++t) {
-          const fa::ItemPlace at = fa::item_place(t, blocks, pairs, chunk);
+          const fa::ItemPlace at = order.place(t);
           const int ck = at.pair / chunk;
           if (at.pair < 0 || at.pair >= pairs || at.block < 0 || at.block >= blocks || !seen.insert({at.pair, at.block}).second ||
               ck < last_chunk || (ck == last_chunk && at.block < last_block)) {
