@@ -618,9 +618,9 @@ bwd_dkv_kernel(const __grid_constant__ BwdParams p, const __grid_constant__ CUte
 // keep it from running two phases ahead.  The elementwise warps do so with s_full (the next S needs their s_free), ds_free
 // (the next dS needs their ds_full) and acc_done (the next item's last product needs their ds_full), but not with
 // qdo_full: the products of an item of one key block need s_free of the item before only, so Q / dO of two further items
-// can land while a warp is still in that item's exponentials or epilogue.  They wait for nothing there and read the LSE
-// and D of their own row from global memory instead.  The issuers release qdo_empty and kv_empty themselves; the dQ
-// issuer's commit is one of the two that release a K tile.
+// (three with two sets of resident tiles, kSets) can land while a warp is still in that item's exponentials or epilogue.
+// They wait for nothing there and read the LSE and D of their own row from global memory instead.  The issuers release
+// qdo_empty and kv_empty themselves; the dQ issuer's commit is one of the two that release a K tile.
 struct BarB {
   uint64_t qdo_full[2], qdo_empty[2];  // per set: Q / dO of the item have landed; the item's last S / dP have read them
   uint64_t kv_full[kDqSlots], kv_empty[kDqSlots];
