@@ -333,14 +333,17 @@ def test_gradient_rows_off_the_sector_boundary(d, where):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("d,s,h", [(64, 130, 1), (64, 700, 30), (128, 128, 2), (128, 1100, 20)])
-def test_what_follows_the_backward_follows_both_kernels(d, s, h):
-    """The dQ kernel starts beside the dK / dV kernel: fewer work items than SMs, and more.  Inputs are overwritten right behind the
-    call, in stream order; the same through a captured graph."""
+@pytest.mark.parametrize("d,s,s_k,h,h_k,causal", [
+    (64, 130, 130, 1, 1, True), (64, 700, 700, 30, 30, True), (128, 128, 128, 2, 2, True), (128, 1100, 1100, 20, 20, True),
+    (64, 4096, 128, 32, 1, False), (128, 4096, 128, 32, 1, False)])
+def test_what_follows_the_backward_follows_both_kernels(d, s, s_k, h, h_k, causal):
+    """The dQ kernel starts beside the dK / dV kernel: fewer work items than SMs, and more; and one dK / dV item of 2048 units, which
+    is at work long after the other SMs are through with all of dQ (head dim 64: 1150 us, and 19 for a dQ kernel by itself, which starts
+    some 10 us later).  Inputs are overwritten right behind the call, in stream order; the same through a captured graph."""
     from flash_b200 import ops
     g = torch.Generator().manual_seed(s)
-    q, k, v, dout = (torch.randn(1, s, h, d, generator=g).to(torch.bfloat16).cuda() for _ in range(4))
-    kw = dict(softmax_scale=d ** -0.5, causal=True)
+    q, k, v, dout = (torch.randn(1, n, heads, d, generator=g).to(torch.bfloat16).cuda() for n, heads in ((s, h), (s_k, h_k), (s_k, h_k), (s, h)))
+    kw = dict(softmax_scale=d ** -0.5, causal=causal)
     out, lse = ops.attention_forward(q, k, v, **kw)
     want = ops.attention_backward(dout, q, k, v, out, lse, **kw)
     torch.cuda.synchronize()
