@@ -49,6 +49,27 @@ int bwd_tc5_launch(const BwdParams& p, const fa_bwd_params& a, cudaStream_t st, 
   const dim3 grid_kv((unsigned)std::min<long long>(items_kv, num_sm)), grid_q((unsigned)std::min<long long>(items_q, num_sm));
   // the two work-item counters: the first 16 bytes of the workspace, cleared by the kernel in front (bwd_delta_kernel)
   int32_t* counters = reinterpret_cast<int32_t*>(p.dq_accum);
+  // The dQ kernel writes nothing that the dK / dV kernel reads and may run beside it, unless a caller has dQ written over an input,
+  // as a whole or, with rows of a wider buffer, over some of its columns: then it is launched behind.  (Address ranges; a dQ that
+  // lies between the rows of an input is launched behind it too.)
+  struct Range {
+    uintptr_t first, end;
+  };
+  auto range = [&](const void* ptr, int64_t rows, int64_t heads, int64_t row_stride, int64_t head_stride, int64_t batch_stride) {
+    int64_t lo = 0, hi = a.d;
+    auto along = [&](int64_t n, int64_t stride) { (stride < 0 ? lo : hi) += (n - 1) * stride; };
+    along(rows, row_stride);
+    along(heads, head_stride);
+    along(outer, batch_stride);
+    return Range{reinterpret_cast<uintptr_t>(ptr) + 2 * lo, reinterpret_cast<uintptr_t>(ptr) + 2 * hi};
+  };
+  const Range out = range(a.dq, q_rows, a.h, a.dq_row_stride, a.dq_head_stride, a.dq_batch_stride);
+  bool apart = true;
+  for (const Range& in : {range(a.q, q_rows, a.h, a.q_row_stride, a.q_head_stride, a.q_batch_stride),
+                          range(a.dout, q_rows, a.h, a.do_row_stride, a.do_head_stride, a.do_batch_stride),
+                          range(a.k, k_rows, a.h_k, a.k_row_stride, a.k_head_stride, a.k_batch_stride),
+                          range(a.v, k_rows, a.h_k, a.v_row_stride, a.v_head_stride, a.v_batch_stride)})
+    apart = apart && (out.end <= in.first || in.end <= out.first);
   cudaError_t e = cudaSuccess;
   auto launch = [&](auto kern, dim3 grid, const CUtensorMap& mq, const CUtensorMap& mdo, int32_t* counter, bool overlap) {
     if (e != cudaSuccess) return;
@@ -68,8 +89,6 @@ int bwd_tc5_launch(const BwdParams& p, const fa_bwd_params& a, cudaStream_t st, 
     constexpr bool C = decltype(cap_tag)::value;
     constexpr int HD = decltype(hd_tag)::value;
     launch(bwd_dkv_kernel<T, F, C, HD>, grid_kv, tq_u, tdo_u, counters, false);
-    // nothing that the dK / dV kernel reads is written by the dQ kernel, unless a caller has dQ written over an input
-    const bool apart = a.dq != a.q && a.dq != a.dout && a.dq != a.k && a.dq != a.v;
     launch(bwd_dq_kernel<T, F, C, HD>, grid_q, tq, tdo, counters + 1, apart);
   };
   auto by_hd = [&](auto t_tag, auto fmt_tag, auto cap_tag) {

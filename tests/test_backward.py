@@ -366,3 +366,30 @@ def test_what_follows_the_backward_follows_both_kernels(d, s, s_k, h, h_k, causa
         graph.replay()
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("over", ["q", "dout", "columns of q", "packed q"])
+def test_dq_over_an_input(d, over):
+    """dQ may be written over q or dout, or over some of their columns: the dQ kernel reads its own rows before it writes them, and does
+    not start beside a dK / dV kernel that still reads them (one item of 2048 units, see above).  The same bits as apart."""
+    from flash_b200 import ops
+    g = torch.Generator().manual_seed(d)
+    s, s_k, h = 4096, 128, 32
+    wide = torch.randn(1, s, h, d + 16, generator=g).to(torch.bfloat16).cuda()
+    q, k, v, dout = (torch.randn(1, n, heads, d, generator=g).to(torch.bfloat16).cuda() for n, heads in ((s, h), (s_k, 1), (s_k, 1), (s, h)))
+    kw = dict(softmax_scale=d ** -0.5, causal=False)
+    if over == "columns of q":
+        q = wide[..., :d]
+    if over == "packed q":
+        q, k, v, dout = (t[0] for t in (q, k, v, dout))
+        cu = [torch.tensor([0, 1000, n], dtype=torch.int32).cuda() for n in (s, s_k)]
+        cu[1][1] = 1
+        kw.update(cu_seqlens_q=cu[0], cu_seqlens_k=cu[1], max_seqlen_q=s - 1000, max_seqlen_k=s_k - 1)
+    out, lse = ops.attention_forward(q, k, v, **kw)
+    want = ops.attention_backward(dout, q, k, v, out, lse, **kw)
+    dq = {"q": q, "dout": dout, "columns of q": wide[..., 16:], "packed q": q}[over]
+    got = ops.attention_backward(dout, q, k, v, out, lse, dq=dq, **kw)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
